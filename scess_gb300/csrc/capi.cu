@@ -9,6 +9,7 @@
 
 #include "adjoint.h"
 #include "ccsd_so.h"
+#include "gemm_slice.h"
 #include "gemm_tc.h"
 #include "rccsd.h"
 #include "triples.h"
@@ -35,6 +36,8 @@ int guard(scess_ctx *ctx, F &&f) {
   try {
     SCESS_CUDA(cudaSetDevice(ctx->impl->device));
     f(*ctx->impl);
+    // (FP64 calls: a bounded wait inside their tensor-core launches)
+    if (ctx->impl->slices) ctx->impl->slices->check_error();
     ctx->err.clear();
   } catch (const Error &e) {
     ctx->err = e.what();
@@ -49,6 +52,7 @@ int guard(scess_ctx *ctx, F &&f) {
   // Packings cached during a plain call are keyed by device pointers of that call.
   cudaStreamSynchronize(ctx->impl->stream);
   if (ctx->impl->tc) ctx->impl->tc->clear_cache(nullptr);
+  if (ctx->impl->slices) ctx->impl->slices->clear_cache(nullptr);
   if (code != SCESS_OK) cudaGetLastError();
   return code;
 }
@@ -472,6 +476,7 @@ void scess_rccsd_state_destroy(scess_rccsd_state *state) {
     const auto t0 = std::chrono::steady_clock::now();
     scess::CurrentCtx cur(state->ctx->impl);  // the state's blocks go to its context's cache
     if (state->ctx->impl->tc) state->ctx->impl->tc->clear_cache(state->impl);
+    if (state->ctx->impl->slices) state->ctx->impl->slices->clear_cache(state->impl);
     delete state->impl;
     state->ctx->impl->timer.host("state_destroy", ms_since(t0));
   }
@@ -486,12 +491,15 @@ int scess_rccsd_state_iterate(scess_rccsd_state *state, int32_t n_iterations,
     ctl.cancel = c.cancel;
     ctl.user = c.user;
     ctl.time_limit_s = state->impl->options().time_limit_s;
-    if (c.tc) c.tc->set_cache_owner(state->impl);
     struct Reset {
       scess::Ctx &c;
-      ~Reset() { if (c.tc) c.tc->set_cache_owner(nullptr); }
+      ~Reset() {
+        c.tensor_cores().set_cache_owner(nullptr);
+        c.slice_engine().set_cache_owner(nullptr);
+      }
     } reset{c};
     c.tensor_cores().set_cache_owner(state->impl);
+    c.slice_engine().set_cache_owner(state->impl);
     state->impl->iterate(n_iterations, ctl);
     if (result) *result = state->impl->result();
     if (device_ms) *device_ms = state->impl->last_device_ms();

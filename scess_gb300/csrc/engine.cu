@@ -5,6 +5,7 @@
 #include <cstring>
 
 #include "engine.h"
+#include "gemm_slice.h"
 #include "gemm_tc.h"
 
 namespace scess {
@@ -173,6 +174,7 @@ Ctx::~Ctx() {
   if (stream) cudaStreamSynchronize(stream);
   blocks.flush();
   tc.reset();
+  slices.reset();
   plans.clear();
   workspace.release();
   scratch.release();
@@ -202,6 +204,11 @@ void Ctx::logf(int level, const char *fmt, ...) const {
 TcEngine &Ctx::tensor_cores() {
   if (!tc) tc = std::make_unique<TcEngine>(*this);
   return *tc;
+}
+
+SliceEngine &Ctx::slice_engine() {
+  if (!slices) slices = std::make_unique<SliceEngine>(*this);
+  return *slices;
 }
 
 void upload(Ctx &ctx, double *dst, const double *src, int64_t n) {
@@ -386,6 +393,21 @@ std::vector<int64_t> offsets(const std::vector<Lbl> &ls, int which) {
 
 }  // namespace
 
+uint64_t table_hash(const std::vector<int64_t> &r, const std::vector<int64_t> &k) {
+  uint64_t x = 1469598103934665603ull;  // FNV-1a over sizes and entries
+  auto mix = [&](uint64_t v) {
+    for (int b = 0; b < 8; b++) {
+      x ^= (v >> (8 * b)) & 0xffu;
+      x *= 1099511628211ull;
+    }
+  };
+  mix(r.size());
+  for (int64_t e : r) mix((uint64_t)e);
+  mix(k.size());
+  for (int64_t e : k) mix((uint64_t)e);
+  return x | 1ull;  // (0 = not yet computed)
+}
+
 const EinsumPlan &plan_einsum(Ctx &ctx, const char *spec, const TV &A, const TV &B, const TV &C) {
   std::string key(spec);
   geom_key(key, A);
@@ -526,6 +548,9 @@ void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, 
     ctx.tensor_cores().contract(pl, alpha, A.p, B.p, beta, C.p, constA, constB);
     return;
   }
+  if (SliceEngine::worth_it(pl.M, pl.N, pl.K) &&
+      ctx.slice_engine().contract(pl, alpha, A.p, B.p, beta, C.p, constA, constB))
+    return;
   TableGemm g;
   g.A = A.p;
   g.B = B.p;
@@ -566,6 +591,12 @@ void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, 
   }
   double *ws = ctx.ensure_workspace(dgemm_table_workspace(g));
   dgemm_table(g, ws, ctx.stream);
+}
+
+void fp64_table_gemm(Ctx &ctx, const TableGemm &g, const char *name) {
+  if (SliceEngine::worth_it(g.M, g.N, g.K) && ctx.slice_engine().table_gemm(g, name)) return;
+  TimedScope ts(ctx.timer, "dgemm_table", 2.0 * g.M * g.N * g.K, 0.0, ctx.stream);
+  dgemm_table(g, ctx.ensure_workspace(dgemm_table_workspace(g)), ctx.stream);
 }
 
 void permute(Ctx &ctx, const char *spec, double alpha, const TV &X, double beta, const TV &Y) {

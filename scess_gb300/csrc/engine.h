@@ -137,7 +137,10 @@ struct EinsumPlan {
   // plans that gather an operand through equal tables pack it identically
   mutable uint64_t hashA = 0, hashB = 0;
 };
-class TcEngine;  // tensor-core (mixed precision) backend, gemm_tc.cu
+// Content hash of an operand's two offset tables (never 0).
+uint64_t table_hash(const std::vector<int64_t> &r, const std::vector<int64_t> &k);
+class TcEngine;     // tensor-core (mixed precision) backend, gemm_tc.cu
+class SliceEngine;  // FP64 contractions on tensor-core slices, gemm_slice.cu
 
 // Forward-op record for the hand-written adjoint: every einsum / permute (and
 // the residual's tau and PlusTranspose steps) issued while Ctx::tape is set is
@@ -223,6 +226,7 @@ struct Ctx {
   double *dscalars = nullptr;  // 64 device doubles
   double *hscalars = nullptr;  // 64 pinned host doubles
   std::unique_ptr<TcEngine> tc;
+  std::unique_ptr<SliceEngine> slices;
   KernelTimer timer;
   Tape *tape = nullptr;  // recording target while an adjoint forward pass runs
   BlockCache blocks;     // released large device blocks (see BlockCache)
@@ -237,7 +241,12 @@ struct Ctx {
   double *ensure_workspace(int64_t doubles);
   void logf(int level, const char *fmt, ...) const;
   TcEngine &tensor_cores();
+  SliceEngine &slice_engine();
 };
+
+// C = alpha A.B + beta C in FP64 through the tables of g: on the tensor cores'
+// exact slices where that pays (SliceEngine::worth_it), else the DFMA kernel.
+void fp64_table_gemm(Ctx &ctx, const TableGemm &g, const char *name);
 
 // FP64: DFMA engine.  MIXED: tensor cores for contractions large enough to pay
 // for packing, FP64 for the rest.  TENSOR: tensor cores for every contraction.

@@ -1,0 +1,939 @@
+// FP64 GEMM on BF16 slices with tcgen05 (see gemm_slice.h for the splitting).
+//
+// A persistent CTA per SM walks work units (problem, 128 x bn output tile, K range),
+// bn <= 80:
+//   warp 0     TMA producer: per 32-wide K block one stage with the 7 slices of
+//              128 A rows and bn B rows (64-byte rows, 64B swizzle);
+//   warp 1     owns TMEM (six accumulators of bn columns: S_0 .. S_4 and S_5 + S_6)
+//              and issues the MMAs (M = 128, N = bn, K = 16);
+//   warps 4-11 two epilogue warpgroups, bn / 2 columns each: add every drained
+//              S_d, an exact integer, into one 64-bit integer per output, and turn
+//              integer + FP32 tail into FP64 at the end of the unit.
+// Each S_d keeps its own accumulator and is drained only as often as its sums
+// stay exact integers in FP32 (every 128, 16, 5, 3, 2 K blocks for d = 0 .. 4), so
+// that a K of 200 takes 12 drains; with three rotating 128-wide accumulators drained
+// every K block (36 drains) the drains took 2.3 x the MMAs' time.
+// Every mbarrier wait is bounded (see mbarrier.cuh).
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
+#include <cstring>
+#include <mutex>
+
+#include "dgemm_tile.cuh"
+#include "gemm_slice.h"
+#include "pack_tiles.cuh"
+#include "slice_math.cuh"
+#include "tcgen05.cuh"
+
+namespace scess {
+
+namespace {
+
+constexpr int BM = 128, BN = 80, BK = kSliceBK;
+constexpr int STAGES = 2;
+constexpr uint32_t A_SLICE = (uint32_t)BM * BK * 2;                  // one slice of 128 rows
+constexpr uint32_t STAGE_BYTES = kSlices * (BM + BN) * BK * 2;       // 91 KiB
+constexpr int NDIAG = 5;                                             // S_0 .. S_4 are drained
+constexpr int NACC = NDIAG + 1;                                      // ... and the tail
+constexpr int HC = BN / 2;                                           // columns of an epilogue thread
+constexpr int THREADS = 384;
+constexpr int kEpiRegs = 224, kCtlRegs = 56, kLaunchRegs = 168;      // 3 x 168 = 56 + 2 x 224
+// K blocks between drains of S_d: |S_d| per K is at most 2^12, 2^15, 1.5 2^16,
+// 2.5 2^16, 3.5 2^16 for d = 0 .. 4 and the sum has to stay within 2^24
+__host__ __device__ constexpr int drain_every(int d) {
+  return d == 0 ? 128 : d == 1 ? 16 : d == 2 ? 5 : d == 3 ? 3 : 2;
+}
+struct Ctl {  // behind the stages
+  uint64_t full[STAGES], empty[STAGES], tfull[NACC], tempty[NACC], done;
+  uint32_t tmem;
+  uint32_t pad;
+  int64_t colOff[BN];
+  int colE[BN];
+};
+constexpr size_t SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + sizeof(Ctl);
+
+enum : unsigned { ERR_FULL_WAIT = 1, ERR_EMPTY_WAIT = 2, ERR_ACCUM_WAIT = 3 };
+
+struct SegArgs {
+  int mapA, mapB;
+  int nkb, kpad;
+  int64_t rowA0[3], rowAy[3], rowAz[3], rowB0[3], rowBy[3], rowBz[3];
+};
+struct SliceMaps {
+  CUtensorMap m[6];
+};
+struct SliceArgs {
+  int M, N, tiles_m, tiles_n;
+  int bn;      // tile width: a multiple of 16, at most 80
+  int fs;      // fraction bits kept of the tail (see slice_value)
+  int ny, nz, ng, nseg;
+  int kb_total, kb_per_split, splits;
+  SegArgs seg[4];
+  int tri[3], gstart[4];
+  const int *expA, *expB;
+  int64_t expA0[3];
+  double *C;
+  int64_t baseC, cy[3], cz[3], cg[3];
+  const int64_t *rowC[3], *colC[3];
+  double alpha, beta;
+  int alpha_pow2, alpha_e, alpha_neg;  // alpha = (-1)^neg 2^e: folded into the exponent
+  double *partial;                     // split-K partial sums [split][n][m], or null
+  int64_t part_stride;
+  unsigned *err;
+  long long wait_cycles;
+  int withhold_first;
+};
+
+// T += i 2^(9 (4 - D)) for the drained S_D = i 2^(-9 D), |i| <= 2^24.
+template <int D>
+__device__ __forceinline__ void add_diag(long long &T, uint32_t raw) {
+  const int i = __float2int_rn(__uint_as_float(raw) * __int_as_float((127 + 9 * D) << 23));
+  if constexpr (D == 0) T += (long long)((unsigned long long)(unsigned)(i << 4) << 32);
+  else asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(T) : "r"(i), "n"(1 << (9 * (4 - D))));
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+// The wait takes the loaded registers as operands: no use is scheduled before it.
+__device__ __forceinline__ void tmem_wait8(uint32_t *r) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+               :
+               : "memory");
+}
+
+// What bounds it: long K, the tensor pipe behind shared memory (28 products of
+// 2 x 128 x bn x 32 a stage; an M = 128, N = 80 MMA reads 6.5 KiB per 40 cycles);
+// short K, the epilogue (about 45 instructions per output).
+__global__ void __launch_bounds__(THREADS, 1)
+    slice_gemm_kernel(const __grid_constant__ SliceMaps maps, const __grid_constant__ SliceArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  Ctl &ctl = *reinterpret_cast<Ctl *>(smem + STAGES * STAGE_BYTES);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tiles = a.tiles_m * a.tiles_n;
+  const int nprob = a.gstart[a.ng];
+  const int units = tiles * nprob * a.splits;
+  const int bn = a.bn;
+  const uint32_t bslice = (uint32_t)bn * BK * 2;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; s++) {
+      mbar_init(&ctl.full[s], 1);
+      mbar_init(&ctl.empty[s], 1);
+    }
+    for (int b = 0; b < NACC; b++) {
+      mbar_init(&ctl.tfull[b], 1);
+      mbar_init(&ctl.tempty[b], 8);  // one arrival per epilogue warp
+    }
+    mbar_init(&ctl.done, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&ctl.tmem)),
+                 "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = ctl.tmem;
+
+  // unit -> (tile m, tile n, problem y, z, g, K-block range, split)
+  auto unit_coords = [&](int u, int &tm, int &tn, int &py, int &pz, int &pg, int &kb0, int &kb1, int &sp) {
+    const int tile = u % tiles;
+    const int rest = u / tiles;
+    const int q = rest % nprob;
+    sp = rest / nprob;
+    tn = tile % a.tiles_n;
+    tm = tile / a.tiles_n;
+    pg = 0;
+    while (pg + 1 < a.ng && q >= a.gstart[pg + 1]) pg++;
+    const int lq = q - a.gstart[pg];
+    if (a.tri[pg]) {  // lq = y (y + 1) / 2 + z, z <= y
+      int y = (int)((sqrtf(8.0f * (float)lq + 1.0f) - 1.0f) * 0.5f);
+      while (y * (y + 1) / 2 > lq) y--;
+      while ((y + 1) * (y + 2) / 2 <= lq) y++;
+      py = y;
+      pz = lq - y * (y + 1) / 2;
+    } else {
+      py = lq % a.ny;
+      pz = lq / a.ny;
+    }
+    kb0 = sp * a.kb_per_split;
+    kb1 = min(a.kb_total, kb0 + a.kb_per_split);
+  };
+  auto seg_at = [&](int kb, int &s, int &lkb) {
+    s = 0;
+    lkb = kb;
+    while (s < a.nseg - 1 && lkb >= a.seg[s].nkb) {
+      lkb -= a.seg[s].nkb;
+      s++;
+    }
+  };
+
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kCtlRegs));
+  if (warp == 0) {
+    if (lane == 0) {
+      int g = 0;
+      int last[STAGES];
+      for (int s = 0; s < STAGES; s++) last[s] = -1;
+      bool ok = true;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        int tm, tn, py, pz, pg, kb0, kb1, sp;
+        unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
+        for (int kb = kb0; kb < kb1; kb++, g++) {
+          int sg, lkb;
+          seg_at(kb, sg, lkb);
+          const SegArgs &S = a.seg[sg];
+          const int ya = (int)(S.rowA0[pg] + py * S.rowAy[pg] + pz * S.rowAz[pg]) + tm * BM;
+          const int yb = (int)(S.rowB0[pg] + py * S.rowBy[pg] + pz * S.rowBz[pg]) + tn * bn;
+          const int s = g % STAGES;
+          const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
+          if (!mbar_wait(&ctl.empty[s], ph ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) { ok = false; break; }
+          // diagnostics: the first stage is taken but never filled (see scess_ctx_arm_wait_expiry)
+          if (a.withhold_first && g == 0) continue;
+          uint8_t *st = smem + s * STAGE_BYTES;
+          mbar_expect_tx(&ctl.full[s], kSlices * (A_SLICE + bslice));
+#pragma unroll
+          for (int p = kSlices - 1; p >= 0; p--) {
+            tma_load_2d(st + p * A_SLICE, &maps.m[S.mapA], p * S.kpad + lkb * BK, ya, &ctl.full[s]);
+            tma_load_2d(st + kSlices * A_SLICE + p * bslice, &maps.m[S.mapB], p * S.kpad + lkb * BK, yb,
+                        &ctl.full[s]);
+          }
+          last[s] = g;
+        }
+      }
+      for (int s = 0; s < STAGES; s++)
+        if (last[s] >= 0) mbar_drain(&ctl.full[s], (uint32_t)(last[s] / STAGES) & 1u);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int g = 0;
+      uint32_t cnt[NACC] = {0, 0, 0, 0, 0, 0};  // fills of each accumulator so far
+      const uint64_t desc_a = sw_desc<64>(smem_u32(smem)), desc_b = sw_desc<64>(smem_u32(smem) + kSlices * A_SLICE);
+      const uint32_t bq = bslice >> 4;
+      bool ok = true;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        int tm, tn, py, pz, pg, kb0, kb1, sp;
+        unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
+        const uint32_t idesc = idesc_f16kind(BM, min(bn, (a.N - tn * bn + 15) & ~15), 1u);  // BF16
+        for (int kb = kb0; kb < kb1 && ok; kb++, g++) {
+          const int s = g % STAGES;
+          const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
+          if (!mbar_wait(&ctl.full[s], ph, a.err, ERR_FULL_WAIT, a.wait_cycles)) { ok = false; break; }
+          tc_fence_after();
+          // slice offsets are added to the stage's descriptors (address field in units
+          // of 16 bytes): building a descriptor per MMA made the issuing thread the
+          // bound (100 cycles per MMA where N = 80 takes 52 and N = 128 takes 64)
+          const uint64_t da = desc_a + (uint64_t)(s * (STAGE_BYTES >> 4));
+          const uint64_t db = desc_b + (uint64_t)(s * (STAGE_BYTES >> 4));
+          auto product = [&](uint32_t d, int p, int q, uint32_t acc) {
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+              mma_bf16(d, da + (uint64_t)(p * (A_SLICE >> 4) + 2 * k), db + (uint64_t)(q * bq + 2 * k), idesc,
+                       k ? 1u : acc);
+          };
+          // an accumulator's first block of a fill waits for its drain and starts from zero
+          auto open = [&](int b, bool first) -> bool {
+            if (!first) return true;
+            if (!mbar_wait(&ctl.tempty[b], (cnt[b] & 1u) ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) return false;
+            tc_fence_after();
+            return true;
+          };
+          // the tail first: the accumulators of the previous unit are drained behind it
+          if (!open(NDIAG, kb == kb0)) { ok = false; break; }
+          {
+            uint32_t acc = kb == kb0 ? 0u : 1u;
+#pragma unroll
+            for (int d = NDIAG; d < kSlices; d++)
+#pragma unroll
+              for (int p = 0; p <= d; p++, acc = 1u) product(tmem + (uint32_t)(NDIAG * bn), p, d - p, acc);
+            if (kb == kb1 - 1) {
+              mma_commit(&ctl.tfull[NDIAG]);
+              cnt[NDIAG]++;
+            }
+          }
+#pragma unroll
+          for (int d = 0; d < NDIAG; d++) {
+            const bool first = (kb - kb0) % drain_every(d) == 0;
+            if (ok && !open(d, first)) ok = false;
+            if (!ok) break;
+#pragma unroll
+            for (int p = 0; p <= d; p++) product(tmem + (uint32_t)(d * bn), p, d - p, (first && p == 0) ? 0u : 1u);
+            if ((kb - kb0) % drain_every(d) == drain_every(d) - 1 || kb == kb1 - 1) {
+              mma_commit(&ctl.tfull[d]);
+              cnt[d]++;
+            }
+          }
+          if (!ok) break;
+          mma_commit(&ctl.empty[s]);
+        }
+      }
+      mma_commit(&ctl.done);
+      mbar_drain(&ctl.done, 0);
+    }
+  }
+  } else {  // epilogue warps
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
+    const int q = warp & 3;
+    const int row = 32 * q + lane;
+    const int h = (warp - 4) >> 2;                  // column half
+    const int hc = bn >> 1;                         // its width: 8, 16, .. 40
+    const int et = threadIdx.x - 128 - 128 * h;     // 0..127 within the half
+    const int bar = 1 + h;
+    uint32_t cnt[NACC] = {0, 0, 0, 0, 0, 0};
+    bool ok = true;
+    const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(hc * h);
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      int tm, tn, py, pz, pg, kb0, kb1, sp;
+      unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
+      const int m = tm * BM + row;
+      asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");  // previous unit's column tables read
+      if (et < hc) {
+        const int nn = tn * bn + hc * h + et;
+        const int e = nn < a.N ? a.expB[nn] : kRowNonFinite;
+        ctl.colE[hc * h + et] = max(e, 1);
+        ctl.colOff[hc * h + et] =
+            e == kRowNonFinite ? -1
+            : a.partial ? (int64_t)sp * a.part_stride + (int64_t)a.M * nn
+                        : a.baseC + py * a.cy[pg] + pz * a.cz[pg] + a.cg[pg] + a.colC[pg][nn];
+      }
+      const int eA = m < a.M ? a.expA[a.expA0[pg] + m] : kRowNonFinite;
+      const int64_t rowOff = m < a.M ? (a.partial ? (int64_t)m : a.rowC[pg][m]) : 0;
+      const unsigned errv = *(volatile unsigned *)a.err;
+      long long T[HC];
+      float F[HC];
+#pragma unroll
+      for (int j = 0; j < HC; j++) T[j] = 0;
+      auto wait_for = [&](int b) -> bool {
+        if (!mbar_wait(&ctl.tfull[b], cnt[b] & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) return false;
+        tc_fence_after();
+        return true;
+      };
+      auto release = [&](int b) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&ctl.tempty[b])) : "memory");
+        cnt[b]++;
+      };
+      auto take = [&](auto diag) -> bool {
+        constexpr int D = decltype(diag)::value;
+        if (!wait_for(D)) return false;
+        uint32_t r[2][8];
+        const uint32_t t0 = tl + (uint32_t)(D * bn);
+        tmem_ld8(t0, r[0]);
+#pragma unroll
+        for (int j = 0; j < HC; j += 8) {
+          if (j < hc) {
+            tmem_wait8(r[(j >> 3) & 1]);
+            if (j + 8 < hc) tmem_ld8(t0 + (uint32_t)(j + 8), r[((j >> 3) & 1) ^ 1]);
+#pragma unroll
+            for (int i = 0; i < 8; i++) add_diag<D>(T[j + i], r[(j >> 3) & 1][i]);
+          }
+        }
+        release(D);
+        return true;
+      };
+      for (int kb = kb0; kb < kb1; kb++) {
+        const int k = kb - kb0;
+        const bool last = kb == kb1 - 1;
+        if (last) {  // the tail, in units 2^-fs below the integer's
+          ok = wait_for(NDIAG);
+          if (!ok) break;
+#pragma unroll
+          for (int j = 0; j < HC; j += 8) {
+            if (j < hc) {
+              uint32_t r[8];
+              tmem_ld8(tl + (uint32_t)(NDIAG * bn + j), r);
+              tmem_wait8(r);
+#pragma unroll
+              for (int i = 0; i < 8; i++) F[j + i] = __uint_as_float(r[i]);
+            }
+          }
+          release(NDIAG);
+        }
+        if (k % drain_every(0) == drain_every(0) - 1 || last) ok = ok && take(std::integral_constant<int, 0>{});
+        if (k % drain_every(1) == drain_every(1) - 1 || last) ok = ok && take(std::integral_constant<int, 1>{});
+        if (k % drain_every(2) == drain_every(2) - 1 || last) ok = ok && take(std::integral_constant<int, 2>{});
+        if (k % drain_every(3) == drain_every(3) - 1 || last) ok = ok && take(std::integral_constant<int, 3>{});
+        if (k % drain_every(4) == drain_every(4) - 1 || last) ok = ok && take(std::integral_constant<int, 4>{});
+        if (!ok) break;
+      }
+      asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");  // column tables of this unit written
+      if (!ok || errv) break;
+      if (eA == kRowNonFinite) continue;
+      const double mul = a.alpha;
+      const bool scaled = !a.partial && !a.alpha_pow2;
+      const uint32_t flip = (!a.partial && a.alpha_pow2 && a.alpha_neg) ? 0x80000000u : 0u;
+      // value = (T 2^-36 + tail) 2^(EA + EB - 12), E = exps - 1022
+      const int sc0 = max(eA, 1) - 2 * 1022 - 12 - 36 + ((!a.partial && a.alpha_pow2) ? a.alpha_e : 0);
+      const float ftail = __int_as_float((127 + 36 + a.fs) << 23);  // 2^(36 + fs)
+      double *base = (a.partial ? a.partial : a.C) + rowOff;
+      const int mode = (a.partial || a.beta == 0.0) ? 0 : (a.beta == 1.0 ? 1 : 2);
+#pragma unroll
+      for (int j = 0; j < HC; j += 8) {
+        if (j < hc) {
+        double v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          v[i] = slice_value(T[j + i], rint_i32(F[j + i] * ftail), a.fs, sc0 + ctl.colE[hc * h + j + i], flip);
+        if (scaled) {
+#pragma unroll
+          for (int i = 0; i < 8; i++) v[i] *= mul;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const int64_t co = ctl.colOff[hc * h + j + i];
+          if (co < 0) continue;
+          double *p = base + co;
+          if (mode == 0) *p = v[i];
+          else if (mode == 1) asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v[i]) : "memory");
+          else *p = fma(a.beta, *p, v[i]);
+        }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+}
+
+// Split-K: C = alpha sum_z partial_z + beta C over unmarked outputs, z in order.
+__global__ void slice_reduce_kernel(SliceArgs a, int splits) {
+  const int64_t MN = (int64_t)a.M * a.N;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < MN;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t m = e % a.M, n = e / a.M;
+    if (a.expA[m] == kRowNonFinite || a.expB[n] == kRowNonFinite) continue;
+    double s = 0.0;
+    for (int z = 0; z < splits; z++) s += a.partial[(int64_t)z * MN + e];
+    double *p = a.C + a.baseC + a.rowC[0][m] + a.colC[0][n];
+    double val = a.alpha * s;
+    if (a.beta != 0.0) val += a.beta * *p;
+    *p = val;
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Packs.  One CTA per 32 rows (RowTiles: along the operand's smallest-stride row
+// label, so that loads coalesce) walks K in chunks of 64.  EXPS: the row
+// exponents only, over the K chunks blockIdx.y, + gridDim.y, ..., folded into exps with
+// atomics.  OWN: the CTA covers the whole K, finds its rows' exponents in a
+// first walk and cuts in a second one (whose loads hit L2).  GIVEN: the exponents
+// are read, K chunks spread over blockIdx.y.  HBM-bound: 8 B read and 14 B
+// written per element (about 50 integer and FP32 instructions).
+enum class PackMode { EXPS, OWN, GIVEN };
+
+template <PackMode MODE, bool AFFINE>
+__global__ void __launch_bounds__(256) slice_pack_kernel(
+    const double *__restrict__ src, const int64_t *__restrict__ rowOff, int64_t rows,
+    const int64_t *__restrict__ kOff, int64_t K, int unitK, uint16_t *__restrict__ dst,
+    int64_t Kpad, int *__restrict__ exps, const int64_t *__restrict__ expIdx, int negate, int64_t rs,
+    int64_t ks, const RowTiles rt) {
+  __shared__ double tile[32][65];
+  __shared__ int64_t sr[32], sk[64], srow[32];
+  __shared__ int se[32];
+  const int t = threadIdx.x;
+  if (t < 32) {
+    const int64_t r = rt.row(blockIdx.x, t);
+    srow[t] = (r >= 0 && r < rows) ? r : -1;
+    sr[t] = srow[t] >= 0 ? (AFFINE ? r * rs : rowOff[r]) : -1;
+    se[t] = MODE == PackMode::GIVEN && srow[t] >= 0 ? exps[expIdx ? expIdx[r] : r] : 0;
+  }
+  const int64_t nchunk = (MODE == PackMode::EXPS ? (K + 63) : (Kpad + 63)) / 64;
+  const int64_t c0 = MODE == PackMode::OWN ? 0 : blockIdx.y, cs = MODE == PackMode::OWN ? 1 : gridDim.y;
+  auto load_offsets = [&](int64_t k0) {
+    __syncthreads();
+    if (t < 64) sk[t] = (k0 + t < K) ? (AFFINE ? (k0 + t) * ks : kOff[k0 + t]) : -1;
+    __syncthreads();
+  };
+  if (MODE != PackMode::GIVEN) {
+    int mx[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int64_t c = c0; c * 64 < K; c += cs) {
+      load_offsets(c * 64);
+      double x[8];
+#pragma unroll
+      for (int p = 0; p < 8; p++) {
+        const int rr = unitK ? (t >> 6) + 4 * p : t & 31, kk = unitK ? t & 63 : (t >> 5) + 8 * p;
+        const int64_t ro = sr[rr], ko = sk[kk];
+        x[p] = (ro >= 0 && ko >= 0) ? src[ro + ko] : 0.0;
+      }
+#pragma unroll
+      for (int p = 0; p < 8; p++) {
+        const int hi = __double2hiint(x[p]) & 0x7fffffff;
+        const int e = (hi >> 20) ? (hi >> 20) : ((hi | __double2loint(x[p])) ? 1 : 0);
+        mx[p] = max(mx[p], e);
+      }
+    }
+    if (unitK) {  // the rows (t >> 6) + 4 p are shared by two warps
+#pragma unroll
+      for (int p = 0; p < 8; p++) {
+        const int m = __reduce_max_sync(0xffffffffu, mx[p]);
+        if ((t & 31) == 0) atomicMax(&se[(t >> 6) + 4 * p], m);
+      }
+    } else {
+      int m = 0;
+#pragma unroll
+      for (int p = 0; p < 8; p++) m = max(m, mx[p]);
+      atomicMax(&se[t & 31], m);
+    }
+    __syncthreads();
+    if (t < 32 && srow[t] >= 0) {
+      if (MODE == PackMode::EXPS) atomicMax(&exps[expIdx ? expIdx[srow[t]] : srow[t]], se[t]);
+      else exps[srow[t]] = se[t];
+    }
+  }
+  for (int64_t c = c0; MODE != PackMode::EXPS && c < nchunk; c += cs) {
+    const int64_t k0 = c * 64;
+    load_offsets(k0);
+#pragma unroll
+    for (int p = 0; p < 8; p++) {
+      const int rr = unitK ? (t >> 6) + 4 * p : t & 31, kk = unitK ? t & 63 : (t >> 5) + 8 * p;
+      const int64_t ro = sr[rr], ko = sk[kk];
+      tile[rr][kk] = (ro >= 0 && ko >= 0) ? src[ro + ko] : 0.0;
+    }
+    __syncthreads();
+    const int rr = t >> 3, ch = t & 7;
+    const int64_t r = srow[rr];
+    if (r < 0 || k0 + ch * 8 >= Kpad) continue;
+    const int e = se[rr];
+    uint32_t w[kSlices][4];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      int64_t F = e == kRowNonFinite ? 0 : slice_fixed(tile[rr][ch * 8 + j], e);
+      if (negate) F = -F;
+      const int64_t G = F + kDigitBias;
+#pragma unroll
+      for (int p = 0; p < kSlices; p++) {
+        // digit 2^(-9 p) as a float (exact), of which BF16 keeps the upper half (exact)
+        float f;
+        if (p == 0)
+          f = __int_as_float(0x4B400000 + (int)(G >> 54)) - 12582912.0f;
+        else
+          f = __int_as_float((0x4B000000 - (9 * p << 23)) | ((int)(G >> (9 * (6 - p))) & 511)) -
+              __int_as_float((0x4B000000 - (9 * p << 23)) | 256);
+        const uint32_t b = __float_as_uint(f) >> 16;
+        if (j & 1) w[p][j >> 1] |= b << 16;
+        else w[p][j >> 1] = b;
+      }
+    }
+    uint16_t *d = dst + r * kSlices * Kpad + k0 + ch * 8;
+#pragma unroll
+    for (int p = 0; p < kSlices; p++)
+      *reinterpret_cast<uint4 *>(d + p * Kpad) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+  }
+}
+
+__global__ void __launch_bounds__(256) dgemm_masked_kernel(TableGemm g, const int *__restrict__ expA,
+                                                           const int *__restrict__ expB) {
+  const int64_t tm = (g.M + kDgemmTile - 1) / kDgemmTile, tn = (g.N + kDgemmTile - 1) / kDgemmTile;
+  const int t = threadIdx.x;
+  for (int64_t tile = blockIdx.x; tile < tm * tn; tile += gridDim.x) {
+    const int64_t m0 = (tile % tm) * kDgemmTile, n0 = (tile / tm) * kDgemmTile;
+    bool bad = false;
+    if (t < kDgemmTile) bad = m0 + t < g.M && expA[m0 + t] == kRowNonFinite;
+    else if (t < 2 * kDgemmTile) bad = n0 + t - kDgemmTile < g.N && expB[n0 + t - kDgemmTile] == kRowNonFinite;
+    if (!__syncthreads_or(bad)) continue;
+    dgemm_tile(g, m0, n0, 0, g.K, [&](int64_t m, int64_t n, double acc) {
+      if (expA[m] != kRowNonFinite && expB[n] != kRowNonFinite) return;
+      const int64_t off = g.baseC + g.rowC[m] + g.colC[n];
+      double val = g.alpha * acc;
+      if (g.beta != 0.0) val += g.beta * g.C[off];
+      g.C[off] = val;
+    });
+    __syncthreads();
+  }
+}
+
+PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
+  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    cudaDriverEntryPointQueryResult q;
+    void *p = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
+                                         &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+  });
+  if (!fn) throw Error(SCESS_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
+  return fn;
+}
+
+// The kernel's setmaxnreg split assumes it is launched with exactly kLaunchRegs
+// registers a thread.
+bool kernel_ok() {
+  static bool ok = false;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    cudaFuncAttributes fa;
+    ok = cudaFuncSetAttribute(slice_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)SMEM_BYTES) == cudaSuccess &&
+         cudaFuncGetAttributes(&fa, slice_gemm_kernel) == cudaSuccess && fa.numRegs == kLaunchRegs;
+    cudaGetLastError();
+  });
+  return ok;
+}
+
+}  // namespace
+
+void dgemm_masked(const TableGemm &g, const int *expA, const int *expB, cudaStream_t stream) {
+  const int64_t tiles = ceil_div(g.M, kDgemmTile) * ceil_div(g.N, kDgemmTile);
+  dgemm_masked_kernel<<<(unsigned)std::min<int64_t>(tiles, 4 * kNumSMs), 256, 0, stream>>>(g, expA, expB);
+  SCESS_CHECK_LAUNCH();
+}
+
+SliceEngine::SliceEngine(Ctx &ctx) : ctx_(ctx) {
+  err_.alloc(sizeof(unsigned) * 4);
+  SCESS_CUDA(cudaMemsetAsync(err_.as<void>(), 0, sizeof(unsigned) * 4, ctx_.stream));
+}
+
+int SliceEngine::tile_n(int64_t N) { return (int)round_up(ceil_div(N, ceil_div(N, BN)), 16); }
+
+bool SliceEngine::worth_it(int64_t M, int64_t N, int64_t K) {
+  if (!kernel_ok() || M > INT32_MAX / 2 || N > INT32_MAX / 2 || K < 1 || std::min(M, N) < 2) return false;
+  // The DFMA kernel computes whole 64 x 64 tiles at about 1 TFLOP/s; packs, GEMM and
+  // mask check take about 25 us before size counts.
+  const double tiles = (double)round_up(M, 64) * (double)round_up(N, 64);
+  return 2.0 * tiles * (double)K >= 3.0e7;
+}
+
+CUtensorMap SliceEngine::map_of(const SlicedPack &p, int box_rows) {
+  CUtensorMap m;
+  std::memset(&m, 0, sizeof(m));
+  cuuint64_t dims[2] = {(cuuint64_t)(kSlices * p.Kpad), (cuuint64_t)p.rows};
+  cuuint64_t strides[1] = {(cuuint64_t)(kSlices * p.Kpad * 2)};
+  cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.mem.as<void>(), dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    throw Error(SCESS_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
+  return m;
+}
+
+void SliceEngine::alloc(SlicedPack &out, int64_t rows, int64_t K) {
+  const int64_t Kpad = round_up(std::max<int64_t>(K, 1), BK);
+  const size_t bytes = (size_t)rows * kSlices * Kpad * sizeof(uint16_t), eb = (size_t)rows * sizeof(int);
+  if (out.mem.bytes() < bytes) out.mem.alloc(bytes);
+  if (out.exps.bytes() < eb) out.exps.alloc(round_up((int64_t)eb, 4096));
+  out.rows = rows;
+  out.K = K;
+  out.Kpad = Kpad;
+}
+
+void SliceEngine::row_exps(const double *src, const int64_t *rowOff, int64_t rows, const int64_t *kOff,
+                           int64_t K, bool unitK, int *exps) {
+  const RowTiles rt = RowTiles::make(rows, 1, rows);
+  const dim3 grid((unsigned)rt.count,
+                  (unsigned)std::max<int64_t>(1, std::min<int64_t>({ceil_div(K, 64), ceil_div(8 * kNumSMs, rt.count), 65535})));
+  slice_pack_kernel<PackMode::EXPS, false><<<grid, 256, 0, ctx_.stream>>>(
+      src, rowOff, rows, kOff, K, unitK ? 1 : 0, nullptr, 0, exps, nullptr, 0, 0, 0, rt);
+  SCESS_CHECK_LAUNCH();
+}
+
+void SliceEngine::pack_with_exps(const double *src, const int64_t *rowOff, int64_t rows, const int64_t *kOff,
+                                 int64_t K, bool unitK, const int *exps, const int64_t *expIdx, bool negate,
+                                 SlicedPack &out) {
+  alloc(out, rows, K);
+  const RowTiles rt = RowTiles::make(rows, 1, rows);
+  TimedScope ts(ctx_.timer, "slice_pack", 0.0, (double)rows * K * 8 + (double)rows * out.Kpad * 14, ctx_.stream);
+  const dim3 grid((unsigned)rt.count, (unsigned)std::min<int64_t>(ceil_div(out.Kpad, 64), 65535));
+  slice_pack_kernel<PackMode::GIVEN, false><<<grid, 256, 0, ctx_.stream>>>(
+      src, rowOff, rows, kOff, K, unitK ? 1 : 0, out.mem.as<uint16_t>(), out.Kpad, const_cast<int *>(exps),
+      expIdx, negate ? 1 : 0, 0, 0, rt);
+  SCESS_CHECK_LAUNCH();
+}
+
+void SliceEngine::pack(const Gather &g, SlicedPack &out) {
+  alloc(out, g.rows, g.K);
+  const bool aff = g.rs >= 0 && g.ks >= 0;
+  const RowTiles rt = RowTiles::make(g.rows, g.P, g.E > 0 ? g.E : g.rows);
+  if (rt.count > INT32_MAX) throw Error(SCESS_ERR_INVALID, "slice pack: too large");
+  TimedScope ts(ctx_.timer, "slice_pack", 0.0, (double)g.rows * g.K * 8 + (double)g.rows * out.Kpad * 14,
+                ctx_.stream);
+  const int u = g.unitK ? 1 : 0;
+  uint16_t *dst = out.mem.as<uint16_t>();
+  int *ex = out.exps.as<int>();
+  const int64_t chunks = ceil_div(out.Kpad, 64);
+  // one walk per CTA over its rows' whole K while that fills the device or K is
+  // short; else the exponents first, then the cut, each spread over K too
+  if (rt.count >= 2 * kNumSMs || chunks <= 4) {
+    if (aff)
+      slice_pack_kernel<PackMode::OWN, true><<<(unsigned)rt.count, 256, 0, ctx_.stream>>>(
+          g.src, nullptr, g.rows, nullptr, g.K, u, dst, out.Kpad, ex, nullptr, 0, g.rs, g.ks, rt);
+    else
+      slice_pack_kernel<PackMode::OWN, false><<<(unsigned)rt.count, 256, 0, ctx_.stream>>>(
+          g.src, g.row, g.rows, g.k, g.K, u, dst, out.Kpad, ex, nullptr, 0, 0, 0, rt);
+    SCESS_CHECK_LAUNCH();
+    return;
+  }
+  SCESS_CUDA(cudaMemsetAsync(ex, 0, (size_t)g.rows * sizeof(int), ctx_.stream));
+  const dim3 ge((unsigned)rt.count, (unsigned)std::min<int64_t>({ceil_div(g.K, 64), ceil_div(8 * kNumSMs, rt.count), 65535}));
+  const dim3 gp((unsigned)rt.count, (unsigned)std::min<int64_t>({chunks, ceil_div(16 * kNumSMs, rt.count), 65535}));
+  if (aff) {
+    slice_pack_kernel<PackMode::EXPS, true><<<ge, 256, 0, ctx_.stream>>>(
+        g.src, nullptr, g.rows, nullptr, g.K, u, nullptr, 0, ex, nullptr, 0, g.rs, g.ks, rt);
+    SCESS_CHECK_LAUNCH();
+    slice_pack_kernel<PackMode::GIVEN, true><<<gp, 256, 0, ctx_.stream>>>(
+        g.src, nullptr, g.rows, nullptr, g.K, u, dst, out.Kpad, ex, nullptr, 0, g.rs, g.ks, rt);
+  } else {
+    slice_pack_kernel<PackMode::EXPS, false><<<ge, 256, 0, ctx_.stream>>>(
+        g.src, g.row, g.rows, g.k, g.K, u, nullptr, 0, ex, nullptr, 0, 0, 0, rt);
+    SCESS_CHECK_LAUNCH();
+    slice_pack_kernel<PackMode::GIVEN, false><<<gp, 256, 0, ctx_.stream>>>(
+        g.src, g.row, g.rows, g.k, g.K, u, dst, out.Kpad, ex, nullptr, 0, 0, 0, rt);
+  }
+  SCESS_CHECK_LAUNCH();
+}
+
+void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial) {
+  if (!kernel_ok()) throw Error(SCESS_ERR_UNSUPPORTED, "slice gemm: kernel unavailable");
+  if (ps.M <= 0 || ps.N <= 0 || ps.ny <= 0 || ps.nz <= 0 || ps.ng <= 0) return;
+  if (ps.ng > 3 || ps.nseg < 1 || ps.nseg > 4) throw Error(SCESS_ERR_INVALID, "slice gemm: groups or segments");
+  SliceArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.M = (int)ps.M;
+  a.N = (int)ps.N;
+  a.tiles_m = (int)ceil_div(ps.M, BM);
+  // column tiles of equal width (the B-side maps have boxes of this many rows)
+  a.bn = tile_n(ps.N);
+  a.tiles_n = (int)ceil_div(ps.N, a.bn);
+  a.ny = ps.ny;
+  a.nz = ps.nz;
+  a.ng = ps.ng;
+  a.nseg = ps.nseg;
+  for (int s = 0; s < ps.nseg; s++) {
+    const SliceSegment &g = ps.seg[s];
+    if (g.Kpad % BK != 0 || g.Kpad <= 0 || kSlices * g.Kpad > INT32_MAX)
+      throw Error(SCESS_ERR_INVALID, "slice gemm: segment K");
+    for (int q = 0; q < ps.ng; q++) {
+      const int64_t maxA = g.rowA0[q] + (int64_t)(ps.ny - 1) * g.rowAy[q] + (int64_t)(ps.nz - 1) * g.rowAz[q] + a.tiles_m * BM;
+      const int64_t maxB = g.rowB0[q] + (int64_t)(ps.ny - 1) * g.rowBy[q] + (int64_t)(ps.nz - 1) * g.rowBz[q] + a.tiles_n * a.bn;
+      if (maxA > INT32_MAX || maxB > INT32_MAX || g.rowA0[q] < 0 || g.rowB0[q] < 0 || g.rowAy[q] < 0 ||
+          g.rowAz[q] < 0 || g.rowBy[q] < 0 || g.rowBz[q] < 0)
+        throw Error(SCESS_ERR_INVALID, "slice gemm: row coordinates");
+    }
+    SegArgs &d = a.seg[s];
+    d.mapA = g.mapA;
+    d.mapB = g.mapB;
+    d.nkb = (int)(g.Kpad / BK);
+    d.kpad = (int)g.Kpad;
+    for (int q = 0; q < 3; q++) {
+      d.rowA0[q] = g.rowA0[q];
+      d.rowAy[q] = g.rowAy[q];
+      d.rowAz[q] = g.rowAz[q];
+      d.rowB0[q] = g.rowB0[q];
+      d.rowBy[q] = g.rowBy[q];
+      d.rowBz[q] = g.rowBz[q];
+    }
+    a.kb_total += d.nkb;
+  }
+  splits = std::max(1, std::min(splits, a.kb_total));
+  a.kb_per_split = (int)ceil_div(a.kb_total, splits);
+  a.splits = (int)ceil_div(a.kb_total, a.kb_per_split);
+  // the 64-bit sum holds 2^12 k 2^36 per output: K <= 2^14 a unit
+  // and the tail, below 2^10 K in units of the integer, in 31 bits
+  a.fs = 20;
+  for (int64_t k = (int64_t)a.kb_per_split * BK; k > 1; k >>= 1) a.fs--;
+  if (a.kb_per_split > 512) throw Error(SCESS_ERR_INVALID, "slice gemm: K of a unit");
+  int64_t start = 0;
+  for (int g = 0; g < ps.ng; g++) {
+    if (ps.tri[g] && ps.ny != ps.nz) throw Error(SCESS_ERR_INVALID, "slice gemm: triangular groups need ny == nz");
+    a.tri[g] = ps.tri[g] ? 1 : 0;
+    a.gstart[g] = (int)start;
+    start += a.tri[g] ? (int64_t)ps.ny * (ps.ny + 1) / 2 : (int64_t)ps.ny * ps.nz;
+    a.expA0[g] = ps.expA0[g];
+    a.cy[g] = ps.cy[g];
+    a.cz[g] = ps.cz[g];
+    a.cg[g] = ps.cg[g];
+    a.rowC[g] = ps.rowC[g];
+    a.colC[g] = ps.colC[g];
+  }
+  if (start > INT32_MAX) throw Error(SCESS_ERR_INVALID, "slice gemm: too many problems");
+  a.gstart[ps.ng] = (int)start;
+  a.expA = ps.expA;
+  a.expB = ps.expB;
+  a.C = ps.C;
+  a.baseC = ps.baseC;
+  a.alpha = ps.alpha;
+  a.beta = ps.beta;
+  int e = 0;
+  const double f = std::frexp(ps.alpha, &e);
+  a.alpha_pow2 = std::fabs(f) == 0.5 && e > -500 && e < 500;
+  a.alpha_e = e - 1;
+  a.alpha_neg = f < 0;
+  a.partial = a.splits > 1 ? partial : nullptr;
+  a.part_stride = ps.M * ps.N;
+  if (a.splits > 1 && (!partial || start > 1)) throw Error(SCESS_ERR_INVALID, "slice gemm: split-K");
+  a.err = err_.as<unsigned>();
+  a.wait_cycles = wait_cycles_;
+  a.withhold_first = withhold_ ? 1 : 0;
+  wait_cycles_ = 1ll << 32;  // (diagnostics are for one launch)
+  withhold_ = false;
+  SliceMaps maps;
+  for (int i = 0; i < 6; i++) maps.m[i] = ps.maps[std::min(i, ps.nmaps - 1)];
+  const int64_t units = (int64_t)a.tiles_m * a.tiles_n * start * a.splits;
+  if (units > INT32_MAX) throw Error(SCESS_ERR_INVALID, "slice gemm: too many work units");
+  launched_ = true;
+  slice_gemm_kernel<<<(unsigned)std::min<int64_t>(units, kNumSMs), THREADS, SMEM_BYTES, ctx_.stream>>>(maps, a);
+  SCESS_CHECK_LAUNCH();
+  if (a.splits > 1) {
+    slice_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div(ps.M * ps.N, 256), 8192), 256, 0, ctx_.stream>>>(
+        a, a.splits);
+    SCESS_CHECK_LAUNCH();
+  }
+}
+
+void SliceEngine::gemm_grouped(const SliceProblemSet &ps, double flops, const char *name) {
+  TimedScope ts(ctx_.timer, name, flops, 0.0, ctx_.stream);
+  launch(ps, 1, nullptr);
+}
+
+void SliceEngine::gemm(const SlicedPack &A, const SlicedPack &B, double alpha, double beta, double *C,
+                       const int64_t *rowC, const int64_t *colC, const char *name) {
+  SliceProblemSet ps;
+  ps.M = A.rows;
+  ps.N = B.rows;
+  const int64_t nkb = A.Kpad / BK, tiles = ceil_div(ps.M, BM) * ceil_div(ps.N, tile_n(ps.N));
+  // split K when the tiles leave SMs idle (at least 4 K blocks a unit) or a
+  // unit's K would pass what its 64-bit sum holds
+  int64_t splits = 1;
+  if (tiles < kNumSMs) splits = std::max<int64_t>(1, std::min<int64_t>(kNumSMs / tiles, nkb / 4));
+  while (splits > 1 && splits * ps.M * ps.N > (int64_t(64) << 20)) splits--;
+  splits = std::max(splits, ceil_div(nkb, 512));
+  double *partial = nullptr;
+  if (splits > 1) {
+    const size_t need = (size_t)splits * ps.M * ps.N * sizeof(double);
+    if (partial_.bytes() < need) partial_.alloc(need);
+    partial = partial_.d();
+  }
+  TimedScope ts(ctx_.timer, name, 2.0 * ps.M * ps.N * A.K, 0.0, ctx_.stream);
+  ps.maps[0] = map_of(A, BM);
+  ps.maps[1] = map_of(B, tile_n(ps.N));
+  ps.nmaps = 2;
+  ps.seg[0].Kpad = A.Kpad;
+  ps.expA = A.e();
+  ps.expB = B.e();
+  ps.C = C;
+  ps.rowC[0] = rowC;
+  ps.colC[0] = colC;
+  ps.alpha = alpha;
+  ps.beta = beta;
+  launch(ps, (int)splits, partial);
+}
+
+bool SliceEngine::table_gemm(const TableGemm &g, const char *name) {
+  try {
+    pack({g.A + g.baseA, g.rowA, g.M, g.kA, g.K, !g.aUnitM}, tmpA_);
+    pack({g.B + g.baseB, g.colB, g.N, g.kB, g.K, !g.bUnitN}, tmpB_);
+    if (g.M <= 64 && g.M < g.N) gemm(tmpB_, tmpA_, g.alpha, g.beta, g.C + g.baseC, g.colC, g.rowC, name);
+    else gemm(tmpA_, tmpB_, g.alpha, g.beta, g.C + g.baseC, g.rowC, g.colC, name);
+  } catch (const Error &e) {
+    if (e.code != SCESS_ERR_OOM) throw;
+    return false;
+  }
+  dgemm_masked(g, tmpA_.e(), tmpB_.e(), ctx_.stream);
+  return true;
+}
+
+void SliceEngine::clear_cache(const void *owner) {
+  for (auto it = cache_.begin(); it != cache_.end();) {
+    if (it->second.first == owner) it = cache_.erase(it);
+    else ++it;
+  }
+}
+
+void SliceEngine::check_error() {
+  if (!launched_) return;
+  launched_ = false;
+  unsigned h = 0;
+  SCESS_CUDA(cudaMemcpyAsync(&h, err_.as<void>(), sizeof(unsigned), cudaMemcpyDeviceToHost, ctx_.stream));
+  ctx_.sync();
+  if (h != 0) {
+    SCESS_CUDA(cudaMemsetAsync(err_.as<void>(), 0, sizeof(unsigned), ctx_.stream));
+    throw Error(SCESS_ERR_CUDA, "tensor-core pipeline wait expired (code " + std::to_string(h) + ")");
+  }
+}
+
+bool SliceEngine::contract(const EinsumPlan &pl, double alpha, const double *A, const double *B, double beta,
+                           double *C, bool constA, bool constB) {
+  // Epilogue lanes walk the GEMM rows: put C's unit-stride index there, unless
+  // that side is short: rows come in tiles of 128, columns in steps of 16.
+  const bool swap = std::min(pl.M, pl.N) <= 64 ? pl.M < pl.N : (!pl.cUnitM && pl.cUnitN);
+  const Gather gA{A, pl.d_rowA, pl.M, pl.d_kA, pl.K, pl.aUnitK, pl.aRowStride, pl.aKStride, pl.aRowP, pl.aRowE};
+  const Gather gB{B, pl.d_colB, pl.N, pl.d_kB, pl.K, pl.bUnitK, pl.bColStride, pl.bKStride, pl.bColP, pl.bColE};
+  auto get = [&](const Gather &g, bool isA, bool isConst, SlicedPack &tmp) -> const SlicedPack & {
+    if (!isConst && !stable_.count(g.src)) {
+      pack(g, tmp);
+      return tmp;
+    }
+    uint64_t &hs = isA ? pl.hashA : pl.hashB;
+    if (!hs) hs = isA ? table_hash(pl.rowA, pl.kA) : table_hash(pl.colB, pl.kB);
+    const std::string key = std::to_string((uintptr_t)g.src) + "|" + std::to_string(hs) + "|" +
+                            std::to_string(g.rows) + "|" + std::to_string(g.K);
+    if (isConst) {
+      auto it = cache_.find(key);
+      if (it != cache_.end() && it->second.first == owner_) return *it->second.second;
+    } else {
+      auto it = reuse_.find(key);
+      if (it != reuse_.end()) return *it->second;
+    }
+    auto pk = std::make_unique<SlicedPack>();
+    pack(g, *pk);
+    SlicedPack &ref = *pk;
+    if (isConst) cache_[key] = std::make_pair(owner_, std::move(pk));
+    else reuse_[key] = std::move(pk);
+    return ref;
+  };
+  const std::string tname = "slice_gemm[" + pl.spec + "]";
+  const SlicedPack *pa = nullptr, *pb = nullptr;
+  try {
+    pa = &get(gA, true, constA, tmpA_);
+    pb = &get(gB, false, constB, tmpB_);
+    if (swap) gemm(*pb, *pa, alpha, beta, C, pl.d_colC, pl.d_rowC, tname.c_str());
+    else gemm(*pa, *pb, alpha, beta, C, pl.d_rowC, pl.d_colC, tname.c_str());
+  } catch (const Error &e) {
+    if (e.code != SCESS_ERR_OOM) throw;
+    // no room for the packs: give the kept ones back, the DFMA kernel needs none
+    reuse_.clear();
+    clear_cache(owner_);
+    return false;
+  }
+  TableGemm g;
+  g.A = A;
+  g.B = B;
+  g.C = C;
+  g.rowA = pl.d_rowA;
+  g.kA = pl.d_kA;
+  g.colB = pl.d_colB;
+  g.kB = pl.d_kB;
+  g.rowC = pl.d_rowC;
+  g.colC = pl.d_colC;
+  g.M = pl.M;
+  g.N = pl.N;
+  g.K = pl.K;
+  g.alpha = alpha;
+  g.beta = beta;
+  g.aUnitM = pl.aUnitM;
+  g.bUnitN = pl.bUnitN;
+  dgemm_masked(g, pa->e(), pb->e(), ctx_.stream);
+  return true;
+}
+
+}  // namespace scess

@@ -1,0 +1,148 @@
+// FP64 contractions on the tensor cores: operands cut into exact BF16 slices.
+//
+// GB300's FP64 units run at about 1 TFLOP/s, 1/1900 of its BF16 tensor rate.  An
+// FP64 value is therefore cut into kSlices = 7 signed base-512 digits of a fixed
+// point number scaled to its row's largest exponent (error-free splitting in
+// the manner of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012; on
+// tensor cores Mukunoki et al., ISC 2020):
+//   x = 2^(E - 6) sum_p d_p 2^(-9 p),  |d_0| <= 64, |d_p| <= 256,
+// E the row's exponent, the last digit rounded: 60 bits below the row's largest
+// value.  Digits d_p 2^(-9 p) are exact in BF16.  A product of two rows is
+//   sum_d 2^(-9 d) S_d,  S_d = sum_k sum_(p + q = d) a_p b_q,
+// and as long as an S_d stays within 2^24 (64 values of k at least, for d <= 4) its
+// FP32 sum inside the tensor core is exact.  The kernel drains S_0 .. S_4 in time
+// into one 64-bit integer per output (exact), lets S_5 and S_6 (weights 2^-45,
+// 2^-54) add up in FP32 in tensor memory over the whole K range, and rounds
+// integer + FP32 tail to FP64 once.  Dropped: S_7 and beyond (2^-63).
+// Per output the error is about 2^-59 |row max| |column max| sqrt(K) and one
+// rounding to 53 bits, where a chain of K fused multiply-adds rounds K times.
+//
+// Rows holding Inf or NaN are marked by the pack kernel; their outputs are left to
+// the DFMA kernel (dgemm_masked), which is launched behind every GEMM and returns
+// at once where nothing is marked.
+#pragma once
+#include <cuda.h>
+
+#include <map>
+#include <memory>
+#include <set>
+#include <string>
+#include <vector>
+
+#include "engine.h"
+
+namespace scess {
+
+constexpr int kSlices = 7;
+constexpr int kSliceBK = 32;        // K block of the kernel: 32 x 16 bit = 64 B rows, SWIZZLE_64B
+constexpr int kRowNonFinite = 2047;  // row exponent of a row that holds Inf or NaN
+
+// rows x [kSlices][Kpad] BF16 digits, Kpad a multiple of 32, and one biased FP64
+// exponent per row (0: all values zero; kRowNonFinite: Inf or NaN).
+struct SlicedPack {
+  DevMem mem, exps;
+  int64_t rows = 0, K = 0, Kpad = 0;
+  const int *e() const { return exps.as<int>(); }
+};
+
+// One K segment of a grouped launch (see TcSegment, gemm_tc.h).
+struct SliceSegment {
+  int mapA = 0, mapB = 1;
+  int64_t Kpad = 0;
+  int64_t rowA0[3] = {0, 0, 0}, rowAy[3] = {0, 0, 0}, rowAz[3] = {0, 0, 0};
+  int64_t rowB0[3] = {0, 0, 0}, rowBy[3] = {0, 0, 0}, rowBz[3] = {0, 0, 0};
+};
+struct SliceProblemSet {
+  CUtensorMap maps[6];
+  int nmaps = 0;
+  int64_t M = 0, N = 0;
+  int ny = 1, nz = 1, ng = 1, nseg = 1;
+  SliceSegment seg[4];
+  bool tri[3] = {false, false, false};  // group g keeps its problems with y >= z
+  // exponents of output row m / column n of group g: expA[expA0[g] + m], expB[n]
+  const int *expA = nullptr, *expB = nullptr;
+  int64_t expA0[3] = {0, 0, 0};
+  // output element (m, n) of problem (y, z, g): C[baseC + y cy + z cz + cg + rowC[m] + colC[n]]
+  double *C = nullptr;
+  int64_t baseC = 0, cy[3] = {0, 0, 0}, cz[3] = {0, 0, 0}, cg[3] = {0, 0, 0};
+  const int64_t *rowC[3] = {nullptr, nullptr, nullptr}, *colC[3] = {nullptr, nullptr, nullptr};
+  double alpha = 1.0, beta = 0.0;
+};
+
+class SliceEngine {
+ public:
+  explicit SliceEngine(Ctx &ctx);
+  // Large enough to pay for the packs (see the definition for the line).
+  static bool worth_it(int64_t M, int64_t N, int64_t K);
+  // C = alpha A.B + beta C through the tables of g (the FP64 engine's GEMM).
+  // False when the packs do not fit into device memory: nothing was launched
+  // and the caller uses the DFMA kernel.
+  bool table_gemm(const TableGemm &g, const char *name);
+  bool contract(const EinsumPlan &pl, double alpha, const double *A, const double *B, double beta,
+                double *C, bool constA, bool constB);
+  void gemm_grouped(const SliceProblemSet &ps, double flops, const char *name);
+
+  // Largest biased exponent of every row of the gather src[rowOff[r] + kOff[k]],
+  // folded into exps[r] (atomic max; the caller clears exps first).
+  void row_exps(const double *src, const int64_t *rowOff, int64_t rows, const int64_t *kOff,
+                int64_t K, bool unitK, int *exps);
+  // Digits of the gather relative to the given row exponents exps[expIdx[r]]
+  // (expIdx null: exps[r]), optionally negated.
+  void pack_with_exps(const double *src, const int64_t *rowOff, int64_t rows, const int64_t *kOff,
+                      int64_t K, bool unitK, const int *exps, const int64_t *expIdx, bool negate,
+                      SlicedPack &out);
+  static CUtensorMap map_of(const SlicedPack &p, int box_rows);
+  // Column-tile width of an N-column product: the box rows of its B-side map
+  // (its A-side map has boxes of 128 rows).
+  static int tile_n(int64_t N);
+
+  // Packs of constant operands, kept for the owner of their source (see TcEngine).
+  void set_cache_owner(const void *o) { owner_ = o; }
+  void clear_cache(const void *owner);
+  // A tensor that stays unchanged until clear_stable(): einsums that gather it
+  // through equal tables share one pack.
+  void add_stable(const double *p) { stable_.insert(p); }
+  void clear_stable() {
+    stable_.clear();
+    reuse_.clear();
+  }
+  // Throws SCESS_ERR_CUDA if a bounded wait of a launch since the last check expired.
+  void check_error();
+  bool launched() const { return launched_; }
+  void arm_wait_expiry(long long wait_cycles) {
+    wait_cycles_ = wait_cycles;
+    withhold_ = true;
+  }
+
+ private:
+  struct Gather {  // an operand seen through its tables
+    const double *src;
+    const int64_t *row;
+    int64_t rows;
+    const int64_t *k;
+    int64_t K;
+    bool unitK;
+    int64_t rs = -1, ks = -1, P = 1, E = 0;
+  };
+  void pack(const Gather &g, SlicedPack &out);
+  void alloc(SlicedPack &out, int64_t rows, int64_t K);
+  void gemm(const SlicedPack &A, const SlicedPack &B, double alpha, double beta, double *C,
+            const int64_t *rowC, const int64_t *colC, const char *name);
+  void launch(const SliceProblemSet &ps, int splits, double *partial);
+
+  Ctx &ctx_;
+  std::map<std::string, std::pair<const void *, std::unique_ptr<SlicedPack>>> cache_;
+  std::map<std::string, std::unique_ptr<SlicedPack>> reuse_;
+  std::set<const double *> stable_;
+  const void *owner_ = nullptr;
+  SlicedPack tmpA_, tmpB_;
+  DevMem err_, partial_;
+  bool launched_ = false;
+  long long wait_cycles_ = 1ll << 32;
+  bool withhold_ = false;
+};
+
+// Outputs of g whose A row or B column is marked in expA / expB (kRowNonFinite).
+void dgemm_masked(const TableGemm &g, const int *expA, const int *expB, cudaStream_t stream);
+
+}  // namespace scess

@@ -6,96 +6,29 @@
 // permutation is fused into the tile loads), deterministic split-K when the
 // output has too few tiles to cover the 152 SMs.
 #include "common.cuh"
+#include "dgemm_tile.cuh"
 #include "kernels.h"
 
 namespace scess {
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16;
+constexpr int BM = kDgemmTile, BN = kDgemmTile, BK = kDgemmBK;
 
 __global__ void __launch_bounds__(256) dgemm_table_kernel(TableGemm g, int64_t kChunk,
                                                           double *partial) {
-  __shared__ double As[BK][BM];
-  __shared__ double Bs[BK][BN];
-  __shared__ int64_t sRowA[BM], sColB[BN], sKA[BK], sKB[BK];
-  const int t = threadIdx.x;
-  const int64_t m0 = (int64_t)blockIdx.x * BM, n0 = (int64_t)blockIdx.y * BN;
   const int64_t kb = (int64_t)blockIdx.z * kChunk;
-  const int64_t ke = min(g.K, kb + kChunk);
-  if (t < BM) {
-    const int64_t m = m0 + t;
-    sRowA[t] = m < g.M ? g.baseA + g.rowA[m] : -1;
-  } else if (t < BM + BN) {
-    const int64_t n = n0 + (t - BM);
-    sColB[t - BM] = n < g.N ? g.baseB + g.colB[n] : -1;
-  }
-  double acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
-  const int tx = t & 15, ty = t >> 4;
-  for (int64_t k0 = kb; k0 < ke; k0 += BK) {
-    __syncthreads();
-    if (t < BK) {
-      const int64_t k = k0 + t;
-      sKA[t] = k < ke ? g.kA[k] : -1;
-    } else if (t >= 32 && t < 32 + BK) {
-      const int64_t k = k0 + (t - 32);
-      sKB[t - 32] = k < ke ? g.kB[k] : -1;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const int idx = t + 256 * r;
-      int mm, kk;
-      if (g.aUnitM) { mm = idx & (BM - 1); kk = idx / BM; }
-      else { kk = idx & (BK - 1); mm = idx / BK; }
-      const int64_t ro = sRowA[mm], ko = sKA[kk];
-      As[kk][mm] = (ro >= 0 && ko >= 0) ? g.A[ro + ko] : 0.0;
-    }
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const int idx = t + 256 * r;
-      int nn, kk;
-      if (g.bUnitN) { nn = idx & (BN - 1); kk = idx / BN; }
-      else { kk = idx & (BK - 1); nn = idx / BK; }
-      const int64_t co = sColB[nn], ko = sKB[kk];
-      Bs[kk][nn] = (co >= 0 && ko >= 0) ? g.B[co + ko] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; kk++) {
-      double a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = As[kk][tx + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = Bs[kk][ty + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int64_t m = m0 + tx + 16 * i;
-    if (m >= g.M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int64_t n = n0 + ty + 16 * j;
-      if (n >= g.N) continue;
-      if (partial) {
-        partial[(int64_t)blockIdx.z * g.M * g.N + m + g.M * n] = acc[i][j];
-      } else {
-        const int64_t off = g.baseC + g.rowC[m] + g.colC[n];
-        double val = g.alpha * acc[i][j];
-        if (g.beta != 0.0) val += g.beta * g.C[off];
-        g.C[off] = val;
-      }
-    }
-  }
+  dgemm_tile(g, (int64_t)blockIdx.x * BM, (int64_t)blockIdx.y * BN, kb, min(g.K, kb + kChunk),
+             [&](int64_t m, int64_t n, double acc) {
+               if (partial) {
+                 partial[(int64_t)blockIdx.z * g.M * g.N + m + g.M * n] = acc;
+               } else {
+                 const int64_t off = g.baseC + g.rowC[m] + g.colC[n];
+                 double val = g.alpha * acc;
+                 if (g.beta != 0.0) val += g.beta * g.C[off];
+                 g.C[off] = val;
+               }
+             });
 }
 
 __global__ void splitk_reduce_kernel(TableGemm g, int splits, const double *partial) {

@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "gemm_slice.h"
 #include "gemm_tc.h"
 #include "rccsd.h"
 
@@ -214,14 +215,18 @@ void RccsdWork::alloc(int64_t o, int64_t v, bool direct_vvvv) {
 // hints), for the calls that run on the tensor cores; cleared on scope exit.
 struct MaxHints {
   TcEngine *tc = nullptr;
+  SliceEngine *slices = nullptr;  // FP64: packs of the tensors shared between einsums
   MaxHints(Ctx &ctx, Backend be) {
     if (be != Backend::FP64) tc = &ctx.tensor_cores();
+    else slices = &ctx.slice_engine();
   }
   void add(const double *p, int64_t n) {
     if (tc) tc->add_max_hint(p, n);
+    else slices->add_stable(p);
   }
   ~MaxHints() {
     if (tc) tc->clear_max_hints();
+    else slices->clear_stable();
   }
   MaxHints(const MaxHints &) = delete;
   MaxHints &operator=(const MaxHints &) = delete;

@@ -637,9 +637,8 @@ void TriplesSetup::build(Ctx &ctx, const double *d_eri, const double *d_t2, cons
 // sum over the six permutations of the raw P.Q - R.t2 product (GetW,
 // RCCSD_T.cpp:62-68), each added at its permuted position (Symmetrise :78-106).
 // tc: the same GEMMs on the tensor cores (TcEngine::table_gemm).
-void w_block_fp64(Ctx &ctx, const TriplesSetup &T, const int64_t U[3], double *W, double *ws,
+void w_block_fp64(Ctx &ctx, const TriplesSetup &T, const int64_t U[3], double *W,
                   bool tc = false) {
-  cudaStream_t s = ctx.stream;
   const int64_t o = T.o, v = T.v, nb = T.nb, vp = T.vp, o2 = o * o, o3 = o2 * o;
   for (int p = 0; p < 6; p++) {
     const int *pi = kPerm[p];
@@ -665,12 +664,8 @@ void w_block_fp64(Ctx &ctx, const TriplesSetup &T, const int64_t U[3], double *W
     g.beta = p == 0 ? 0.0 : 1.0;
     g.aUnitM = 1;
     g.bUnitN = 0;
-    if (tc) {
-      ctx.tensor_cores().table_gemm(g, "triples_w");
-    } else {
-      TimedScope ts(ctx.timer, "dgemm_table", 2.0 * g.M * g.N * g.K, 0.0, s);
-      dgemm_table(g, ws, s);
-    }
+    if (tc) ctx.tensor_cores().table_gemm(g, "triples_w");
+    else fp64_table_gemm(ctx, g, "slice_gemm[triples_w]");
     TableGemm h;
     h.A = T.Rt.p();
     h.B = T.T2p.p();
@@ -690,12 +685,8 @@ void w_block_fp64(Ctx &ctx, const TriplesSetup &T, const int64_t U[3], double *W
     h.beta = 1.0;
     h.aUnitM = r_swapped(pi) ? 0 : 1;
     h.bUnitN = 0;
-    if (tc) {
-      ctx.tensor_cores().table_gemm(h, "triples_w");
-    } else {
-      TimedScope ts(ctx.timer, "dgemm_table", 2.0 * h.M * h.N * h.K, 0.0, s);
-      dgemm_table(h, ws, s);
-    }
+    if (tc) ctx.tensor_cores().table_gemm(h, "triples_w");
+    else fp64_table_gemm(ctx, h, "slice_gemm[triples_w]");
   }
 }
 
@@ -825,18 +816,13 @@ __global__ void __launch_bounds__(256) triples_grad_kernel(
 // per permutation, G read through that permutation's W tables.
 // tc: the same GEMMs on the tensor cores (TcEngine::table_gemm).
 void g_block_fp64(Ctx &ctx, const TriplesSetup &T, const int64_t U[3], const double *G, double *gP,
-                  double *gQt, double *gRt, double *gT2p, bool integrals, double *ws,
+                  double *gQt, double *gRt, double *gT2p, bool integrals,
                   bool tc = false) {
-  cudaStream_t s = ctx.stream;
   const int64_t o = T.o, v = T.v, nb = T.nb, vp = T.vp, o2 = o * o, o3 = o2 * o;
   const size_t K0 = T.kOperand;
   auto run = [&](TableGemm &g) {
-    if (tc) {
-      ctx.tensor_cores().table_gemm(g, "triples_vjp");
-      return;
-    }
-    TimedScope ts(ctx.timer, "dgemm_table", 2.0 * g.M * g.N * g.K, 0.0, s);
-    dgemm_table(g, ws, s);
+    if (tc) ctx.tensor_cores().table_gemm(g, "triples_vjp");
+    else fp64_table_gemm(ctx, g, "slice_gemm[triples_vjp]");
   };
   for (int p = 0; p < 6; p++) {
     const int *pi = kPerm[p];
@@ -996,7 +982,6 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
   DevMem Sf;    // (ia|jb) as FP32 for the energy kernel (padded rows)
   DevMem etab;  // eps as FP32 hi + lo (nmo float2), then t1 in FP32
   const int64_t Mg = o * nb, Ng = o2;
-  const int64_t Mpq = o * nb * nb, Npq = o2 * nb, Mr = o2 * nb, Nr = o * nb * nb;  // FP64 GEMMs
   if (mixed) {
     TimedScope ts(ctx.timer, "phase:triples_pack", 0.0, 0.0, s);
     TcEngine &tc = ctx.tensor_cores();
@@ -1063,19 +1048,6 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
   // (i, j) pairs spread evenly over at most 256 threads
   const unsigned e3threads =
       (unsigned)round_up(ceil_div(o2, ceil_div(o2, 256)), 32);
-  double *ws = nullptr;
-  if (!mixed) {
-    TableGemm probe;
-    probe.M = Mpq;
-    probe.N = Npq;
-    probe.K = v;
-    TableGemm probe2;
-    probe2.M = Mr;
-    probe2.N = Nr;
-    probe2.K = o;
-    ws = ctx.ensure_workspace(std::max(dgemm_table_workspace(probe), dgemm_table_workspace(probe2)));
-  }
-
   // MIXED: consecutive launches overlap (programmatic dependent launches);
   // SCESS_TUNE t_pdl = 0 serialises them, for comparison
   const bool pdl = tune_value("t_pdl", 1) != 0;
@@ -1171,7 +1143,7 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
           ps.pdl = pdl && blocks_done > 0;
           tc.gemm_grouped(ps, out, flops, "tc_gemm[triples]");
         } else {
-          w_block_fp64(ctx, T, U, W.d(), ws);
+          w_block_fp64(ctx, T, U, W.d());
         }
         const unsigned nblk = (unsigned)(nb * nb * nb);
         TimedScope ts(ctx.timer, "triples_energy", 0.0,
@@ -1252,26 +1224,13 @@ double rccsd_triples_vjp(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o,
   if (gsmem > 200 * 1024) throw Error(SCESS_ERR_UNSUPPORTED, "(T) gradient: o^3 too large for one CTA");
   SCESS_CUDA(cudaFuncSetAttribute(triples_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)gsmem));
-  int64_t need = 0;
-  {
-    const int64_t shapes[6][3] = {{T.Mpq(), T.Npq(), v}, {T.Mr(), T.Nr(), o}, {T.Mpq(), v, T.Npq()},
-                                  {T.Npq(), v, T.Mpq()}, {T.Mr(), o, T.Nr()}, {T.Nr(), o, T.Mr()}};
-    for (auto &sh : shapes) {
-      TableGemm probe;
-      probe.M = sh[0];
-      probe.N = sh[1];
-      probe.K = sh[2];
-      need = std::max(need, dgemm_table_workspace(probe));
-    }
-  }
-  double *ws = ctx.ensure_workspace(need);
   int64_t blocks_done = 0;
   for (int64_t A = 0; A < NB; A++)
     for (int64_t Bk = 0; Bk <= A; Bk++)
       for (int64_t C = 0; C <= Bk; C++) {
         if ((blocks_done & 15) == 0) ctl.poll();
         const int64_t U[3] = {A, Bk, C};
-        w_block_fp64(ctx, T, U, W.d(), ws, mixed);
+        w_block_fp64(ctx, T, U, W.d(), mixed);
         {
           TimedScope ts(ctx.timer, "triples_grad", 0.0, 0.0, s);
           triples_grad_kernel<<<(unsigned)(nb * nb * nb), 256, gsmem, s>>>(
@@ -1280,7 +1239,7 @@ double rccsd_triples_vjp(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o,
           SCESS_CHECK_LAUNCH();
         }
         g_block_fp64(ctx, T, U, G.d(), integrals ? gP.p() : nullptr, gQt.p(),
-                     integrals ? gRt.p() : nullptr, gT2p.p(), integrals, ws, mixed);
+                     integrals ? gRt.p() : nullptr, gT2p.p(), integrals, mixed);
         blocks_done++;
       }
   sum_energies_kernel<<<1, 1024, 0, s>>>(ntrip, energies.p(), ctx.dscalars);
