@@ -168,6 +168,8 @@ Ctx::Ctx(int dev) : device(dev) {
   partials = scratch.d();
   dscalars = partials + kDotBlocks;
   SCESS_CUDA(cudaMallocHost(&hscalars, 64 * sizeof(double)));
+  counters.alloc(kSmallCounters * sizeof(int));
+  SCESS_CUDA(cudaMemsetAsync(counters.as<void>(), 0, kSmallCounters * sizeof(int), stream));
 }
 
 Ctx::~Ctx() {
@@ -178,6 +180,7 @@ Ctx::~Ctx() {
   plans.clear();
   workspace.release();
   scratch.release();
+  counters.release();
   if (hscalars) cudaFreeHost(hscalars);
   if (stream) cudaStreamDestroy(stream);
 }
@@ -505,6 +508,19 @@ const EinsumPlan &plan_einsum(Ctx &ctx, const char *spec, const TV &A, const TV 
   return ref;
 }
 
+namespace {
+// C = alpha A.B + beta C on the FP64 units.
+void dfma_gemm(Ctx &ctx, const TableGemm &g) {
+  if (dgemm_small_ok(g)) {
+    TimedScope ts(ctx.timer, "dgemm_small", 2.0 * g.M * g.N * g.K, 0.0, ctx.stream);
+    dgemm_small(g, ctx.ensure_workspace(dgemm_small_workspace(g)), ctx.counters.as<int>(), ctx.stream);
+    return;
+  }
+  TimedScope ts(ctx.timer, "dgemm_table", 2.0 * g.M * g.N * g.K, 0.0, ctx.stream);
+  dgemm_table(g, ctx.ensure_workspace(dgemm_table_workspace(g)), ctx.stream);
+}
+}  // namespace
+
 void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, double beta,
             const TV &C, Backend be, bool constA, bool constB) {
   if (ctx.tape) {
@@ -548,9 +564,6 @@ void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, 
     ctx.tensor_cores().contract(pl, alpha, A.p, B.p, beta, C.p, constA, constB);
     return;
   }
-  if (SliceEngine::worth_it(pl.M, pl.N, pl.K) &&
-      ctx.slice_engine().contract(pl, alpha, A.p, B.p, beta, C.p, constA, constB))
-    return;
   TableGemm g;
   g.A = A.p;
   g.B = B.p;
@@ -568,14 +581,13 @@ void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, 
   g.beta = beta;
   g.aUnitM = pl.aUnitM;
   g.bUnitN = pl.bUnitN;
-  TimedScope ts(ctx.timer, (pl.N == 1 || pl.M == 1) ? "dgemv_table" : "dgemm_table",
-                2.0 * pl.M * pl.N * pl.K, 0.0, ctx.stream);
-  if (pl.N == 1 && pl.K > 0) {
-    dgemv_table(g, ctx.stream);
-    return;
-  }
-  if (pl.M == 1 && pl.K > 0) {  // C^T = B^T A^T
-    TableGemm h = g;
+  if ((pl.N == 1 || pl.M == 1) && pl.K > 0) {
+    TimedScope ts(ctx.timer, "dgemv_table", 2.0 * pl.M * pl.N * pl.K, 0.0, ctx.stream);
+    if (pl.N == 1) {
+      dgemv_table(g, ctx.stream);
+      return;
+    }
+    TableGemm h = g;  // C^T = B^T A^T
     h.A = B.p;
     h.B = A.p;
     h.rowA = pl.d_colB;
@@ -589,14 +601,16 @@ void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, 
     dgemv_table(h, ctx.stream);
     return;
   }
-  double *ws = ctx.ensure_workspace(dgemm_table_workspace(g));
-  dgemm_table(g, ws, ctx.stream);
+  if (!dgemm_small_ok(g) && SliceEngine::usable(pl.M, pl.N) &&
+      ctx.slice_engine().contract(pl, alpha, A.p, B.p, beta, C.p, constA, constB))
+    return;
+  dfma_gemm(ctx, g);
 }
 
 void fp64_table_gemm(Ctx &ctx, const TableGemm &g, const char *name) {
-  if (SliceEngine::worth_it(g.M, g.N, g.K) && ctx.slice_engine().table_gemm(g, name)) return;
-  TimedScope ts(ctx.timer, "dgemm_table", 2.0 * g.M * g.N * g.K, 0.0, ctx.stream);
-  dgemm_table(g, ctx.ensure_workspace(dgemm_table_workspace(g)), ctx.stream);
+  if (!dgemm_small_ok(g) && SliceEngine::usable(g.M, g.N) && ctx.slice_engine().table_gemm(g, name))
+    return;
+  dfma_gemm(ctx, g);
 }
 
 void permute(Ctx &ctx, const char *spec, double alpha, const TV &X, double beta, const TV &Y) {

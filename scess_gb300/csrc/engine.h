@@ -222,6 +222,7 @@ struct Ctx {
   std::map<std::string, std::unique_ptr<EinsumPlan>> plans;
   DevMem workspace;          // split-K partials
   DevMem scratch;            // partial sums of reductions + device scalars
+  DevMem counters;           // dgemm_small's tile counters (zero between launches)
   double *partials = nullptr;
   double *dscalars = nullptr;  // 64 device doubles
   double *hscalars = nullptr;  // 64 pinned host doubles
@@ -244,8 +245,8 @@ struct Ctx {
   SliceEngine &slice_engine();
 };
 
-// C = alpha A.B + beta C in FP64 through the tables of g: on the tensor cores'
-// exact slices where that pays (SliceEngine::worth_it), else the DFMA kernel.
+// C = alpha A.B + beta C in FP64 through the tables of g: small products on the
+// FP64 units (dgemm_small_ok), the others on the tensor cores' exact slices.
 void fp64_table_gemm(Ctx &ctx, const TableGemm &g, const char *name);
 
 // FP64: DFMA engine.  MIXED: tensor cores for contractions large enough to pay

@@ -604,12 +604,8 @@ SliceEngine::SliceEngine(Ctx &ctx) : ctx_(ctx) {
 
 int SliceEngine::tile_n(int64_t N) { return (int)round_up(ceil_div(N, ceil_div(N, BN)), 16); }
 
-bool SliceEngine::worth_it(int64_t M, int64_t N, int64_t K) {
-  if (!kernel_ok() || M > INT32_MAX / 2 || N > INT32_MAX / 2 || K < 1 || std::min(M, N) < 2) return false;
-  // The DFMA kernel computes whole 64 x 64 tiles at about 1 TFLOP/s; packs, GEMM and
-  // mask check take about 25 us before size counts.
-  const double tiles = (double)round_up(M, 64) * (double)round_up(N, 64);
-  return 2.0 * tiles * (double)K >= 3.0e7;
+bool SliceEngine::usable(int64_t M, int64_t N) {
+  return kernel_ok() && M <= INT32_MAX / 2 && N <= INT32_MAX / 2;
 }
 
 CUtensorMap SliceEngine::map_of(const SlicedPack &p, int box_rows) {

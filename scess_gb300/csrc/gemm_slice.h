@@ -72,8 +72,8 @@ struct SliceProblemSet {
 class SliceEngine {
  public:
   explicit SliceEngine(Ctx &ctx);
-  // Large enough to pay for the packs (see the definition for the line).
-  static bool worth_it(int64_t M, int64_t N, int64_t K);
+  // The device runs the kernel and the sizes are within its coordinates.
+  static bool usable(int64_t M, int64_t N);
   // C = alpha A.B + beta C through the tables of g (the FP64 engine's GEMM).
   // False when the packs do not fit into device memory: nothing was launched
   // and the caller uses the DFMA kernel.

@@ -59,18 +59,118 @@ int choose_splits(const TableGemm &g) {
 }  // namespace
 
 namespace {
-__global__ void dgemv_table_kernel(TableGemm g) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+
+// Small FP64 contraction: GB300 issues about two FP64 lanes per cycle and SM, so one
+// 64 x 64 x 16 step of dgemm_table_kernel takes an SM 18 us.  Small products are
+// therefore cut finely over the whole device: 8 x 8 outputs a CTA, K in ranges of
+// at most kSmallKB staged at once (two dependent loads, then arithmetic), the four
+// 64-thread groups taking every fourth k.  With several K ranges per tile the last
+// CTA of the tile to finish adds the partial sums in order (deterministic) and
+// leaves the tile's counter at zero.  90 x 10 x 90: 107 -> 4 us.
+constexpr int kSmallT = 8, kSmallKB = 128;
+__global__ void __launch_bounds__(256) dgemm_small_kernel(TableGemm g, int64_t kper, int splits,
+                                                          double *__restrict__ partial,
+                                                          int *__restrict__ counters) {
+  __shared__ double As[kSmallKB][kSmallT + 1], Bs[kSmallKB][kSmallT + 1];
+  __shared__ double red[4][64];
+  __shared__ int last;
+  const int t = threadIdx.x, grp = t >> 6, o = t & 63, i = o & 7, j = o >> 3;
+  const int64_t tm = (g.M + kSmallT - 1) / kSmallT;
+  const int64_t tile = blockIdx.x / splits, z = blockIdx.x % splits;
+  const int64_t m0 = (tile % tm) * kSmallT, n0 = (tile / tm) * kSmallT;
+  const int64_t kb = z * kper, ke = min(g.K, kb + kper);
+  double acc = 0.0;
+  for (int64_t k0 = kb; k0 < ke; k0 += kSmallKB) {
+    const int nk = (int)min((int64_t)kSmallKB, ke - k0);
+    int64_t ra[4], rb[4];
+    double a[4], b[4];
+    // along the operand's unit-stride side, eight rows / columns of up to 128 k
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+      const int e = t + 256 * p;
+      const int am = g.aUnitM ? e & 7 : e >> 7, ak = g.aUnitM ? e >> 3 : e & 127;
+      const int bm = g.bUnitN ? e & 7 : e >> 7, bk = g.bUnitN ? e >> 3 : e & 127;
+      ra[p] = (m0 + am < g.M && ak < nk) ? g.rowA[m0 + am] + g.kA[k0 + ak] : -1;
+      rb[p] = (n0 + bm < g.N && bk < nk) ? g.colB[n0 + bm] + g.kB[k0 + bk] : -1;
+    }
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+      a[p] = ra[p] >= 0 ? g.A[g.baseA + ra[p]] : 0.0;
+      b[p] = rb[p] >= 0 ? g.B[g.baseB + rb[p]] : 0.0;
+    }
+    __syncthreads();  // the previous range is used up
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+      const int e = t + 256 * p;
+      if (g.aUnitM) As[e >> 3][e & 7] = a[p];
+      else As[e & 127][e >> 7] = a[p];
+      if (g.bUnitN) Bs[e >> 3][e & 7] = b[p];
+      else Bs[e & 127][e >> 7] = b[p];
+    }
+    __syncthreads();
+    if (m0 + i < g.M && n0 + j < g.N)
+      for (int k = grp; k < nk; k += 4) acc = fma(As[k][i], Bs[k][j], acc);
+  }
+  red[grp][o] = acc;
+  __syncthreads();
+  double s = 0.0;
+  if (t < 64) s = (red[0][t] + red[1][t]) + (red[2][t] + red[3][t]);
+  if (splits > 1) {
+    double *p = partial + tile * splits * 64;
+    if (t < 64) p[z * 64 + t] = s;
+    __threadfence();
+    __syncthreads();
+    if (t == 0) last = atomicAdd(&counters[tile], 1) == splits - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double v = 0.0;
+    for (int q = grp; q < splits; q += 4) v += __ldcg(p + q * 64 + o);
+    red[grp][o] = v;
+    __syncthreads();
+    if (t < 64) s = (red[0][t] + red[1][t]) + (red[2][t] + red[3][t]);
+    if (t == 0) counters[tile] = 0;
+  }
+  if (t < 64 && m0 + i < g.M && n0 + j < g.N) {
+    const int64_t off = g.baseC + g.rowC[m0 + i] + g.colC[n0 + j];
+    double val = g.alpha * s;
+    if (g.beta != 0.0) val += g.beta * g.C[off];
+    g.C[off] = val;
+  }
+}
+
+struct SmallShape {
+  int64_t tiles, kper;
+  int splits;
+};
+SmallShape small_shape(const TableGemm &g) {
+  SmallShape s;
+  s.tiles = ceil_div(g.M, kSmallT) * ceil_div(g.N, kSmallT);
+  // about two CTAs an SM, at least 16 k each; a range beyond 128 k is walked in steps
+  const int64_t want = s.tiles >= 2 * kNumSMs ? 1 : ceil_div(2 * kNumSMs, s.tiles);
+  const int64_t n = std::max<int64_t>(1, std::min(want, ceil_div(g.K, 16)));
+  s.kper = round_up(ceil_div(g.K, n), 4);
+  s.splits = (int)ceil_div(g.K, s.kper);
+  return s;
+}
+
+// One row of a matrix-vector product per warp, or, with few rows, per CTA (its
+// eight warps then share the K range): four independent partial sums a lane, so
+// that four loads are in flight, added in a fixed order.
+template <bool CTA>
+__global__ void __launch_bounds__(256) dgemv_table_kernel(TableGemm g) {
+  __shared__ double red[8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t step = CTA ? 256 : 32, k0 = CTA ? threadIdx.x : lane;
+  const int64_t m1 = CTA ? gridDim.x : ((int64_t)gridDim.x * blockDim.x) >> 5;
   const double *__restrict__ B = g.B + g.baseB + g.colB[0];
-  for (int64_t m = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; m < g.M; m += warps) {
+  for (int64_t m = CTA ? blockIdx.x : ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; m < g.M; m += m1) {
     const double *__restrict__ A = g.A + g.baseA + g.rowA[m];
-    // four independent partial sums a lane: four loads in flight, fixed order
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    int64_t k = lane;
-    for (; k + 96 < g.K; k += 128) {
-      const int64_t ka0 = g.kA[k], ka1 = g.kA[k + 32], ka2 = g.kA[k + 64], ka3 = g.kA[k + 96];
-      const int64_t kb0 = g.kB[k], kb1 = g.kB[k + 32], kb2 = g.kB[k + 64], kb3 = g.kB[k + 96];
+    int64_t k = k0;
+    for (; k + 3 * step < g.K; k += 4 * step) {
+      const int64_t ka0 = g.kA[k], ka1 = g.kA[k + step], ka2 = g.kA[k + 2 * step], ka3 = g.kA[k + 3 * step];
+      const int64_t kb0 = g.kB[k], kb1 = g.kB[k + step], kb2 = g.kB[k + 2 * step], kb3 = g.kB[k + 3 * step];
       const double a0 = A[ka0], a1 = A[ka1], a2 = A[ka2], a3 = A[ka3];
       const double b0 = B[kb0], b1 = B[kb1], b2 = B[kb2], b3 = B[kb3];
       s0 = fma(a0, b0, s0);
@@ -78,10 +178,17 @@ __global__ void dgemv_table_kernel(TableGemm g) {
       s2 = fma(a2, b2, s2);
       s3 = fma(a3, b3, s3);
     }
-    for (; k < g.K; k += 32) s0 = fma(A[g.kA[k]], B[g.kB[k]], s0);
+    for (; k < g.K; k += step) s0 = fma(A[g.kA[k]], B[g.kB[k]], s0);
     double s = (s0 + s1) + (s2 + s3);
     for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-    if (lane == 0) {
+    if (CTA) {
+      __syncthreads();
+      if (lane == 0) red[w] = s;
+      __syncthreads();
+      if (threadIdx.x == 0)
+        s = ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
+    }
+    if (CTA ? threadIdx.x == 0 : lane == 0) {
       const int64_t off = g.baseC + g.rowC[m] + g.colC[0];
       double val = g.alpha * s;
       if (g.beta != 0.0) val += g.beta * g.C[off];
@@ -90,6 +197,25 @@ __global__ void dgemv_table_kernel(TableGemm g) {
   }
 }
 }  // namespace
+
+bool dgemm_small_ok(const TableGemm &g) {
+  // padded to whole 8 x 8 tiles: 6e6 multiply-adds take the device's FP64 units 10 us,
+  // what the packs and launches of the sliced form (gemm_slice.h) take at least
+  const double fma = (double)round_up(g.M, kSmallT) * (double)round_up(g.N, kSmallT) * (double)g.K;
+  // (many outputs of a short K: the 8 x 8 tiles' own overhead, 1805 x 475 x 5 takes 50 us)
+  return g.M > 0 && g.N > 0 && g.K > 0 && fma <= 6.0e6 && g.M * g.N <= (1 << 17);
+}
+
+int64_t dgemm_small_workspace(const TableGemm &g) {
+  const SmallShape s = small_shape(g);
+  return s.splits > 1 ? s.tiles * s.splits * 64 : 0;
+}
+
+void dgemm_small(const TableGemm &g, double *workspace, int *counters, cudaStream_t stream) {
+  const SmallShape s = small_shape(g);
+  dgemm_small_kernel<<<(unsigned)(s.tiles * s.splits), 256, 0, stream>>>(g, s.kper, s.splits, workspace, counters);
+  SCESS_CHECK_LAUNCH();
+}
 
 namespace {
 // Tables of a skinny contraction seen from its small side (Sm, s indices) and
@@ -237,8 +363,10 @@ void skinny_table(const TableGemm &g, bool small_is_a, bool stage, cudaStream_t 
 
 void dgemv_table(const TableGemm &g, cudaStream_t stream) {
   if (g.M <= 0) return;
-  const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(g.M * 32, 256), 16 * kNumSMs);
-  dgemv_table_kernel<<<blocks, 256, 0, stream>>>(g);
+  if (g.M < 8 * kNumSMs && g.K >= 512)  // too few rows for a warp each to fill the device
+    dgemv_table_kernel<true><<<(unsigned)std::min<int64_t>(g.M, 8 * kNumSMs), 256, 0, stream>>>(g);
+  else
+    dgemv_table_kernel<false><<<(unsigned)std::min<int64_t>(ceil_div(g.M * 32, 256), 16 * kNumSMs), 256, 0, stream>>>(g);
   SCESS_CHECK_LAUNCH();
 }
 

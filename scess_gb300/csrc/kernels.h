@@ -33,6 +33,14 @@ struct TableGemm {
 constexpr int kSkinnyMaxK = 32, kSkinnyMaxS = 256;
 void skinny_table(const TableGemm &g, bool small_is_a, bool stage, cudaStream_t stream);
 
+// The same contraction for products of at most about 6e6 multiply-adds, cut finely
+// over the device (dgemm_small_ok); workspace of dgemm_small_workspace doubles for
+// the K ranges' partial sums, counters: kSmallCounters zeroed ints (left zero).
+constexpr int kSmallCounters = 1024;
+bool dgemm_small_ok(const TableGemm &g);
+int64_t dgemm_small_workspace(const TableGemm &g);
+void dgemm_small(const TableGemm &g, double *workspace, int *counters, cudaStream_t stream);
+
 // FP64 matrix-vector form of the same contraction (N == 1), one warp per row,
 // deterministic.  Used instead of dgemm_table when N == 1 (or M == 1, swapped).
 void dgemv_table(const TableGemm &g, cudaStream_t stream);

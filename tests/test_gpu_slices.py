@@ -1,9 +1,10 @@
-"""FP64 contractions on the tensor cores' exact BF16 slices (SliceEngine).
+"""FP64 contractions: on the tensor cores' exact BF16 slices (SliceEngine) and, for
+small products, on the FP64 units.
 
 Sizes sit where the kernel can go wrong: tiles of 128 x 128 and K blocks of 32
 with remainders, one narrow side, K beyond what one unit's integer sum takes
 (16384: split), few tiles (split K) and many.  Every contraction is above the
-4e7 FLOPs from which the engine is used.
+6e6 multiply-adds from which the engine is used.
 
 Tolerance: an output is one rounding of a sum whose operands are cut 60 bits
 below their row's largest value and whose products below 2^-63 of
@@ -62,6 +63,34 @@ def test_alpha_beta_and_permuted_output(gctx, alpha, beta):
     got = gctx.einsum('iak,kbj->bija', A, B, C_init=C0, alpha=alpha, beta=beta)
     want = alpha * np.einsum('iak,kbj->bija', A, B, optimize=True) + beta * C0
     assert np.max(np.abs(got - want)) <= 2.0**-50 * np.max(np.abs(want))
+
+
+SMALL = [(1 + 8, 8, 3), (7, 9, 128), (8, 8, 129), (25, 19, 361), (5, 5, 9025), (90, 10, 90), (361, 25, 131),
+         (2, 3, 1), (700, 700, 11)]
+
+
+@pytest.mark.parametrize('M,N,K', SMALL)
+@pytest.mark.parametrize('spec', ['mk,kn->mn', 'km,nk->nm'])
+def test_small_products_are_exact(gctx, M, N, K, spec):
+    # 8 x 8 tiles and K ranges of 128 with remainders, one tile split over many CTAs
+    rng = np.random.default_rng(M * N + K)
+    A = rng.integers(-1000, 1001, (M, K)).astype(float)
+    B = rng.integers(-1000, 1001, (K, N)).astype(float)
+    C0 = rng.integers(-1000, 1001, (M, N)).astype(float)
+    want = 2.0 * (A @ B) - 3.0 * C0
+    if spec == 'km,nk->nm':
+        got = gctx.einsum(spec, A.T, B.T, C_init=C0.T, alpha=2.0, beta=-3.0).T
+    else:
+        got = gctx.einsum(spec, A, B, C_init=C0, alpha=2.0, beta=-3.0)
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize('M,K', [(1, 600), (95, 1805), (1215, 513), (1216, 700), (1217, 511), (3000, 33)])
+def test_matrix_vector_products_are_exact(gctx, M, K):
+    rng = np.random.default_rng(M + K)
+    A = rng.integers(-1000, 1001, (M, K)).astype(float)
+    x = rng.integers(-1000, 1001, (K, 1)).astype(float)
+    assert np.array_equal(gctx.einsum('mk,kn->mn', A, x, out_shape=(M, 1)), A @ x)
 
 
 def test_zero_tiny_and_huge_rows(gctx):
