@@ -381,6 +381,7 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
     if (lane == 0 && (!PAIR || rank == 0)) {  // (pair: the rank-0 CTA issues for both)
       int g = 0, c = 0;
       bool ok = true;
+      const uint64_t desc = sw_desc<SH::SWZ>(smem_u32(smem)), desc64 = sw_desc<64>(smem_u32(smem));
       for (int it = 0; it * nwork < units && ok; it++) {
         const int u = unit_at(it);
         if (u >= units) continue;
@@ -404,37 +405,35 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
           if (first && !mbar_wait(&tempty[b], bph ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) { ok = false; break; }
           if (!mbar_wait(&full[s], ph, a.err, ERR_FULL_WAIT, a.wait_cycles)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t st = smem_u32(smem + s * SH::STAGE_BYTES);
-          const uint32_t ahi = st, bhi = st + SH::A_BYTES;
-          const uint32_t alo = st + SH::A_BYTES + SH::B_BYTES;
-          const uint32_t blo = st + 2 * SH::A_BYTES + SH::B_BYTES;
+          // operand descriptors of the stage: the four tiles lie at fixed offsets (the
+          // address field counts 16 bytes), K steps of 32 bytes.  Building one per MMA
+          // costs the issuing thread ~100 cycles each, more than an N = 128 MMA takes.
+          const uint64_t off = (uint64_t)s * (SH::STAGE_BYTES >> 4);
+          constexpr uint64_t oBhi = SH::A_BYTES >> 4, oAlo = (SH::A_BYTES + SH::B_BYTES) >> 4,
+                             oBlo = (2 * SH::A_BYTES + SH::B_BYTES) >> 4;
           const uint32_t d = tmem + (uint32_t)(b * BN);
           uint32_t acc = first ? 0u : 1u;
           if (SH::BK == 64 && a.seg[sg].bk == 32) {
             // half-filled stage of a 32-wide segment: 64-byte rows, 64-byte swizzle
+            const uint64_t st = desc64 + off;
             if (a.split3) {
 #pragma unroll
-              for (int k = 0; k < 2; k++, acc = 1)
-                MMA_(d, sw_desc<64>(alo + 32 * k), sw_desc<64>(bhi + 32 * k), id, acc);
+              for (int k = 0; k < 2; k++, acc = 1) MMA_(d, st + oAlo + 2 * k, st + oBhi + 2 * k, id, acc);
 #pragma unroll
-              for (int k = 0; k < 2; k++)
-                MMA_(d, sw_desc<64>(ahi + 32 * k), sw_desc<64>(blo + 32 * k), id, 1u);
+              for (int k = 0; k < 2; k++) MMA_(d, st + 2 * k, st + oBlo + 2 * k, id, 1u);
             }
 #pragma unroll
-            for (int k = 0; k < 2; k++, acc = 1)
-              MMA_(d, sw_desc<64>(ahi + 32 * k), sw_desc<64>(bhi + 32 * k), id, acc);
+            for (int k = 0; k < 2; k++, acc = 1) MMA_(d, st + 2 * k, st + oBhi + 2 * k, id, acc);
           } else {
+            const uint64_t st = desc + off;
             if (a.split3) {
 #pragma unroll
-              for (int k = 0; k < SH::BK / 16; k++, acc = 1)
-                MMA_(d, sw_desc<SH::SWZ>(alo + 32 * k), sw_desc<SH::SWZ>(bhi + 32 * k), id, acc);
+              for (int k = 0; k < SH::BK / 16; k++, acc = 1) MMA_(d, st + oAlo + 2 * k, st + oBhi + 2 * k, id, acc);
 #pragma unroll
-              for (int k = 0; k < SH::BK / 16; k++)
-                MMA_(d, sw_desc<SH::SWZ>(ahi + 32 * k), sw_desc<SH::SWZ>(blo + 32 * k), id, 1u);
+              for (int k = 0; k < SH::BK / 16; k++) MMA_(d, st + 2 * k, st + oBlo + 2 * k, id, 1u);
             }
 #pragma unroll
-            for (int k = 0; k < SH::BK / 16; k++, acc = 1)
-              MMA_(d, sw_desc<SH::SWZ>(ahi + 32 * k), sw_desc<SH::SWZ>(bhi + 32 * k), id, acc);
+            for (int k = 0; k < SH::BK / 16; k++, acc = 1) MMA_(d, st + 2 * k, st + oBhi + 2 * k, id, acc);
           }
           if constexpr (PAIR) {
             mma2_commit_both(&empty[s]);
