@@ -634,12 +634,12 @@ void SliceEngine::alloc(SlicedPack &out, int64_t rows, int64_t K) {
 }
 
 void SliceEngine::row_exps(const double *src, const int64_t *rowOff, int64_t rows, const int64_t *kOff,
-                           int64_t K, bool unitK, int *exps) {
+                           int64_t K, bool unitK, int *exps, const int64_t *expIdx) {
   const RowTiles rt = RowTiles::make(rows, 1, rows);
   const dim3 grid((unsigned)rt.count,
                   (unsigned)std::max<int64_t>(1, std::min<int64_t>({ceil_div(K, 64), ceil_div(8 * kNumSMs, rt.count), 65535})));
   slice_pack_kernel<PackMode::EXPS, false><<<grid, 256, 0, ctx_.stream>>>(
-      src, rowOff, rows, kOff, K, unitK ? 1 : 0, nullptr, 0, exps, nullptr, 0, 0, 0, rt);
+      src, rowOff, rows, kOff, K, unitK ? 1 : 0, nullptr, 0, exps, expIdx, 0, 0, 0, rt);
   SCESS_CHECK_LAUNCH();
 }
 

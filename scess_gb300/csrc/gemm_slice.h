@@ -83,11 +83,11 @@ class SliceEngine {
   void gemm_grouped(const SliceProblemSet &ps, double flops, const char *name);
 
   // Largest biased exponent of every row of the gather src[rowOff[r] + kOff[k]],
-  // folded into exps[r] (atomic max; the caller clears exps first).
+  // folded into exps[expIdx[r]] (atomic max; the caller clears exps first).
   void row_exps(const double *src, const int64_t *rowOff, int64_t rows, const int64_t *kOff,
-                int64_t K, bool unitK, int *exps);
-  // Digits of the gather relative to the given row exponents exps[expIdx[r]]
-  // (expIdx null: exps[r]), optionally negated.
+                int64_t K, bool unitK, int *exps, const int64_t *expIdx);
+  // Digits of the gather relative to the given exponents exps[expIdx[r]] (no smaller
+  // than the row's own), optionally negated.
   void pack_with_exps(const double *src, const int64_t *rowOff, int64_t rows, const int64_t *kOff,
                       int64_t K, bool unitK, const int *exps, const int64_t *expIdx, bool negate,
                       SlicedPack &out);

@@ -26,6 +26,7 @@
 #include <cstring>
 #include <vector>
 
+#include "gemm_slice.h"
 #include "gemm_tc.h"
 #include "triples.h"
 
@@ -387,6 +388,117 @@ __global__ void __launch_bounds__(256) triples_energy_orbit_kernel(
     if (a == c) deg = 6.0;
     else if (a == b || b == c) deg = 2.0;
     energies[triple_id(a, b, c)] = total / deg;
+  }
+}
+
+// FP64 form: one CTA per local triple (a_l, b_l, c_l) of the block triple.  W is
+// read from the three group buffers of the sliced GEMM, problem-major with the
+// GEMM rows contiguous:
+//   W_g[y + nb z][s + o t][u + o x_l], (x, y, z) = (a, b, c), (b, a, c), (c, a, b),
+// u the occupied partner of x and (s, t) the other two occupied indices in order;
+// W = (W_0 + W_1) + W_2 is formed in shared memory.  Then as the mixed form: one
+// thread per orbit of (i, j, k), six orderings sharing one denominator.  GB300
+// issues about two FP64 lanes per cycle and SM, so this kernel is FP64-bound: 18 FMAs
+// for W + V of an orbit, 18 for r3 and its products, one division, and 12 adds for
+// the sum of the buffers (10 FP64 operations per element; a thread per element with
+// its own denominator took about 30).
+__global__ void __launch_bounds__(256) triples_energy_orbit64_kernel(
+    const double *__restrict__ W, int64_t o, int64_t v, int64_t nb, int64_t A, int64_t Bk, int64_t C,
+    const double *__restrict__ eps, const double *__restrict__ t1, const double *__restrict__ S,
+    const uint32_t *__restrict__ orbits, int norbits, double *__restrict__ energies) {
+  const int n = (int)nb;
+  const int al = blockIdx.x / (n * n), bl = (blockIdx.x / n) % n, cl = blockIdx.x % n;
+  const int64_t a = A * nb + al, b = Bk * nb + bl, c = C * nb + cl;
+  if (a >= v || b >= v || c >= v || b > a || c > b) return;
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  __shared__ double red[8];
+  const int oo = (int)o, o2 = oo * oo, o3 = o2 * oo;
+  // W(i,j,k) at i + p1 j + p2 k and the slices at x + p1 y, p1 and p2 odd: reads along
+  // any one index are free of bank conflicts
+  const int p1 = oo | 1, p2 = (p1 * oo) | 1;
+  double *Ws = reinterpret_cast<double *>(sm_raw);
+  double *Sbc = Ws + p2 * oo, *Sac = Sbc + p1 * oo, *Sab = Sac + p1 * oo;
+  double *ta = Sab + p1 * oo, *tb = ta + oo, *tc = tb + oo, *eo = tc + oo;
+  const int64_t Mg = o * nb, prob = Mg * o2, grp = nb * nb * prob;
+  const double *W0 = W + (bl + nb * cl) * prob + o * al, *W1 = W + grp + (al + nb * cl) * prob + o * bl,
+               *W2 = W + 2 * grp + (al + nb * bl) * prob + o * cl;
+  for (int e = threadIdx.x; e < o2; e += blockDim.x) {
+    const int x = e % oo, y = e / oo;
+    Sbc[x + p1 * y] = S[e + o2 * (b + v * c)];
+    Sac[x + p1 * y] = S[e + o2 * (a + v * c)];
+    Sab[x + p1 * y] = S[e + o2 * (a + v * b)];
+  }
+  for (int i = threadIdx.x; i < oo; i += blockDim.x) {
+    ta[i] = t1[i + o * a];
+    tb[i] = t1[i + o * b];
+    tc[i] = t1[i + o * c];
+    eo[i] = eps[i];
+  }
+  // element e of a buffer: u = e % o, column e / o = s + o t; (su, ss, st) are the
+  // strides of u, s, t in Ws.  Eight loads in flight a thread.
+  auto add = [&](const double *Wg, int su, int ss, int st, bool first) {
+    for (int e0 = threadIdx.x; e0 < o3; e0 += 8 * blockDim.x) {
+      double x[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int e = e0 + q * blockDim.x;
+        if (e < o3) x[q] = Wg[e % oo + Mg * (e / oo)];
+      }
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int e = e0 + q * blockDim.x;
+        if (e < o3) {
+          const int u = e % oo, col = e / oo;
+          double *p = Ws + u * su + (col % oo) * ss + (col / oo) * st;
+          *p = first ? x[q] : *p + x[q];
+        }
+      }
+    }
+    __syncthreads();
+  };
+  add(W0, 1, p1, p2, true);    // (u, s, t) = (i, j, k)
+  add(W1, p1, 1, p2, false);   // (j, i, k)
+  add(W2, p2, 1, p1, false);   // (k, i, j)
+  const double evirt = eps[o + a] + eps[o + b] + eps[o + c];
+  double acc = 0.0;
+  for (int q = threadIdx.x; q < norbits; q += blockDim.x) {
+    const uint32_t code = __ldg(orbits + q);
+    const int i = code & 255, j = (code >> 8) & 255, k = (code >> 16) & 255, m = code >> 24;
+    const double ai = ta[i], aj = ta[j], ak = ta[k], bi = tb[i], bj = tb[j], bk = tb[k], ci = tc[i], cj = tc[j],
+                 ck = tc[k];
+    const int pi = p1 * i, pj = p1 * j, pk = p1 * k, qi = p2 * i, qj = p2 * j, qk = p2 * k;
+    // V_xyz = t1_xa (yb|zc) + t1_yb (xa|zc) + t1_zc (xa|yb)                       :70-75
+    const double we0 = Ws[i + pj + qk], we1 = Ws[j + pk + qi], we2 = Ws[k + pi + qj];
+    const double wo0 = Ws[i + pk + qj], wo1 = Ws[k + pj + qi], wo2 = Ws[j + pi + qk];
+    const double ye0 = fma(ai, Sbc[j + pk], fma(bj, Sac[i + pk], fma(ck, Sab[i + pj], we0)));
+    const double ye1 = fma(aj, Sbc[k + pi], fma(bk, Sac[j + pi], fma(ci, Sab[j + pk], we1)));
+    const double ye2 = fma(ak, Sbc[i + pj], fma(bi, Sac[k + pj], fma(cj, Sab[k + pi], we2)));
+    const double yo0 = fma(ai, Sbc[k + pj], fma(bk, Sac[i + pj], fma(cj, Sab[i + pk], wo0)));
+    const double yo1 = fma(ak, Sbc[j + pi], fma(bj, Sac[k + pi], fma(ci, Sab[k + pj], wo1)));
+    const double yo2 = fma(aj, Sbc[i + pk], fma(bi, Sac[j + pk], fma(ck, Sab[j + pi], wo2)));
+    const double Se = (ye0 + ye1) + ye2, So = (yo0 + yo1) + yo2;
+    const double ce = fma(-2.0, So, Se), co = fma(-2.0, Se, So);                   // :152-154
+    double num = we0 * fma(3.0, ye0, ce);
+    num = fma(we1, fma(3.0, ye1, ce), num);
+    num = fma(we2, fma(3.0, ye2, ce), num);
+    num = fma(wo0, fma(3.0, yo0, co), num);
+    num = fma(wo1, fma(3.0, yo1, co), num);
+    num = fma(wo2, fma(3.0, yo2, co), num);
+    const double d = ((eo[i] + eo[j]) + eo[k]) - evirt;                             // :155
+    // an orbit with two (three) equal indices visits its elements twice (six times)
+    acc += num / (m == 0 ? d : (m == 1 ? d + d : 6.0 * d));                         // :156
+  }
+  for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0) red[w] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int q = 0; q < (int)(blockDim.x >> 5); q++) s += red[q];
+    double deg = 1.0;                                                               // :135-139
+    if (a == c) deg = 6.0;
+    else if (a == b || b == c) deg = 2.0;
+    energies[triple_id(a, b, c)] = s / deg;
   }
 }
 
@@ -893,6 +1005,184 @@ int choose_nb_grouped(int64_t o, int64_t v) {
   return best;
 }
 
+// Block size of the sliced FP64 form: rows (u, x_l) in 128-row tiles, padded
+// virtuals close to v, the three FP64 W buffers within 96 MiB so that they stay in L2
+// between the GEMM and the energy kernel; ties go to the larger block.
+int choose_nb_sliced(int64_t o, int64_t v) {
+  const int64_t forced = tune_value("t_nb", 0);
+  if (forced >= 1) return (int)std::min<int64_t>(forced, v);
+  int best = 1;
+  double best_score = -1.0;
+  const double o3 = (double)o * o * o;
+  for (int nb = 1; nb <= std::min<int64_t>(v, 64); nb++) {
+    if (nb > 1 && (double)nb * nb * nb * o3 * 24.0 > double(96 << 20)) break;
+    const double rows = (double)o * nb;
+    const double vp = (double)ceil_div(v, nb) * nb;
+    const double score = rows / (128.0 * std::ceil(rows / 128.0)) * std::pow((double)v / vp, 3.0);
+    if (score >= best_score * (1.0 - 1e-9)) {
+      best = nb;
+      best_score = std::max(score, best_score);
+    }
+  }
+  return best;
+}
+
+// FP64 (T) with the 12 products of a block triple as one grouped launch on the
+// tensor cores' exact slices (gemm_slice.h), in the three groups of four K segments
+// described in rccsd_triples.  All segments of a group add up in one sum per output,
+// so P and t2 rows share the exponent of their (u, x) and Q and R rows that of their
+// (s, t).  False (nothing computed) when the packs do not fit into device memory.
+bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, const double *d_eps,
+                         const double *d_t1, const double *d_t2, const Control &ctl, TriplesStats *stats,
+                         const double *d_B, int64_t naux, double &e_t) {
+  const int64_t v = nmo - o, N = nmo, o2 = o * o, o3 = o2 * o;
+  cudaStream_t s = ctx.stream;
+  const int nb = choose_nb_sliced(o, v);
+  const int64_t NB = ceil_div(v, nb), vp = NB * nb;
+  const int64_t Mg = o * nb, Ng = o2, prob = Mg * Ng;
+  if (!SliceEngine::usable(o * vp * vp, o2 * vp)) return false;
+  const int64_t ntrip = v * (v + 1) * (v + 2) / 6;
+  TriplesSetup T;
+  T.o = o;
+  T.v = v;
+  T.N = N;
+  T.nb = nb;
+  T.NB = NB;
+  T.vp = vp;
+  SliceEngine &se = ctx.slice_engine();
+  SlicedPack pP, pQ, pQ2, pR, pR2, pTx;
+  DevTables pdt, gdt;
+  DevMem exps, W, orbits;
+  DTensor energies;
+  std::vector<uint32_t> ot = orbit_table(o);
+  const int norbits = (int)ot.size();
+  try {
+    {
+      TimedScope ts(ctx.timer, "phase:triples_setup", 0.0, 0.0, s);
+      T.build(ctx, d_eri, d_t2, d_B, naux, Backend::FP64);
+    }
+    TimedScope ts(ctx.timer, "phase:triples_pack", 0.0, 0.0, s);
+    // rows as in the mixed form: P (i,x | y,Y,X), Q (j,k | z,Z), R (i,j | x,X),
+    // t2 (u,x | z,X,Z), Q (k,j | z,Z), R (j,i | x,X); then the exponent index of each:
+    // i + o x over all virtuals (P, t2), s + o t (Q, R)
+    pdt.build(ctx, {table({{o, 1}, {nb, o * v}, {nb, o * v * vp}, {NB, o * v * vp * nb}, {NB, o * v * nb}}),
+                    table({{o, v}, {o, v * o}, {nb, v * o2}, {NB, v * o2 * nb}}),
+                    table({{o, 1}, {o, o}, {nb, o3}, {NB, o3 * nb}}),
+                    table({{o, o}, {nb, o2 * vp}, {nb, o2}, {NB, o2 * vp * nb}, {NB, o2 * nb}}),
+                    table({{o, v * o}, {o, v}, {nb, v * o2}, {NB, v * o2 * nb}}),
+                    table({{o, o}, {o, 1}, {nb, o3}, {NB, o3 * nb}}),
+                    table({{o, 1}, {nb, o}, {nb, 0}, {NB, 0}, {NB, o * nb}}),
+                    table({{o, 1}, {nb, o}, {nb, 0}, {NB, o * nb}, {NB, 0}}),
+                    table({{o, 1}, {o, o}, {nb, 0}, {NB, 0}})});
+    exps.alloc((size_t)(o * vp + o2) * sizeof(int));
+    int *eA = exps.as<int>(), *eB = eA + o * vp;
+    SCESS_CUDA(cudaMemsetAsync(eA, 0, (size_t)(o * vp + o2) * sizeof(int), s));
+    const int64_t *kP = T.dt.ptr[T.kOperand + 1], *kT = T.dt.ptr[T.kOperand + 7], *kQ = T.dt.ptr[T.kOperand + 3],
+                  *kR = T.dt.ptr[T.kOperand + 5];
+    const int64_t rP = o * vp * vp, rQ = o2 * vp;
+    struct Op {
+      const DTensor &t;
+      int row;
+      int64_t rows;
+      const int64_t *k;
+      int64_t K;
+      bool unitK;
+      int *e;
+      int idx;
+      bool neg;
+      SlicedPack &out;
+    };
+    const Op ops[6] = {{T.P, 0, rP, kP, v, false, eA, 6, false, pP},  {T.T2p, 3, rP, kT, o, true, eA, 7, true, pTx},
+                       {T.Qt, 1, rQ, kQ, v, true, eB, 8, false, pQ},  {T.Qt, 4, rQ, kQ, v, true, eB, 8, false, pQ2},
+                       {T.Rt, 2, rQ, kR, o, false, eB, 8, false, pR}, {T.Rt, 5, rQ, kR, o, false, eB, 8, false, pR2}};
+    for (const Op &q : ops)
+      se.row_exps(q.t.p(), pdt.ptr[q.row], q.rows, q.k, q.K, q.unitK, q.e, pdt.ptr[q.idx]);
+    for (const Op &q : ops)
+      se.pack_with_exps(q.t.p(), pdt.ptr[q.row], q.rows, q.k, q.K, q.unitK, q.e, pdt.ptr[q.idx], q.neg, q.out);
+    gdt.build(ctx, {table({{Mg, 1}}), table({{Ng, Mg}})});
+    W.alloc((size_t)(3 * nb * nb * prob) * sizeof(double));
+    energies = DTensor({std::max<int64_t>(ntrip, 1)});
+    orbits.alloc(ot.size() * sizeof(uint32_t));
+  } catch (const Error &e) {
+    if (e.code != SCESS_ERR_OOM) throw;
+    return false;
+  }
+  SCESS_CUDA(cudaMemsetAsync(energies.p(), 0, energies.size() * sizeof(double), s));
+  SCESS_CUDA(cudaMemcpyAsync(orbits.as<void>(), ot.data(), ot.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+  ctx.sync();  // (ot is a host vector of this scope)
+  const int64_t p1 = o | 1, p2 = (p1 * o) | 1;
+  const size_t smem = (size_t)(p2 * o + 3 * p1 * o + 4 * o) * 8;
+  SCESS_CUDA(cudaFuncSetAttribute(triples_energy_orbit64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const unsigned threads = (unsigned)std::min<int64_t>(256, round_up(norbits, 32));
+  SliceProblemSet ps;
+  const SlicedPack *packs[6] = {&pP, &pQ, &pQ2, &pR, &pR2, &pTx};
+  const int bn = SliceEngine::tile_n(Ng);
+  for (int i = 0; i < 6; i++) ps.maps[i] = SliceEngine::map_of(*packs[i], i == 0 || i == 5 ? 128 : bn);
+  ps.nmaps = 6;
+  ps.M = Mg;
+  ps.N = Ng;
+  ps.ny = ps.nz = nb;
+  ps.ng = 3;
+  ps.nseg = 4;
+  const int mA[4] = {0, 0, 5, 5}, mB[4] = {1, 2, 3, 4};
+  for (int q = 0; q < 4; q++) {
+    ps.seg[q].mapA = mA[q];
+    ps.seg[q].mapB = mB[q];
+    ps.seg[q].Kpad = q < 2 ? pP.Kpad : pTx.Kpad;
+  }
+  ps.expA = exps.as<int>();
+  ps.expB = ps.expA + o * vp;
+  ps.C = W.d();
+  for (int g = 0; g < 3; g++) {
+    ps.cy[g] = prob;
+    ps.cz[g] = nb * prob;
+    ps.cg[g] = g * nb * nb * prob;
+    ps.rowC[g] = gdt.ptr[0];
+    ps.colC[g] = gdt.ptr[1];
+  }
+  int64_t blocks_done = 0;
+  for (int64_t A = 0; A < NB; A++)
+    for (int64_t Bk = 0; Bk <= A; Bk++)
+      for (int64_t C = 0; C <= Bk; C++) {
+        if ((blocks_done & 15) == 0) ctl.poll();                                     // :123
+        const int64_t U[3] = {A, Bk, C};
+        const int kRoles[3][3] = {{0, 1, 2}, {1, 0, 2}, {2, 0, 1}};  // (x, y, z) of group g
+        const int64_t rp = o * nb * nb, rq = o2 * nb;
+        double nprob = 0.0;
+        for (int g = 0; g < 3; g++) {
+          const int64_t X = U[kRoles[g][0]], Yb = U[kRoles[g][1]], Z = U[kRoles[g][2]];
+          SliceSegment &s0 = ps.seg[0], &s1 = ps.seg[1], &s2 = ps.seg[2], &s3 = ps.seg[3];
+          s0.rowA0[g] = rp * (Yb + NB * X); s0.rowAy[g] = Mg;   // P(u,f,x,y) Q(f,s,t,z)
+          s0.rowB0[g] = rq * Z;             s0.rowBz[g] = o2;
+          s1.rowA0[g] = rp * (Z + NB * X);  s1.rowAz[g] = Mg;   // P(u,f,x,z) Q(f,t,s,y)
+          s1.rowB0[g] = rq * Yb;            s1.rowBy[g] = o2;
+          s2.rowA0[g] = rp * (X + NB * Z);  s2.rowAz[g] = Mg;   // -t2(m,u,z,x) R(s,t,m,y)
+          s2.rowB0[g] = rq * Yb;            s2.rowBy[g] = o2;
+          s3.rowA0[g] = rp * (X + NB * Yb); s3.rowAy[g] = Mg;   // -t2(m,u,y,x) R(t,s,m,z)
+          s3.rowB0[g] = rq * Z;             s3.rowBz[g] = o2;
+          ps.expA0[g] = Mg * X;
+          ps.tri[g] = Yb == Z;  // problems y < z of a diagonal block feed no unique triple
+          nprob += ps.tri[g] ? nb * (nb + 1) / 2.0 : (double)nb * nb;
+        }
+        se.gemm_grouped(ps, nprob * 2.0 * (double)Mg * Ng * (2.0 * v + 2.0 * o), "slice_gemm[triples]");
+        TimedScope ts(ctx.timer, "triples_energy", 0.0, 24.0 * nb * nb * prob, s);
+        triples_energy_orbit64_kernel<<<(unsigned)(nb * nb * nb), threads, smem, s>>>(
+            W.d(), o, v, nb, A, Bk, C, d_eps, d_t1, T.S.p(), orbits.as<uint32_t>(), norbits, energies.p());
+        SCESS_CHECK_LAUNCH();
+        blocks_done++;
+      }
+  sum_energies_kernel<<<1, 1024, 0, s>>>(ntrip, energies.p(), ctx.dscalars);
+  SCESS_CHECK_LAUNCH();
+  SCESS_CUDA(cudaMemcpyAsync(ctx.hscalars, ctx.dscalars, sizeof(double), cudaMemcpyDeviceToHost, s));
+  ctx.sync();
+  if (stats) {
+    stats->nb = nb;
+    stats->block_triples = blocks_done;
+  }
+  e_t = ctx.hscalars[0];
+  return true;
+}
+
 }  // namespace
 
 double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, const double *d_eps,
@@ -900,6 +1190,13 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
                      TriplesStats *stats, const double *d_B, int64_t naux) {
   const int64_t v = nmo - o, N = nmo;
   cudaStream_t s = ctx.stream;
+  {
+    const int64_t q1 = o | 1, q2 = (q1 * o) | 1;
+    if (!mixed && (q2 * o + 3 * o * o + 4 * o) * 8 <= 200 * 1024 && o <= 255) {  // (else refused below)
+      double e_t = 0.0;
+      if (triples_fp64_sliced(ctx, d_eri, nmo, o, d_eps, d_t1, d_t2, ctl, stats, d_B, naux, e_t)) return e_t;
+    }
+  }
   const int nb = mixed ? choose_nb_grouped(o, v) : choose_nb(o, v, 8, size_t(128) << 20);
   const int64_t NB = ceil_div(v, nb), vp = NB * nb;
   const int64_t o2 = o * o, o3 = o2 * o;
