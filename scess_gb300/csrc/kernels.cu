@@ -658,6 +658,29 @@ __global__ void mp2_partial_kernel(int64_t o, int64_t v, const double *__restric
   if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 
+// Non-negative doubles order like their bits; a NaN (sign cleared) is above all of them.
+__global__ void pair_asymmetry_kernel(const double *__restrict__ x, Ext4 n, Ext4 st, double *__restrict__ out) {
+  const int64_t total = n.e[0] * n.e[1] * n.e[2] * n.e[3];
+  unsigned long long d = 0, m = 0;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = e % n.e[0], q = (e / n.e[0]) % n.e[1], rs = e / (n.e[0] * n.e[1]), r = rs % n.e[2], s = rs / n.e[2];
+    if (s < r || (s == r && q < p)) continue;  // each pair once
+    const double a = x[p * st.e[0] + q * st.e[1] + r * st.e[2] + s * st.e[3]];
+    const double b = x[q * st.e[0] + p * st.e[1] + s * st.e[2] + r * st.e[3]];
+    d = max(d, (unsigned long long)__double_as_longlong(fabs(a - b)));
+    m = max(m, (unsigned long long)__double_as_longlong(fabs(a)));
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    d = max(d, __shfl_down_sync(0xffffffffu, d, off));
+    m = max(m, __shfl_down_sync(0xffffffffu, m, off));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(reinterpret_cast<unsigned long long *>(out), d);
+    atomicMax(reinterpret_cast<unsigned long long *>(out) + 1, m);
+  }
+}
+
 __global__ void lincomb_kernel(int64_t n, int nv, const double *const *__restrict__ vecs,
                                const double *__restrict__ coef, double *__restrict__ out) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
@@ -765,6 +788,13 @@ void mp2_energy(int64_t o, int64_t v, const double *g, int64_t si, int64_t sa, i
   mp2_partial_kernel<<<kDotBlocks, 256, 0, stream>>>(o, v, g, si, sa, sj, sb, eps, partials);
   SCESS_CHECK_LAUNCH();
   sum_partials_kernel<<<1, 1024, 0, stream>>>(kDotBlocks, partials, result);
+  SCESS_CHECK_LAUNCH();
+}
+
+void pair_asymmetry(const double *x, Ext4 ext, Ext4 str, double *out, cudaStream_t stream) {
+  const int64_t n = ext.e[0] * ext.e[1] * ext.e[2] * ext.e[3];
+  pair_asymmetry_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), 8 * kNumSMs)), 256, 0, stream>>>(
+      x, ext, str, out);
   SCESS_CHECK_LAUNCH();
 }
 

@@ -112,6 +112,12 @@ void tau_energy(int64_t o, int64_t v, const double *L, const double *t1, const d
 void mp2_energy(int64_t o, int64_t v, const double *g, int64_t si, int64_t sa, int64_t sj,
                 int64_t sb, const double *eps, double *partials, double *result,
                 cudaStream_t stream);
+// out[0] = max|x(p,q,r,s) - x(q,p,s,r)|, out[1] = max|x| (folded in with atomic maxima; out
+// zeroed by the caller) over extents ext = (n, n, m, m) and element strides str
+struct Ext4 {
+  int64_t e[4];
+};
+void pair_asymmetry(const double *x, Ext4 ext, Ext4 str, double *out, cudaStream_t stream);
 // any non-finite value in x -> flag[0] = 1
 void check_finite(int64_t n, const double *x, int *flag, cudaStream_t stream);
 

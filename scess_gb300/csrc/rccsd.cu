@@ -598,8 +598,7 @@ void RccsdState::init(const SolveInput &in, const scess_rccsd_options &opts) {
   diis_err_.alloc((size_t)maxv_ * n_ * sizeof(double));
   vecptr_.alloc((size_t)maxv_ * sizeof(double *));
   coefd_.alloc((size_t)(maxv_ + 1) * sizeof(double));
-  w_.alloc(o, v, !mixed_);
-  have_wvvvv_ = !mixed_;
+  w_.alloc(o, v, false);
   phase_ = mixed_ ? Phase::MIXED : Phase::FP64;
   std::memset(&res_, 0, sizeof(res_));
   SCESS_CUDA(cudaEventCreate(&ev0_));
@@ -636,6 +635,7 @@ void RccsdState::get_amplitudes(double *t1, double *t2) {
 void RccsdState::reset_history() {
   order_.clear();
   gram_.clear();
+  symmetric_ = -1;
   E_last_ = DBL_MAX;
   it_ = 0;
   phase_start_ = 0;
@@ -643,6 +643,26 @@ void RccsdState::reset_history() {
   phase_ = mixed_ ? Phase::MIXED : Phase::FP64;
   converged_ = false;
   std::memset(&res_, 0, sizeof(res_));
+}
+
+bool RccsdState::inputs_symmetric() {
+  const int64_t o = B_.o, v = B_.v;
+  cudaStream_t s = ctx_.stream;
+  double *d = ctx_.dscalars;
+  SCESS_CUDA(cudaMemsetAsync(d, 0, 6 * sizeof(double), s));
+  pair_asymmetry(amp_.p() + n1_, {{o, o, v, v}}, {{1, o, o * o, o * o * v}}, d, s);
+  if (drv_.p()) pair_asymmetry(drv_.p(), {{o, o, v, v}}, {{1, o, o * o, o * o * v}}, d + 2, s);
+  if (eri_.p()) {  // (a DF state's <ab|cd> is symmetric as it is formed)
+    const int64_t *st = B_.vvvv.str;
+    pair_asymmetry(B_.vvvv.p, {{v, v, v, v}}, {{st[0], st[1], st[2], st[3]}}, d + 4, s);
+  }
+  SCESS_CUDA(cudaMemcpyAsync(ctx_.hscalars, d, 6 * sizeof(double), cudaMemcpyDeviceToHost, s));
+  ctx_.sync();
+  const double *h = ctx_.hscalars;
+  // rounding of a solver's own amplitudes, no more
+  for (int q = 0; q < 3; q++)
+    if (!(h[2 * q] <= 16.0 * DBL_EPSILON * h[2 * q + 1])) return false;
+  return true;
 }
 
 double RccsdState::energy_of_amplitudes() {
@@ -668,11 +688,12 @@ bool RccsdState::iterate(int max_steps, const Control &ctl) {
     if (ph == Phase::MIXED) {
       rccsd_residual(ctx_, B_, amp_.p(), drv_.p(), Backend::MIXED, w_, R_.p());       // :350
     } else if (ph == Phase::FP64) {
-      if (!have_wvvvv_) {
-        w_.Wvvvv = DTensor({v, v, v, v});
-        have_wvvvv_ = true;
-      }
-      rccsd_residual(ctx_, B_, amp_.p(), drv_.p(), Backend::FP64, w_, R_.p());
+      // the reassociated list has a quarter of the ladder's FLOPs and forms no v^4
+      // intermediate, but takes t2(ijab) = t2(jiba) and <ab|cd> = <ba|dc> for granted
+      if (symmetric_ < 0) symmetric_ = inputs_symmetric() ? 1 : 0;
+      if (!symmetric_ && !w_.Wvvvv.p()) w_.Wvvvv = DTensor({v, v, v, v});
+      rccsd_residual(ctx_, B_, amp_.p(), drv_.p(), Backend::FP64, w_, R_.p(),
+                     symmetric_ ? ResidualList::REASSOCIATED : ResidualList::LITERAL);
     } else if (ph == Phase::REFINED) {
       // R = R0 + dR(T0, T - T0)
       SCESS_CUDA(cudaMemcpyAsync(damp_.p(), amp_.p(), n_ * sizeof(double), cudaMemcpyDeviceToDevice, s));

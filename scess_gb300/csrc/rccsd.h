@@ -123,6 +123,7 @@ class RccsdState {
   int64_t nmo() const { return B_.N; }
 
  private:
+  bool inputs_symmetric();  // t2 and the driver under (ia <-> jb), <ab|cd> under (ac <-> bd)
   void reset_history();
   void init(const SolveInput &in, const scess_rccsd_options &opts);
   Ctx &ctx_;
@@ -132,7 +133,8 @@ class RccsdState {
   RccsdBlocks B_;
   scess_rccsd_options opts_;
   int64_t n1_ = 0, n2_ = 0, n_ = 0;
-  bool mixed_ = false, have_f12_ = false, have_wvvvv_ = false;
+  bool mixed_ = false, have_f12_ = false;
+  int symmetric_ = -1;  // FP64: inputs_symmetric() of the amplitudes set last (-1: not yet known)
   DTensor eps_, amp_, prev_, R_, drv_, Lf12_;
   int maxv_ = 8;
   DevMem diis_amp_, diis_err_, vecptr_, coefd_;
