@@ -1,18 +1,22 @@
 // FP64 GEMM on BF16 slices with tcgen05 (see gemm_slice.h for the splitting).
 //
 // A persistent CTA per SM walks work units (problem, 128 x bn output tile, K range),
-// bn <= 80:
+// bn <= 128:
 //   warp 0     TMA producer: per 32-wide K block one stage with the 7 slices of
 //              128 A rows and bn B rows (64-byte rows, 64B swizzle);
-//   warp 1     owns TMEM (six accumulators of bn columns: S_0 .. S_4 and S_5 + S_6)
-//              and issues the MMAs (M = 128, N = bn, K = 16);
-//   warps 4-11 two epilogue warpgroups, bn / 2 columns each: add every drained
+//   warp 1     owns TMEM (three rotating accumulators of bn columns for S_4 .. S_0,
+//              one for S_5 + S_6) and issues the MMAs (M = 128, N = bn, K = 16);
+//   warps 4-19 four epilogue warpgroups, bn / 4 columns each: add every drained
 //              S_d, an exact integer, into one 64-bit integer per output, and turn
 //              integer + FP32 tail into FP64 at the end of the unit.
-// Each S_d keeps its own accumulator and is drained only as often as its sums
-// stay exact integers in FP32 (every 128, 16, 5, 3, 2 K blocks for d = 0 .. 4), so
-// that a K of 200 takes 12 drains; with three rotating 128-wide accumulators drained
-// every K block (36 drains) the drains took 2.3 x the MMAs' time.
+// Shared memory bounds the tensor pipe: operand reads (128 B a cycle) and TMA writes
+// (70 B a cycle, measured, on every SM alone) share its port, so an MMA of N = 128
+// costs 64 + 29 cycles (0.73 per column) and one of N = 80 52 + 24 (0.95).  The wide
+// tile leaves TMEM room for four accumulators only, hence the rotation and five
+// drains per K block, which run beside the MMAs.  A TMEM load takes about 200 cycles
+// whatever its width, so four epilogue warps share a scheduler (two: 39 TFLOP/s at
+// 4096^3 and 0.74 ms for 8192 x 8192 x 32; four: 41.8 and 0.38).  Six accumulators of
+// 80 columns with a third of the drains and two warps: 34 TFLOP/s.
 // Every mbarrier wait is bounded (see mbarrier.cuh).
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -30,20 +34,17 @@ namespace scess {
 
 namespace {
 
-constexpr int BM = 128, BN = 80, BK = kSliceBK;
+constexpr int BM = 128, BN = 128, BK = kSliceBK;
 constexpr int STAGES = 2;
 constexpr uint32_t A_SLICE = (uint32_t)BM * BK * 2;                  // one slice of 128 rows
-constexpr uint32_t STAGE_BYTES = kSlices * (BM + BN) * BK * 2;       // 91 KiB
+constexpr uint32_t STAGE_BYTES = kSlices * (BM + BN) * BK * 2;       // 112 KiB
 constexpr int NDIAG = 5;                                             // S_0 .. S_4 are drained
-constexpr int NACC = NDIAG + 1;                                      // ... and the tail
-constexpr int HC = BN / 2;                                           // columns of an epilogue thread
-constexpr int THREADS = 384;
-constexpr int kEpiRegs = 224, kCtlRegs = 56, kLaunchRegs = 168;      // 3 x 168 = 56 + 2 x 224
-// K blocks between drains of S_d: |S_d| per K is at most 2^12, 2^15, 1.5 2^16,
-// 2.5 2^16, 3.5 2^16 for d = 0 .. 4 and the sum has to stay within 2^24
-__host__ __device__ constexpr int drain_every(int d) {
-  return d == 0 ? 128 : d == 1 ? 16 : d == 2 ? 5 : d == 3 ? 3 : 2;
-}
+constexpr int NROT = 3, TAIL = NROT, NACC = NROT + 1;                // accumulators
+constexpr int EPI = 4;                                               // epilogue warpgroups
+constexpr int HC = BN / EPI;                                         // columns of an epilogue thread
+constexpr int THREADS = 128 * (1 + EPI);
+constexpr int kEpiRegs = 104, kCtlRegs = 56, kLaunchRegs = 96;       // 56 + 4 x 104 <= 5 x 96
+static_assert(kCtlRegs + EPI * kEpiRegs <= (1 + EPI) * kLaunchRegs, "setmaxnreg draws on the launch's registers");
 struct Ctl {  // behind the stages
   uint64_t full[STAGES], empty[STAGES], tfull[NACC], tempty[NACC], done;
   uint32_t tmem;
@@ -65,7 +66,7 @@ struct SliceMaps {
 };
 struct SliceArgs {
   int M, N, tiles_m, tiles_n;
-  int bn;      // tile width: a multiple of 16, at most 80
+  int bn;      // tile width: a multiple of 32, at most 128
   int fs;      // fraction bits kept of the tail (see slice_value)
   int ny, nz, ng, nseg;
   int kb_total, kb_per_split, splits;
@@ -85,12 +86,36 @@ struct SliceArgs {
   int withhold_first;
 };
 
-// T += i 2^(9 (4 - D)) for the drained S_D = i 2^(-9 D), |i| <= 2^24.
+// T += i 2^(9 (4 - D)) for the drained S_D = i 2^(-9 D) of one K block: |i| is at most
+// 2^17, 2^20, 0.75 2^22, 0.63 2^23, 0.88 2^23 for D = 0 .. 4.  S_0 .. S_2 become
+// integers by adding 1.5 2^(23 - 9 D), whose bit pattern then holds the integer in its
+// low bits (the constants' own patterns are taken off once per unit); S_3 and S_4 are
+// converted.
+constexpr int kMagic0 = 0x4B400000;                    // 1.5 2^23
+constexpr int kMagic1 = kMagic0 - (9 << 23);           // 1.5 2^14
+constexpr int kMagic2 = kMagic0 - (18 << 23);          // 1.5 2^5
 template <int D>
 __device__ __forceinline__ void add_diag(long long &T, uint32_t raw) {
-  const int i = __float2int_rn(__uint_as_float(raw) * __int_as_float((127 + 9 * D) << 23));
-  if constexpr (D == 0) T += (long long)((unsigned long long)(unsigned)(i << 4) << 32);
-  else asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(T) : "r"(i), "n"(1 << (9 * (4 - D))));
+  const float s = __uint_as_float(raw);
+  if constexpr (D == 0) {
+    const int b = __float_as_int(s + __int_as_float(kMagic0));
+    T += (long long)((unsigned long long)(unsigned)(b << 4) << 32);
+  } else if constexpr (D == 1) {
+    const int b = __float_as_int(s + __int_as_float(kMagic1));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(T) : "r"(b), "n"(1 << 27));
+  } else if constexpr (D == 2) {
+    const int b = __float_as_int(s + __int_as_float(kMagic2));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(T) : "r"(b), "n"(1 << 18));
+  } else {
+    const int b = __float2int_rn(s * __int_as_float((127 + 9 * D) << 23));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(T) : "r"(b), "n"(1 << (9 * (4 - D))));
+  }
+}
+// What the magic constants have added to T after n K blocks (modulo 2^64).
+__device__ __forceinline__ long long magic_sum(int n) {
+  const unsigned long long c = ((unsigned long long)(unsigned)(kMagic0 << 4) << 32) +
+                               ((unsigned long long)kMagic1 << 27) + ((unsigned long long)kMagic2 << 18);
+  return (long long)(c * (unsigned long long)n);
 }
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *r) {
@@ -106,9 +131,8 @@ __device__ __forceinline__ void tmem_wait8(uint32_t *r) {
                : "memory");
 }
 
-// What bounds it: long K, the tensor pipe behind shared memory (28 products of
-// 2 x 128 x bn x 32 a stage; an M = 128, N = 80 MMA reads 6.5 KiB per 40 cycles);
-// short K, the epilogue (about 45 instructions per output).
+// What bounds it: long K, the shared-memory port (above); short K, the epilogue
+// (about 45 instructions per output).
 __global__ void __launch_bounds__(THREADS, 1)
     slice_gemm_kernel(const __grid_constant__ SliceMaps maps, const __grid_constant__ SliceArgs a) {
   extern __shared__ uint8_t smem_raw[];
@@ -128,7 +152,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     for (int b = 0; b < NACC; b++) {
       mbar_init(&ctl.tfull[b], 1);
-      mbar_init(&ctl.tempty[b], 8);  // one arrival per epilogue warp
+      mbar_init(&ctl.tempty[b], 4 * EPI);  // one arrival per epilogue warp
     }
     mbar_init(&ctl.done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -217,12 +241,11 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      int g = 0;
-      uint32_t cnt[NACC] = {0, 0, 0, 0, 0, 0};  // fills of each accumulator so far
+      int g = 0, c = 0, w = 0;  // stages, rotating fills and units so far
       const uint64_t desc_a = sw_desc<64>(smem_u32(smem)), desc_b = sw_desc<64>(smem_u32(smem) + kSlices * A_SLICE);
       const uint32_t bq = bslice >> 4;
       bool ok = true;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x, w++) {
         int tm, tn, py, pz, pg, kb0, kb1, sp;
         unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
         const uint32_t idesc = idesc_f16kind(BM, min(bn, (a.N - tn * bn + 15) & ~15), 1u);  // BF16
@@ -232,51 +255,41 @@ __global__ void __launch_bounds__(THREADS, 1)
           if (!mbar_wait(&ctl.full[s], ph, a.err, ERR_FULL_WAIT, a.wait_cycles)) { ok = false; break; }
           tc_fence_after();
           // slice offsets are added to the stage's descriptors (address field in units
-          // of 16 bytes): building a descriptor per MMA made the issuing thread the
-          // bound (100 cycles per MMA where N = 80 takes 52 and N = 128 takes 64)
+          // of 16 bytes): building a descriptor per MMA costs the issuing thread 100
+          // cycles, more than the MMA takes
           const uint64_t da = desc_a + (uint64_t)(s * (STAGE_BYTES >> 4));
           const uint64_t db = desc_b + (uint64_t)(s * (STAGE_BYTES >> 4));
-          auto product = [&](uint32_t d, int p, int q, uint32_t acc) {
+          auto product = [&](uint32_t col, int p, int q, uint32_t acc) {
 #pragma unroll
             for (int k = 0; k < 2; k++)
-              mma_bf16(d, da + (uint64_t)(p * (A_SLICE >> 4) + 2 * k), db + (uint64_t)(q * bq + 2 * k), idesc,
+              mma_bf16(tmem + col, da + (uint64_t)(p * (A_SLICE >> 4) + 2 * k), db + (uint64_t)(q * bq + 2 * k), idesc,
                        k ? 1u : acc);
           };
-          // an accumulator's first block of a fill waits for its drain and starts from zero
-          auto open = [&](int b, bool first) -> bool {
-            if (!first) return true;
-            if (!mbar_wait(&ctl.tempty[b], (cnt[b] & 1u) ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) return false;
-            tc_fence_after();
-            return true;
-          };
-          // the tail first: the accumulators of the previous unit are drained behind it
-          if (!open(NDIAG, kb == kb0)) { ok = false; break; }
-          {
-            uint32_t acc = kb == kb0 ? 0u : 1u;
+          // the longest first, so that a drain is done when its accumulator comes round
 #pragma unroll
-            for (int d = NDIAG; d < kSlices; d++)
-#pragma unroll
-              for (int p = 0; p <= d; p++, acc = 1u) product(tmem + (uint32_t)(NDIAG * bn), p, d - p, acc);
-            if (kb == kb1 - 1) {
-              mma_commit(&ctl.tfull[NDIAG]);
-              cnt[NDIAG]++;
-            }
-          }
-#pragma unroll
-          for (int d = 0; d < NDIAG; d++) {
-            const bool first = (kb - kb0) % drain_every(d) == 0;
-            if (ok && !open(d, first)) ok = false;
+          for (int d = NDIAG - 1; d >= 0; d--) {
+            const int b = c % NROT;
+            if (ok && !mbar_wait(&ctl.tempty[b], (((uint32_t)(c / NROT)) & 1u) ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) ok = false;
             if (!ok) break;
+            tc_fence_after();
 #pragma unroll
-            for (int p = 0; p <= d; p++) product(tmem + (uint32_t)(d * bn), p, d - p, (first && p == 0) ? 0u : 1u);
-            if ((kb - kb0) % drain_every(d) == drain_every(d) - 1 || kb == kb1 - 1) {
-              mma_commit(&ctl.tfull[d]);
-              cnt[d]++;
-            }
+            for (int p = 0; p <= d; p++) product((uint32_t)(b * bn), p, d - p, p ? 1u : 0u);
+            mma_commit(&ctl.tfull[b]);
+            c++;
           }
           if (!ok) break;
+          if (kb == kb0) {
+            if (!mbar_wait(&ctl.tempty[TAIL], ((uint32_t)w & 1u) ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) { ok = false; break; }
+            tc_fence_after();
+          }
+          uint32_t acc = kb == kb0 ? 0u : 1u;
+#pragma unroll
+          for (int d = NDIAG; d < kSlices; d++)
+#pragma unroll
+            for (int p = 0; p <= d; p++, acc = 1u) product((uint32_t)(TAIL * bn), p, d - p, acc);
           mma_commit(&ctl.empty[s]);
         }
+        if (ok) mma_commit(&ctl.tfull[TAIL]);
       }
       mma_commit(&ctl.done);
       mbar_drain(&ctl.done, 0);
@@ -286,14 +299,14 @@ __global__ void __launch_bounds__(THREADS, 1)
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
     const int q = warp & 3;
     const int row = 32 * q + lane;
-    const int h = (warp - 4) >> 2;                  // column half
-    const int hc = bn >> 1;                         // its width: 8, 16, .. 40
-    const int et = threadIdx.x - 128 - 128 * h;     // 0..127 within the half
+    const int h = (warp - 4) >> 2;                  // column group
+    const int hc = bn / EPI;                        // its width: 8, 16, 24 or 32
+    const int et = threadIdx.x - 128 - 128 * h;     // 0..127 within the group
     const int bar = 1 + h;
-    uint32_t cnt[NACC] = {0, 0, 0, 0, 0, 0};
+    int c = 0, w = 0;
     bool ok = true;
     const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(hc * h);
-    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x, w++) {
       int tm, tn, py, pz, pg, kb0, kb1, sp;
       unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
       const int m = tm * BM + row;
@@ -311,67 +324,47 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int64_t rowOff = m < a.M ? (a.partial ? (int64_t)m : a.rowC[pg][m]) : 0;
       const unsigned errv = *(volatile unsigned *)a.err;
       long long T[HC];
-      float F[HC];
 #pragma unroll
       for (int j = 0; j < HC; j++) T[j] = 0;
-      auto wait_for = [&](int b) -> bool {
-        if (!mbar_wait(&ctl.tfull[b], cnt[b] & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) return false;
-        tc_fence_after();
-        return true;
-      };
       auto release = [&](int b) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0)
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&ctl.tempty[b])) : "memory");
-        cnt[b]++;
       };
       auto take = [&](auto diag) -> bool {
         constexpr int D = decltype(diag)::value;
-        if (!wait_for(D)) return false;
-        uint32_t r[2][8];
-        const uint32_t t0 = tl + (uint32_t)(D * bn);
-        tmem_ld8(t0, r[0]);
+        const int b = c % NROT;
+        if (!mbar_wait(&ctl.tfull[b], (uint32_t)(c / NROT) & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) return false;
+        tc_fence_after();
+        const uint32_t t0 = tl + (uint32_t)(b * bn);
+        // (16 columns a load, four warps a scheduler: a TMEM load takes about 200 cycles
+        // whatever its width)
 #pragma unroll
-        for (int j = 0; j < HC; j += 8) {
-          if (j < hc) {
-            tmem_wait8(r[(j >> 3) & 1]);
-            if (j + 8 < hc) tmem_ld8(t0 + (uint32_t)(j + 8), r[((j >> 3) & 1) ^ 1]);
+        for (int j = 0; j < HC; j += 16) {
+          if (j < hc) {  // (columns past hc, within TMEM, are not used)
+            uint32_t r[16];
+            tmem_ld16_async(t0 + (uint32_t)j, r);
+            tmem_wait16(r);
 #pragma unroll
-            for (int i = 0; i < 8; i++) add_diag<D>(T[j + i], r[(j >> 3) & 1][i]);
+            for (int i = 0; i < 16; i++) add_diag<D>(T[j + i], r[i]);
           }
         }
-        release(D);
+        release(b);
+        c++;
         return true;
       };
       for (int kb = kb0; kb < kb1; kb++) {
-        const int k = kb - kb0;
-        const bool last = kb == kb1 - 1;
-        if (last) {  // the tail, in units 2^-fs below the integer's
-          ok = wait_for(NDIAG);
-          if (!ok) break;
-#pragma unroll
-          for (int j = 0; j < HC; j += 8) {
-            if (j < hc) {
-              uint32_t r[8];
-              tmem_ld8(tl + (uint32_t)(NDIAG * bn + j), r);
-              tmem_wait8(r);
-#pragma unroll
-              for (int i = 0; i < 8; i++) F[j + i] = __uint_as_float(r[i]);
-            }
-          }
-          release(NDIAG);
-        }
-        if (k % drain_every(0) == drain_every(0) - 1 || last) ok = ok && take(std::integral_constant<int, 0>{});
-        if (k % drain_every(1) == drain_every(1) - 1 || last) ok = ok && take(std::integral_constant<int, 1>{});
-        if (k % drain_every(2) == drain_every(2) - 1 || last) ok = ok && take(std::integral_constant<int, 2>{});
-        if (k % drain_every(3) == drain_every(3) - 1 || last) ok = ok && take(std::integral_constant<int, 3>{});
-        if (k % drain_every(4) == drain_every(4) - 1 || last) ok = ok && take(std::integral_constant<int, 4>{});
+        ok = take(std::integral_constant<int, 4>{}) && take(std::integral_constant<int, 3>{}) &&
+             take(std::integral_constant<int, 2>{}) && take(std::integral_constant<int, 1>{}) &&
+             take(std::integral_constant<int, 0>{});
         if (!ok) break;
       }
+      if (ok && !mbar_wait(&ctl.tfull[TAIL], (uint32_t)w & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) ok = false;
       asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");  // column tables of this unit written
       if (!ok || errv) break;
-      if (eA == kRowNonFinite) continue;
+      tc_fence_after();
+      const long long off = magic_sum(kb1 - kb0);
       const double mul = a.alpha;
       const bool scaled = !a.partial && !a.alpha_pow2;
       const uint32_t flip = (!a.partial && a.alpha_pow2 && a.alpha_neg) ? 0x80000000u : 0u;
@@ -382,11 +375,15 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int mode = (a.partial || a.beta == 0.0) ? 0 : (a.beta == 1.0 ? 1 : 2);
 #pragma unroll
       for (int j = 0; j < HC; j += 8) {
-        if (j < hc) {
+        if (j >= hc) continue;
+        uint32_t r[8];
+        tmem_ld8(tl + (uint32_t)(TAIL * bn + j), r);
+        tmem_wait8(r);
         double v[8];
 #pragma unroll
         for (int i = 0; i < 8; i++)
-          v[i] = slice_value(T[j + i], rint_i32(F[j + i] * ftail), a.fs, sc0 + ctl.colE[hc * h + j + i], flip);
+          v[i] = slice_value(T[j + i] - off, rint_i32(__uint_as_float(r[i]) * ftail), a.fs,
+                             sc0 + ctl.colE[hc * h + j + i], flip);
         if (scaled) {
 #pragma unroll
           for (int i = 0; i < 8; i++) v[i] *= mul;
@@ -394,14 +391,14 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
         for (int i = 0; i < 8; i++) {
           const int64_t co = ctl.colOff[hc * h + j + i];
-          if (co < 0) continue;
+          if (co < 0 || eA == kRowNonFinite) continue;
           double *p = base + co;
           if (mode == 0) *p = v[i];
           else if (mode == 1) asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v[i]) : "memory");
           else *p = fma(a.beta, *p, v[i]);
         }
-        }
       }
+      release(TAIL);
     }
   }
   tc_fence_before();
@@ -602,7 +599,7 @@ SliceEngine::SliceEngine(Ctx &ctx) : ctx_(ctx) {
   SCESS_CUDA(cudaMemsetAsync(err_.as<void>(), 0, sizeof(unsigned) * 4, ctx_.stream));
 }
 
-int SliceEngine::tile_n(int64_t N) { return (int)round_up(ceil_div(N, ceil_div(N, BN)), 16); }
+int SliceEngine::tile_n(int64_t N) { return (int)round_up(ceil_div(N, ceil_div(N, BN)), 8 * EPI); }
 
 bool SliceEngine::usable(int64_t M, int64_t N) {
   return kernel_ok() && M <= INT32_MAX / 2 && N <= INT32_MAX / 2;
@@ -807,12 +804,23 @@ void SliceEngine::gemm(const SlicedPack &A, const SlicedPack &B, double alpha, d
   ps.M = A.rows;
   ps.N = B.rows;
   const int64_t nkb = A.Kpad / BK, tiles = ceil_div(ps.M, BM) * ceil_div(ps.N, tile_n(ps.N));
-  // split K when the tiles leave SMs idle (at least 4 K blocks a unit) or a
-  // unit's K would pass what its 64-bit sum holds
-  int64_t splits = 1;
-  if (tiles < kNumSMs) splits = std::max<int64_t>(1, std::min<int64_t>(kNumSMs / tiles, nkb / 4));
-  while (splits > 1 && splits * ps.M * ps.N > (int64_t(64) << 20)) splits--;
-  splits = std::max(splits, ceil_div(nkb, 512));
+  // Split K where it shortens the launch: rounds of units over the SMs times the K
+  // blocks of a unit, in units of one K block (2.8 us): a unit's epilogue costs about
+  // 1.5, partial sums are written and read again at 5 TB/s, their reduction is one more
+  // launch (1.5).  (9870 x 136 x 9870: 156 tiles take two rounds of 309 blocks; 19 splits
+  // take 20 of 17.)  A unit's K is at most what its 64-bit sums hold.
+  int64_t splits = ceil_div(nkb, 512);
+  double best = 1e300;
+  const int64_t most = std::min<int64_t>(nkb / 2, std::max<int64_t>(64, ceil_div(2 * kNumSMs, tiles)));
+  for (int64_t z = splits; z <= std::max(splits, most); z++) {
+    if (z > splits && z * ps.M * ps.N > (int64_t(64) << 20)) break;
+    double cost = (double)ceil_div(tiles * z, kNumSMs) * ((double)ceil_div(nkb, z) + 1.5);
+    if (z > 1) cost += 1.5 + (double)z * ps.M * ps.N * 16.0 / 5.0e12 / 2.8e-6;
+    if (cost < 0.97 * best) {
+      best = cost;
+      splits = z;
+    }
+  }
   double *partial = nullptr;
   if (splits > 1) {
     const size_t need = (size_t)splits * ps.M * ps.N * sizeof(double);
