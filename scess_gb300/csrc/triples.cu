@@ -981,19 +981,21 @@ void g_block_fp64(Ctx &ctx, const TriplesSetup &T, const int64_t U[3], const dou
 }
 
 // Block size of the grouped tensor-core form: GEMM rows (u, x_l) = o nb fill
-// the 128-row tiles well, the padded virtual range vp = NB nb stays close to v,
-// and W (nb^3 o^3 floats per buffer) stays within 64 MiB a buffer; ties go to
-// the larger block (fewer, larger launches).  The tuning key t_nb overrides it.
+// the units' rows well (256 on cluster pairs, else 128), the padded virtual range
+// vp = NB nb stays close to v, and W (nb^3 o^3 floats per buffer) stays within 64 MiB a
+// buffer; ties go to the larger block (fewer, larger launches).  With rows counted in
+// 128s on pairs, o = 13, v = 117 took nb = 9 (117 of 256 rows, 455 launches, 27.5 ms)
+// where nb = 17 (84 launches) takes 16.8 ms.  The tuning key t_nb overrides it.
 int choose_nb_grouped(int64_t o, int64_t v) {
   const int64_t forced = tune_value("t_nb", 0);
   if (forced >= 1) return (int)std::min<int64_t>(forced, v);
   int best = 1;
   double best_score = -1.0;
-  const double o3 = (double)o * o * o;
+  const double o3 = (double)o * o * o, bm = TcEngine::pair_available() ? 256.0 : 128.0;
   for (int nb = 1; nb <= std::min<int64_t>(v, 64); nb++) {
     if (nb > 1 && (double)nb * nb * nb * o3 * 4.0 > double(64 << 20)) break;
     const double rows = (double)o * nb;
-    const double effM = rows / (128.0 * std::ceil(rows / 128.0));
+    const double effM = rows / (bm * std::ceil(rows / bm));
     const double vp = (double)ceil_div(v, nb) * nb;
     const double effV = std::pow((double)v / vp, 3.0);
     const double score = effM * effV;
