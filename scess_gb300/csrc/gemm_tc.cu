@@ -614,10 +614,12 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
         __syncwarp();  // rowOffS read before the next unit rewrites it
         continue;
       }
-      if (a.stcol[pg] && out.fp32 && out.beta == 0.0 && !a.partial) {  // (beta = 1: the generic path)
+      if (a.stcol[pg] && out.fp32 && (out.beta == 0.0 || accum) && !a.partial) {
         // Tile staged through shared memory CH columns at a time, then each warp
-        // stores its 32 rows with the lanes along the columns: for outputs whose
-        // unit-stride index is a column index this writes contiguous runs.
+        // stores (beta = 1: adds) its 32 rows with the lanes along the columns: for
+        // outputs whose unit-stride index is a column index this writes contiguous runs.
+        // (The (T) launch with o not a multiple of 4: with every lane in a row of its own
+        // the reductions of o = 13, v = 117 took 154 us a launch, now 96.)
         float *C = (float *)out.C;
         const float fa = s_falpha;
         constexpr int CH = SH::CH;
@@ -629,7 +631,7 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
 #pragma unroll
           for (int jj = 0; jj < CH; jj++) stage[h][jj][row] = fa * acc[j0 + jj];
           __syncwarp();
-          if (BN == 256 && a.stvec[pg]) {  // (the (T) launch; einsums keep the scalar form)
+          if (BN == 256 && a.stvec[pg] && !accum) {  // (the (T) launch; einsums keep the scalar form)
             // every aligned quad of columns is a contiguous 16-byte run: lanes
             // take quad lane % QPR of row rr + lane / QPR (conflict-free reads:
             // the staging pitch is 2 mod 32 words)
@@ -660,11 +662,20 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
             const int rsub = lane / CH;
             constexpr int RSTEP = 32 / CH;
             const int64_t co = colH[j0 + cl];
+            if (accum) {
 #pragma unroll 4
-            for (int rr = 0; rr < 32; rr += RSTEP) {
-              const int r = 32 * q + rr + rsub;
-              const int64_t ro = rowOffS[h][r];
-              if (ro >= 0 && co >= 0) C[ro + co] = stage[h][cl][r];
+              for (int rr = 0; rr < 32; rr += RSTEP) {
+                const int r = 32 * q + rr + rsub;
+                const int64_t ro = rowOffS[h][r];
+                if (ro >= 0 && co >= 0) atomicAdd(C + ro + co, stage[h][cl][r]);
+              }
+            } else {
+#pragma unroll 4
+              for (int rr = 0; rr < 32; rr += RSTEP) {
+                const int r = 32 * q + rr + rsub;
+                const int64_t ro = rowOffS[h][r];
+                if (ro >= 0 && co >= 0) C[ro + co] = stage[h][cl][r];
+              }
             }
           }
         }
