@@ -81,6 +81,10 @@ void DevMem::alloc(size_t bytes) {
   }
   if (c && c->mem_limit) {
     if (c->mem_held + bytes > c->mem_limit && c->blocks.bytes() > 0) flush_cache(c);
+    if (c->mem_held + bytes > c->mem_limit && c->slices) {
+      c->slices->reclaim();
+      flush_cache(c);
+    }
     if (c->mem_held + bytes > c->mem_limit)
       throw Error(SCESS_ERR_OOM, "device memory limit of the context reached: " +
                                      std::to_string(c->mem_held) + " B held + " +
@@ -88,8 +92,9 @@ void DevMem::alloc(size_t bytes) {
                                      std::to_string(c->mem_limit) + " B");
   }
   cudaError_t e = cudaMalloc(&p_, bytes);
-  if (e == cudaErrorMemoryAllocation && c && c->blocks.bytes() > 0) {
+  if (e == cudaErrorMemoryAllocation && c) {
     cudaGetLastError();
+    if (c->slices) c->slices->reclaim();
     flush_cache(c);
     e = cudaMalloc(&p_, bytes);
   }

@@ -426,49 +426,80 @@ __global__ void slice_reduce_kernel(SliceArgs a, int splits) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Packs.  One CTA per 32 rows (RowTiles: along the operand's smallest-stride row
-// label, so that loads coalesce) walks K in chunks of 64.  EXPS: the row
-// exponents only, over the K chunks blockIdx.y, + gridDim.y, ..., folded into exps with
-// atomics.  OWN: the CTA covers the whole K, finds its rows' exponents in a
-// first walk and cuts in a second one (whose loads hit L2).  GIVEN: the exponents
-// are read, K chunks spread over blockIdx.y.  HBM-bound: 8 B read and 14 B
-// written per element (about 50 integer and FP32 instructions).
-enum class PackMode { EXPS, OWN, GIVEN };
+// Packs.  One CTA per tile of 2048 / KT rows x KT values of k (KT = 64, or 32, 16 for a K
+// that short; rows in the order of RowTiles, so that loads coalesce) and range of K
+// chunks.  A launch takes up to two operands.  OWN: the CTA covers the whole K, finds
+// its rows' exponents in a first walk (kept in registers when K <= KT) and cuts in a
+// second one, whose loads hit L2.  PART / FROM_PART: K spread over CTAs, partial
+// exponents first, the cut in a second launch.  EXPS: exponents only, folded into
+// exps[expIdx[row]] with atomics.  GIVEN: exponents exps[expIdx[row]], K spread over
+// CTAs.
+// HBM-bound with long rows (8 B read and 14 B written per element, 3.2 TB/s at
+// 4096 x 4096, 2.3 before the loads of the next chunk were in flight while one is cut).
+enum PackMode { PACK_OWN, PACK_PART, PACK_FROM_PART, PACK_EXPS, PACK_GIVEN };
+struct PackOp {
+  const double *src;
+  const int64_t *row, *k;  // offset tables, or null: r rs and k ks
+  int64_t rs, ks;
+  int64_t rows, K, Kpad;
+  RowTiles rt;
+  int mode, unitK, negate, parts;
+  uint16_t *dst;
+  int *exps, *part;
+  const int64_t *expIdx;
+  int64_t blocks;  // rt.count times the K ranges
+};
+struct PackOps {
+  PackOp op[2];
+};
 
-template <PackMode MODE, bool AFFINE>
-__global__ void __launch_bounds__(256) slice_pack_kernel(
-    const double *__restrict__ src, const int64_t *__restrict__ rowOff, int64_t rows,
-    const int64_t *__restrict__ kOff, int64_t K, int unitK, uint16_t *__restrict__ dst,
-    int64_t Kpad, int *__restrict__ exps, const int64_t *__restrict__ expIdx, int negate, int64_t rs,
-    int64_t ks, const RowTiles rt) {
-  __shared__ double tile[32][65];
-  __shared__ int64_t sr[32], sk[64], srow[32];
-  __shared__ int se[32];
+__device__ __forceinline__ int tile_col(int k) { return k + (k >> 3); }
+
+template <int KT>
+__global__ void __launch_bounds__(256) slice_pack_kernel(const __grid_constant__ PackOps ops) {
+  const bool second = blockIdx.x >= ops.op[0].blocks;
+  const PackOp &op = ops.op[second ? 1 : 0];
+  const int64_t blk = second ? blockIdx.x - ops.op[0].blocks : blockIdx.x;
+  // doubles with a gap every 8 columns and a pitch of 1 mod 16: free of bank conflicts both ways
+  constexpr int ROWS = 2048 / KT, PITCH = KT == 64 ? 81 : KT == 32 ? 49 : 33;
+  __shared__ double tile[ROWS][PITCH];
+  __shared__ int64_t sr[ROWS], sk[KT], srow[ROWS];
+  __shared__ int se[ROWS];
   const int t = threadIdx.x;
-  if (t < 32) {
-    const int64_t r = rt.row(blockIdx.x, t);
-    srow[t] = (r >= 0 && r < rows) ? r : -1;
-    sr[t] = srow[t] >= 0 ? (AFFINE ? r * rs : rowOff[r]) : -1;
-    se[t] = MODE == PackMode::GIVEN && srow[t] >= 0 ? exps[expIdx ? expIdx[r] : r] : 0;
+  const int mode = op.mode, unitK = op.unitK;
+  const int64_t x0 = blk % op.rt.count, c0 = blk / op.rt.count, cs = op.blocks / op.rt.count;
+  const int64_t K = op.K;
+  const double *__restrict__ src = op.src;
+  if (t < ROWS) {
+    const int64_t r = op.rt.row(x0 * ROWS + t);
+    srow[t] = r;
+    sr[t] = r < 0 ? -1 : (op.row ? op.row[r] : r * op.rs);
+    int e = 0;
+    if (r >= 0 && mode == PACK_GIVEN) e = op.exps[op.expIdx ? op.expIdx[r] : r];
+    if (r >= 0 && mode == PACK_FROM_PART) {
+      for (int q = 0; q < op.parts; q++) e = max(e, op.part[(int64_t)q * op.rows + r]);
+      if (c0 == 0) op.exps[r] = e;
+    }
+    se[t] = e;
   }
-  const int64_t nchunk = (MODE == PackMode::EXPS ? (K + 63) : (Kpad + 63)) / 64;
-  const int64_t c0 = MODE == PackMode::OWN ? 0 : blockIdx.y, cs = MODE == PackMode::OWN ? 1 : gridDim.y;
-  auto load_offsets = [&](int64_t k0) {
-    __syncthreads();
-    if (t < 64) sk[t] = (k0 + t < K) ? (AFFINE ? (k0 + t) * ks : kOff[k0 + t]) : -1;
-    __syncthreads();
-  };
-  if (MODE != PackMode::GIVEN) {
-    int mx[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int64_t c = c0; c * 64 < K; c += cs) {
-      load_offsets(c * 64);
-      double x[8];
+  auto koff = [&](int64_t k) -> int64_t { return k < K ? (op.k ? op.k[k] : k * op.ks) : -1; };
+  double x[8];
+  auto load = [&]() {
 #pragma unroll
-      for (int p = 0; p < 8; p++) {
-        const int rr = unitK ? (t >> 6) + 4 * p : t & 31, kk = unitK ? t & 63 : (t >> 5) + 8 * p;
-        const int64_t ro = sr[rr], ko = sk[kk];
-        x[p] = (ro >= 0 && ko >= 0) ? src[ro + ko] : 0.0;
-      }
+    for (int p = 0; p < 8; p++) {
+      const int rr = unitK ? t / KT + (256 / KT) * p : t % ROWS, kk = unitK ? t % KT : t / ROWS + (256 / ROWS) * p;
+      const int64_t ro = sr[rr], ko = sk[kk];
+      x[p] = (ro >= 0 && ko >= 0) ? src[ro + ko] : 0.0;
+    }
+  };
+  const bool find = mode == PACK_OWN || mode == PACK_PART || mode == PACK_EXPS;
+  if (find) {
+    int mx[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int64_t c = c0; c * KT < K; c += cs) {
+      __syncthreads();
+      if (t < KT) sk[t] = koff(c * KT + t);
+      __syncthreads();
+      load();
 #pragma unroll
       for (int p = 0; p < 8; p++) {
         const int hi = __double2hiint(x[p]) & 0x7fffffff;
@@ -476,43 +507,56 @@ __global__ void __launch_bounds__(256) slice_pack_kernel(
         mx[p] = max(mx[p], e);
       }
     }
-    if (unitK) {  // the rows (t >> 6) + 4 p are shared by two warps
+    if (unitK) {  // KT lanes share a row (two warps with KT = 64)
 #pragma unroll
       for (int p = 0; p < 8; p++) {
-        const int m = __reduce_max_sync(0xffffffffu, mx[p]);
-        if ((t & 31) == 0) atomicMax(&se[(t >> 6) + 4 * p], m);
+        int m = mx[p];
+#pragma unroll
+        for (int off = (KT < 32 ? KT : 32) / 2; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
+        if (t % (KT < 32 ? KT : 32) == 0) atomicMax(&se[t / KT + (256 / KT) * p], m);
       }
     } else {
       int m = 0;
 #pragma unroll
       for (int p = 0; p < 8; p++) m = max(m, mx[p]);
-      atomicMax(&se[t & 31], m);
+      atomicMax(&se[t % ROWS], m);
     }
     __syncthreads();
-    if (t < 32 && srow[t] >= 0) {
-      if (MODE == PackMode::EXPS) atomicMax(&exps[expIdx ? expIdx[srow[t]] : srow[t]], se[t]);
-      else exps[srow[t]] = se[t];
+    if (t < ROWS && srow[t] >= 0) {
+      if (mode == PACK_EXPS) atomicMax(&op.exps[op.expIdx ? op.expIdx[srow[t]] : srow[t]], se[t]);
+      else if (mode == PACK_PART) op.part[c0 * op.rows + srow[t]] = se[t];
+      else op.exps[srow[t]] = se[t];
     }
+    if (mode != PACK_OWN) return;
   }
-  for (int64_t c = c0; MODE != PackMode::EXPS && c < nchunk; c += cs) {
-    const int64_t k0 = c * 64;
-    load_offsets(k0);
+  const int64_t Kpad = op.Kpad, nchunk = (Kpad + KT - 1) / KT;
+  if (!(find && K <= KT)) {  // (else x holds the chunk already)
+    __syncthreads();
+    if (t < KT) sk[t] = koff(c0 * KT + t);
+    __syncthreads();
+    load();
+  }
+  const int rr = t / (KT / 8), ch = t % (KT / 8);
+  for (int64_t c = c0; c < nchunk; c += cs) {
+    const bool more = c + cs < nchunk;
+    const int64_t nk = (t < KT && more) ? koff((c + cs) * KT + t) : -1;
+    __syncthreads();  // the previous chunk's tile and offsets are used up
 #pragma unroll
     for (int p = 0; p < 8; p++) {
-      const int rr = unitK ? (t >> 6) + 4 * p : t & 31, kk = unitK ? t & 63 : (t >> 5) + 8 * p;
-      const int64_t ro = sr[rr], ko = sk[kk];
-      tile[rr][kk] = (ro >= 0 && ko >= 0) ? src[ro + ko] : 0.0;
+      const int r = unitK ? t / KT + (256 / KT) * p : t % ROWS, kk = unitK ? t % KT : t / ROWS + (256 / ROWS) * p;
+      tile[r][tile_col(kk)] = x[p];
     }
+    if (t < KT) sk[t] = nk;
     __syncthreads();
-    const int rr = t >> 3, ch = t & 7;
-    const int64_t r = srow[rr];
+    if (more) load();  // in flight while this chunk is cut
+    const int64_t k0 = c * KT, r = srow[rr];
     if (r < 0 || k0 + ch * 8 >= Kpad) continue;
     const int e = se[rr];
     uint32_t w[kSlices][4];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      int64_t F = e == kRowNonFinite ? 0 : slice_fixed(tile[rr][ch * 8 + j], e);
-      if (negate) F = -F;
+      int64_t F = e == kRowNonFinite ? 0 : slice_fixed(tile[rr][9 * ch + j], e);
+      if (op.negate) F = -F;
       const int64_t G = F + kDigitBias;
 #pragma unroll
       for (int p = 0; p < kSlices; p++) {
@@ -528,11 +572,27 @@ __global__ void __launch_bounds__(256) slice_pack_kernel(
         else w[p][j >> 1] = b;
       }
     }
-    uint16_t *d = dst + r * kSlices * Kpad + k0 + ch * 8;
+    uint16_t *d = op.dst + r * kSlices * Kpad + k0 + ch * 8;
 #pragma unroll
     for (int p = 0; p < kSlices; p++)
       *reinterpret_cast<uint4 *>(d + p * Kpad) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
   }
+}
+
+// Tile width of a K: no wider than needed.
+int pack_kt(int64_t K) { return K <= 16 ? 16 : K <= 32 ? 32 : 64; }
+
+void launch_packs(const PackOp *op, int n, cudaStream_t stream) {  // (the operands have one K)
+  PackOps p;
+  p.op[0] = op[0];
+  p.op[1] = op[n - 1];
+  const int64_t blocks = op[0].blocks + (n > 1 ? op[1].blocks : 0);
+  if (blocks > INT32_MAX) throw Error(SCESS_ERR_INVALID, "slice pack: too large");
+  const int kt = pack_kt(op[0].K);
+  if (kt == 16) slice_pack_kernel<16><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  else if (kt == 32) slice_pack_kernel<32><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  else slice_pack_kernel<64><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  SCESS_CHECK_LAUNCH();
 }
 
 __global__ void __launch_bounds__(256) dgemm_masked_kernel(TableGemm g, const int *__restrict__ expA,
@@ -632,67 +692,89 @@ void SliceEngine::alloc(SlicedPack &out, int64_t rows, int64_t K) {
 
 void SliceEngine::row_exps(const double *src, const int64_t *rowOff, int64_t rows, const int64_t *kOff,
                            int64_t K, bool unitK, int *exps, const int64_t *expIdx) {
-  const RowTiles rt = RowTiles::make(rows, 1, rows);
-  const dim3 grid((unsigned)rt.count,
-                  (unsigned)std::max<int64_t>(1, std::min<int64_t>({ceil_div(K, 64), ceil_div(8 * kNumSMs, rt.count), 65535})));
-  slice_pack_kernel<PackMode::EXPS, false><<<grid, 256, 0, ctx_.stream>>>(
-      src, rowOff, rows, kOff, K, unitK ? 1 : 0, nullptr, 0, exps, expIdx, 0, 0, 0, rt);
-  SCESS_CHECK_LAUNCH();
+  PackOp op = {};
+  op.src = src;
+  op.row = rowOff;
+  op.k = kOff;
+  op.rows = rows;
+  op.K = K;
+  op.rt = RowTiles::make(rows, 1, rows, 2048 / pack_kt(K));
+  op.mode = PACK_EXPS;
+  op.unitK = unitK ? 1 : 0;
+  op.exps = exps;
+  op.expIdx = expIdx;
+  op.blocks = op.rt.count * std::max<int64_t>(1, std::min(ceil_div(K, 64), ceil_div(8 * kNumSMs, op.rt.count)));
+  launch_packs(&op, 1, ctx_.stream);
 }
 
 void SliceEngine::pack_with_exps(const double *src, const int64_t *rowOff, int64_t rows, const int64_t *kOff,
                                  int64_t K, bool unitK, const int *exps, const int64_t *expIdx, bool negate,
                                  SlicedPack &out) {
   alloc(out, rows, K);
-  const RowTiles rt = RowTiles::make(rows, 1, rows);
   TimedScope ts(ctx_.timer, "slice_pack", 0.0, (double)rows * K * 8 + (double)rows * out.Kpad * 14, ctx_.stream);
-  const dim3 grid((unsigned)rt.count, (unsigned)std::min<int64_t>(ceil_div(out.Kpad, 64), 65535));
-  slice_pack_kernel<PackMode::GIVEN, false><<<grid, 256, 0, ctx_.stream>>>(
-      src, rowOff, rows, kOff, K, unitK ? 1 : 0, out.mem.as<uint16_t>(), out.Kpad, const_cast<int *>(exps),
-      expIdx, negate ? 1 : 0, 0, 0, rt);
-  SCESS_CHECK_LAUNCH();
+  PackOp op = {};
+  op.src = src;
+  op.row = rowOff;
+  op.k = kOff;
+  op.rows = rows;
+  op.K = K;
+  op.Kpad = out.Kpad;
+  op.rt = RowTiles::make(rows, 1, rows, 2048 / pack_kt(K));
+  op.mode = PACK_GIVEN;
+  op.unitK = unitK ? 1 : 0;
+  op.negate = negate ? 1 : 0;
+  op.dst = out.mem.as<uint16_t>();
+  op.exps = const_cast<int *>(exps);
+  op.expIdx = expIdx;
+  op.blocks = op.rt.count * std::max<int64_t>(1, std::min(ceil_div(out.Kpad, 64), ceil_div(16 * kNumSMs, op.rt.count)));
+  launch_packs(&op, 1, ctx_.stream);
 }
 
-void SliceEngine::pack(const Gather &g, SlicedPack &out) {
-  alloc(out, g.rows, g.K);
-  const bool aff = g.rs >= 0 && g.ks >= 0;
-  const RowTiles rt = RowTiles::make(g.rows, g.P, g.E > 0 ? g.E : g.rows);
-  if (rt.count > INT32_MAX) throw Error(SCESS_ERR_INVALID, "slice pack: too large");
-  TimedScope ts(ctx_.timer, "slice_pack", 0.0, (double)g.rows * g.K * 8 + (double)g.rows * out.Kpad * 14,
-                ctx_.stream);
-  const int u = g.unitK ? 1 : 0;
-  uint16_t *dst = out.mem.as<uint16_t>();
-  int *ex = out.exps.as<int>();
-  const int64_t chunks = ceil_div(out.Kpad, 64);
-  // one walk per CTA over its rows' whole K while that fills the device or K is
-  // short; else the exponents first, then the cut, each spread over K too
-  if (rt.count >= 2 * kNumSMs || chunks <= 4) {
-    if (aff)
-      slice_pack_kernel<PackMode::OWN, true><<<(unsigned)rt.count, 256, 0, ctx_.stream>>>(
-          g.src, nullptr, g.rows, nullptr, g.K, u, dst, out.Kpad, ex, nullptr, 0, g.rs, g.ks, rt);
-    else
-      slice_pack_kernel<PackMode::OWN, false><<<(unsigned)rt.count, 256, 0, ctx_.stream>>>(
-          g.src, g.row, g.rows, g.k, g.K, u, dst, out.Kpad, ex, nullptr, 0, 0, 0, rt);
-    SCESS_CHECK_LAUNCH();
-    return;
+void SliceEngine::pack(const Gather *g, SlicedPack *const *out, int n) {
+  PackOp first[2], second[2];
+  int ns = 0;
+  double bytes = 0.0;
+  for (int i = 0; i < n; i++) {
+    SlicedPack &o = *out[i];
+    alloc(o, g[i].rows, g[i].K);
+    PackOp &op = first[i];
+    op = PackOp{};
+    const bool aff = g[i].rs >= 0 && g[i].ks >= 0;
+    op.src = g[i].src;
+    op.row = aff ? nullptr : g[i].row;
+    op.k = aff ? nullptr : g[i].k;
+    op.rs = g[i].rs;
+    op.ks = g[i].ks;
+    op.rows = g[i].rows;
+    op.K = g[i].K;
+    op.Kpad = o.Kpad;
+    op.rt = RowTiles::make(g[i].rows, g[i].P, g[i].E > 0 ? g[i].E : g[i].rows, 2048 / pack_kt(g[i].K));
+    op.unitK = g[i].unitK ? 1 : 0;
+    op.dst = o.mem.as<uint16_t>();
+    op.exps = o.exps.as<int>();
+    bytes += (double)g[i].rows * g[i].K * 8 + (double)g[i].rows * o.Kpad * 14;
+    const int64_t chunks = ceil_div(o.Kpad, 64);
+    // one walk per CTA over its rows' whole K while that fills the device or K is
+    // short; else the exponents first, then the cut, each spread over K too
+    if (op.rt.count >= 2 * kNumSMs || chunks <= 4) {
+      op.mode = PACK_OWN;
+      op.blocks = op.rt.count;
+      continue;
+    }
+    op.mode = PACK_PART;
+    op.parts = (int)std::min<int64_t>({ceil_div(g[i].K, 64), ceil_div(8 * kNumSMs, op.rt.count), 64});
+    op.blocks = op.rt.count * op.parts;
+    const size_t need = (size_t)op.parts * g[i].rows * sizeof(int);
+    if (o.part.bytes() < need) o.part.alloc(round_up((int64_t)need, 4096));
+    op.part = o.part.as<int>();
+    PackOp &cut = second[ns++];
+    cut = op;
+    cut.mode = PACK_FROM_PART;
+    cut.blocks = op.rt.count * std::min(chunks, ceil_div(16 * kNumSMs, op.rt.count));
   }
-  SCESS_CUDA(cudaMemsetAsync(ex, 0, (size_t)g.rows * sizeof(int), ctx_.stream));
-  const dim3 ge((unsigned)rt.count, (unsigned)std::min<int64_t>({ceil_div(g.K, 64), ceil_div(8 * kNumSMs, rt.count), 65535}));
-  const dim3 gp((unsigned)rt.count, (unsigned)std::min<int64_t>({chunks, ceil_div(16 * kNumSMs, rt.count), 65535}));
-  if (aff) {
-    slice_pack_kernel<PackMode::EXPS, true><<<ge, 256, 0, ctx_.stream>>>(
-        g.src, nullptr, g.rows, nullptr, g.K, u, nullptr, 0, ex, nullptr, 0, g.rs, g.ks, rt);
-    SCESS_CHECK_LAUNCH();
-    slice_pack_kernel<PackMode::GIVEN, true><<<gp, 256, 0, ctx_.stream>>>(
-        g.src, nullptr, g.rows, nullptr, g.K, u, dst, out.Kpad, ex, nullptr, 0, g.rs, g.ks, rt);
-  } else {
-    slice_pack_kernel<PackMode::EXPS, false><<<ge, 256, 0, ctx_.stream>>>(
-        g.src, g.row, g.rows, g.k, g.K, u, nullptr, 0, ex, nullptr, 0, 0, 0, rt);
-    SCESS_CHECK_LAUNCH();
-    slice_pack_kernel<PackMode::GIVEN, false><<<gp, 256, 0, ctx_.stream>>>(
-        g.src, g.row, g.rows, g.k, g.K, u, dst, out.Kpad, ex, nullptr, 0, 0, 0, rt);
-  }
-  SCESS_CHECK_LAUNCH();
+  TimedScope ts(ctx_.timer, "slice_pack", 0.0, bytes, ctx_.stream);
+  launch_packs(first, n, ctx_.stream);
+  if (ns) launch_packs(second, ns, ctx_.stream);
 }
 
 void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial) {
@@ -842,10 +924,30 @@ void SliceEngine::gemm(const SlicedPack &A, const SlicedPack &B, double alpha, d
   launch(ps, (int)splits, partial);
 }
 
+void SliceEngine::reclaim() {
+  if (busy_) return;
+  tmpA_ = SlicedPack();
+  tmpB_ = SlicedPack();
+  partial_.release();
+  spare_.clear();
+  cache_.clear();
+}
+
+namespace {
+struct Busy {
+  bool &b;
+  explicit Busy(bool &x) : b(x) { b = true; }
+  ~Busy() { b = false; }
+};
+}  // namespace
+
 bool SliceEngine::table_gemm(const TableGemm &g, const char *name) {
+  Busy busy(busy_);
   try {
-    pack({g.A + g.baseA, g.rowA, g.M, g.kA, g.K, !g.aUnitM}, tmpA_);
-    pack({g.B + g.baseB, g.colB, g.N, g.kB, g.K, !g.bUnitN}, tmpB_);
+    const Gather ga[2] = {{g.A + g.baseA, g.rowA, g.M, g.kA, g.K, !g.aUnitM},
+                          {g.B + g.baseB, g.colB, g.N, g.kB, g.K, !g.bUnitN}};
+    SlicedPack *const out[2] = {&tmpA_, &tmpB_};
+    pack(ga, out, 2);
     if (g.M <= 64 && g.M < g.N) gemm(tmpB_, tmpA_, g.alpha, g.beta, g.C + g.baseC, g.colC, g.rowC, name);
     else gemm(tmpA_, tmpB_, g.alpha, g.beta, g.C + g.baseC, g.rowC, g.colC, name);
   } catch (const Error &e) {
@@ -858,9 +960,18 @@ bool SliceEngine::table_gemm(const TableGemm &g, const char *name) {
 
 void SliceEngine::clear_cache(const void *owner) {
   for (auto it = cache_.begin(); it != cache_.end();) {
-    if (it->second.first == owner) it = cache_.erase(it);
+    if (it->first.owner == owner) it = cache_.erase(it);
     else ++it;
   }
+  if (!owner) spare_.clear();  // (the end of an API call)
+}
+
+void SliceEngine::clear_stable() {
+  // the packs' memory serves the next residual's (at most kSpare of them)
+  for (auto &kv : reuse_)
+    if ((int)spare_.size() < kSpare) spare_.push_back(std::move(kv.second));
+  reuse_.clear();
+  stable_.clear();
 }
 
 void SliceEngine::check_error() {
@@ -877,47 +988,55 @@ void SliceEngine::check_error() {
 
 bool SliceEngine::contract(const EinsumPlan &pl, double alpha, const double *A, const double *B, double beta,
                            double *C, bool constA, bool constB) {
+  Busy busy(busy_);
   // Epilogue lanes walk the GEMM rows: put C's unit-stride index there, unless
   // that side is short: rows come in tiles of 128, columns in steps of 16.
   const bool swap = std::min(pl.M, pl.N) <= 64 ? pl.M < pl.N : (!pl.cUnitM && pl.cUnitN);
   const Gather gA{A, pl.d_rowA, pl.M, pl.d_kA, pl.K, pl.aUnitK, pl.aRowStride, pl.aKStride, pl.aRowP, pl.aRowE};
   const Gather gB{B, pl.d_colB, pl.N, pl.d_kB, pl.K, pl.bUnitK, pl.bColStride, pl.bKStride, pl.bColP, pl.bColE};
-  auto get = [&](const Gather &g, bool isA, bool isConst, SlicedPack &tmp) -> const SlicedPack & {
-    if (!isConst && !stable_.count(g.src)) {
-      pack(g, tmp);
-      return tmp;
+  Gather todo[2];
+  SlicedPack *out[2];
+  int n = 0;
+  // the operand's pack: kept (constant operands, stable tensors) or still to be made
+  auto get = [&](const Gather &g, bool isA, bool isConst, SlicedPack &tmp) -> SlicedPack * {
+    SlicedPack *p = &tmp;
+    if (isConst || stable_.count(g.src)) {
+      uint64_t &hs = isA ? pl.hashA : pl.hashB;
+      if (!hs) hs = isA ? table_hash(pl.rowA, pl.kA) : table_hash(pl.colB, pl.kB);
+      const Key key{g.src, hs, g.rows, g.K, isConst ? owner_ : nullptr};
+      auto &kept = isConst ? cache_ : reuse_;
+      auto it = kept.find(key);
+      if (it != kept.end()) return it->second.get();
+      std::unique_ptr<SlicedPack> np;
+      if (!isConst && !spare_.empty()) {
+        np = std::move(spare_.back());
+        spare_.pop_back();
+      } else {
+        np = std::make_unique<SlicedPack>();
+      }
+      p = np.get();
+      alloc(*p, g.rows, g.K);  // (before it is listed: an allocation may fail)
+      kept[key] = std::move(np);
     }
-    uint64_t &hs = isA ? pl.hashA : pl.hashB;
-    if (!hs) hs = isA ? table_hash(pl.rowA, pl.kA) : table_hash(pl.colB, pl.kB);
-    const std::string key = std::to_string((uintptr_t)g.src) + "|" + std::to_string(hs) + "|" +
-                            std::to_string(g.rows) + "|" + std::to_string(g.K);
-    if (isConst) {
-      auto it = cache_.find(key);
-      if (it != cache_.end() && it->second.first == owner_) return *it->second.second;
-    } else {
-      auto it = reuse_.find(key);
-      if (it != reuse_.end()) return *it->second;
-    }
-    auto pk = std::make_unique<SlicedPack>();
-    pack(g, *pk);
-    SlicedPack &ref = *pk;
-    if (isConst) cache_[key] = std::make_pair(owner_, std::move(pk));
-    else reuse_[key] = std::move(pk);
-    return ref;
+    todo[n] = g;
+    out[n++] = p;
+    return p;
   };
   const std::string tname = "slice_gemm[" + pl.spec + "]";
   const SlicedPack *pa = nullptr, *pb = nullptr;
   try {
-    pa = &get(gA, true, constA, tmpA_);
-    pb = &get(gB, false, constB, tmpB_);
+    pa = get(gA, true, constA, tmpA_);
+    pb = get(gB, false, constB, tmpB_);
+    if (n) pack(todo, out, n);
     if (swap) gemm(*pb, *pa, alpha, beta, C, pl.d_colC, pl.d_rowC, tname.c_str());
     else gemm(*pa, *pb, alpha, beta, C, pl.d_rowC, pl.d_colC, tname.c_str());
   } catch (const Error &e) {
-    if (e.code != SCESS_ERR_OOM) throw;
-    // no room for the packs: give the kept ones back, the DFMA kernel needs none
+    // packs listed above may not have been made
     reuse_.clear();
-    clear_cache(owner_);
-    return false;
+    spare_.clear();
+    cache_.clear();
+    if (e.code != SCESS_ERR_OOM) throw;
+    return false;  // no room for the packs: the DFMA kernel needs none
   }
   TableGemm g;
   g.A = A;

@@ -27,6 +27,7 @@
 #include <memory>
 #include <set>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "engine.h"
@@ -41,6 +42,7 @@ constexpr int kRowNonFinite = 2047;  // row exponent of a row that holds Inf or 
 // exponent per row (0: all values zero; kRowNonFinite: Inf or NaN).
 struct SlicedPack {
   DevMem mem, exps;
+  DevMem part;  // partial row exponents of long rows
   int64_t rows = 0, K = 0, Kpad = 0;
   const int *e() const { return exps.as<int>(); }
 };
@@ -99,13 +101,13 @@ class SliceEngine {
   // Packs of constant operands, kept for the owner of their source (see TcEngine).
   void set_cache_owner(const void *o) { owner_ = o; }
   void clear_cache(const void *owner);
+  // Gives back what it keeps (packs, workspaces) unless a contraction is being set up:
+  // called when an allocation fails.
+  void reclaim();
   // A tensor that stays unchanged until clear_stable(): einsums that gather it
   // through equal tables share one pack.
   void add_stable(const double *p) { stable_.insert(p); }
-  void clear_stable() {
-    stable_.clear();
-    reuse_.clear();
-  }
+  void clear_stable();
   // Throws SCESS_ERR_CUDA if a bounded wait of a launch since the last check expired.
   void check_error();
   bool launched() const { return launched_; }
@@ -116,28 +118,39 @@ class SliceEngine {
 
  private:
   struct Gather {  // an operand seen through its tables
-    const double *src;
-    const int64_t *row;
-    int64_t rows;
-    const int64_t *k;
-    int64_t K;
-    bool unitK;
+    const double *src = nullptr;
+    const int64_t *row = nullptr;
+    int64_t rows = 0;
+    const int64_t *k = nullptr;
+    int64_t K = 0;
+    bool unitK = false;
     int64_t rs = -1, ks = -1, P = 1, E = 0;
   };
-  void pack(const Gather &g, SlicedPack &out);
+  // Packs of up to two operands in one launch (two where K is long).
+  void pack(const Gather *g, SlicedPack *const *out, int n);
   void alloc(SlicedPack &out, int64_t rows, int64_t K);
   void gemm(const SlicedPack &A, const SlicedPack &B, double alpha, double beta, double *C,
             const int64_t *rowC, const int64_t *colC, const char *name);
   void launch(const SliceProblemSet &ps, int splits, double *partial);
 
   Ctx &ctx_;
-  std::map<std::string, std::pair<const void *, std::unique_ptr<SlicedPack>>> cache_;
-  std::map<std::string, std::unique_ptr<SlicedPack>> reuse_;
+  struct Key {  // a gather: source, content hash of its tables, sizes; owner of a kept pack
+    const double *src;
+    uint64_t hash;
+    int64_t rows, K;
+    const void *owner;
+    bool operator<(const Key &o) const {
+      return std::tie(src, hash, rows, K, owner) < std::tie(o.src, o.hash, o.rows, o.K, o.owner);
+    }
+  };
+  std::map<Key, std::unique_ptr<SlicedPack>> cache_, reuse_;
+  static constexpr int kSpare = 12;
+  std::vector<std::unique_ptr<SlicedPack>> spare_;  // packs of stable tensors, done with
   std::set<const double *> stable_;
   const void *owner_ = nullptr;
   SlicedPack tmpA_, tmpB_;
   DevMem err_, partial_;
-  bool launched_ = false;
+  bool launched_ = false, busy_ = false;
   long long wait_cycles_ = 1ll << 32;
   bool withhold_ = false;
 };

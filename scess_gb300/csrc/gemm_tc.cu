@@ -847,7 +847,7 @@ __global__ void __launch_bounds__(256) maxabs_kernel(
     const int64_t k0 = (tile / trow) * 64;
     __syncthreads();  // previous tile's table reads done
     if (t < 32) {
-      const int64_t r = rt.row(tile % trow, t);
+      const int64_t r = rt.row((tile % trow) * 32 + t);
       sr[t] = (r >= 0 && r < rows) ? (AFFINE ? r * rs : rowOff[r]) : -1;
     }
     else if (t < 96) sk[t - 32] = (k0 + t - 32 < K) ? (AFFINE ? (k0 + t - 32) * ks : kOff[k0 + t - 32]) : -1;
@@ -934,7 +934,7 @@ __global__ void __launch_bounds__(256) pack_split_kernel(
   // row tiles on grid.x (up to 2^31 - 1), K blocks on grid.y (<= 65535)
   const int64_t k0 = (int64_t)blockIdx.y * 64;
   if (t < 32) {
-    const int64_t r = rt.row(blockIdx.x, t);
+    const int64_t r = rt.row((int64_t)blockIdx.x * 32 + t);
     srow[t] = (r >= 0 && r < rows) ? r : -1;
     sr[t] = srow[t] >= 0 ? (AFFINE ? r * rs : rowOff[r]) : -1;
   }

@@ -1,31 +1,36 @@
-// Row tiling shared by the pack kernels of the tensor-core GEMMs.
+// Row order of the pack kernels of the tensor-core GEMMs.
 #pragma once
 #include <algorithm>
 #include <cstdint>
 
 namespace scess {
 
-// Row tiles of 32 rows along a group's smallest-stride label: row tile x holds
-// rows r = pre + P (32 ft + t + E post), t < 32 (-1 past the label's extent),
-// so that a tile's source values are contiguous when that stride is 1.
+// A pack walks an operand's rows along its smallest-stride row label first, so that
+// the source values of consecutive rows lie together.  Rows r = pre + P (f + E post) with
+// f < E that label's index, P the product of the extents before it; the q-th row of
+// the order has f = q mod E, then pre, then post.  Tiles are cut from this order, so
+// that a label shorter than a tile leaves no rows of it empty (with one label per tile
+// the packs of o = 10 filled 10 rows of 32).
 struct RowTiles {
-  int64_t P = 1, E = 1, nft = 1, count = 0;
-  static RowTiles make(int64_t rows, int64_t P, int64_t E) {
+  int64_t P = 1, E = 1, rows = 0, count = 0;  // count: tiles of T rows
+  static RowTiles make(int64_t rows, int64_t P, int64_t E, int T = 32) {
     RowTiles r;
-    if (P < 1 || E < 1 || rows % (P * E) != 0) {  // not a product grouping: plain tiles
+    if (P < 1 || E < 1 || rows % (P * E) != 0) {  // not a product grouping: consecutive rows
       P = 1;
       E = std::max<int64_t>(rows, 1);
     }
     r.P = P;
     r.E = E;
-    r.nft = (E + 31) / 32;
-    r.count = P * r.nft * (std::max<int64_t>(rows, 1) / (P * E));
+    r.rows = rows;
+    r.count = (std::max<int64_t>(rows, 1) + T - 1) / T;
     return r;
   }
-  __device__ int64_t row(int64_t x, int t) const {
-    const int64_t pre = x % P, rem = x / P, ft = rem % nft, post = rem / nft;
-    const int64_t f = ft * 32 + t;
-    return f < E ? pre + P * (f + E * post) : -1;
+  // The q-th row, -1 past the last.
+  __device__ int64_t row(int64_t q) const {
+    if (q >= rows) return -1;
+    if (P == 1) return q;
+    const int64_t f = q % E, rest = q / E;
+    return rest % P + P * (f + E * (rest / P));
   }
 };
 
