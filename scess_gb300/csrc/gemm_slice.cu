@@ -48,9 +48,8 @@ static_assert(kCtlRegs + EPI * kEpiRegs <= (1 + EPI) * kLaunchRegs, "setmaxnreg 
 struct Ctl {  // behind the stages
   uint64_t full[STAGES], empty[STAGES], tfull[NACC], tempty[NACC], done;
   uint32_t tmem;
-  uint32_t pad;
-  int64_t colOff[BN];
-  int colE[BN];
+  alignas(16) int64_t colOff[BN];
+  alignas(16) int colE[BN];
 };
 constexpr size_t SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + sizeof(Ctl);
 
@@ -314,7 +313,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       if (et < hc) {
         const int nn = tn * bn + hc * h + et;
         const int e = nn < a.N ? a.expB[nn] : kRowNonFinite;
-        ctl.colE[hc * h + et] = max(e, 1);
+        ctl.colE[hc * h + et] = e == 0 ? 1023 : e;  // (all zero: any scale)
         ctl.colOff[hc * h + et] =
             e == kRowNonFinite ? -1
             : a.partial ? (int64_t)sp * a.part_stride + (int64_t)a.M * nn
@@ -324,8 +323,9 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int64_t rowOff = m < a.M ? (a.partial ? (int64_t)m : a.rowC[pg][m]) : 0;
       const unsigned errv = *(volatile unsigned *)a.err;
       long long T[HC];
+      const long long off = magic_sum(kb1 - kb0);
 #pragma unroll
-      for (int j = 0; j < HC; j++) T[j] = 0;
+      for (int j = 0; j < HC; j++) T[j] = -off;
       auto release = [&](int b) {
         tc_fence_before();
         __syncwarp();
@@ -364,40 +364,55 @@ __global__ void __launch_bounds__(THREADS, 1)
       asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");  // column tables of this unit written
       if (!ok || errv) break;
       tc_fence_after();
-      const long long off = magic_sum(kb1 - kb0);
       const double mul = a.alpha;
       const bool scaled = !a.partial && !a.alpha_pow2;
       const uint32_t flip = (!a.partial && a.alpha_pow2 && a.alpha_neg) ? 0x80000000u : 0u;
       // value = (T 2^-36 + tail) 2^(EA + EB - 12), E = exps - 1022
-      const int sc0 = max(eA, 1) - 2 * 1022 - 12 - 36 + ((!a.partial && a.alpha_pow2) ? a.alpha_e : 0);
+      const int sc0 = (eA == 0 ? 1023 : eA) - 2 * 1022 - 12 - 36 + ((!a.partial && a.alpha_pow2) ? a.alpha_e : 0);
       const float ftail = __int_as_float((127 + 36 + a.fs) << 23);  // 2^(36 + fs)
       double *base = (a.partial ? a.partial : a.C) + rowOff;
       const int mode = (a.partial || a.beta == 0.0) ? 0 : (a.beta == 1.0 ? 1 : 2);
+      // Plain warps (every row and column inside the product, finite and of a scale that
+      // keeps results normal) skip the checks of each output: 42 instructions instead of 90.
+      auto fits = [](int e) { return e >= 640 && e <= 1400; };
+      const bool rok = fits(eA == 0 ? 1023 : eA) && sc0 >= -1500 && sc0 <= -600;
+      const bool cok = lane >= hc || (ctl.colOff[hc * h + lane] >= 0 && fits(ctl.colE[hc * h + lane]));
+      const bool plain = __all_sync(0xffffffffu, rok && cok) && !scaled && mode != 2;
+      auto finish = [&](auto is_plain) {
+        constexpr bool PLAIN = decltype(is_plain)::value;
 #pragma unroll
-      for (int j = 0; j < HC; j += 8) {
-        if (j >= hc) continue;
-        uint32_t r[8];
-        tmem_ld8(tl + (uint32_t)(TAIL * bn + j), r);
-        tmem_wait8(r);
-        double v[8];
+        for (int j = 0; j < HC; j += 8) {
+          if (j >= hc) continue;
+          uint32_t r[8];
+          tmem_ld8(tl + (uint32_t)(TAIL * bn + j), r);
+          int e[8];
+          long long co[8];
+          *reinterpret_cast<int4 *>(e) = *reinterpret_cast<const int4 *>(&ctl.colE[hc * h + j]);
+          *reinterpret_cast<int4 *>(e + 4) = *reinterpret_cast<const int4 *>(&ctl.colE[hc * h + j + 4]);
 #pragma unroll
-        for (int i = 0; i < 8; i++)
-          v[i] = slice_value(T[j + i] - off, rint_i32(__uint_as_float(r[i]) * ftail), a.fs,
-                             sc0 + ctl.colE[hc * h + j + i], flip);
-        if (scaled) {
+          for (int i = 0; i < 8; i += 2)
+            *reinterpret_cast<longlong2 *>(co + i) = *reinterpret_cast<const longlong2 *>(&ctl.colOff[hc * h + j + i]);
+          tmem_wait8(r);
 #pragma unroll
-          for (int i = 0; i < 8; i++) v[i] *= mul;
+          for (int i = 0; i < 8; i++) {
+            const int w = rint_i32(__uint_as_float(r[i]) * ftail);
+            double *p = base + co[i];
+            if (PLAIN) {
+              const double v = slice_value_plain(T[j + i], w, a.fs, sc0 + e[i], flip);
+              if (mode == 0) *p = v;
+              else asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+            } else if (co[i] >= 0 && eA != kRowNonFinite) {
+              double v = slice_value(T[j + i], w, a.fs, sc0 + e[i], flip);
+              if (scaled) v *= mul;
+              if (mode == 0) *p = v;
+              else if (mode == 1) asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+              else *p = fma(a.beta, *p, v);
+            }
+          }
         }
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const int64_t co = ctl.colOff[hc * h + j + i];
-          if (co < 0 || eA == kRowNonFinite) continue;
-          double *p = base + co;
-          if (mode == 0) *p = v[i];
-          else if (mode == 1) asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v[i]) : "memory");
-          else *p = fma(a.beta, *p, v[i]);
-        }
-      }
+      };
+      if (plain) finish(std::true_type{});
+      else finish(std::false_type{});
       release(TAIL);
     }
   }

@@ -86,10 +86,10 @@ SCESS_HD double power_of_two(int n) {
   return double_of(n < -1022 ? 1ull << (n + 1074) : (uint64_t)(n + 1023) << 52);
 }
 
-// (T + w 2^-fs) 2^sc rounded to FP64 (|T| < 2^62, 1 <= fs <= 31), its sign bit
-// xor-ed by flip unless it is zero.  A negative sum is complemented rather than
-// negated: one part in 2^32 of T's last place.
-SCESS_HD double slice_value(int64_t T, int w, int fs, int sc, uint32_t flip) {
+// (T + w 2^-fs) 2^sc rounded to FP64 (|T| < 2^62, 1 <= fs <= 31, -900 <= sc <= 800),
+// its sign bit xor-ed by flip unless it is zero.  A negative sum is complemented
+// rather than negated: one part in 2^32 of T's last place.
+SCESS_HD double slice_value_plain(int64_t T, int w, int fs, int sc, uint32_t flip) {
   const uint64_t H = (uint64_t)(T + (int64_t)(w >> fs));
   const uint32_t f = (uint32_t)w << (32 - fs);
   const uint32_t sgn = (uint32_t)((int64_t)H >> 63);
@@ -99,16 +99,19 @@ SCESS_HD double slice_value(int64_t T, int w, int fs, int sc, uint32_t flip) {
   const uint32_t a = m2 ? l : (m1 ? h0 : h1), b = m2 ? 0u : (m1 ? l : h0), c = m1 ? 0u : l;
   const int lz = clz32(a);
   const uint32_t x1 = funnel_l(a, b, lz & 31), x0 = funnel_l(b, c, lz & 31);
-  const int scc = sc < -900 ? -900 : (sc > 800 ? 800 : sc);
-  const int be = scc + 1023 + 63 - lz - (m1 ? 32 : 0) - (m2 ? 32 : 0);
+  const int be = sc + 1023 + 63 - lz - (m1 ? 32 : 0) - (m2 ? 32 : 0);
   // 53 bits of (x1, x0), the half bit rounded up; the carry runs into the exponent
   const uint64_t mant = ((((uint64_t)x1 << 32) | x0) >> 11) + ((x0 >> 10) & 1u);
-  double v = double_of(((uint64_t)(((uint32_t)(be - 1) << 20) + ((sgn & 0x80000000u) ^ flip)) << 32) + mant);
-  if (a == 0u) v = 0.0;
-  if (sc != scc) {  // beyond the normal numbers: one more rounding, to the place or to infinity
-    if (sc < scc) v = v * power_of_two(-100) * power_of_two(sc - scc + 100);
-    else v *= power_of_two(sc - scc);
-  }
+  const double v = double_of(((uint64_t)(((uint32_t)(be - 1) << 20) + ((sgn & 0x80000000u) ^ flip)) << 32) + mant);
+  return a == 0u ? 0.0 : v;
+}
+// The same for any sc.
+SCESS_HD double slice_value(int64_t T, int w, int fs, int sc, uint32_t flip) {
+  const int scc = sc < -900 ? -900 : (sc > 800 ? 800 : sc);
+  double v = slice_value_plain(T, w, fs, scc, flip);
+  // beyond the normal numbers: one more rounding, to the place or to infinity
+  if (sc < scc) v = v * power_of_two(-100) * power_of_two(sc - scc + 100);
+  else if (sc > scc) v *= power_of_two(sc - scc);
   return v;
 }
 
