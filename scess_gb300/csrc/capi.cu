@@ -172,6 +172,7 @@ int solve_common(scess_ctx *ctx, const double *eri, const double *B, int64_t nau
     in.eps_host = eps;
     in.f12_residual = f12_residual;
     in.f12_energy = f12_energy;
+    scess::HostPages pages(t2_out, nocc * nocc * v * v);  // (done long before the download)
     std::unique_ptr<scess::RccsdState> stp;
     if (B)  // DF: the integral blocks are contracted from B, no nmo^4 eri
       stp.reset(new scess::RccsdState(c, device_B(c, B, naux, nmo), naux, nmo, nocc, in, o));
@@ -365,6 +366,7 @@ static int triples_vjp_common(scess_ctx *ctx, const double *eri, const double *B
     scess::Control ctl;
     ctl.cancel = c.cancel;
     ctl.user = c.user;
+    scess::HostPages pe(g_eri, N4), pb(g_B, naux * N * N), p2(g_t2, n2);
     scess::DTensor d_eri({N, N, N, N}), dB;
     scess::Tape dfTape;
     if (eri) {
@@ -538,6 +540,8 @@ int scess_rccsd_state_amplitudes(scess_rccsd_state *state, double *t1_out, doubl
   if (!state || !state->impl) return SCESS_ERR_INVALID;
   return guard(state->ctx, [&](scess::Ctx &c) {
     const auto t0 = std::chrono::steady_clock::now();
+    const int64_t o = state->impl->nocc(), v = state->impl->nmo() - o;
+    scess::HostPages(t2_out, o * o * v * v).wait();
     state->impl->get_amplitudes(t1_out, t2_out);
     c.timer.host("amplitudes_download", ms_since(t0));
   });
@@ -650,6 +654,7 @@ static int residual_vjp_common(scess_ctx *ctx, const double *eri, const double *
       throw Error(SCESS_ERR_INVALID, "bad precision");
     const int64_t o = nocc, v = nmo - nocc, N = nmo, n1 = o * v, n2 = o * o * v * v;
     const int64_t N4 = N * N * N * N;
+    scess::HostPages pe(g_eri, N4), pb(g_B, naux * N * N), p2(g_t2, n2);
     scess::DTensor d_eri({N, N, N, N}), dB;
     scess::Tape dfTape;
     if (eri) {
@@ -835,6 +840,7 @@ int scess_transform_tei(scess_ctx *ctx, const double *tei, int64_t nao, const do
     const scess::Backend be =
         precision == SCESS_PRECISION_MIXED ? scess::Backend::TENSOR : scess::Backend::FP64;
     const int64_t n = nao, n4 = n * n * n * n;
+    scess::HostPages pages(out, na * nb * nc * nd);
     auto mat = [&](const double *h, int64_t cols, const char *name) {
       scess::DTensor m({n, cols});
       scess::upload(c, m.p(), h, n * cols);
@@ -858,8 +864,10 @@ int scess_transform_tei(scess_ctx *ctx, const double *tei, int64_t nao, const do
     if (chem_to_phys) {                                                // :57-59, pqrs -> prqs
       y = scess::DTensor({na, nc, nb, nd});
       scess::permute(c, "pqrs->prqs", 1.0, x.v, 0.0, y.v);
+      pages.wait();
       scess::download(c, out, y.p(), na * nb * nc * nd);
     } else {
+      pages.wait();
       scess::download(c, out, x.p(), na * nb * nc * nd);
     }
     if (precision == SCESS_PRECISION_MIXED) c.tensor_cores().check_error();
@@ -1009,6 +1017,7 @@ int scess_ccsd_so_solve(scess_ctx *ctx, const double *mo_eri, const double *eps,
     scess::Control ctl;
     ctl.cancel = c.cancel;
     ctl.user = c.user;
+    scess::HostPages pg(g_out, N * N * N * N);
     scess::DTensor g({N, N, N, N});
     {
       scess::DTensor chem = device_eri(c, mo_eri, nmo);
