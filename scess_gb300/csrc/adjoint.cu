@@ -356,7 +356,6 @@ LambdaResult rccsd_lambda(Ctx &ctx, const double *d_eri, const double *eps_host,
 
   const int maxv = std::max(1, opts.max_diis_vectors);
   DevMem dv((size_t)maxv * n * sizeof(double)), de((size_t)maxv * n * sizeof(double));
-  DevMem vecptr((size_t)maxv * sizeof(double *)), coefd((size_t)maxv * sizeof(double));
   std::deque<int> order;
   std::vector<std::vector<double>> gram;
   LambdaResult res;
@@ -380,8 +379,9 @@ LambdaResult rccsd_lambda(Ctx &ctx, const double *d_eri, const double *eps_host,
     axpby(n, -1.0, d_lambda, 1.0, ve, s);
     order.push_back(slot);
     const int nv = (int)order.size();
-    for (int q = 0; q < nv; q++)
-      dot(n, de.d() + (size_t)order[q] * n, ve, ctx.partials, ctx.dscalars + q, s);
+    std::vector<const double *> hp(nv);
+    for (int q = 0; q < nv; q++) hp[q] = de.d() + (size_t)order[q] * n;
+    dots(n, hp.data(), nv, ve, ctx.partials, ctx.dscalars, s);
     SCESS_CUDA(cudaMemcpyAsync(ctx.hscalars, ctx.dscalars, nv * sizeof(double), cudaMemcpyDeviceToHost, s));
     ctx.sync();
     for (int q = 0; q < nv - 1; q++) gram[q].push_back(ctx.hscalars[q]);
@@ -389,12 +389,8 @@ LambdaResult rccsd_lambda(Ctx &ctx, const double *d_eri, const double *eps_host,
     const double rms = std::sqrt(ctx.hscalars[nv - 1] / (double)n);
     if (it >= opts.diis_start) {
       std::vector<double> c = diis_coefficients(gram);
-      std::vector<const double *> hp(nv);
       for (int q = 0; q < nv; q++) hp[q] = dv.d() + (size_t)order[q] * n;
-      SCESS_CUDA(cudaMemcpyAsync(vecptr.as<void>(), hp.data(), nv * sizeof(double *), cudaMemcpyHostToDevice, s));
-      SCESS_CUDA(cudaMemcpyAsync(coefd.d(), c.data(), nv * sizeof(double), cudaMemcpyHostToDevice, s));
-      linear_combination(n, nv, vecptr.as<const double *>(), coefd.d(), d_lambda, s);
-      ctx.sync();
+      linear_combination(n, nv, hp.data(), c.data(), d_lambda, s);
     } else {
       SCESS_CUDA(cudaMemcpyAsync(d_lambda, lnew.p(), n * sizeof(double), cudaMemcpyDeviceToDevice, s));
     }

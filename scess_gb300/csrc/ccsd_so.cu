@@ -302,8 +302,9 @@ SoResult so_ccsd(Ctx &ctx, const double *d_g, const double *d_eps, int64_t nmo, 
       axpby(n, -1.0, prev.p(), 1.0, ve, s);
       order.push_back(slot);
       const int m = (int)order.size();
-      for (int q = 0; q < m; q++)
-        dot(n, verr.d() + (size_t)order[q] * n, ve, ctx.partials, ctx.dscalars + q, s);
+      std::vector<const double *> hp(m);
+      for (int q = 0; q < m; q++) hp[q] = verr.d() + (size_t)order[q] * n;
+      dots(n, hp.data(), m, ve, ctx.partials, ctx.dscalars, s);
       SCESS_CUDA(cudaMemcpyAsync(ctx.hscalars, ctx.dscalars, m * sizeof(double),
                                  cudaMemcpyDeviceToHost, s));
       ctx.sync();
@@ -330,13 +331,8 @@ SoResult so_ccsd(Ctx &ctx, const double *d_g, const double *d_eps, int64_t nmo, 
         rhs[k] = -1.0;
         std::vector<double> c = partial_piv_lu_solve(B, rhs, k + 1);
         c.resize(k);
-        std::vector<const double *> hp(k);
         for (int q = 0; q < k; q++) hp[q] = vamp.d() + (size_t)order[q] * n;
-        SCESS_CUDA(cudaMemcpyAsync(vptr.as<void>(), hp.data(), k * sizeof(double *),
-                                   cudaMemcpyHostToDevice, s));
-        SCESS_CUDA(cudaMemcpyAsync(vcoef.d(), c.data(), k * sizeof(double), cudaMemcpyHostToDevice, s));
-        linear_combination(n, k, vptr.as<const double *>(), vcoef.d(), amp.p(), s);
-        ctx.sync();  // hp / c are host buffers of this scope
+        linear_combination(n, k, hp.data(), c.data(), amp.p(), s);
       }
     }
     E = so_energy(ctx, goovv, amp.p(), o, v, xe);                                  // :161-165

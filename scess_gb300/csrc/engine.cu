@@ -173,9 +173,9 @@ Ctx::Ctx(int dev) : device(dev) {
                                            "); this library is built for sm_103a (GB300)");
   SCESS_CUDA(cudaSetDevice(dev));
   SCESS_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-  scratch.alloc((kDotBlocks + 64) * sizeof(double));
+  scratch.alloc((kDotVectors * kDotBlocks + 64) * sizeof(double));
   partials = scratch.d();
-  dscalars = partials + kDotBlocks;
+  dscalars = partials + kDotVectors * kDotBlocks;
   SCESS_CUDA(cudaMallocHost(&hscalars, 64 * sizeof(double)));
   counters.alloc(kSmallCounters * sizeof(int));
   SCESS_CUDA(cudaMemsetAsync(counters.as<void>(), 0, kSmallCounters * sizeof(int), stream));
@@ -549,9 +549,17 @@ const EinsumPlan &plan_einsum(Ctx &ctx, const char *spec, const TV &A, const TV 
 }
 
 namespace {
-// C = alpha A.B + beta C on the FP64 units.
+// Whether the sliced form is usable and faster than the FP64 units (estimates of both;
+// tuning key f64: 1 = sliced, 2 = FP64 units).
+bool prefer_slices(const TableGemm &g) {
+  const int64_t route = tune_value("f64", 0);
+  if (route == 1) return g.K > 0 && SliceEngine::usable(g.M, g.N);
+  return route != 2 && g.K > 0 && SliceEngine::usable(g.M, g.N) && SliceEngine::estimate_us(g.M, g.N, g.K) < dgemm_small_us(g);
+}
+
+// C = alpha A.B + beta C on the FP64 units: cut finely unless that takes too many CTAs.
 void dfma_gemm(Ctx &ctx, const TableGemm &g) {
-  if (dgemm_small_ok(g)) {
+  if (g.K > 0 && dgemm_small_us(g) < 2000.0) {
     TimedScope ts(ctx.timer, "dgemm_small", 2.0 * g.M * g.N * g.K, 0.0, ctx.stream);
     dgemm_small(g, ctx.ensure_workspace(dgemm_small_workspace(g)), ctx.counters.as<int>(), ctx.stream);
     return;
@@ -641,14 +649,14 @@ void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, 
     dgemv_table(h, ctx.stream);
     return;
   }
-  if (!dgemm_small_ok(g) && SliceEngine::usable(pl.M, pl.N) &&
+  if (prefer_slices(g) &&
       ctx.slice_engine().contract(pl, alpha, A.p, B.p, beta, C.p, constA, constB))
     return;
   dfma_gemm(ctx, g);
 }
 
 void fp64_table_gemm(Ctx &ctx, const TableGemm &g, const char *name) {
-  if (!dgemm_small_ok(g) && SliceEngine::usable(g.M, g.N) && ctx.slice_engine().table_gemm(g, name))
+  if (prefer_slices(g) && ctx.slice_engine().table_gemm(g, name))
     return;
   dfma_gemm(ctx, g);
 }

@@ -39,7 +39,8 @@ class BlockCache {
 // variable SCESS_TUNE holds "key=value" pairs separated by commas, read at
 // every call.  Keys: t_nb (virtual block size of (T), both forms; default: the
 // size chosen from o and v), t_kbd (K blocks of 64 per TMEM drain in the
-// mixed (T) launch: 1, 2 or 4) and t_wbuf (W buffers of the mixed (T): 1 or 3).
+// mixed (T) launch: 1, 2 or 4), t_wbuf (W buffers of the mixed (T): 1 or 3) and f64
+// (FP64 products: 1 on the tensor cores' slices, 2 on the FP64 units).
 // Returns `def` for an unset key.
 int64_t tune_value(const char *key, int64_t def);
 // TMEM drain cadence of the mixed (T) launch (K blocks of 64 per drain).
@@ -247,7 +248,7 @@ struct Ctx {
 };
 
 // C = alpha A.B + beta C in FP64 through the tables of g: small products on the
-// FP64 units (dgemm_small_ok), the others on the tensor cores' exact slices.
+// FP64 units, the others on the tensor cores' exact slices.
 void fp64_table_gemm(Ctx &ctx, const TableGemm &g, const char *name);
 
 // FP64: DFMA engine.  MIXED: tensor cores for contractions large enough to pay

@@ -676,6 +676,46 @@ SliceEngine::SliceEngine(Ctx &ctx) : ctx_(ctx) {
 
 int SliceEngine::tile_n(int64_t N) { return (int)round_up(ceil_div(N, ceil_div(N, BN)), 8 * EPI); }
 
+namespace {
+// Cycles an SM spends on one K block of a unit of bn columns: 56 MMAs (no faster than 40
+// cycles each: issue and the A reads) and the fill of the stage share the shared-memory
+// port, about 10 % is lost between them.
+double block_cycles(int bn) {
+  return 1.1 * (56.0 * std::max(40.0, bn / 2.0) + kSlices * (BM + bn) * 64.0 / 70.0) + 500.0;
+}
+
+// Split-K of a product and its estimated time in us.  Rounds of units over the SMs times
+// the K blocks of a unit; a unit's epilogue costs about 90 cycles a column, partial sums
+// are written and read again at 5 TB/s, their reduction is one more launch (4 us).
+// (9870 x 136 x 9870: 156 tiles take two rounds of 309 blocks; 19 splits take 20 of 17.)
+// A unit's K is at most what its 64-bit sums hold.
+double plan_us(int64_t M, int64_t N, int64_t Kpad, int64_t &splits) {
+  const int bn = SliceEngine::tile_n(N);
+  const int64_t nkb = ceil_div(Kpad, BK), tiles = ceil_div(M, BM) * ceil_div(N, bn);
+  const double blk = block_cycles(bn) / 1900.0, epi = 90.0 * bn / 1900.0;
+  const int64_t least = ceil_div(nkb, 512);
+  const int64_t most = std::min<int64_t>(nkb / 2, std::max<int64_t>(64, ceil_div(2 * kNumSMs, tiles)));
+  double best = 1e300;
+  splits = least;
+  for (int64_t z = least; z <= std::max(least, most); z++) {
+    if (z > least && z * M * N > (int64_t(64) << 20)) break;
+    double us = (double)ceil_div(tiles * z, kNumSMs) * ((double)ceil_div(nkb, z) * blk + epi);
+    if (z > 1) us += 4.0 + (double)z * M * N * 16.0 / 5.0e6;
+    if (us < 0.97 * best) {
+      best = us;
+      splits = z;
+    }
+  }
+  return best;
+}
+}  // namespace
+
+double SliceEngine::estimate_us(int64_t M, int64_t N, int64_t K) {
+  int64_t z = 1;
+  // packs at 2.5 TB/s, 14 us of launches and latencies
+  return 14.0 + (double)(M + N) * (double)K * 22.0 / 2.5e6 + plan_us(M, N, round_up(std::max<int64_t>(K, 1), BK), z);
+}
+
 bool SliceEngine::usable(int64_t M, int64_t N) {
   return kernel_ok() && M <= INT32_MAX / 2 && N <= INT32_MAX / 2;
 }
@@ -900,24 +940,8 @@ void SliceEngine::gemm(const SlicedPack &A, const SlicedPack &B, double alpha, d
   SliceProblemSet ps;
   ps.M = A.rows;
   ps.N = B.rows;
-  const int64_t nkb = A.Kpad / BK, tiles = ceil_div(ps.M, BM) * ceil_div(ps.N, tile_n(ps.N));
-  // Split K where it shortens the launch: rounds of units over the SMs times the K
-  // blocks of a unit, in units of one K block (2.8 us): a unit's epilogue costs about
-  // 1.5, partial sums are written and read again at 5 TB/s, their reduction is one more
-  // launch (1.5).  (9870 x 136 x 9870: 156 tiles take two rounds of 309 blocks; 19 splits
-  // take 20 of 17.)  A unit's K is at most what its 64-bit sums hold.
-  int64_t splits = ceil_div(nkb, 512);
-  double best = 1e300;
-  const int64_t most = std::min<int64_t>(nkb / 2, std::max<int64_t>(64, ceil_div(2 * kNumSMs, tiles)));
-  for (int64_t z = splits; z <= std::max(splits, most); z++) {
-    if (z > splits && z * ps.M * ps.N > (int64_t(64) << 20)) break;
-    double cost = (double)ceil_div(tiles * z, kNumSMs) * ((double)ceil_div(nkb, z) + 1.5);
-    if (z > 1) cost += 1.5 + (double)z * ps.M * ps.N * 16.0 / 5.0e12 / 2.8e-6;
-    if (cost < 0.97 * best) {
-      best = cost;
-      splits = z;
-    }
-  }
+  int64_t splits = 1;
+  plan_us(ps.M, ps.N, A.Kpad, splits);
   double *partial = nullptr;
   if (splits > 1) {
     const size_t need = (size_t)splits * ps.M * ps.N * sizeof(double);

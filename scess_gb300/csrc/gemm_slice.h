@@ -76,6 +76,8 @@ class SliceEngine {
   explicit SliceEngine(Ctx &ctx);
   // The device runs the kernel and the sizes are within its coordinates.
   static bool usable(int64_t M, int64_t N);
+  // Estimated time of a product with its packs, in us.
+  static double estimate_us(int64_t M, int64_t N, int64_t K);
   // C = alpha A.B + beta C through the tables of g (the FP64 engine's GEMM).
   // False when the packs do not fit into device memory: nothing was launched
   // and the caller uses the DFMA kernel.

@@ -62,62 +62,69 @@ namespace {
 
 // Small FP64 contraction: GB300 issues about two FP64 lanes per cycle and SM, so one
 // 64 x 64 x 16 step of dgemm_table_kernel takes an SM 18 us.  Small products are
-// therefore cut finely over the whole device: 8 x 8 outputs a CTA, K in ranges of
-// at most kSmallKB staged at once (two dependent loads, then arithmetic), the four
-// 64-thread groups taking every fourth k.  With several K ranges per tile the last
-// CTA of the tile to finish adds the partial sums in order (deterministic) and
-// leaves the tile's counter at zero.  90 x 10 x 90: 107 -> 4 us.
-constexpr int kSmallT = 8, kSmallKB = 128;
-__global__ void __launch_bounds__(256) dgemm_small_kernel(TableGemm g, int64_t kper, int splits,
+// therefore cut finely over the whole device: up to 64 outputs a CTA (tm x tn, chosen
+// for the least padding), K in ranges of at most kSmallKB staged at once (two dependent
+// loads, then arithmetic), the four 64-thread groups taking every fourth k.  With
+// several K ranges per tile the last CTA of the tile to finish adds the partial sums in
+// order (deterministic) and leaves the tile's counter at zero.  90 x 10 x 90:
+// 107 -> 4 us; 10 x 10 x 81000: 134 us on the tensor cores' slices (packs included), 47 here.
+constexpr int kSmallOut = 64, kSmallKB = 128, kSmallSide = 16;
+__global__ void __launch_bounds__(256) dgemm_small_kernel(TableGemm g, int64_t kper, int splits, int tm, int tn,
                                                           double *__restrict__ partial,
                                                           int *__restrict__ counters) {
-  __shared__ double As[kSmallKB][kSmallT + 1], Bs[kSmallKB][kSmallT + 1];
-  __shared__ double red[4][64];
+  __shared__ double As[kSmallKB][kSmallSide + 1], Bs[kSmallKB][kSmallSide + 1];
+  __shared__ double red[4][kSmallOut];
   __shared__ int last;
-  const int t = threadIdx.x, grp = t >> 6, o = t & 63, i = o & 7, j = o >> 3;
-  const int64_t tm = (g.M + kSmallT - 1) / kSmallT;
+  const int t = threadIdx.x, grp = t >> 6, o = t & 63, i = o % tm, j = o / tm;
+  const int im = 65536 / tm + 1, in = 65536 / tn + 1;  // (exact for e below 4096)
+  const int64_t ntm = (g.M + tm - 1) / tm;
   const int64_t tile = blockIdx.x / splits, z = blockIdx.x % splits;
-  const int64_t m0 = (tile % tm) * kSmallT, n0 = (tile / tm) * kSmallT;
+  const int64_t m0 = (tile % ntm) * tm, n0 = (tile / ntm) * tn;
   const int64_t kb = z * kper, ke = min(g.K, kb + kper);
+  const bool out = j < tn && m0 + i < g.M && n0 + j < g.N;
   double acc = 0.0;
   for (int64_t k0 = kb; k0 < ke; k0 += kSmallKB) {
     const int nk = (int)min((int64_t)kSmallKB, ke - k0);
-    int64_t ra[4], rb[4];
-    double a[4], b[4];
-    // along the operand's unit-stride side, eight rows / columns of up to 128 k
-#pragma unroll
-    for (int p = 0; p < 4; p++) {
-      const int e = t + 256 * p;
-      const int am = g.aUnitM ? e & 7 : e >> 7, ak = g.aUnitM ? e >> 3 : e & 127;
-      const int bm = g.bUnitN ? e & 7 : e >> 7, bk = g.bUnitN ? e >> 3 : e & 127;
-      ra[p] = (m0 + am < g.M && ak < nk) ? g.rowA[m0 + am] + g.kA[k0 + ak] : -1;
-      rb[p] = (n0 + bm < g.N && bk < nk) ? g.colB[n0 + bm] + g.kB[k0 + bk] : -1;
-    }
-#pragma unroll
-    for (int p = 0; p < 4; p++) {
-      a[p] = ra[p] >= 0 ? g.A[g.baseA + ra[p]] : 0.0;
-      b[p] = rb[p] >= 0 ? g.B[g.baseB + rb[p]] : 0.0;
-    }
     __syncthreads();  // the previous range is used up
+    // element e of a side: along its unit-stride index, else along k
+    for (int e0 = t; e0 < max(tm, tn) * kSmallKB; e0 += 4 * 256) {
+      int64_t ra[4], rb[4];
+      double a[4], b[4];
 #pragma unroll
-    for (int p = 0; p < 4; p++) {
-      const int e = t + 256 * p;
-      if (g.aUnitM) As[e >> 3][e & 7] = a[p];
-      else As[e & 127][e >> 7] = a[p];
-      if (g.bUnitN) Bs[e >> 3][e & 7] = b[p];
-      else Bs[e & 127][e >> 7] = b[p];
+      for (int p = 0; p < 4; p++) {
+        const int e = e0 + 256 * p;
+        const int qm = (e * im) >> 16, qn = (e * in) >> 16;  // e / tm, e / tn
+        const int am = g.aUnitM ? e - qm * tm : e >> 7, ak = g.aUnitM ? qm : e & 127;
+        const int bm = g.bUnitN ? e - qn * tn : e >> 7, bk = g.bUnitN ? qn : e & 127;
+        ra[p] = (am < tm && m0 + am < g.M && ak < nk) ? g.rowA[m0 + am] + g.kA[k0 + ak] : -1;
+        rb[p] = (bm < tn && n0 + bm < g.N && bk < nk) ? g.colB[n0 + bm] + g.kB[k0 + bk] : -1;
+      }
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        a[p] = ra[p] >= 0 ? g.A[g.baseA + ra[p]] : 0.0;
+        b[p] = rb[p] >= 0 ? g.B[g.baseB + rb[p]] : 0.0;
+      }
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const int e = e0 + 256 * p;
+        const int qm = (e * im) >> 16, qn = (e * in) >> 16;  // e / tm, e / tn
+        const int am = g.aUnitM ? e - qm * tm : e >> 7, ak = g.aUnitM ? qm : e & 127;
+        const int bm = g.bUnitN ? e - qn * tn : e >> 7, bk = g.bUnitN ? qn : e & 127;
+        if (am < tm && ak < nk) As[ak][am] = a[p];
+        if (bm < tn && bk < nk) Bs[bk][bm] = b[p];
+      }
     }
     __syncthreads();
-    if (m0 + i < g.M && n0 + j < g.N)
+    if (out)
       for (int k = grp; k < nk; k += 4) acc = fma(As[k][i], Bs[k][j], acc);
   }
   red[grp][o] = acc;
   __syncthreads();
   double s = 0.0;
-  if (t < 64) s = (red[0][t] + red[1][t]) + (red[2][t] + red[3][t]);
+  if (t < kSmallOut) s = (red[0][t] + red[1][t]) + (red[2][t] + red[3][t]);
   if (splits > 1) {
-    double *p = partial + tile * splits * 64;
-    if (t < 64) p[z * 64 + t] = s;
+    double *p = partial + tile * splits * kSmallOut;
+    if (t < kSmallOut) p[z * kSmallOut + t] = s;
     __threadfence();
     __syncthreads();
     if (t == 0) last = atomicAdd(&counters[tile], 1) == splits - 1;
@@ -125,13 +132,13 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(TableGemm g, int64_t k
     if (!last) return;
     __threadfence();
     double v = 0.0;
-    for (int q = grp; q < splits; q += 4) v += __ldcg(p + q * 64 + o);
+    for (int q = grp; q < splits; q += 4) v += __ldcg(p + q * kSmallOut + o);
     red[grp][o] = v;
     __syncthreads();
-    if (t < 64) s = (red[0][t] + red[1][t]) + (red[2][t] + red[3][t]);
+    if (t < kSmallOut) s = (red[0][t] + red[1][t]) + (red[2][t] + red[3][t]);
     if (t == 0) counters[tile] = 0;
   }
-  if (t < 64 && m0 + i < g.M && n0 + j < g.N) {
+  if (t < kSmallOut && out) {
     const int64_t off = g.baseC + g.rowC[m0 + i] + g.colC[n0 + j];
     double val = g.alpha * s;
     if (g.beta != 0.0) val += g.beta * g.C[off];
@@ -140,12 +147,24 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(TableGemm g, int64_t k
 }
 
 struct SmallShape {
-  int64_t tiles, kper;
-  int splits;
+  int tm = 8, tn = 8, splits = 1;
+  int64_t tiles = 0, kper = 0;
 };
 SmallShape small_shape(const TableGemm &g) {
   SmallShape s;
-  s.tiles = ceil_div(g.M, kSmallT) * ceil_div(g.N, kSmallT);
+  // the tile with the fewest padded outputs (whole warps of 32), then the fewest tiles
+  int64_t best = INT64_MAX;
+  for (int tm = 4; tm <= kSmallSide; tm++) {
+    const int tn = std::min(kSmallOut / tm, kSmallSide);
+    const int64_t tiles = ceil_div(g.M, tm) * ceil_div(g.N, tn);
+    const int64_t cost = tiles * round_up(tm * tn, 32) * 1024 + std::min<int64_t>(tiles, 1023);
+    if (cost < best) {
+      best = cost;
+      s.tm = tm;
+      s.tn = tn;
+      s.tiles = tiles;
+    }
+  }
   // about two CTAs an SM, at least 16 k each; a range beyond 128 k is walked in steps
   const int64_t want = s.tiles >= 2 * kNumSMs ? 1 : ceil_div(2 * kNumSMs, s.tiles);
   const int64_t n = std::max<int64_t>(1, std::min(want, ceil_div(g.K, 16)));
@@ -198,22 +217,25 @@ __global__ void __launch_bounds__(256) dgemv_table_kernel(TableGemm g) {
 }
 }  // namespace
 
-bool dgemm_small_ok(const TableGemm &g) {
-  // padded to whole 8 x 8 tiles: 6e6 multiply-adds take the device's FP64 units 10 us,
-  // what the packs and launches of the sliced form (gemm_slice.h) take at least
-  const double fma = (double)round_up(g.M, kSmallT) * (double)round_up(g.N, kSmallT) * (double)g.K;
-  // (many outputs of a short K: the 8 x 8 tiles' own overhead, 1805 x 475 x 5 takes 50 us)
-  return g.M > 0 && g.N > 0 && g.K > 0 && fma <= 6.0e6 && g.M * g.N <= (1 << 17);
+double dgemm_small_us(const TableGemm &g) {
+  if (g.M <= 0 || g.N <= 0 || g.K <= 0) return 1e30;
+  const SmallShape s = small_shape(g);
+  if ((double)s.tiles * s.splits > 2.0e9) return 1e30;
+  // 4 us of latency, padded multiply-adds at two lanes a cycle and SM, 2.5 us for every
+  // six CTAs of an SM
+  const double fma = (double)s.tiles * (double)round_up(s.tm * s.tn, 32) * (double)g.K;
+  return 4.0 + fma / (2.0 * kNumSMs * 1900.0) + 2.5 * (double)(s.tiles * s.splits) / (6.0 * kNumSMs);
 }
 
 int64_t dgemm_small_workspace(const TableGemm &g) {
   const SmallShape s = small_shape(g);
-  return s.splits > 1 ? s.tiles * s.splits * 64 : 0;
+  return s.splits > 1 ? s.tiles * s.splits * kSmallOut : 0;
 }
 
 void dgemm_small(const TableGemm &g, double *workspace, int *counters, cudaStream_t stream) {
   const SmallShape s = small_shape(g);
-  dgemm_small_kernel<<<(unsigned)(s.tiles * s.splits), 256, 0, stream>>>(g, s.kper, s.splits, workspace, counters);
+  dgemm_small_kernel<<<(unsigned)(s.tiles * s.splits), 256, 0, stream>>>(g, s.kper, s.splits, s.tm, s.tn, workspace,
+                                                                         counters);
   SCESS_CHECK_LAUNCH();
 }
 
@@ -616,12 +638,24 @@ __global__ void dot_partial_kernel(int64_t n, const double *__restrict__ x,
   if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 
+// Dots of nv vectors xs[q] with y, one per blockIdx.y: each is dot_partial_kernel's sum.
+__global__ void dots_partial_kernel(int64_t n, DotVectors xs, const double *__restrict__ y,
+                                    double *__restrict__ partials) {
+  const double *__restrict__ x = xs.p[blockIdx.y];
+  double s = 0.0;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
+       e += (int64_t)gridDim.x * blockDim.x)
+    s = fma(x[e], y[e], s);
+  s = block_sum(s);
+  if (threadIdx.x == 0) partials[blockIdx.y * gridDim.x + blockIdx.x] = s;
+}
+
 __global__ void sum_partials_kernel(int np, const double *__restrict__ partials,
                                     double *__restrict__ result) {
   double s = 0.0;
-  for (int e = threadIdx.x; e < np; e += blockDim.x) s += partials[e];
+  for (int e = threadIdx.x; e < np; e += blockDim.x) s += partials[(int64_t)blockIdx.x * np + e];
   s = block_sum(s);
-  if (threadIdx.x == 0) result[0] = s;
+  if (threadIdx.x == 0) result[blockIdx.x] = s;
 }
 
 __global__ void tau_energy_partial_kernel(int64_t o, int64_t v, const double *__restrict__ L,
@@ -681,12 +715,11 @@ __global__ void pair_asymmetry_kernel(const double *__restrict__ x, Ext4 n, Ext4
   }
 }
 
-__global__ void lincomb_kernel(int64_t n, int nv, const double *const *__restrict__ vecs,
-                               const double *__restrict__ coef, double *__restrict__ out) {
+__global__ void lincomb_kernel(int64_t n, int nv, LinComb lc, bool first, double *__restrict__ out) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int c = 0; c < nv; c++) s += coef[c] * vecs[c][e];
+    double s = first ? 0.0 : out[e];
+    for (int c = 0; c < nv; c++) s += lc.coef[c] * lc.p[c][e];
     out[e] = s;
   }
 }
@@ -768,10 +801,31 @@ void dot(int64_t n, const double *x, const double *y, double *partials, double *
   SCESS_CHECK_LAUNCH();
 }
 
+void dots(int64_t n, const double *const *xs, int nv, const double *y, double *partials, double *result,
+          cudaStream_t stream) {
+  for (int q0 = 0; q0 < nv; q0 += kDotVectors) {
+    DotVectors v{};
+    const int m = std::min(kDotVectors, nv - q0);
+    for (int q = 0; q < m; q++) v.p[q] = xs[q0 + q];
+    dots_partial_kernel<<<dim3(kDotBlocks, (unsigned)m), 256, 0, stream>>>(n, v, y, partials);
+    SCESS_CHECK_LAUNCH();
+    sum_partials_kernel<<<(unsigned)m, 1024, 0, stream>>>(kDotBlocks, partials, result + q0);
+    SCESS_CHECK_LAUNCH();
+  }
+}
+
 void linear_combination(int64_t n, int nv, const double *const *vecs, const double *coef,
                         double *out, cudaStream_t stream) {
-  lincomb_kernel<<<grid_for(n), 256, 0, stream>>>(n, nv, vecs, coef, out);
-  SCESS_CHECK_LAUNCH();
+  for (int c0 = 0; c0 < nv; c0 += kDotVectors) {
+    LinComb lc{};
+    const int m = std::min(kDotVectors, nv - c0);
+    for (int c = 0; c < m; c++) {
+      lc.p[c] = vecs[c0 + c];
+      lc.coef[c] = coef[c0 + c];
+    }
+    lincomb_kernel<<<grid_for(n), 256, 0, stream>>>(n, m, lc, c0 == 0, out);
+    SCESS_CHECK_LAUNCH();
+  }
 }
 
 void tau_energy(int64_t o, int64_t v, const double *L, const double *t1, const double *t2,

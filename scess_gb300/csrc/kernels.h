@@ -33,11 +33,11 @@ struct TableGemm {
 constexpr int kSkinnyMaxK = 32, kSkinnyMaxS = 256;
 void skinny_table(const TableGemm &g, bool small_is_a, bool stage, cudaStream_t stream);
 
-// The same contraction for products of at most about 6e6 multiply-adds, cut finely
-// over the device (dgemm_small_ok); workspace of dgemm_small_workspace doubles for
-// the K ranges' partial sums, counters: kSmallCounters zeroed ints (left zero).
+// The same contraction for small products, cut finely over the device; workspace of
+// dgemm_small_workspace doubles for the K ranges' partial sums, counters: kSmallCounters
+// zeroed ints (left zero).  dgemm_small_us: estimated time in us.
 constexpr int kSmallCounters = 1024;
-bool dgemm_small_ok(const TableGemm &g);
+double dgemm_small_us(const TableGemm &g);
 int64_t dgemm_small_workspace(const TableGemm &g);
 void dgemm_small(const TableGemm &g, double *workspace, int *counters, cudaStream_t stream);
 
@@ -100,7 +100,19 @@ void axpby(int64_t n, double a, const double *x, double b, double *y, cudaStream
 void dot(int64_t n, const double *x, const double *y, double *partials, double *result,
          cudaStream_t stream);
 constexpr int kDotBlocks = 608;   // 4 x 152 SMs
-// out = sum_c coef[c] * vecs[c] for nv vectors of length n (coef on device).
+// result[q] = xs[q] . y for nv vectors (host array of device pointers), each as dot() gives
+// it, in one launch pair per kDotVectors; partials: kDotVectors kDotBlocks doubles.
+constexpr int kDotVectors = 16;
+struct DotVectors {
+  const double *p[kDotVectors];
+};
+void dots(int64_t n, const double *const *xs, int nv, const double *y, double *partials, double *result,
+          cudaStream_t stream);
+struct LinComb {
+  const double *p[kDotVectors];
+  double coef[kDotVectors];
+};
+// out = sum_c coef[c] * vecs[c] for nv vectors of length n (vecs and coef on the host; out none of them).
 void linear_combination(int64_t n, int nv, const double *const *vecs, const double *coef,
                         double *out, cudaStream_t stream);
 // result[0] = sum L(i,j,a,b) * (t2 + t1 t1)(i,j,a,b)  (CorrelationEnergy) deterministic

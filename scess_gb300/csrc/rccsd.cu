@@ -596,8 +596,6 @@ void RccsdState::init(const SolveInput &in, const scess_rccsd_options &opts) {
   maxv_ = std::max(1, opts.max_diis_vectors);
   diis_amp_.alloc((size_t)maxv_ * n_ * sizeof(double));
   diis_err_.alloc((size_t)maxv_ * n_ * sizeof(double));
-  vecptr_.alloc((size_t)maxv_ * sizeof(double *));
-  coefd_.alloc((size_t)(maxv_ + 1) * sizeof(double));
   w_.alloc(o, v, false);
   phase_ = mixed_ ? Phase::MIXED : Phase::FP64;
   std::memset(&res_, 0, sizeof(res_));
@@ -733,8 +731,9 @@ bool RccsdState::iterate(int max_steps, const Control &ctl) {
     axpby(n_, -1.0, prev_.p(), 1.0, ve, s);                                           // :352
     order_.push_back(slot);
     const int nv = (int)order_.size();
-    for (int q = 0; q < nv; q++)
-      dot(n_, diis_err_.d() + (size_t)order_[q] * n_, ve, ctx_.partials, ctx_.dscalars + q, s);
+    std::vector<const double *> vecs(nv);
+    for (int q = 0; q < nv; q++) vecs[q] = diis_err_.d() + (size_t)order_[q] * n_;
+    dots(n_, vecs.data(), nv, ve, ctx_.partials, ctx_.dscalars, s);
     SCESS_CUDA(cudaMemcpyAsync(ctx_.hscalars, ctx_.dscalars, nv * sizeof(double),
                                cudaMemcpyDeviceToHost, s));
     ctx_.sync();
@@ -744,13 +743,8 @@ bool RccsdState::iterate(int max_steps, const Control &ctl) {
     if (it_ - phase_start_ >= opts_.diis_start) {                                    // :354-357
       if (it_ - phase_start_ == opts_.diis_start) ctx_.logf(1, "Turning on DIIS");
       std::vector<double> c = diis_coefficients(gram_);
-      std::vector<const double *> hptr(nv);
-      for (int q = 0; q < nv; q++) hptr[q] = diis_amp_.d() + (size_t)order_[q] * n_;
-      SCESS_CUDA(cudaMemcpyAsync(vecptr_.as<void>(), hptr.data(), nv * sizeof(double *),
-                                 cudaMemcpyHostToDevice, s));
-      SCESS_CUDA(cudaMemcpyAsync(coefd_.d(), c.data(), nv * sizeof(double), cudaMemcpyHostToDevice, s));
-      linear_combination(n_, nv, vecptr_.as<const double *>(), coefd_.d(), amp_.p(), s);
-      ctx_.sync();  // hptr / c are host buffers of this scope
+      for (int q = 0; q < nv; q++) vecs[q] = diis_amp_.d() + (size_t)order_[q] * n_;
+      linear_combination(n_, nv, vecs.data(), c.data(), amp_.p(), s);
     }
     const double E = energy_of_amplitudes();                                          // :361
     const double dE = std::fabs(E - E_last_);                                         // :362

@@ -137,7 +137,7 @@ class RccsdState {
   int symmetric_ = -1;  // FP64: inputs_symmetric() of the amplitudes set last (-1: not yet known)
   DTensor eps_, amp_, prev_, R_, drv_, Lf12_;
   int maxv_ = 8;
-  DevMem diis_amp_, diis_err_, vecptr_, coefd_;
+  DevMem diis_amp_, diis_err_;
   RccsdWork w_;
   std::deque<int> order_;  // DIIS slots, oldest first
   std::vector<std::vector<double>> gram_;

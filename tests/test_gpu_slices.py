@@ -1,10 +1,9 @@
 """FP64 contractions: on the tensor cores' exact BF16 slices (SliceEngine) and, for
-small products, on the FP64 units.
+small products, on the FP64 units; the tuning key f64 selects either for any size.
 
-Sizes sit where the kernel can go wrong: tiles of 128 x 128 and K blocks of 32
+Sizes sit where the kernels can go wrong: tiles of 128 x 128 and K blocks of 32
 with remainders, one narrow side, K beyond what one unit's integer sum takes
-(16384: split), few tiles (split K) and many.  Every contraction is above the
-6e6 multiply-adds from which the engine is used.
+(16384: split), few tiles (split K) and many.
 
 Tolerance: an output is one rounding of a sum whose operands are cut 60 bits
 below their row's largest value and whose products below 2^-63 of
@@ -19,7 +18,12 @@ from tests.gpu_common import gctx  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(129, 128, 1217), (128, 127, 1300), (2000, 17, 600), (8, 4001, 700), (1025, 641, 33),
+@pytest.fixture
+def sliced(monkeypatch):
+    monkeypatch.setenv('SCESS_TUNE', 'f64=1')
+
+
+SHAPES = [(1, 1, 1), (3, 2, 5), (129, 128, 1217), (128, 127, 1300), (2000, 17, 600), (8, 4001, 700), (1025, 641, 33),
           (600, 520, 65), (300, 31, 16401), (24, 24, 36000), (2111, 1301, 8)]
 
 
@@ -31,7 +35,7 @@ def reference(A, B):
 
 
 @pytest.mark.parametrize('M,N,K', SHAPES)
-def test_integers_are_exact(gctx, M, N, K):
+def test_integers_are_exact(gctx, sliced, M, N, K):
     rng = np.random.default_rng(M + N + K)
     lim = 1 << 18
     A = rng.integers(-lim, lim + 1, (M, K)).astype(float)
@@ -43,7 +47,7 @@ def test_integers_are_exact(gctx, M, N, K):
 
 
 @pytest.mark.parametrize('M,N,K', [(129, 128, 1217), (2000, 17, 600), (1025, 641, 33), (24, 24, 36000)])
-def test_random_values_round_once(gctx, M, N, K):
+def test_random_values_round_once(gctx, sliced, M, N, K):
     rng = np.random.default_rng(K)
     A = rng.standard_normal((M, K)) * np.exp(2.0 * rng.standard_normal((M, 1)))
     B = rng.standard_normal((K, N)) * np.exp(2.0 * rng.standard_normal((1, N)))
@@ -55,7 +59,7 @@ def test_random_values_round_once(gctx, M, N, K):
 
 
 @pytest.mark.parametrize('alpha,beta', [(1.0, 0.0), (-2.0, 1.0), (0.3, 1.0), (-0.5, 0.7), (1.5, 0.0)])
-def test_alpha_beta_and_permuted_output(gctx, alpha, beta):
+def test_alpha_beta_and_permuted_output(gctx, sliced, alpha, beta):
     rng = np.random.default_rng(5)
     A = rng.integers(-512, 513, (20, 90, 45)).astype(float)       # (i, a, k)
     B = rng.integers(-512, 513, (45, 33, 21)).astype(float)       # (k, b, j)
@@ -65,14 +69,15 @@ def test_alpha_beta_and_permuted_output(gctx, alpha, beta):
     assert np.max(np.abs(got - want)) <= 2.0**-50 * np.max(np.abs(want))
 
 
-SMALL = [(1 + 8, 8, 3), (7, 9, 128), (8, 8, 129), (25, 19, 361), (5, 5, 9025), (90, 10, 90), (361, 25, 131),
+SMALL = [(9, 8, 3), (10, 10, 2000), (16, 4, 33), (17, 5, 260), (7, 9, 128), (8, 8, 129), (25, 19, 361), (5, 5, 9025), (90, 10, 90), (361, 25, 131),
          (2, 3, 1), (700, 700, 11)]
 
 
 @pytest.mark.parametrize('M,N,K', SMALL)
 @pytest.mark.parametrize('spec', ['mk,kn->mn', 'km,nk->nm'])
-def test_small_products_are_exact(gctx, M, N, K, spec):
-    # 8 x 8 tiles and K ranges of 128 with remainders, one tile split over many CTAs
+def test_small_products_are_exact(gctx, monkeypatch, M, N, K, spec):
+    monkeypatch.setenv('SCESS_TUNE', 'f64=2')
+    # tiles of up to 64 outputs, K ranges of 128 with remainders, one tile split over many CTAs
     rng = np.random.default_rng(M * N + K)
     A = rng.integers(-1000, 1001, (M, K)).astype(float)
     B = rng.integers(-1000, 1001, (K, N)).astype(float)
@@ -93,7 +98,7 @@ def test_matrix_vector_products_are_exact(gctx, M, K):
     assert np.array_equal(gctx.einsum('mk,kn->mn', A, x, out_shape=(M, 1)), A @ x)
 
 
-def test_zero_tiny_and_huge_rows(gctx):
+def test_zero_tiny_and_huge_rows(gctx, sliced):
     rng = np.random.default_rng(6)
     M, N, K = 140, 150, 1000
     A = rng.integers(-999, 1000, (M, K)).astype(float)
@@ -108,7 +113,7 @@ def test_zero_tiny_and_huge_rows(gctx):
     assert np.array_equal(got, want)
 
 
-def test_infinities_and_nans_reach_their_outputs(gctx):
+def test_infinities_and_nans_reach_their_outputs(gctx, sliced):
     rng = np.random.default_rng(7)
     M, N, K = 200, 170, 700
     A = rng.integers(-99, 100, (M, K)).astype(float)
