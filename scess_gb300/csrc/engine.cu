@@ -63,6 +63,11 @@ size_t BlockCache::flush() {
 }
 
 namespace {
+// What the engines keep between contractions goes back to the block cache.
+void reclaim(Ctx *c) {
+  if (c->slices) c->slices->reclaim();
+  if (c->tc) c->tc->reclaim();
+}
 // Frees the context's cached blocks (after its queued work) and stops counting them.
 void flush_cache(Ctx *c) {
   cudaStreamSynchronize(c->stream);
@@ -74,7 +79,10 @@ void flush_cache(Ctx *c) {
 void DevMem::alloc(size_t bytes) {
   release();
   if (bytes == 0) return;
+  bytes = (bytes + 511) & ~size_t(511);
   Ctx *c = current_ctx();
+  // a cap set below what is held: the cached blocks go first
+  if (c && c->mem_limit && c->mem_held > c->mem_limit && c->blocks.bytes() > 0) flush_cache(c);
   if (c && bytes >= BlockCache::kMinBytes) {
     if (void *p = c->blocks.take(bytes)) {  // (cached bytes are already counted as held)
       p_ = p;
@@ -85,8 +93,8 @@ void DevMem::alloc(size_t bytes) {
   }
   if (c && c->mem_limit) {
     if (c->mem_held + bytes > c->mem_limit && c->blocks.bytes() > 0) flush_cache(c);
-    if (c->mem_held + bytes > c->mem_limit && c->slices) {
-      c->slices->reclaim();
+    if (c->mem_held + bytes > c->mem_limit) {
+      reclaim(c);
       flush_cache(c);
     }
     if (c->mem_held + bytes > c->mem_limit)
@@ -98,7 +106,7 @@ void DevMem::alloc(size_t bytes) {
   cudaError_t e = cudaMalloc(&p_, bytes);
   if (e == cudaErrorMemoryAllocation && c) {
     cudaGetLastError();
-    if (c->slices) c->slices->reclaim();
+    reclaim(c);
     flush_cache(c);
     e = cudaMalloc(&p_, bytes);
   }

@@ -15,15 +15,17 @@ namespace scess {
 // Owning device allocation (freed on destruction).
 struct Ctx;
 
-// Large device blocks released while an API call of their context runs are
-// kept by that context (exact sizes) instead of going back through cudaFree,
-// which synchronises the whole device; later allocations of the same size in
-// the same context reuse them.  All of a context's kernels run on its one
+// Device blocks released while an API call of their context runs are
+// kept by that context (exact sizes, multiples of 512 bytes) instead of going back
+// through cudaFree, which synchronises the whole device (a small call's dozens of small
+// blocks too: a residual gradient at o = 8 v = 47 took 10.7 ms instead of 6.7 in a process
+// with a history of allocations); later allocations of the same size in the same
+// context reuse them.  All of a context's kernels run on its one
 // stream, so a reused block's earlier work precedes its new work.  The cache
 // is emptied when an allocation fails and with the context.
 class BlockCache {
  public:
-  static constexpr size_t kMinBytes = size_t(1) << 20;
+  static constexpr size_t kMinBytes = 512;
   static constexpr size_t kMaxCached = size_t(96) << 30;
   void *take(size_t bytes);
   bool give(void *p, size_t bytes);  // false: the caller frees it

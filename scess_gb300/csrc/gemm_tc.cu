@@ -1321,7 +1321,6 @@ void TcEngine::pack(const double *src, const int64_t *rowOff, int64_t rows, cons
   const int64_t rows_pad = round_up(std::max<int64_t>(rows, 1), std::max<int64_t>(row_align, 32));
   const size_t bytes = (size_t)rows_pad * 2 * Kpad * sizeof(uint16_t);
   if (out.mem.bytes() < bytes || !out.aux.bytes()) {
-    ctx_.sync();
     if (out.mem.bytes() < bytes) out.mem.alloc(bytes);
     if (!out.aux.bytes()) out.aux.alloc(16);
   }
@@ -1405,6 +1404,10 @@ void TcEngine::add_max_hint(const double *p, int64_t n) {
 }
 
 void TcEngine::clear_max_hints() {
+  // the packs' memory serves the next residual's (at most kSpare of them): allocating
+  // and freeing them per residual synchronised the device dozens of times
+  for (auto &kv : reuse_)
+    if ((int)spare_.size() < kSpare) spare_.push_back(std::move(kv.second));
   hints_.clear();
   reuse_.clear();
 }
@@ -1426,7 +1429,6 @@ void TcEngine::pack_with_max(const double *src, const int64_t *rowOff, int64_t r
   const int64_t rows_pad = round_up(std::max<int64_t>(rows, 1), std::max<int64_t>(row_align, 32));
   const size_t bytes = (size_t)rows_pad * 2 * Kpad * sizeof(uint16_t);
   if (out.mem.bytes() < bytes || !out.aux.bytes()) {
-    ctx_.sync();
     if (out.mem.bytes() < bytes) out.mem.alloc(bytes);
     if (!out.aux.bytes()) out.aux.alloc(16);
   }
@@ -1488,7 +1490,25 @@ void TcEngine::gemm(const Packed &A, int64_t rowA0, int64_t M, const Packed &B, 
                       err_.as<unsigned>(), ctx_.stream, take_diag());
 }
 
+std::unique_ptr<Packed> TcEngine::take_spare(size_t bytes) {
+  // the smallest one that is large enough, else the largest
+  int best = -1;
+  for (int i = 0; i < (int)spare_.size(); i++) {
+    if (best < 0) {
+      best = i;
+      continue;
+    }
+    const size_t b = spare_[best]->mem.bytes(), x = spare_[i]->mem.bytes();
+    if (b >= bytes ? (x >= bytes && x < b) : x > b) best = i;
+  }
+  if (best < 0) return std::make_unique<Packed>();
+  std::unique_ptr<Packed> p = std::move(spare_[best]);
+  spare_.erase(spare_.begin() + best);
+  return p;
+}
+
 void TcEngine::clear_cache(const void *owner) {
+  if (!owner) spare_.clear();  // (the end of an API call)
   for (auto it = cache_.begin(); it != cache_.end();) {
     if (it->second.first == owner) it = cache_.erase(it);
     else ++it;
@@ -1557,7 +1577,8 @@ void TcEngine::contract(const EinsumPlan &pl, double alpha, const double *A, con
                               std::to_string(nrows) + "|" + std::to_string(pl.K) + (unitK ? "u" : "s");
       auto it = reuse_.find(key);
       if (it != reuse_.end()) return *it->second;
-      auto pk = std::make_unique<Packed>();
+      std::unique_ptr<Packed> pk = take_spare((size_t)round_up(std::max<int64_t>(nrows, 1), TC_BM) * 4 *
+                                              round_up(std::max<int64_t>(pl.K, 1), TC_BK));
       pack(src, rows, nrows, ks, pl.K, unitK, TC_BM, *pk, h.rs, h.ks, h.P, h.E, h.dense);
       auto &ref = *pk;
       reuse_[key] = std::move(pk);

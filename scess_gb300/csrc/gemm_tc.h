@@ -202,6 +202,8 @@ class TcEngine {
   // the tensor unchanged until clear_max_hints().
   void add_max_hint(const double *p, int64_t n);
   void clear_max_hints();
+  // Gives the spare packs back (when an allocation fails).
+  void reclaim() { spare_.clear(); }
 
  private:
   Ctx &ctx_;
@@ -219,6 +221,9 @@ class TcEngine {
   // gathers the same tensor through equal tables reuses the first one's pack
   // (dropped with the hints)
   std::map<std::string, std::unique_ptr<Packed>> reuse_;
+  static constexpr int kSpare = 12;
+  std::vector<std::unique_ptr<Packed>> spare_;  // packs of hinted tensors, done with
+  std::unique_ptr<Packed> take_spare(size_t bytes);
   DevMem hint_words_;  // one max word per hint slot
   DevMem partial_;
   DevMem err_;
