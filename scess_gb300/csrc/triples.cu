@@ -24,6 +24,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "gemm_slice.h"
@@ -156,18 +157,29 @@ __host__ __device__ inline int64_t pad4(int64_t n) { return (n + 3) & ~int64_t(3
 
 // FP32 tables of the mixed energy kernel, built once per (T) call: every
 // orbital energy as hi + lo (hi = the FP32 rounding of eps, lo = the FP32
-// rounding of the remainder) and t1 in FP32.
+// rounding of the remainder), t1 in FP32, and for every orbit (see orbit_table)
+// its code, e_i + e_j + e_k as hi + lo and the weight of its six orderings.
 __global__ void energy_tables_kernel(const double *__restrict__ eps, int64_t n,
                                      const double *__restrict__ t1, int64_t nt1,
-                                     float2 *__restrict__ ehl, float *__restrict__ t1f) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n + nt1;
+                                     const uint32_t *__restrict__ codes, int64_t norbits,
+                                     float2 *__restrict__ ehl, float *__restrict__ t1f,
+                                     uint4 *__restrict__ orbits) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n + nt1 + norbits;
        e += (int64_t)gridDim.x * blockDim.x) {
     if (e < n) {
       const double x = eps[e];
       const float h = (float)x;
       ehl[e] = make_float2(h, (float)(x - (double)h));
-    } else {
+    } else if (e < n + nt1) {
       t1f[e - n] = (float)t1[e - n];
+    } else {
+      const uint32_t code = codes[e - n - nt1];
+      const double x = (eps[code & 255] + eps[(code >> 8) & 255]) + eps[(code >> 16) & 255];
+      const float h = (float)x;
+      const uint32_t m = code >> 24;
+      const float mult = m == 0 ? 1.0f : (m == 1 ? 0.5f : (1.0f / 6.0f));
+      orbits[e - n - nt1] = make_uint4(code, __float_as_uint(h), __float_as_uint((float)(x - (double)h)),
+                                       __float_as_uint(mult));
     }
   }
 }
@@ -203,34 +215,41 @@ std::vector<uint32_t> orbit_table(int64_t o) {
 // block is o^3 floats in (i, j, k) order, i + o j + o2p k.  One CTA per local
 // triple (a_l, b_l, c_l).
 //
-// Pass 1 (threads own (i, j) pairs and walk k; a pair's loads are all issued
-// before any is used): Y = W + V in shared memory, V_ijk = t1_ia (jb|kc) +
-// t1_jb (ia|kc) + t1_kc (ia|jb) (GetV, RCCSD_T.cpp:70-75).
+// Pass 1: Y = W + V in shared memory, V_ijk = t1_ia (jb|kc) + t1_jb (ia|kc) +
+// t1_kc (ia|jb) (GetV, RCCSD_T.cpp:70-75).  A thread owns a pair (i, j), or four
+// with consecutive i where o is a multiple of four, and some of the k; the loads of
+// several k are issued before any is used, and what was read is cleared at once.
 // Pass 2 (threads own orbits of (i, j, k)): r3 (:152-154) of an even ordering
 // of the orbit is 3 Y + (S_e - 2 S_o), of an odd one 3 Y + (S_o - 2 S_e)
 // (S_e, S_o: sums of Y over the even / odd orderings), and the denominator
 // (:155) is the same for the whole orbit:
 //   sum_orbit W r3(Y) / D = [sum_even W (3 Y + S_e - 2 S_o) + sum_odd W (3 Y + S_o - 2 S_e)] / D,
 // one division per orbit instead of six; r3 is formed per ordering before it
-// multiplies W (it is a small difference of similar Y values), and W = Y - V
-// with V recomputed from the (ia|jb) slices, so that shared memory holds only
-// Y and the slices.  D comes from the FP64 orbital energies without FP64
-// arithmetic per orbit: every energy is split into FP32 hi + lo, the sum is
-// formed in double-float (two_sum) and rounded once.  The orbit sums are
-// compensated (Kahan), the sums over the warp double-float, the CTA's FP64.
-constexpr int kEnergyMaxO = 32;  // pass 1 keeps a pair's o loads in registers
-template <int NW>
-__global__ void __launch_bounds__(256) triples_energy_orbit_kernel(
+// multiplies W (it is a small difference of similar Y values).  D needs no FP64
+// arithmetic per orbit: energies are FP32 hi + lo pairs, e_i + e_j + e_k comes from
+// the orbit table, and the difference is formed in double-float (two_sum) and rounded
+// once.  The orbit sums are compensated (Kahan), the sums over the warp
+// double-float, the CTA's FP64.
+//
+// The kernel is bound by instruction issue and shared-memory wavefronts (W comes from
+// L2).  WS keeps (Y, W) pairs in shared memory: six 8-byte reads per orbit.  Where two
+// such CTAs don't fit an SM (o >= 24) only Y is kept and W = Y - V recomputed from the
+// (ia|jb) slices: 24 reads and 18 multiply-adds per orbit.  At o = 20 and 1728 triples:
+// 45.5 us with V recomputed and the energies added per orbit, 38.3 this way; o = 13: 37.1, 34.0.
+constexpr int kEnergyMaxO = 32;
+template <int NW, bool WS>
+__global__ void __launch_bounds__(256, 4) triples_energy_orbit_kernel(
     float *__restrict__ W, int64_t o, int64_t v, int64_t nb, int64_t A, int64_t Bk, int64_t C,
     const float2 *__restrict__ ehl, const float *__restrict__ t1f, const float *__restrict__ S,
-    const uint32_t *__restrict__ orbits, int norbits, double *__restrict__ energies) {
+    const uint4 *__restrict__ orbits, int norbits, double *__restrict__ energies) {
   const int al = (int)(blockIdx.x / (nb * nb)), bl = (int)((blockIdx.x / nb) % nb),
             cl = (int)(blockIdx.x % nb);
   const int64_t a = A * nb + al, b = Bk * nb + bl, c = C * nb + cl;
   const int oo = (int)o, o2 = oo * oo;
   const int o2p = (int)pad4(o2), o3p = oo * o2p;
   const int64_t nb3o3 = nb * nb * nb * (int64_t)o3p;
-  const float *W0, *W1 = nullptr, *W2 = nullptr;
+  float *W0;
+  const float *W1 = nullptr, *W2 = nullptr;
   if (NW == 3) {
     W0 = W + ((bl * nb + cl) * nb + al) * (int64_t)o3p;
     W1 = W + nb3o3 + ((al * nb + cl) * nb + bl) * (int64_t)o3p;
@@ -247,34 +266,41 @@ __global__ void __launch_bounds__(256) triples_energy_orbit_kernel(
     // and visible only after this wait (no-op for an ordinary launch)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (NW == 1) {  // its block received the launch's sums all the same: clear it
-      float4 *w4 = reinterpret_cast<float4 *>(const_cast<float *>(W0));
+      float4 *w4 = reinterpret_cast<float4 *>(W0);
       for (int e = threadIdx.x; e < o3p / 4; e += blockDim.x) w4[e] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     return;
   }
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  __shared__ float red_hi[32], red_lo[32];
+  __shared__ double red[8];
   __shared__ float s_ev[2];
-  // ek[x] = (e_x hi, e_x lo, t1_xc, 0), tab[x] = (t1_xa, t1_xb); Y at
-  // i + p1 j + p2 k with odd p1, p2, the (ia|jb) slices at x + p1 y, so that
-  // reads along any one index are free of bank conflicts
-  const int p1 = oo | 1, p2 = (p1 * oo) | 1;
-  float4 *ek = reinterpret_cast<float4 *>(sm_raw);
-  float2 *tab = reinterpret_cast<float2 *>(ek + oo);
-  float *Y = reinterpret_cast<float *>(tab + oo);
-  float *Sbc = Y + p2 * oo, *Sac = Sbc + p1 * oo, *Sab = Sac + p1 * oo;
+  // tab[x] = (t1_xa, t1_xb, t1_xc); the (ia|jb) slices at x + ps y; Y or (Y, W) at
+  // i + p1 j + p2 k.  Odd pitches keep reads along any one index free of bank conflicts
+  // (the slices are read that way in pass 2 alone).
+  constexpr int EL = WS ? 8 : 4;  // bytes of an element
+  const int p1 = oo | 1, p2 = (p1 * oo) | 1, ps = WS ? oo : p1, slice = WS ? o2p : p1 * oo;
+  float4 *tab = reinterpret_cast<float4 *>(sm_raw);
+  float *Sbc = reinterpret_cast<float *>(tab + oo), *Sac = Sbc + slice, *Sab = Sac + slice;
+  float *Y = Sab + slice;
+  if (!WS) Y = reinterpret_cast<float *>(sm_raw + ((reinterpret_cast<unsigned char *>(Y) - sm_raw + 7) & ~7));
+  unsigned char *yb = reinterpret_cast<unsigned char *>(Y);
   const float *S_bc = S + (b + v * c) * o2p, *S_ac = S + (a + v * c) * o2p, *S_ab = S + (a + v * b) * o2p;
-  for (int e = threadIdx.x; e < o2; e += blockDim.x) {
-    const int x = e % oo, y = e / oo;
-    Sbc[x + p1 * y] = S_bc[e];
-    Sac[x + p1 * y] = S_ac[e];
-    Sab[x + p1 * y] = S_ab[e];
+  if (WS) {
+    for (int e = threadIdx.x; e < o2p / 4; e += blockDim.x) {
+      reinterpret_cast<float4 *>(Sbc)[e] = reinterpret_cast<const float4 *>(S_bc)[e];
+      reinterpret_cast<float4 *>(Sac)[e] = reinterpret_cast<const float4 *>(S_ac)[e];
+      reinterpret_cast<float4 *>(Sab)[e] = reinterpret_cast<const float4 *>(S_ab)[e];
+    }
+  } else {
+    for (int e = threadIdx.x; e < o2; e += blockDim.x) {
+      const int x = e % oo, y = e / oo;
+      Sbc[x + p1 * y] = S_bc[e];
+      Sac[x + p1 * y] = S_ac[e];
+      Sab[x + p1 * y] = S_ab[e];
+    }
   }
-  for (int i = threadIdx.x; i < oo; i += blockDim.x) {
-    const float2 e = ehl[i];
-    ek[i] = make_float4(e.x, e.y, t1f[i + o * c], 0.f);
-    tab[i] = make_float2(t1f[i + o * a], t1f[i + o * b]);
-  }
+  for (int i = threadIdx.x; i < oo; i += blockDim.x)
+    tab[i] = make_float4(t1f[i + o * a], t1f[i + o * b], t1f[i + o * c], 0.f);
   if (threadIdx.x == 0) {  // e_a + e_b + e_c in double-float
     const float2 ea = ehl[o + a], eb = ehl[o + b], ec = ehl[o + c];
     float s1, e1, s2, e2;
@@ -288,63 +314,136 @@ __global__ void __launch_bounds__(256) triples_energy_orbit_kernel(
   // the tables above come from the call's setup; W from the grouped GEMM just
   // before, complete after this wait
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  // pass 1: Y = W + V (loads only; NW = 1 clears W after the barrier below).
-  // A pair's o loads are all issued before any is used; the first pair's go
-  // out before the barrier that publishes the tables.
-  float wr[kEnergyMaxO];
-  auto load_pair = [&](int pr) {
+  // pass 1; the first loads go out before the barrier that publishes the tables
+  auto pass1 = [&](auto quad) {
+    constexpr int Q = decltype(quad)::value;
+    using Vec = std::conditional_t<Q == 4, float4, float>;
+    constexpr int CH = Q == 4 ? 4 : 8;  // k loads of a thread in flight (more would spill)
+    const int nu = o2 / Q, kgn = max(1, (int)blockDim.x / nu), units = nu * kgn;
+    int t = threadIdx.x, i = 0, j = 0, k0 = 0;
+    Vec r[CH];
+    float *w = W0;
+    auto begin = [&]() {
+      const int kg = t / nu, pr = (t - kg * nu) * Q;
+      j = pr / oo;
+      i = pr - j * oo;
+      k0 = kg;
+      w = W0 + pr;
+    };
+    auto load = [&]() {
 #pragma unroll
-    for (int k = 0; k < kEnergyMaxO; k++) {
-      if (k < oo) {
-        const int e = pr + o2p * k;
-        wr[k] = W0[e];
-        if (NW == 3) wr[k] += W1[e] + W2[e];
+      for (int n = 0; n < CH; n++) {
+        const int k = k0 + n * kgn;
+        if (k < oo) {
+          r[n] = *reinterpret_cast<const Vec *>(w + k * o2p);
+          if (NW == 3) {
+            const Vec x = *reinterpret_cast<const Vec *>(W1 + (w - W0) + k * o2p),
+                      y = *reinterpret_cast<const Vec *>(W2 + (w - W0) + k * o2p);
+            if constexpr (Q == 4)
+              r[n] = make_float4(r[n].x + (x.x + y.x), r[n].y + (x.y + y.y), r[n].z + (x.z + y.z),
+                                 r[n].w + (x.w + y.w));
+            else
+              r[n] += x + y;
+          }
+        }
       }
+    };
+    if (t < units) {
+      begin();
+      load();
+    }
+    __syncthreads();
+    while (t < units) {
+      const float tbj = tab[j].y;
+      float tai[Q], sab[Q];
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        tai[q] = tab[i + q].x;
+        sab[q] = Sab[i + q + ps * j];
+      }
+      unsigned char *y0 = yb + EL * (i + p1 * j);
+#pragma unroll
+      for (int n = 0; n < CH; n++) {
+        const int k = k0 + n * kgn;
+        if (k < oo) {
+          const float bc = Sbc[j + ps * k], tck = tab[k].z;
+          const Vec sac = *reinterpret_cast<const Vec *>(Sac + i + ps * k);
+          const float *ac = reinterpret_cast<const float *>(&sac), *wr = reinterpret_cast<const float *>(&r[n]);
+#pragma unroll
+          for (int q = 0; q < Q; q++) {
+            const float y = wr[q] + (tai[q] * bc + tbj * ac[q] + tck * sab[q]);
+            if (WS)
+              *reinterpret_cast<float2 *>(y0 + EL * (p2 * k + q)) = make_float2(y, wr[q]);
+            else
+              *reinterpret_cast<float *>(y0 + EL * (p2 * k + q)) = y;
+          }
+          // W is read: cleared for the next block triple's reductions
+          if (NW == 1) *reinterpret_cast<Vec *>(w + k * o2p) = Vec{};
+        }
+      }
+      k0 += CH * kgn;
+      if (k0 >= oo) {
+        t += blockDim.x;
+        if (kgn > 1 || t >= units) break;
+        begin();
+      }
+      load();
     }
   };
-  if ((int)threadIdx.x < o2) load_pair(threadIdx.x);
+  if (WS && (oo & 3) == 0)
+    pass1(std::integral_constant<int, 4>{});
+  else
+    pass1(std::integral_constant<int, 1>{});
+  // (shared memory leaves the L1 cache little room: the orbit table comes from L2, an
+  // entry ahead of its use)
+  int q = threadIdx.x;
+  uint4 next = q < norbits ? __ldg(orbits + q) : make_uint4(0, 0, 0, 0);
   __syncthreads();
-  for (int pr = threadIdx.x; pr < o2; pr += blockDim.x) {
-    if (pr != (int)threadIdx.x) load_pair(pr);
-    const int i = pr % oo, j = pr / oo;
-    const float tai = tab[i].x, tbj = tab[j].y, sab = Sab[i + p1 * j];
-    const int yo = i + p1 * j;
-#pragma unroll
-    for (int k = 0; k < kEnergyMaxO; k++)
-      if (k < oo)
-        Y[yo + p2 * k] = wr[k] + (tai * Sbc[j + p1 * k] + tbj * Sac[i + p1 * k] + ek[k].z * sab);
-  }
-  __syncthreads();
-  if (NW == 1) {  // the block of W is read: clear it for the next block triple's reductions
-    float4 *w4 = reinterpret_cast<float4 *>(const_cast<float *>(W0));
-    for (int e = threadIdx.x; e < o3p / 4; e += blockDim.x) w4[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
   // pass 2: orbits
   const float evh = s_ev[0], evl = s_ev[1];
+  const int s1 = EL * p1, s2 = EL * p2;
   float sum = 0.0f, comp = 0.0f;
-  for (int q = threadIdx.x; q < norbits; q += blockDim.x) {
-    const uint32_t code = __ldg(orbits + q);
-    const int i = code & 255, j = (code >> 8) & 255, k = (code >> 16) & 255;
-    const int m = code >> 24;
-    const float2 ti = tab[i], tj = tab[j], tk = tab[k];
-    const float4 ei = ek[i], ej = ek[j], ekk = ek[k];
-    const int pi = p1 * i, pj = p1 * j, pk = p1 * k, qi = p2 * i, qj = p2 * j, qk = p2 * k;
-    // V_xyz = t1_xa Sbc(y,z) + t1_yb Sac(x,z) + t1_zc Sab(x,y) over the orderings
-    const float bc_jk = Sbc[j + pk], bc_kj = Sbc[k + pj], bc_ki = Sbc[k + pi],
-                bc_ik = Sbc[i + pk], bc_ij = Sbc[i + pj], bc_ji = Sbc[j + pi];
-    const float ac_jk = Sac[j + pk], ac_kj = Sac[k + pj], ac_ki = Sac[k + pi],
-                ac_ik = Sac[i + pk], ac_ij = Sac[i + pj], ac_ji = Sac[j + pi];
-    const float ab_jk = Sab[j + pk], ab_kj = Sab[k + pj], ab_ki = Sab[k + pi],
-                ab_ik = Sab[i + pk], ab_ij = Sab[i + pj], ab_ji = Sab[j + pi];
+  while (q < norbits) {
+    const uint4 ob = next;
+    q += blockDim.x;
+    if (q < norbits) next = __ldg(orbits + q);
+    const int i = ob.x & 255, j = (ob.x >> 8) & 255, k = (ob.x >> 16) & 255;
+    const int bi = EL * i, bj = EL * j, bk = EL * k;
+    const int pi = s1 * i, pj = s1 * j, pk = s1 * k, qi = s2 * i, qj = s2 * j, qk = s2 * k;
     // even orderings ijk, jki, kij; odd ikj, kji, jik
-    const float ye0 = Y[i + pj + qk], ye1 = Y[j + pk + qi], ye2 = Y[k + pi + qj];
-    const float yo0 = Y[i + pk + qj], yo1 = Y[k + pj + qi], yo2 = Y[j + pi + qk];
-    const float we0 = ye0 - (ti.x * bc_jk + tj.y * ac_ik + ekk.z * ab_ij);
-    const float we1 = ye1 - (tj.x * bc_ki + tk.y * ac_ji + ei.z * ab_jk);
-    const float we2 = ye2 - (tk.x * bc_ij + ti.y * ac_kj + ej.z * ab_ki);
-    const float wo0 = yo0 - (ti.x * bc_kj + tk.y * ac_ij + ej.z * ab_ik);
-    const float wo1 = yo1 - (tk.x * bc_ji + tj.y * ac_ki + ei.z * ab_kj);
-    const float wo2 = yo2 - (tj.x * bc_ik + ti.y * ac_jk + ekk.z * ab_ji);
+    float ye0, ye1, ye2, yo0, yo1, yo2, we0, we1, we2, wo0, wo1, wo2;
+    if (WS) {
+      auto at = [&](int off, float &y, float &w) {
+        const float2 x = *reinterpret_cast<const float2 *>(yb + off);
+        y = x.x;
+        w = x.y;
+      };
+      at(bi + pj + qk, ye0, we0);
+      at(bj + pk + qi, ye1, we1);
+      at(bk + pi + qj, ye2, we2);
+      at(bi + pk + qj, yo0, wo0);
+      at(bk + pj + qi, yo1, wo1);
+      at(bj + pi + qk, yo2, wo2);
+    } else {
+      auto at = [&](int off) { return *reinterpret_cast<const float *>(yb + off); };
+      ye0 = at(bi + pj + qk), ye1 = at(bj + pk + qi), ye2 = at(bk + pi + qj);
+      yo0 = at(bi + pk + qj), yo1 = at(bk + pj + qi), yo2 = at(bj + pi + qk);
+      // V_xyz = t1_xa Sbc(y,z) + t1_yb Sac(x,z) + t1_zc Sab(x,y) over the orderings
+      const float4 ti = tab[i], tj = tab[j], tk = tab[k];
+      const int si = p1 * i, sj = p1 * j, sk = p1 * k;
+      const float bc_jk = Sbc[j + sk], bc_kj = Sbc[k + sj], bc_ki = Sbc[k + si],
+                  bc_ik = Sbc[i + sk], bc_ij = Sbc[i + sj], bc_ji = Sbc[j + si];
+      const float ac_jk = Sac[j + sk], ac_kj = Sac[k + sj], ac_ki = Sac[k + si],
+                  ac_ik = Sac[i + sk], ac_ij = Sac[i + sj], ac_ji = Sac[j + si];
+      const float ab_jk = Sab[j + sk], ab_kj = Sab[k + sj], ab_ki = Sab[k + si],
+                  ab_ik = Sab[i + sk], ab_ij = Sab[i + sj], ab_ji = Sab[j + si];
+      we0 = ye0 - (ti.x * bc_jk + tj.y * ac_ik + tk.z * ab_ij);
+      we1 = ye1 - (tj.x * bc_ki + tk.y * ac_ji + ti.z * ab_jk);
+      we2 = ye2 - (tk.x * bc_ij + ti.y * ac_kj + tj.z * ab_ki);
+      wo0 = yo0 - (ti.x * bc_kj + tk.y * ac_ij + tj.z * ab_ik);
+      wo1 = yo1 - (tk.x * bc_ji + tj.y * ac_ki + ti.z * ab_kj);
+      wo2 = yo2 - (tj.x * bc_ik + ti.y * ac_jk + tk.z * ab_ji);
+    }
     const float Se = (ye0 + ye1) + ye2, So = (yo0 + yo1) + yo2;
     const float ce = Se - 2.0f * So, co = So - 2.0f * Se;                          // :152-154
     float num = we0 * fmaf(3.0f, ye0, ce);
@@ -354,13 +453,10 @@ __global__ void __launch_bounds__(256) triples_energy_orbit_kernel(
     num = fmaf(wo1, fmaf(3.0f, yo1, co), num);
     num = fmaf(wo2, fmaf(3.0f, yo2, co), num);
     // D = e_i + e_j + e_k - (e_a + e_b + e_c) in double-float, rounded once   :155
-    float s1, e1, s2, e2, s3, e3;
-    two_sum(ei.x, ej.x, s1, e1);
-    two_sum(s1, ekk.x, s2, e2);
-    two_sum(s2, -evh, s3, e3);
-    const float d = s3 + (((e1 + e2) + e3) + (((ei.y + ej.y) + ekk.y) - evl));
-    const float mult = m == 0 ? 1.0f : (m == 1 ? 0.5f : (1.0f / 6.0f));
-    const float term = __fdividef(num * mult, d) - comp;                           // :156
+    float dh, de;
+    two_sum(__uint_as_float(ob.y), -evh, dh, de);
+    const float d = dh + (de + (__uint_as_float(ob.z) - evl));
+    const float term = __fdividef(num * __uint_as_float(ob.w), d) - comp;          // :156
     const float t = sum + term;
     comp = (t - sum) - term;
     sum = t;
@@ -375,19 +471,15 @@ __global__ void __launch_bounds__(256) triples_energy_orbit_kernel(
     acc_hi = h;
     acc_lo += e + ol;
   }
-  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-  if (lane == 0) {
-    red_hi[wi] = acc_hi;
-    red_lo[wi] = acc_lo;
-  }
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = (double)acc_hi + (double)acc_lo;
   __syncthreads();
   if (threadIdx.x == 0) {
     double total = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); q++) total += (double)red_hi[q] + (double)red_lo[q];
-    double deg = 1.0;                                                               // :135-139
-    if (a == c) deg = 6.0;
-    else if (a == b || b == c) deg = 2.0;
-    energies[triple_id(a, b, c)] = total / deg;
+    for (int q = 0; q < (int)(blockDim.x >> 5); q++) total += red[q];
+    // degeneracy of the virtual indices                                            :135-139
+    if (a == c) total /= 6.0;
+    else if (a == b || b == c) total *= 0.5;
+    energies[triple_id(a, b, c)] = total;
   }
 }
 
@@ -1231,8 +1323,13 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
   DevMem W(wbytes);
   if (mixed && nw == 1) SCESS_CUDA(cudaMemsetAsync(W.as<void>(), 0, wbytes, s));
   const int64_t p1 = o | 1, p2 = (p1 * o) | 1;
-  const size_t ysmem = mixed ? (size_t)(4 * o + 2 * o + p2 * o + 3 * p1 * o) * 4
+  // the mixed energy kernel keeps (Y, W) in shared memory where two CTAs fit an SM
+  const size_t wsmem = (size_t)(16 * o + 12 * o2p + 8 * p2 * o);
+  const bool ws = 2 * (wsmem + 1024) <= 228 * 1024;
+  const size_t ysmem = mixed ? (ws ? wsmem : (size_t)(16 * o + 12 * p1 * o + 4 * p2 * o + 8))
                              : (size_t)(p2 * o + 3 * o2 + 4 * o) * 8;
+  const auto orbit_kernel = nw == 1 ? (ws ? triples_energy_orbit_kernel<1, true> : triples_energy_orbit_kernel<1, false>)
+                                    : (ws ? triples_energy_orbit_kernel<3, true> : triples_energy_orbit_kernel<3, false>);
   if (ysmem > 200 * 1024) throw Error(SCESS_ERR_UNSUPPORTED, "(T): o^3 too large for one CTA");
   if (o > 255) throw Error(SCESS_ERR_UNSUPPORTED, "(T): more than 255 occupied orbitals");
   if (mixed && o > kEnergyMaxO)
@@ -1240,8 +1337,7 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
   DevMem orbits;
   int norbits = 0;
   if (mixed) {
-    SCESS_CUDA(cudaFuncSetAttribute(nw == 1 ? triples_energy_orbit_kernel<1> : triples_energy_orbit_kernel<3>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ysmem));
+    SCESS_CUDA(cudaFuncSetAttribute(orbit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ysmem));
     const std::vector<uint32_t> ot = orbit_table(o);
     norbits = (int)ot.size();
     orbits.alloc(ot.size() * sizeof(uint32_t));
@@ -1279,7 +1375,10 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
   CUtensorMap mP{}, mQ{}, mQ2{}, mR{}, mR2{}, mTx{};
   DevTables gdt;  // W_g row / column tables
   DevMem Sf;    // (ia|jb) as FP32 for the energy kernel (padded rows)
-  DevMem etab;  // eps as FP32 hi + lo (nmo float2), then t1 in FP32
+  DevMem etab;  // the orbits (uint4), eps as FP32 hi + lo (nmo float2), then t1 in FP32
+  uint4 *orb = nullptr;
+  float2 *ehl = nullptr;
+  float *t1f = nullptr;
   const int64_t Mg = o * nb, Ng = o2;
   if (mixed) {
     TimedScope ts(ctx.timer, "phase:triples_pack", 0.0, 0.0, s);
@@ -1336,9 +1435,12 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
                  table({{o, o}, {nb, nb * o3p}}), table({{o, 1}, {o, o2p}}),
                  table({{o, o2p}, {nb, o3p}}), table({{o, 1}, {o, o}})});
     Sf.alloc((size_t)o2p * v * v * sizeof(float));
-    etab.alloc((size_t)N * sizeof(float2) + (size_t)o * v * sizeof(float));
-    energy_tables_kernel<<<(unsigned)std::min<int64_t>(ceil_div(N + o * v, 256), 4 * kNumSMs), 256, 0, s>>>(
-        d_eps, N, d_t1, o * v, etab.as<float2>(), reinterpret_cast<float *>(etab.as<float2>() + N));
+    etab.alloc((size_t)norbits * sizeof(uint4) + (size_t)N * sizeof(float2) + (size_t)o * v * sizeof(float));
+    orb = etab.as<uint4>();
+    ehl = reinterpret_cast<float2 *>(orb + norbits);
+    t1f = reinterpret_cast<float *>(ehl + N);
+    energy_tables_kernel<<<(unsigned)std::min<int64_t>(ceil_div(N + o * v + norbits, 256), 4 * kNumSMs), 256, 0, s>>>(
+        d_eps, N, d_t1, o * v, orbits.as<uint32_t>(), norbits, ehl, t1f, orb);
     SCESS_CHECK_LAUNCH();
     to_f32_rows_kernel<<<(unsigned)std::min<int64_t>(ceil_div(o2p * v * v, 256), 16 * kNumSMs), 256, 0, s>>>(
         T.S.p(), v * v, o2, o2p, Sf.as<float>());
@@ -1461,11 +1563,9 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
           cfg.stream = s;
           cfg.attrs = at;
           cfg.numAttrs = pdl ? 1 : 0;
-          const float *t1f = reinterpret_cast<const float *>(etab.as<float2>() + N);
-          SCESS_CUDA(cudaLaunchKernelEx(&cfg, nw == 1 ? triples_energy_orbit_kernel<1> : triples_energy_orbit_kernel<3>,
-                                        W.as<float>(), (int64_t)o, (int64_t)v, (int64_t)nb, (int64_t)A,
-                                        (int64_t)Bk, (int64_t)C, (const float2 *)etab.as<float2>(), t1f,
-                                        (const float *)Sf.as<float>(), (const uint32_t *)orbits.as<uint32_t>(),
+          SCESS_CUDA(cudaLaunchKernelEx(&cfg, orbit_kernel, W.as<float>(), (int64_t)o, (int64_t)v, (int64_t)nb,
+                                        (int64_t)A, (int64_t)Bk, (int64_t)C, (const float2 *)ehl,
+                                        (const float *)t1f, (const float *)Sf.as<float>(), (const uint4 *)orb,
                                         norbits, energies.p()));
         } else
           triples_energy_kernel<double, double><<<nblk, 256, ysmem, s>>>(
