@@ -9,14 +9,15 @@
 //   warps 4-19 four epilogue warpgroups, bn / 4 columns each: add every drained
 //              S_d, an exact integer, into one 64-bit integer per output, and turn
 //              integer + FP32 tail into FP64 at the end of the unit.
-// Shared memory bounds the tensor pipe: operand reads (128 B a cycle) and TMA writes
-// (70 B a cycle, measured, on every SM alone) share its port, so an MMA of N = 128
-// costs 64 + 29 cycles (0.73 per column) and one of N = 80 52 + 24 (0.95).  The wide
-// tile leaves TMEM room for four accumulators only, hence the rotation and five
-// drains per K block, which run beside the MMAs.  A TMEM load takes about 200 cycles
-// whatever its width, so four epilogue warps share a scheduler (two: 39 TFLOP/s at
-// 4096^3 and 0.74 ms for 8192 x 8192 x 32; four: 41.8 and 0.38).  Six accumulators of
-// 80 columns with a third of the drains and two warps: 34 TFLOP/s.
+// The wide tile (an MMA of N = 128 takes 64 cycles, one of N = 80 still 52) leaves TMEM
+// room for four accumulators only, hence the rotation and five drains per K block, which
+// run beside the MMAs.  They bound it: 56 MMAs take 3600 cycles of a K block's 5750, the
+// drains' arithmetic (about four cycles of a scheduler per column, warp and drain) and their waits and
+// releases the rest.  What got it there, TFLOP/s at 4096^3 (68.7 at the tensor pipe's
+// measured rate): two epilogue warps a scheduler 38.8, four 41.8 (they hide each other's
+// waits); MMAs issued from uniform registers (see elect_one) 51.6; S_5 between S_2 and
+// S_1, and accumulators released before their arithmetic, 52.3.  Six accumulators of 80
+// columns with a third of the drains: 34 when issue bound it.
 // Every mbarrier wait is bounded (see mbarrier.cuh).
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -44,6 +45,7 @@ constexpr int EPI = 4;                                               // epilogue
 constexpr int HC = BN / EPI;                                         // columns of an epilogue thread
 constexpr int THREADS = 128 * (1 + EPI);
 constexpr int kEpiRegs = 104, kCtlRegs = 56, kLaunchRegs = 96;       // 56 + 4 x 104 <= 5 x 96
+static_assert(kSlices == NDIAG + 2, "the tail is S_5 + S_6");
 static_assert(kCtlRegs + EPI * kEpiRegs <= (1 + EPI) * kLaunchRegs, "setmaxnreg draws on the launch's registers");
 struct Ctl {  // behind the stages
   uint64_t full[STAGES], empty[STAGES], tfull[NACC], tempty[NACC], done;
@@ -130,14 +132,13 @@ __device__ __forceinline__ void tmem_wait8(uint32_t *r) {
                : "memory");
 }
 
-// What bounds it: long K, the shared-memory port (above); short K, the epilogue
-// (about 45 instructions per output).
+// What bounds it: long K, the drains (above); short K, the outputs (about 45 instructions each).
 __global__ void __launch_bounds__(THREADS, 1)
     slice_gemm_kernel(const __grid_constant__ SliceMaps maps, const __grid_constant__ SliceArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   Ctl &ctl = *reinterpret_cast<Ctl *>(smem + STAGES * STAGE_BYTES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int tiles = a.tiles_m * a.tiles_n;
   const int nprob = a.gstart[a.ng];
   const int units = tiles * nprob * a.splits;
@@ -239,60 +240,69 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (last[s] >= 0) mbar_drain(&ctl.full[s], (uint32_t)(last[s] / STAGES) & 1u);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int g = 0, c = 0, w = 0;  // stages, rotating fills and units so far
-      const uint64_t desc_a = sw_desc<64>(smem_u32(smem)), desc_b = sw_desc<64>(smem_u32(smem) + kSlices * A_SLICE);
-      const uint32_t bq = bslice >> 4;
-      bool ok = true;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x, w++) {
-        int tm, tn, py, pz, pg, kb0, kb1, sp;
-        unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
-        const uint32_t idesc = idesc_f16kind(BM, min(bn, (a.N - tn * bn + 15) & ~15), 1u);  // BF16
-        for (int kb = kb0; kb < kb1 && ok; kb++, g++) {
-          const int s = g % STAGES;
-          const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
-          if (!mbar_wait(&ctl.full[s], ph, a.err, ERR_FULL_WAIT, a.wait_cycles)) { ok = false; break; }
+    // all lanes, issues by the elected one (see elect_one)
+    int g = 0, c = 0, w = 0;  // stages, rotating fills and units so far
+    const uint64_t desc = sw_desc<64>(smem_u32(smem));
+    const uint32_t hi = (uint32_t)(desc >> 32), lo = (uint32_t)desc;
+    const uint32_t bq = bslice >> 4;
+    const bool issuer = elect_one();
+    auto wait = [&](uint64_t *barrier, uint32_t parity, unsigned code) {
+      return __all_sync(0xffffffffu, mbar_wait(barrier, parity, a.err, code, a.wait_cycles)) != 0;
+    };
+    bool ok = true;
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x, w++) {
+      int tm, tn, py, pz, pg, kb0, kb1, sp;
+      unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
+      const uint32_t idesc = idesc_f16kind(BM, min(bn, (a.N - tn * bn + 15) & ~15), 1u);  // BF16
+      for (int kb = kb0; kb < kb1 && ok; kb++, g++) {
+        const int s = g % STAGES;
+        const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
+        if (!wait(&ctl.full[s], ph, ERR_FULL_WAIT)) { ok = false; break; }
+        tc_fence_after();
+        // slice offsets are added to the stage's descriptors (address field in units of 16 bytes)
+        const uint32_t da = lo + (uint32_t)s * (STAGE_BYTES >> 4), db = da + (kSlices * A_SLICE >> 4);
+        auto product = [&](uint32_t col, int p, int q, uint32_t acc) {
+#pragma unroll
+          for (int k = 0; k < 2; k++)
+            mma_f16kind(tmem + col, da + p * (A_SLICE >> 4) + 2 * k, db + q * bq + 2 * k, hi, idesc, k ? 1u : acc);
+        };
+        auto tail = [&](auto diag, uint32_t acc) {
+          constexpr int d = decltype(diag)::value;
+#pragma unroll
+          for (int p = 0; p <= d; p++, acc = 1u) product((uint32_t)(TAIL * bn), p, d - p, acc);
+        };
+        // The longest diagonals first and S_5 between S_2 and S_1: a drain is then done
+        // when its accumulator comes round.
+#pragma unroll
+        for (int d = NDIAG - 1; d >= 0; d--) {
+          if (d == 1) {
+            if (kb == kb0) {
+              if (!wait(&ctl.tempty[TAIL], ((uint32_t)w & 1u) ^ 1u, ERR_EMPTY_WAIT)) { ok = false; break; }
+              tc_fence_after();
+            }
+            if (issuer) tail(std::integral_constant<int, NDIAG>{}, kb == kb0 ? 0u : 1u);
+          }
+          const int b = c % NROT;
+          if (ok && !wait(&ctl.tempty[b], (((uint32_t)(c / NROT)) & 1u) ^ 1u, ERR_EMPTY_WAIT)) ok = false;
+          if (!ok) break;
           tc_fence_after();
-          // slice offsets are added to the stage's descriptors (address field in units
-          // of 16 bytes): building a descriptor per MMA costs the issuing thread 100
-          // cycles, more than the MMA takes
-          const uint64_t da = desc_a + (uint64_t)(s * (STAGE_BYTES >> 4));
-          const uint64_t db = desc_b + (uint64_t)(s * (STAGE_BYTES >> 4));
-          auto product = [&](uint32_t col, int p, int q, uint32_t acc) {
-#pragma unroll
-            for (int k = 0; k < 2; k++)
-              mma_bf16(tmem + col, da + (uint64_t)(p * (A_SLICE >> 4) + 2 * k), db + (uint64_t)(q * bq + 2 * k), idesc,
-                       k ? 1u : acc);
-          };
-          // the longest first, so that a drain is done when its accumulator comes round
-#pragma unroll
-          for (int d = NDIAG - 1; d >= 0; d--) {
-            const int b = c % NROT;
-            if (ok && !mbar_wait(&ctl.tempty[b], (((uint32_t)(c / NROT)) & 1u) ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) ok = false;
-            if (!ok) break;
-            tc_fence_after();
+          if (issuer) {
 #pragma unroll
             for (int p = 0; p <= d; p++) product((uint32_t)(b * bn), p, d - p, p ? 1u : 0u);
             mma_commit(&ctl.tfull[b]);
-            c++;
           }
-          if (!ok) break;
-          if (kb == kb0) {
-            if (!mbar_wait(&ctl.tempty[TAIL], ((uint32_t)w & 1u) ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) { ok = false; break; }
-            tc_fence_after();
-          }
-          uint32_t acc = kb == kb0 ? 0u : 1u;
-#pragma unroll
-          for (int d = NDIAG; d < kSlices; d++)
-#pragma unroll
-            for (int p = 0; p <= d; p++, acc = 1u) product((uint32_t)(TAIL * bn), p, d - p, acc);
+          c++;
+        }
+        if (!ok) break;
+        if (issuer) {
+          tail(std::integral_constant<int, NDIAG + 1>{}, 1u);
           mma_commit(&ctl.empty[s]);
         }
-        if (ok) mma_commit(&ctl.tfull[TAIL]);
       }
-      mma_commit(&ctl.done);
-      mbar_drain(&ctl.done, 0);
+      if (ok && issuer) mma_commit(&ctl.tfull[TAIL]);
     }
+    if (issuer) mma_commit(&ctl.done);
+    mbar_drain(&ctl.done, 0);
   }
   } else {  // epilogue warps
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
@@ -338,19 +348,18 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!mbar_wait(&ctl.tfull[b], (uint32_t)(c / NROT) & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) return false;
         tc_fence_after();
         const uint32_t t0 = tl + (uint32_t)(b * bn);
-        // (16 columns a load, four warps a scheduler: a TMEM load takes about 200 cycles
-        // whatever its width)
+        // (16 columns a load: the sums take most of the registers)
 #pragma unroll
         for (int j = 0; j < HC; j += 16) {
           if (j < hc) {  // (columns past hc, within TMEM, are not used)
             uint32_t r[16];
             tmem_ld16_async(t0 + (uint32_t)j, r);
             tmem_wait16(r);
+            if (j + 16 >= hc) release(b);  // (all columns are in registers)
 #pragma unroll
             for (int i = 0; i < 16; i++) add_diag<D>(T[j + i], r[i]);
           }
         }
-        release(b);
         c++;
         return true;
       };
@@ -677,12 +686,9 @@ SliceEngine::SliceEngine(Ctx &ctx) : ctx_(ctx) {
 int SliceEngine::tile_n(int64_t N) { return (int)round_up(ceil_div(N, ceil_div(N, BN)), 8 * EPI); }
 
 namespace {
-// Cycles an SM spends on one K block of a unit of bn columns: 56 MMAs (no faster than 40
-// cycles each: issue and the A reads) and the fill of the stage share the shared-memory
-// port, about 10 % is lost between them.
-double block_cycles(int bn) {
-  return 1.1 * (56.0 * std::max(40.0, bn / 2.0) + kSlices * (BM + bn) * 64.0 / 70.0) + 500.0;
-}
+// Cycles an SM spends on one K block of a unit, measured: the five drains, one after the
+// other, take as long for few columns as for many.
+double block_cycles(int) { return 5750.0; }
 
 // Split-K of a product and its estimated time in us.  Rounds of units over the SMs times
 // the K blocks of a unit; a unit's epilogue costs about 90 cycles a column, partial sums

@@ -169,8 +169,8 @@ __device__ __forceinline__ void seg_of(const TcArgs &a, int kb, int &s, int &lkb
 // the MMA of the kernel's form (one CTA, or the pair)
 #define MMA_(...)                         \
   do {                                    \
-    if constexpr (PAIR) mma2_bf16(__VA_ARGS__); \
-    else mma_bf16(__VA_ARGS__);           \
+    if constexpr (PAIR) mma2_f16kind(__VA_ARGS__); \
+    else mma_f16kind(__VA_ARGS__);            \
   } while (0)
 
 template <int BN, int BK, bool PAIR = false>
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
   __shared__ float s_falpha, s_fuser;
   __shared__ int s_shift, s_shift_ok;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int tiles = a.tiles_m * a.tiles_n;
   const int nprob = a.gstart[a.ng];
   const int units = tiles * nprob * a.splits;
@@ -378,10 +378,15 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && (!PAIR || rank == 0)) {  // (pair: the rank-0 CTA issues for both)
+    if (!PAIR || rank == 0) {  // (pair: the rank-0 CTA issues for both)
+      // all lanes, issues by the elected one (see elect_one)
       int g = 0, c = 0;
       bool ok = true;
       const uint64_t desc = sw_desc<SH::SWZ>(smem_u32(smem)), desc64 = sw_desc<64>(smem_u32(smem));
+      const bool issuer = elect_one();
+      auto wait = [&](uint64_t *barrier, uint32_t parity, unsigned code) {
+        return __all_sync(0xffffffffu, mbar_wait(barrier, parity, a.err, code, a.wait_cycles)) != 0;
+      };
       for (int it = 0; it * nwork < units && ok; it++) {
         const int u = unit_at(it);
         if (u >= units) continue;
@@ -402,52 +407,48 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
           const uint32_t bph = (uint32_t)(c / NBUF) & 1u;
           const bool first = (kb - kb0) % a.kbd == 0;
           const bool last = (kb - kb0) % a.kbd == a.kbd - 1 || kb == kb1 - 1;
-          if (first && !mbar_wait(&tempty[b], bph ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) { ok = false; break; }
-          if (!mbar_wait(&full[s], ph, a.err, ERR_FULL_WAIT, a.wait_cycles)) { ok = false; break; }
+          if (first && !wait(&tempty[b], bph ^ 1u, ERR_EMPTY_WAIT)) { ok = false; break; }
+          if (!wait(&full[s], ph, ERR_FULL_WAIT)) { ok = false; break; }
           tc_fence_after();
           // operand descriptors of the stage: the four tiles lie at fixed offsets (the
-          // address field counts 16 bytes), K steps of 32 bytes.  Building one per MMA
-          // costs the issuing thread ~100 cycles each, more than an N = 128 MMA takes.
-          const uint64_t off = (uint64_t)s * (SH::STAGE_BYTES >> 4);
-          constexpr uint64_t oBhi = SH::A_BYTES >> 4, oAlo = (SH::A_BYTES + SH::B_BYTES) >> 4,
+          // address field counts 16 bytes), K steps of 32 bytes
+          const uint32_t off = (uint32_t)s * (SH::STAGE_BYTES >> 4);
+          constexpr uint32_t oBhi = SH::A_BYTES >> 4, oAlo = (SH::A_BYTES + SH::B_BYTES) >> 4,
                              oBlo = (2 * SH::A_BYTES + SH::B_BYTES) >> 4;
           const uint32_t d = tmem + (uint32_t)(b * BN);
-          uint32_t acc = first ? 0u : 1u;
-          if (SH::BK == 64 && a.seg[sg].bk == 32) {
-            // half-filled stage of a 32-wide segment: 64-byte rows, 64-byte swizzle
-            const uint64_t st = desc64 + off;
-            if (a.split3) {
+          if (issuer) {
+            uint32_t acc = first ? 0u : 1u;
+            auto products = [&](uint64_t base, auto steps) {
+              constexpr int KS = decltype(steps)::value;
+              const uint32_t st = (uint32_t)base + off, hi = (uint32_t)(base >> 32);
+              if (a.split3) {
 #pragma unroll
-              for (int k = 0; k < 2; k++, acc = 1) MMA_(d, st + oAlo + 2 * k, st + oBhi + 2 * k, id, acc);
+                for (int k = 0; k < KS; k++, acc = 1) MMA_(d, st + oAlo + 2 * k, st + oBhi + 2 * k, hi, id, acc);
 #pragma unroll
-              for (int k = 0; k < 2; k++) MMA_(d, st + 2 * k, st + oBlo + 2 * k, id, 1u);
+                for (int k = 0; k < KS; k++) MMA_(d, st + 2 * k, st + oBlo + 2 * k, hi, id, 1u);
+              }
+#pragma unroll
+              for (int k = 0; k < KS; k++, acc = 1) MMA_(d, st + 2 * k, st + oBhi + 2 * k, hi, id, acc);
+            };
+            // (a half-filled stage of a 32-wide segment: 64-byte rows, 64-byte swizzle)
+            if (SH::BK == 64 && a.seg[sg].bk == 32) products(desc64, std::integral_constant<int, 2>{});
+            else products(desc, std::integral_constant<int, SH::BK / 16>{});
+            if constexpr (PAIR) {
+              mma2_commit_both(&empty[s]);
+              if (last) mma2_commit_both(&tfull[b]);
+            } else {
+              mma_commit(&empty[s]);
+              if (last) mma_commit(&tfull[b]);
             }
-#pragma unroll
-            for (int k = 0; k < 2; k++, acc = 1) MMA_(d, st + 2 * k, st + oBhi + 2 * k, id, acc);
-          } else {
-            const uint64_t st = desc + off;
-            if (a.split3) {
-#pragma unroll
-              for (int k = 0; k < SH::BK / 16; k++, acc = 1) MMA_(d, st + oAlo + 2 * k, st + oBhi + 2 * k, id, acc);
-#pragma unroll
-              for (int k = 0; k < SH::BK / 16; k++) MMA_(d, st + 2 * k, st + oBlo + 2 * k, id, 1u);
-            }
-#pragma unroll
-            for (int k = 0; k < SH::BK / 16; k++, acc = 1) MMA_(d, st + 2 * k, st + oBhi + 2 * k, id, acc);
-          }
-          if constexpr (PAIR) {
-            mma2_commit_both(&empty[s]);
-            if (last) mma2_commit_both(&tfull[b]);
-          } else {
-            mma_commit(&empty[s]);
-            if (last) mma_commit(&tfull[b]);
           }
           if (last) c++;
         }
       }
       // every MMA issued above has completed once `done` fires
-      if constexpr (PAIR) mma2_commit(done);
-      else mma_commit(done);
+      if (issuer) {
+        if constexpr (PAIR) mma2_commit(done);
+        else mma_commit(done);
+      }
       mbar_drain(done, 0);
     }
   }

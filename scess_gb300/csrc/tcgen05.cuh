@@ -103,13 +103,31 @@ __device__ __forceinline__ uint32_t idesc_f16kind(int M, int N, uint32_t ab_fmt)
          ((uint32_t)(M >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                         uint32_t idesc, uint32_t accum) {
+// One lane of a converged warp, the same at every call.  The issuing warp runs its loop
+// with all lanes and issues under this predicate: what the loop computes is then uniform
+// and stays in uniform registers.  With the loop inside `if (lane == 0)` every operand of
+// every MMA is moved there one by one: beside four busy warps a scheduler that took 88
+// cycles per MMA, more than an N = 128 MMA's 64, against 47 this way.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum));
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(one));
+  return one != 0;
+}
+
+// Operands by the low words of their descriptors (address field) and the high word they share.
+__device__ __forceinline__ void mma_f16kind(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t hi,
+                                            uint32_t idesc, uint32_t accum) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %3};\n\t"
+      "mov.b64 b, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}\n" ::"r"(tmem_d),
+      "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accum));
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {
@@ -122,13 +140,15 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
 // M = 256 over the pair: A rows 0-127 from this CTA's shared memory, 128-255
 // from the peer's at the same offset; B columns split likewise (N/2 each); D
 // rows 0-127 in this SM's TMEM, 128-255 in the peer's.
-__device__ __forceinline__ void mma2_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                          uint32_t idesc, uint32_t accum) {
+__device__ __forceinline__ void mma2_f16kind(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t hi,
+                                             uint32_t idesc, uint32_t accum) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum));
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %3};\n\t"
+      "mov.b64 b, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %4, p;\n\t}\n" ::"r"(tmem_d),
+      "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accum));
 }
 // Arrive on the barrier at this offset in both CTAs of the pair once the
 // issued MMAs have completed.

@@ -235,7 +235,7 @@ std::vector<uint32_t> orbit_table(int64_t o) {
 // L2).  WS keeps (Y, W) pairs in shared memory: six 8-byte reads per orbit.  Where two
 // such CTAs don't fit an SM (o >= 24) only Y is kept and W = Y - V recomputed from the
 // (ia|jb) slices: 24 reads and 18 multiply-adds per orbit.  At o = 20 and 1728 triples:
-// 45.5 us with V recomputed and the energies added per orbit, 38.3 this way; o = 13: 37.1, 34.0.
+// 45.5 us with V recomputed and the energies added per orbit, 38.3 this way.
 constexpr int kEnergyMaxO = 32;
 template <int NW, bool WS>
 __global__ void __launch_bounds__(256, 4) triples_energy_orbit_kernel(
