@@ -562,11 +562,19 @@ namespace {
 bool prefer_slices(const TableGemm &g) {
   const int64_t route = tune_value("f64", 0);
   if (route == 1) return g.K > 0 && SliceEngine::usable(g.M, g.N);
-  return route != 2 && g.K > 0 && SliceEngine::usable(g.M, g.N) && SliceEngine::estimate_us(g.M, g.N, g.K) < dgemm_small_us(g);
+  return route != 2 && g.K > 0 && SliceEngine::usable(g.M, g.N) && 
+         SliceEngine::estimate_us(g.M, g.N, g.K) < std::min(dgemm_small_us(g), skinny64_us(g));
 }
 
-// C = alpha A.B + beta C on the FP64 units: cut finely unless that takes too many CTAs.
-void dfma_gemm(Ctx &ctx, const TableGemm &g) {
+// C = alpha A.B + beta C on the FP64 units: short K against a long side, or cut finely
+// unless that takes too many CTAs.  cUnitM, cUnitN: C's unit stride, if known.
+void dfma_gemm(Ctx &ctx, const TableGemm &g, bool cUnitM, bool cUnitN) {
+  if (skinny64_us(g) < dgemm_small_us(g)) {
+    const bool small_is_a = g.M <= g.N;
+    TimedScope ts(ctx.timer, "skinny64", 2.0 * g.M * g.N * g.K, 0.0, ctx.stream);
+    skinny_table(g, small_is_a, small_is_a ? cUnitM : cUnitN, true, ctx.stream);
+    return;
+  }
   if (g.K > 0 && dgemm_small_us(g) < 2000.0) {
     TimedScope ts(ctx.timer, "dgemm_small", 2.0 * g.M * g.N * g.K, 0.0, ctx.stream);
     dgemm_small(g, ctx.ensure_workspace(dgemm_small_workspace(g)), ctx.counters.as<int>(), ctx.stream);
@@ -613,7 +621,7 @@ void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, 
     g.beta = beta;
     const std::string tname = std::string("skinny[") + spec + "]";
     TimedScope ts(ctx.timer, tname.c_str(), 2.0 * pl.M * pl.N * pl.K, 0.0, ctx.stream);
-    skinny_table(g, small_is_a, small_is_a ? pl.cUnitM : pl.cUnitN, ctx.stream);
+    skinny_table(g, small_is_a, small_is_a ? pl.cUnitM : pl.cUnitN, false, ctx.stream);
     return;
   }
   if ((be == Backend::MIXED && TcEngine::worth_it(pl)) || be == Backend::TENSOR) {
@@ -660,13 +668,13 @@ void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, 
   if (prefer_slices(g) &&
       ctx.slice_engine().contract(pl, alpha, A.p, B.p, beta, C.p, constA, constB))
     return;
-  dfma_gemm(ctx, g);
+  dfma_gemm(ctx, g, pl.cUnitM, pl.cUnitN);
 }
 
 void fp64_table_gemm(Ctx &ctx, const TableGemm &g, const char *name) {
   if (prefer_slices(g) && ctx.slice_engine().table_gemm(g, name))
     return;
-  dfma_gemm(ctx, g);
+  dfma_gemm(ctx, g, false, false);
 }
 
 void permute(Ctx &ctx, const char *spec, double alpha, const TV &X, double beta, const TV &Y) {

@@ -77,6 +77,8 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(TableGemm g, int64_t k
   __shared__ int last;
   const int t = threadIdx.x, grp = t >> 6, o = t & 63, i = o % tm, j = o / tm;
   const int im = 65536 / tm + 1, in = 65536 / tn + 1;  // (exact for e below 4096)
+  // a staged range: K or kSmallKB, rounded up to a power of two
+  const int ks = 32 - __clz((int)min((int64_t)kSmallKB, min(kper, g.K)) - 1), km = (1 << ks) - 1;
   const int64_t ntm = (g.M + tm - 1) / tm;
   const int64_t tile = blockIdx.x / splits, z = blockIdx.x % splits;
   const int64_t m0 = (tile % ntm) * tm, n0 = (tile / ntm) * tn;
@@ -87,15 +89,15 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(TableGemm g, int64_t k
     const int nk = (int)min((int64_t)kSmallKB, ke - k0);
     __syncthreads();  // the previous range is used up
     // element e of a side: along its unit-stride index, else along k
-    for (int e0 = t; e0 < max(tm, tn) * kSmallKB; e0 += 4 * 256) {
+    for (int e0 = t; e0 < max(tm, tn) << ks; e0 += 4 * 256) {
       int64_t ra[4], rb[4];
       double a[4], b[4];
 #pragma unroll
       for (int p = 0; p < 4; p++) {
         const int e = e0 + 256 * p;
         const int qm = (e * im) >> 16, qn = (e * in) >> 16;  // e / tm, e / tn
-        const int am = g.aUnitM ? e - qm * tm : e >> 7, ak = g.aUnitM ? qm : e & 127;
-        const int bm = g.bUnitN ? e - qn * tn : e >> 7, bk = g.bUnitN ? qn : e & 127;
+        const int am = g.aUnitM ? e - qm * tm : e >> ks, ak = g.aUnitM ? qm : e & km;
+        const int bm = g.bUnitN ? e - qn * tn : e >> ks, bk = g.bUnitN ? qn : e & km;
         ra[p] = (am < tm && m0 + am < g.M && ak < nk) ? g.rowA[m0 + am] + g.kA[k0 + ak] : -1;
         rb[p] = (bm < tn && n0 + bm < g.N && bk < nk) ? g.colB[n0 + bm] + g.kB[k0 + bk] : -1;
       }
@@ -108,8 +110,8 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(TableGemm g, int64_t k
       for (int p = 0; p < 4; p++) {
         const int e = e0 + 256 * p;
         const int qm = (e * im) >> 16, qn = (e * in) >> 16;  // e / tm, e / tn
-        const int am = g.aUnitM ? e - qm * tm : e >> 7, ak = g.aUnitM ? qm : e & 127;
-        const int bm = g.bUnitN ? e - qn * tn : e >> 7, bk = g.bUnitN ? qn : e & 127;
+        const int am = g.aUnitM ? e - qm * tm : e >> ks, ak = g.aUnitM ? qm : e & km;
+        const int bm = g.bUnitN ? e - qn * tn : e >> ks, bk = g.bUnitN ? qn : e & km;
         if (am < tm && ak < nk) As[ak][am] = a[p];
         if (bm < tn && bk < nk) Bs[bk][bm] = b[p];
       }
@@ -221,10 +223,10 @@ double dgemm_small_us(const TableGemm &g) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0) return 1e30;
   const SmallShape s = small_shape(g);
   if ((double)s.tiles * s.splits > 2.0e9) return 1e30;
-  // 4 us of latency, padded multiply-adds at two lanes a cycle and SM, 2.5 us for every
-  // six CTAs of an SM
-  const double fma = (double)s.tiles * (double)round_up(s.tm * s.tn, 32) * (double)g.K;
-  return 4.0 + fma / (2.0 * kNumSMs * 1900.0) + 2.5 * (double)(s.tiles * s.splits) / (6.0 * kNumSMs);
+  // Measured: 6 us, and the larger of padded multiply-adds at two lanes a cycle and SM
+  // (80 % reached) and 88 ns for a thousand outputs (staging, tables, C).
+  const double fma = 1.25 * (double)s.tiles * (double)round_up(s.tm * s.tn, 32) * (double)g.K / (2.0 * kNumSMs * 1900.0);
+  return 6.0 + std::hypot(fma, 8.8e-5 * (double)g.M * (double)g.N);
 }
 
 int64_t dgemm_small_workspace(const TableGemm &g) {
@@ -246,13 +248,15 @@ struct SkinnyArgs {
   const double *Sm, *Lg;
   double *C;
   const int64_t *sR, *sK, *lR, *lK, *cS, *cL;
-  int s, sp, K;  // sp: s rounded up to 4
+  int s, sp, K;        // sp: s rounded up to 4
+  int chunk, nchunks;  // small indices of a warp's item (a multiple of 32, or all)
   int64_t l;
-  float alpha;
+  double alpha;
   double beta;
 };
 
-__device__ __forceinline__ void skinny_out(double *p, float v, double beta) {
+template <typename T>
+__device__ __forceinline__ void skinny_out(double *p, T v, double beta) {
   if (beta == 1.0) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"((double)v) : "memory");
   } else if (beta == 0.0) {
@@ -262,78 +266,77 @@ __device__ __forceinline__ void skinny_out(double *p, float v, double beta) {
   }
 }
 
-// Persistent: each block stages the small operand once (FP32, [k][m]) and its
-// warps walk tiles of 32 long indices, one per lane, with the lane's K long
-// values in registers; every shared load of four small-side values (a 16-byte
-// broadcast) feeds four FMAs.
-template <bool STAGE>
+// Persistent: each block stages the small operand once ([k][m], T = FP32 of the mixed form
+// or FP64) and its warps walk items of 32 long indices, one per lane, and a chunk of the
+// small ones, with the lane's K long values in registers; every shared load of four
+// small-side values (16-byte broadcasts) feeds four multiply-adds.  Neighbouring items go
+// to different SMs: with few of them (9000 x 10 x 90: 282 tiles of 32) eight to a block would
+// leave most SMs idle.  FP64 is bound by its units: 10 x 81000 x 10 takes 42 us
+// (dgemm_small 130; sliced 29 and 27 for the packs).
+template <typename T, bool STAGE>
 __global__ void __launch_bounds__(256) skinny_kernel(SkinnyArgs a) {
   extern __shared__ __align__(16) unsigned char sk_raw[];
-  float4 *sS4 = reinterpret_cast<float4 *>(sk_raw);                  // [K][sp / 4]
-  int64_t *cSs = reinterpret_cast<int64_t *>(sS4 + a.K * (a.sp / 4));  // [s]
+  T *sS = reinterpret_cast<T *>(sk_raw);                             // [K][sp]
+  int64_t *cSs = reinterpret_cast<int64_t *>(sS + a.K * a.sp);       // [s]
   int64_t *lKs = cSs + a.sp;                                         // [K]
-  float *stage = reinterpret_cast<float *>(lKs + kSkinnyMaxK);       // [8][32][33] (STAGE)
-  float *sS = reinterpret_cast<float *>(sS4);
+  T *stage = reinterpret_cast<T *>(lKs + kSkinnyMaxK);               // [8][32][33] (STAGE)
   for (int e = threadIdx.x; e < a.K * a.sp; e += blockDim.x) {
     const int m = e % a.sp, k = e / a.sp;
-    sS[e] = m < a.s ? (float)a.Sm[a.sR[m] + a.sK[k]] : 0.0f;
+    sS[e] = m < a.s ? (T)a.Sm[a.sR[m] + a.sK[k]] : T(0);
   }
   for (int m = threadIdx.x; m < a.s; m += blockDim.x) cSs[m] = a.cS[m];
   for (int k = threadIdx.x; k < a.K; k += blockDim.x) lKs[k] = a.lK[k];
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t tiles = (a.l + 31) / 32;
-  for (int64_t t = (int64_t)blockIdx.x * 8 + w; t < tiles; t += (int64_t)gridDim.x * 8) {
+  const T alpha = (T)a.alpha;
+  const int64_t items = (a.l + 31) / 32 * a.nchunks;
+  for (int64_t it = (int64_t)w * gridDim.x + blockIdx.x; it < items; it += (int64_t)gridDim.x * 8) {
+    const int64_t t = it / a.nchunks;
+    const int ms = (int)(it - t * a.nchunks) * a.chunk, me = min(a.s, ms + a.chunk);
     const int64_t n = t * 32 + lane;
     const bool ok = n < a.l;
     const int64_t lr = ok ? a.lR[n] : 0, cl = ok ? a.cL[n] : 0;
-    float lv[kSkinnyMaxK];
+    T lv[kSkinnyMaxK];
 #pragma unroll
-    for (int k = 0; k < kSkinnyMaxK; k++) lv[k] = (ok && k < a.K) ? (float)a.Lg[lr + lKs[k]] : 0.0f;
-    if (!STAGE) {
-      for (int m4 = 0; m4 < a.sp / 4; m4++) {
-        float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
+    for (int k = 0; k < kSkinnyMaxK; k++) lv[k] = (ok && k < a.K) ? (T)a.Lg[lr + lKs[k]] : T(0);
+    // four results C(m .. m + 3, n)
+    auto quad = [&](int m, T *c) {
+      c[0] = c[1] = c[2] = c[3] = T(0);
 #pragma unroll
-        for (int k = 0; k < kSkinnyMaxK; k++) {
-          if (k < a.K) {
-            const float4 q = sS4[k * (a.sp / 4) + m4];
-            c0 = fmaf(q.x, lv[k], c0);
-            c1 = fmaf(q.y, lv[k], c1);
-            c2 = fmaf(q.z, lv[k], c2);
-            c3 = fmaf(q.w, lv[k], c3);
+      for (int k = 0; k < kSkinnyMaxK; k++) {
+        if (k < a.K) {
+          alignas(16) T q[4];
+          const T *src = sS + k * a.sp + m;
+          if constexpr (sizeof(T) == 4) {
+            *reinterpret_cast<float4 *>(q) = *reinterpret_cast<const float4 *>(src);
+          } else {
+            *reinterpret_cast<double2 *>(q) = *reinterpret_cast<const double2 *>(src);
+            *reinterpret_cast<double2 *>(q + 2) = *reinterpret_cast<const double2 *>(src + 2);
           }
+#pragma unroll
+          for (int x = 0; x < 4; x++) c[x] = fma(q[x], lv[k], c[x]);
         }
+      }
+    };
+    if (!STAGE) {
+      for (int m = ms; m < me; m += 4) {
+        T c[4];
+        quad(m, c);
         if (!ok) continue;
-        const int m = 4 * m4;
-        skinny_out(a.C + cSs[m] + cl, a.alpha * c0, a.beta);
-        if (m + 1 < a.s) skinny_out(a.C + cSs[m + 1] + cl, a.alpha * c1, a.beta);
-        if (m + 2 < a.s) skinny_out(a.C + cSs[m + 2] + cl, a.alpha * c2, a.beta);
-        if (m + 3 < a.s) skinny_out(a.C + cSs[m + 3] + cl, a.alpha * c3, a.beta);
+#pragma unroll
+        for (int x = 0; x < 4; x++)
+          if (m + x < a.s) skinny_out(a.C + cSs[m + x] + cl, alpha * c[x], a.beta);
       }
     } else {
-      float *st = stage + w * 32 * 33;
-      for (int m0 = 0; m0 < a.s; m0 += 32) {
+      T *st = stage + w * 32 * 33;
+      for (int m0 = ms; m0 < me; m0 += 32) {
         // this lane's 32 results C(m0 .. m0 + 31, n) into its row of the stage
+#pragma unroll 1
+        for (int j = 0; j < 32 && m0 + j < a.sp; j += 4) {
+          T c[4];
+          quad(m0 + j, c);
 #pragma unroll
-        for (int j4 = 0; j4 < 8; j4++) {
-          float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
-          const int m4 = m0 / 4 + j4;
-          if (4 * m4 < a.sp) {
-#pragma unroll
-            for (int k = 0; k < kSkinnyMaxK; k++) {
-              if (k < a.K) {
-                const float4 q = sS4[k * (a.sp / 4) + m4];
-                c0 = fmaf(q.x, lv[k], c0);
-                c1 = fmaf(q.y, lv[k], c1);
-                c2 = fmaf(q.z, lv[k], c2);
-                c3 = fmaf(q.w, lv[k], c3);
-              }
-            }
-          }
-          st[lane * 33 + 4 * j4] = a.alpha * c0;
-          st[lane * 33 + 4 * j4 + 1] = a.alpha * c1;
-          st[lane * 33 + 4 * j4 + 2] = a.alpha * c2;
-          st[lane * 33 + 4 * j4 + 3] = a.alpha * c3;
+          for (int x = 0; x < 4; x++) st[lane * 33 + j + x] = alpha * c[x];
         }
         __syncwarp();
         // lanes along the small side: column n' of the tile, rows m0 + lane
@@ -347,9 +350,31 @@ __global__ void __launch_bounds__(256) skinny_kernel(SkinnyArgs a) {
     }
   }
 }
+
+// Small indices of an item: with few tiles of 32 long ones, chunks of 32 apart.
+int64_t skinny_chunk(int64_t s, int64_t l) {
+  const int64_t sp = round_up(s, 4);
+  return ceil_div(l, 32) >= 16 * kNumSMs ? sp : std::min<int64_t>(32, sp);
+}
+
+template <typename T>
+void skinny_launch(SkinnyArgs a, bool stage, cudaStream_t stream) {
+  const int64_t tiles = ceil_div(a.l, 32);
+  a.chunk = (int)skinny_chunk(a.s, a.l);
+  a.nchunks = (int)ceil_div(a.s, a.chunk);
+  const int64_t items = tiles * a.nchunks;
+  const unsigned blocks = (unsigned)std::max<int64_t>(std::min<int64_t>(items, kNumSMs),
+                                                      std::min<int64_t>(ceil_div(items, 8), (sizeof(T) == 4 ? 4 : 2) * kNumSMs));
+  const size_t smem = (size_t)a.K * a.sp * sizeof(T) + (size_t)(a.sp + kSkinnyMaxK) * sizeof(int64_t) +
+                      (stage ? (size_t)8 * 32 * 33 * sizeof(T) : 0);
+  const auto kernel = stage ? skinny_kernel<T, true> : skinny_kernel<T, false>;
+  SCESS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<blocks, 256, smem, stream>>>(a);
+  SCESS_CHECK_LAUNCH();
+}
 }  // namespace
 
-void skinny_table(const TableGemm &g, bool small_is_a, bool stage, cudaStream_t stream) {
+void skinny_table(const TableGemm &g, bool small_is_a, bool stage, bool fp64, cudaStream_t stream) {
   SkinnyArgs a;
   a.Sm = (small_is_a ? g.A + g.baseA : g.B + g.baseB);
   a.Lg = (small_is_a ? g.B + g.baseB : g.A + g.baseA);
@@ -367,20 +392,19 @@ void skinny_table(const TableGemm &g, bool small_is_a, bool stage, cudaStream_t 
   a.sp = (int)round_up(s, 4);
   a.K = (int)g.K;
   a.l = l;
-  a.alpha = (float)g.alpha;
+  a.alpha = g.alpha;
   a.beta = g.beta;
-  const size_t smem = (size_t)a.K * a.sp * sizeof(float) + (size_t)(a.sp + kSkinnyMaxK) * sizeof(int64_t) +
-                      (stage ? (size_t)8 * 32 * 33 * sizeof(float) : 0);
-  const int64_t tiles = ceil_div(l, 32);
-  const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(tiles, 8), 4 * kNumSMs));
-  if (stage) {
-    SCESS_CUDA(cudaFuncSetAttribute(skinny_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    skinny_kernel<true><<<blocks, 256, smem, stream>>>(a);
-  } else {
-    SCESS_CUDA(cudaFuncSetAttribute(skinny_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    skinny_kernel<false><<<blocks, 256, smem, stream>>>(a);
-  }
-  SCESS_CHECK_LAUNCH();
+  if (fp64) skinny_launch<double>(a, stage, stream);
+  else skinny_launch<float>(a, stage, stream);
+}
+
+double skinny64_us(const TableGemm &g) {
+  const int64_t s = std::min(g.M, g.N), l = std::max(g.M, g.N);
+  if (g.K < 1 || g.K > kSkinnyMaxK || s < 1 || s > kSkinnyMaxS) return 1e30;
+  // 6 us of latency, then the FP64 units of the SM with the most items, or C written and read
+  const int64_t chunk = skinny_chunk(s, l), items = ceil_div(l, 32) * ceil_div(s, chunk);
+  const double fma = (double)ceil_div(items, kNumSMs) * 32.0 * (double)chunk * (double)(g.K + 2);
+  return 6.0 + std::max(fma / (2.0 * 1900.0), (double)s * (double)l * 16.0 / 5.0e6);
 }
 
 void dgemv_table(const TableGemm &g, cudaStream_t stream) {

@@ -31,7 +31,9 @@ struct TableGemm {
 // stage: C's unit-stride index is on the small side (stores are then staged
 // through shared memory so that lanes run along it).
 constexpr int kSkinnyMaxK = 32, kSkinnyMaxS = 256;
-void skinny_table(const TableGemm &g, bool small_is_a, bool stage, cudaStream_t stream);
+void skinny_table(const TableGemm &g, bool small_is_a, bool stage, bool fp64, cudaStream_t stream);
+// Estimated time of the FP64 form (1e30 where the shape is none of its).
+double skinny64_us(const TableGemm &g);
 
 // The same contraction for small products, cut finely over the device; workspace of
 // dgemm_small_workspace doubles for the K ranges' partial sums, counters: kSmallCounters
