@@ -29,6 +29,7 @@
 #include "gemm_slice.h"
 #include "pack_tiles.cuh"
 #include "slice_math.cuh"
+#include "split_sum.cuh"
 #include "tcgen05.cuh"
 
 namespace scess {
@@ -433,20 +434,16 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
 }
 
-// Split-K: C = alpha sum_z partial_z + beta C over unmarked outputs, z in order.
-__global__ void slice_reduce_kernel(SliceArgs a, int splits) {
-  const int64_t MN = (int64_t)a.M * a.N;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < MN;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t m = e % a.M, n = e / a.M;
-    if (a.expA[m] == kRowNonFinite || a.expB[n] == kRowNonFinite) continue;
-    double s = 0.0;
-    for (int z = 0; z < splits; z++) s += a.partial[(int64_t)z * MN + e];
+// Split-K: C = alpha sum_z partial_z + beta C over unmarked outputs.
+template <int ZG>
+__global__ void __launch_bounds__(256) slice_reduce_kernel(const __grid_constant__ SliceArgs a, int splits) {
+  split_sum<ZG>(a.partial, a.M, a.N, splits, [&](int64_t m, int64_t n, double s) {
+    if (a.expA[m] == kRowNonFinite || a.expB[n] == kRowNonFinite) return;
     double *p = a.C + a.baseC + a.rowC[0][m] + a.colC[0][n];
     double val = a.alpha * s;
     if (a.beta != 0.0) val += a.beta * *p;
     *p = val;
-  }
+  });
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -930,8 +927,9 @@ void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial)
   slice_gemm_kernel<<<(unsigned)std::min<int64_t>(units, kNumSMs), THREADS, SMEM_BYTES, ctx_.stream>>>(maps, a);
   SCESS_CHECK_LAUNCH();
   if (a.splits > 1) {
-    slice_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div(ps.M * ps.N, 256), 8192), 256, 0, ctx_.stream>>>(
-        a, a.splits);
+    const bool groups = split_groups(ps.M * ps.N, a.splits);
+    const auto reduce = groups ? slice_reduce_kernel<kSplitGroups> : slice_reduce_kernel<1>;
+    reduce<<<split_blocks(ps.M * ps.N, groups), 256, 0, ctx_.stream>>>(a, a.splits);
     SCESS_CHECK_LAUNCH();
   }
 }
