@@ -27,6 +27,7 @@
 
 #include "dgemm_tile.cuh"
 #include "gemm_slice.h"
+#include "launch.cuh"
 #include "pack_tiles.cuh"
 #include "slice_math.cuh"
 #include "split_sum.cuh"
@@ -170,6 +171,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = ctl.tmem;
+  chain();
 
   // unit -> (tile m, tile n, problem y, z, g, K-block range, split)
   auto unit_coords = [&](int u, int &tm, int &tn, int &py, int &pz, int &pg, int &kb0, int &kb1, int &sp) {
@@ -437,6 +439,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 // Split-K: C = alpha sum_z partial_z + beta C over unmarked outputs.
 template <int ZG>
 __global__ void __launch_bounds__(256) slice_reduce_kernel(const __grid_constant__ SliceArgs a, int splits) {
+  chain();
   split_sum<ZG>(a.partial, a.M, a.N, splits, [&](int64_t m, int64_t n, double s) {
     if (a.expA[m] == kRowNonFinite || a.expB[n] == kRowNonFinite) return;
     double *p = a.C + a.baseC + a.rowC[0][m] + a.colC[0][n];
@@ -478,6 +481,7 @@ __device__ __forceinline__ int tile_col(int k) { return k + (k >> 3); }
 
 template <int KT>
 __global__ void __launch_bounds__(256) slice_pack_kernel(const __grid_constant__ PackOps ops) {
+  chain();
   const bool second = blockIdx.x >= ops.op[0].blocks;
   const PackOp &op = ops.op[second ? 1 : 0];
   const int64_t blk = second ? blockIdx.x - ops.op[0].blocks : blockIdx.x;
@@ -610,14 +614,15 @@ void launch_packs(const PackOp *op, int n, cudaStream_t stream) {  // (the opera
   const int64_t blocks = op[0].blocks + (n > 1 ? op[1].blocks : 0);
   if (blocks > INT32_MAX) throw Error(SCESS_ERR_INVALID, "slice pack: too large");
   const int kt = pack_kt(op[0].K);
-  if (kt == 16) slice_pack_kernel<16><<<(unsigned)blocks, 256, 0, stream>>>(p);
-  else if (kt == 32) slice_pack_kernel<32><<<(unsigned)blocks, 256, 0, stream>>>(p);
-  else slice_pack_kernel<64><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  if (kt == 16) launch(slice_pack_kernel<16>, (unsigned)blocks, 256, 0, stream, p);
+  else if (kt == 32) launch(slice_pack_kernel<32>, (unsigned)blocks, 256, 0, stream, p);
+  else launch(slice_pack_kernel<64>, (unsigned)blocks, 256, 0, stream, p);
   SCESS_CHECK_LAUNCH();
 }
 
 __global__ void __launch_bounds__(256) dgemm_masked_kernel(TableGemm g, const int *__restrict__ expA,
                                                            const int *__restrict__ expB) {
+  chain();
   const int64_t tm = (g.M + kDgemmTile - 1) / kDgemmTile, tn = (g.N + kDgemmTile - 1) / kDgemmTile;
   const int t = threadIdx.x;
   for (int64_t tile = blockIdx.x; tile < tm * tn; tile += gridDim.x) {
@@ -671,7 +676,7 @@ bool kernel_ok() {
 
 void dgemm_masked(const TableGemm &g, const int *expA, const int *expB, cudaStream_t stream) {
   const int64_t tiles = ceil_div(g.M, kDgemmTile) * ceil_div(g.N, kDgemmTile);
-  dgemm_masked_kernel<<<(unsigned)std::min<int64_t>(tiles, 4 * kNumSMs), 256, 0, stream>>>(g, expA, expB);
+  launch(dgemm_masked_kernel, (unsigned)std::min<int64_t>(tiles, 4 * kNumSMs), 256, 0, stream, g, expA, expB);
   SCESS_CHECK_LAUNCH();
 }
 
@@ -924,12 +929,12 @@ void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial)
   const int64_t units = (int64_t)a.tiles_m * a.tiles_n * start * a.splits;
   if (units > INT32_MAX) throw Error(SCESS_ERR_INVALID, "slice gemm: too many work units");
   launched_ = true;
-  slice_gemm_kernel<<<(unsigned)std::min<int64_t>(units, kNumSMs), THREADS, SMEM_BYTES, ctx_.stream>>>(maps, a);
+  scess::launch(slice_gemm_kernel, (unsigned)std::min<int64_t>(units, kNumSMs), THREADS, SMEM_BYTES, ctx_.stream, maps, a);
   SCESS_CHECK_LAUNCH();
   if (a.splits > 1) {
     const bool groups = split_groups(ps.M * ps.N, a.splits);
     const auto reduce = groups ? slice_reduce_kernel<kSplitGroups> : slice_reduce_kernel<1>;
-    reduce<<<split_blocks(ps.M * ps.N, groups), 256, 0, ctx_.stream>>>(a, a.splits);
+    scess::launch(reduce, split_blocks(ps.M * ps.N, groups), 256, 0, ctx_.stream, a, a.splits);
     SCESS_CHECK_LAUNCH();
   }
 }

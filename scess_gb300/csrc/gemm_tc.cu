@@ -24,6 +24,7 @@
 #include <mutex>
 
 #include "gemm_tc.h"
+#include "launch.cuh"
 #include "pack_tiles.cuh"
 #include "split_sum.cuh"
 #include "tcgen05.cuh"
@@ -177,6 +178,7 @@ __device__ __forceinline__ void seg_of(const TcArgs &a, int kb, int &s, int &lkb
 template <int BN, int BK, bool PAIR = false>
 __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcOut out, TcArgs a) {
+  if constexpr (BN == 128) chain();  // (the grouped launches wait later: see below)
   using SH = TcShape<BN, BK, PAIR>;
   constexpr int STAGES = SH::STAGES, NBUF = SH::NBUF, HC = 128;
   extern __shared__ uint8_t smem_raw[];
@@ -814,6 +816,7 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
 template <int ZG>
 __global__ void __launch_bounds__(256) tc_reduce_kernel(TcOut out, int64_t M, int64_t N, int splits,
                                                         const float *__restrict__ partial) {
+  chain();
   __shared__ double s_alpha;
   if (threadIdx.x == 0) {
     double alpha = out.alpha;
@@ -851,6 +854,7 @@ __global__ void __launch_bounds__(256) maxabs_kernel(
     const double *__restrict__ src, const int64_t *__restrict__ rowOff, int64_t rows,
     const int64_t *__restrict__ kOff, int64_t K, int unitK, unsigned *__restrict__ maxbits,
     int64_t rs, int64_t ks, const RowTiles rt) {
+  chain();
   __shared__ int64_t sr[32], sk[64];
   __shared__ float red[8];
   const int t = threadIdx.x;
@@ -890,6 +894,7 @@ __global__ void __launch_bounds__(256) maxabs_kernel(
 // max|x| over n contiguous values (a gather that covers its source span).
 __global__ void __launch_bounds__(256) maxabs_flat_kernel(const double *__restrict__ src, int64_t n,
                                                           unsigned *__restrict__ maxbits) {
+  chain();
   __shared__ float red[8];
   float m = 0.0f;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -941,6 +946,7 @@ __global__ void __launch_bounds__(256) pack_split_kernel(
     const int64_t *__restrict__ kOff, int64_t K, int unitK, uint16_t *__restrict__ dst,
     int64_t Kpad, const unsigned *__restrict__ maxbits, double *__restrict__ scale_out,
     int negate, int64_t rs, int64_t ks, const RowTiles rt) {
+  chain();
   __shared__ double tile[32][65];
   __shared__ int64_t sr[32], sk[64], srow[32];
   const int t = threadIdx.x;
@@ -1238,13 +1244,12 @@ void tc_gemm_launch_grouped(const TcProblemSet &ps, TcFormat fmt, const TcOut &o
     tc_gemm_kernel<256, 64><<<grid, TcShape<256, 64>::THREADS, TcShape<256, 64>::SMEM_BYTES, stream>>>(
         maps, out, a);
   else
-    tc_gemm_kernel<128, 64><<<grid, TcShape<128, 64>::THREADS, TcShape<128, 64>::SMEM_BYTES, stream>>>(
-        maps, out, a);
+    launch(tc_gemm_kernel<128, 64>, grid, TcShape<128, 64>::THREADS, TcShape<128, 64>::SMEM_BYTES, stream, maps, out, a);
   SCESS_CHECK_LAUNCH();
   if (splits > 1) {
     const bool groups = split_groups(ps.M * ps.N, splits);
     const auto reduce = groups ? tc_reduce_kernel<kSplitGroups> : tc_reduce_kernel<1>;
-    reduce<<<split_blocks(ps.M * ps.N, groups), 256, 0, stream>>>(out, ps.M, ps.N, splits, partial);
+    launch(reduce, split_blocks(ps.M * ps.N, groups), 256, 0, stream, out, ps.M, ps.N, splits, partial);
     SCESS_CHECK_LAUNCH();
   }
 }
@@ -1360,41 +1365,41 @@ void TcEngine::pack(const double *src, const int64_t *rowOff, int64_t rows, cons
     if (h.p == src) hint = hint_words_.as<unsigned>() + h.slot;
   if (fmt_ == TcFormat::FP16 && hint) {  // the tensor's maximum, reduced once
     if (aff)
-      pack_split_kernel<true, true><<<grid, 256, 0, ctx_.stream>>>(src, nullptr, rows, nullptr, K, u, dst,
-                                                                   Kpad, hint, scale, 0, rs, ks, rt);
+      launch(pack_split_kernel<true, true>, grid, 256, 0, ctx_.stream, src, nullptr, rows, nullptr, K, u, dst,
+             Kpad, hint, scale, 0, rs, ks, rt);
     else
-      pack_split_kernel<true, false><<<grid, 256, 0, ctx_.stream>>>(src, rowOff, rows, kOff, K, u, dst,
-                                                                    Kpad, hint, scale, 0, 0, 0, rt);
+      launch(pack_split_kernel<true, false>, grid, 256, 0, ctx_.stream, src, rowOff, rows, kOff, K, u, dst,
+             Kpad, hint, scale, 0, 0, 0, rt);
   } else if (fmt_ == TcFormat::FP16) {
     SCESS_CUDA(cudaMemsetAsync(maxbits, 0, sizeof(unsigned), ctx_.stream));
     const int64_t n = rows * K;
     if (dense || (aff && ((rs == 1 && ks == rows) || (ks == 1 && rs == K)))) {  // the gather is src[0, n)
       const unsigned blocks =
           (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256 * 8), 8 * kNumSMs));
-      maxabs_flat_kernel<<<blocks, 256, 0, ctx_.stream>>>(src, n, maxbits);
+      launch(maxabs_flat_kernel, blocks, 256, 0, ctx_.stream, src, n, maxbits);
     } else if (aff) {
-      maxabs_kernel<true><<<maxabs_blocks(rt, K), 256, 0, ctx_.stream>>>(src, nullptr, rows, nullptr,
-                                                                        K, u, maxbits, rs, ks, rt);
+      launch(maxabs_kernel<true>, maxabs_blocks(rt, K), 256, 0, ctx_.stream, src, nullptr, rows, nullptr, K, u,
+             maxbits, rs, ks, rt);
     } else {
-      maxabs_kernel<false><<<maxabs_blocks(rt, K), 256, 0, ctx_.stream>>>(src, rowOff, rows, kOff, K,
-                                                                         u, maxbits, 0, 0, rt);
+      launch(maxabs_kernel<false>, maxabs_blocks(rt, K), 256, 0, ctx_.stream, src, rowOff, rows, kOff, K, u,
+             maxbits, 0, 0, rt);
     }
     SCESS_CHECK_LAUNCH();
     if (aff)
-      pack_split_kernel<true, true><<<grid, 256, 0, ctx_.stream>>>(src, nullptr, rows, nullptr, K, u, dst,
-                                                                   Kpad, maxbits, scale, 0, rs, ks, rt);
+      launch(pack_split_kernel<true, true>, grid, 256, 0, ctx_.stream, src, nullptr, rows, nullptr, K, u, dst,
+             Kpad, maxbits, scale, 0, rs, ks, rt);
     else
-      pack_split_kernel<true, false><<<grid, 256, 0, ctx_.stream>>>(src, rowOff, rows, kOff, K, u, dst,
-                                                                    Kpad, maxbits, scale, 0, 0, 0, rt);
+      launch(pack_split_kernel<true, false>, grid, 256, 0, ctx_.stream, src, rowOff, rows, kOff, K, u, dst,
+             Kpad, maxbits, scale, 0, 0, 0, rt);
   } else {
     const double one = 1.0;
     SCESS_CUDA(cudaMemcpyAsync(scale, &one, sizeof(double), cudaMemcpyHostToDevice, ctx_.stream));
     if (aff)
-      pack_split_kernel<false, true><<<grid, 256, 0, ctx_.stream>>>(src, nullptr, rows, nullptr, K, u, dst,
-                                                                    Kpad, maxbits, scale, 0, rs, ks, rt);
+      launch(pack_split_kernel<false, true>, grid, 256, 0, ctx_.stream, src, nullptr, rows, nullptr, K, u, dst,
+             Kpad, maxbits, scale, 0, rs, ks, rt);
     else
-      pack_split_kernel<false, false><<<grid, 256, 0, ctx_.stream>>>(src, rowOff, rows, kOff, K, u, dst,
-                                                                     Kpad, maxbits, scale, 0, 0, 0, rt);
+      launch(pack_split_kernel<false, false>, grid, 256, 0, ctx_.stream, src, rowOff, rows, kOff, K, u, dst,
+             Kpad, maxbits, scale, 0, 0, 0, rt);
   }
   SCESS_CHECK_LAUNCH();
 }
@@ -1411,7 +1416,7 @@ void TcEngine::add_max_hint(const double *p, int64_t n) {
   TimedScope ts(ctx_.timer, "pack_max", 0.0, (double)n * 8, ctx_.stream);
   SCESS_CUDA(cudaMemsetAsync(word, 0, sizeof(unsigned), ctx_.stream));
   const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256 * 8), 8 * kNumSMs));
-  maxabs_flat_kernel<<<blocks, 256, 0, ctx_.stream>>>(p, n, word);
+  launch(maxabs_flat_kernel, blocks, 256, 0, ctx_.stream, p, n, word);
   SCESS_CHECK_LAUNCH();
   hints_.push_back({p, slot});
 }
@@ -1429,8 +1434,8 @@ void TcEngine::maxabs_into(const double *src, const int64_t *rowOff, int64_t row
                            const int64_t *kOff, int64_t K, bool unitK, unsigned *maxbits) {
   if (rows <= 0 || K <= 0) return;
   const RowTiles rt = RowTiles::make(rows, 1, rows);
-  maxabs_kernel<false><<<maxabs_blocks(rt, K), 256, 0, ctx_.stream>>>(src, rowOff, rows, kOff, K,
-                                                                     unitK ? 1 : 0, maxbits, 0, 0, rt);
+  launch(maxabs_kernel<false>, maxabs_blocks(rt, K), 256, 0, ctx_.stream, src, rowOff, rows, kOff, K,
+         unitK ? 1 : 0, maxbits, 0, 0, rt);
   SCESS_CHECK_LAUNCH();
 }
 
@@ -1458,15 +1463,13 @@ void TcEngine::pack_with_max(const double *src, const int64_t *rowOff, int64_t r
   dim3 grid((unsigned)rt.count, (unsigned)ceil_div(Kpad, 64));
   clear_pad_rows(out.mem.as<uint16_t>(), rows, rows_pad, Kpad, ctx_.stream);
   if (fmt_ == TcFormat::FP16) {
-    pack_split_kernel<true, false><<<grid, 256, 0, ctx_.stream>>>(src, rowOff, rows, kOff, K, unitK ? 1 : 0,
-                                                                  out.mem.as<uint16_t>(), Kpad, maxbits,
-                                                                  scale, negate ? 1 : 0, 0, 0, rt);
+    launch(pack_split_kernel<true, false>, grid, 256, 0, ctx_.stream, src, rowOff, rows, kOff, K,
+           unitK ? 1 : 0, out.mem.as<uint16_t>(), Kpad, maxbits, scale, negate ? 1 : 0, 0, 0, rt);
   } else {
     const double one = 1.0;
     SCESS_CUDA(cudaMemcpyAsync(scale, &one, sizeof(double), cudaMemcpyHostToDevice, ctx_.stream));
-    pack_split_kernel<false, false><<<grid, 256, 0, ctx_.stream>>>(src, rowOff, rows, kOff, K, unitK ? 1 : 0,
-                                                                   out.mem.as<uint16_t>(), Kpad, maxbits,
-                                                                   scale, negate ? 1 : 0, 0, 0, rt);
+    launch(pack_split_kernel<false, false>, grid, 256, 0, ctx_.stream, src, rowOff, rows, kOff, K,
+           unitK ? 1 : 0, out.mem.as<uint16_t>(), Kpad, maxbits, scale, negate ? 1 : 0, 0, 0, rt);
   }
   SCESS_CHECK_LAUNCH();
 }

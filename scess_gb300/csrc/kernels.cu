@@ -8,6 +8,7 @@
 #include "common.cuh"
 #include "dgemm_tile.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace scess {
 
@@ -17,6 +18,7 @@ constexpr int BM = kDgemmTile, BN = kDgemmTile, BK = kDgemmBK;
 
 __global__ void __launch_bounds__(256) dgemm_table_kernel(TableGemm g, int64_t kChunk,
                                                           double *partial) {
+  chain();
   const int64_t kb = (int64_t)blockIdx.z * kChunk;
   dgemm_tile(g, (int64_t)blockIdx.x * BM, (int64_t)blockIdx.y * BN, kb, min(g.K, kb + kChunk),
              [&](int64_t m, int64_t n, double acc) {
@@ -32,6 +34,7 @@ __global__ void __launch_bounds__(256) dgemm_table_kernel(TableGemm g, int64_t k
 }
 
 __global__ void splitk_reduce_kernel(TableGemm g, int splits, const double *partial) {
+  chain();
   const int64_t MN = g.M * g.N;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < MN;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -72,6 +75,7 @@ constexpr int kSmallOut = 64, kSmallKB = 128, kSmallSide = 16;
 __global__ void __launch_bounds__(256) dgemm_small_kernel(TableGemm g, int64_t kper, int splits, int tm, int tn,
                                                           double *__restrict__ partial,
                                                           int *__restrict__ counters) {
+  chain();
   __shared__ double As[kSmallKB][kSmallSide + 1], Bs[kSmallKB][kSmallSide + 1];
   __shared__ double red[4][kSmallOut];
   __shared__ int last;
@@ -180,6 +184,7 @@ SmallShape small_shape(const TableGemm &g) {
 // that four loads are in flight, added in a fixed order.
 template <bool CTA>
 __global__ void __launch_bounds__(256) dgemv_table_kernel(TableGemm g) {
+  chain();
   __shared__ double red[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t step = CTA ? 256 : 32, k0 = CTA ? threadIdx.x : lane;
@@ -236,8 +241,8 @@ int64_t dgemm_small_workspace(const TableGemm &g) {
 
 void dgemm_small(const TableGemm &g, double *workspace, int *counters, cudaStream_t stream) {
   const SmallShape s = small_shape(g);
-  dgemm_small_kernel<<<(unsigned)(s.tiles * s.splits), 256, 0, stream>>>(g, s.kper, s.splits, s.tm, s.tn, workspace,
-                                                                         counters);
+  launch(dgemm_small_kernel, (unsigned)(s.tiles * s.splits), 256, 0, stream, g, s.kper, s.splits, s.tm, s.tn,
+         workspace, counters);
   SCESS_CHECK_LAUNCH();
 }
 
@@ -275,6 +280,7 @@ __device__ __forceinline__ void skinny_out(double *p, T v, double beta) {
 // (dgemm_small 130; sliced 29 and 27 for the packs).
 template <typename T, bool STAGE>
 __global__ void __launch_bounds__(256) skinny_kernel(SkinnyArgs a) {
+  chain();
   extern __shared__ __align__(16) unsigned char sk_raw[];
   T *sS = reinterpret_cast<T *>(sk_raw);                             // [K][sp]
   int64_t *cSs = reinterpret_cast<int64_t *>(sS + a.K * a.sp);       // [s]
@@ -369,7 +375,7 @@ void skinny_launch(SkinnyArgs a, bool stage, cudaStream_t stream) {
                       (stage ? (size_t)8 * 32 * 33 * sizeof(T) : 0);
   const auto kernel = stage ? skinny_kernel<T, true> : skinny_kernel<T, false>;
   SCESS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<blocks, 256, smem, stream>>>(a);
+  launch(kernel, blocks, 256, smem, stream, a);
   SCESS_CHECK_LAUNCH();
 }
 }  // namespace
@@ -410,9 +416,10 @@ double skinny64_us(const TableGemm &g) {
 void dgemv_table(const TableGemm &g, cudaStream_t stream) {
   if (g.M <= 0) return;
   if (g.M < 8 * kNumSMs && g.K >= 512)  // too few rows for a warp each to fill the device
-    dgemv_table_kernel<true><<<(unsigned)std::min<int64_t>(g.M, 8 * kNumSMs), 256, 0, stream>>>(g);
+    launch(dgemv_table_kernel<true>, (unsigned)std::min<int64_t>(g.M, 8 * kNumSMs), 256, 0, stream, g);
   else
-    dgemv_table_kernel<false><<<(unsigned)std::min<int64_t>(ceil_div(g.M * 32, 256), 16 * kNumSMs), 256, 0, stream>>>(g);
+    launch(dgemv_table_kernel<false>, (unsigned)std::min<int64_t>(ceil_div(g.M * 32, 256), 16 * kNumSMs), 256,
+           0, stream, g);
   SCESS_CHECK_LAUNCH();
 }
 
@@ -427,8 +434,8 @@ void dgemm_table(const TableGemm &g, double *workspace, cudaStream_t stream) {
     // C = beta * C
     TableGemm h = g;
     h.alpha = 0.0;
-    splitk_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div(g.M * g.N, 256), 4096), 256, 0,
-                           stream>>>(h, 0, nullptr);
+    launch(splitk_reduce_kernel, (unsigned)std::min<int64_t>(ceil_div(g.M * g.N, 256), 4096), 256, 0, stream,
+           h, 0, nullptr);
     SCESS_CHECK_LAUNCH();
     return;
   }
@@ -438,12 +445,12 @@ void dgemm_table(const TableGemm &g, double *workspace, cudaStream_t stream) {
   dim3 grid((unsigned)ceil_div(g.M, BM), (unsigned)ceil_div(g.N, BN), (unsigned)nz);
   if (nz > 1) {
     if (!workspace) throw Error(SCESS_ERR_INVALID, "dgemm_table: split-K needs a workspace");
-    dgemm_table_kernel<<<grid, 256, 0, stream>>>(g, kChunk, workspace);
+    launch(dgemm_table_kernel, grid, 256, 0, stream, g, kChunk, workspace);
     SCESS_CHECK_LAUNCH();
-    splitk_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div(g.M * g.N, 256), 4096), 256, 0,
-                           stream>>>(g, nz, workspace);
+    launch(splitk_reduce_kernel, (unsigned)std::min<int64_t>(ceil_div(g.M * g.N, 256), 4096), 256, 0, stream,
+           g, nz, workspace);
   } else {
-    dgemm_table_kernel<<<grid, 256, 0, stream>>>(g, kChunk, nullptr);
+    launch(dgemm_table_kernel, grid, 256, 0, stream, g, kChunk, nullptr);
   }
   SCESS_CHECK_LAUNCH();
 }
@@ -455,7 +462,7 @@ void dgemm_table_bounded(const TableGemm &g, double *workspace, int64_t ws_doubl
   if (g.K <= 0) {
     TableGemm h = g;
     h.alpha = 0.0;
-    splitk_reduce_kernel<<<rblocks, 256, 0, stream>>>(h, 0, nullptr);
+    launch(splitk_reduce_kernel, rblocks, 256, 0, stream, h, 0, nullptr);
     SCESS_CHECK_LAUNCH();
     return;
   }
@@ -465,11 +472,11 @@ void dgemm_table_bounded(const TableGemm &g, double *workspace, int64_t ws_doubl
   const int nz = (int)ceil_div(g.K, kChunk);
   dim3 grid((unsigned)ceil_div(g.M, BM), (unsigned)ceil_div(g.N, BN), (unsigned)nz);
   if (nz > 1) {
-    dgemm_table_kernel<<<grid, 256, 0, stream>>>(g, kChunk, workspace);
+    launch(dgemm_table_kernel, grid, 256, 0, stream, g, kChunk, workspace);
     SCESS_CHECK_LAUNCH();
-    splitk_reduce_kernel<<<rblocks, 256, 0, stream>>>(g, nz, workspace);
+    launch(splitk_reduce_kernel, rblocks, 256, 0, stream, g, nz, workspace);
   } else {
-    dgemm_table_kernel<<<grid, 256, 0, stream>>>(g, kChunk, nullptr);
+    launch(dgemm_table_kernel, grid, 256, 0, stream, g, kChunk, nullptr);
   }
   SCESS_CHECK_LAUNCH();
 }
@@ -480,6 +487,7 @@ namespace {
 
 __global__ void permute_add_kernel(PermDesc d, double alpha, const double *__restrict__ X,
                                    double beta, double *__restrict__ Y, int64_t n) {
+  chain();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
     int64_t r = e, xo = 0, yo = 0;
@@ -504,6 +512,7 @@ unsigned grid_for(int64_t n, int threads = 256) {
 
 __global__ void tau_kernel(int64_t o, int64_t v, const double *__restrict__ t1,
                            const double *__restrict__ t2, double s, double *__restrict__ tau) {
+  chain();
   const int64_t n = o * o * v * v;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -517,6 +526,7 @@ __global__ void tau_kernel(int64_t o, int64_t v, const double *__restrict__ t1,
 __global__ void tau_delta_kernel(int64_t o, int64_t v, const double *__restrict__ t1_0,
                                  const double *__restrict__ dt1, const double *__restrict__ dt2,
                                  double *__restrict__ dtau) {
+  chain();
   const int64_t n = o * o * v * v;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -539,6 +549,7 @@ __global__ void ladder_vpm_kernel(const double *__restrict__ V, int64_t s0, int6
                                   int64_t s3, const int2 *__restrict__ pu, int64_t nu,
                                   const int2 *__restrict__ ps, int64_t ns, double *__restrict__ Vp,
                                   double *__restrict__ Vm) {
+  chain();
   const int64_t total = nu * nu + ns * ns;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -564,6 +575,7 @@ __global__ void ladder_tpm_kernel(int64_t o, int64_t v, const double *__restrict
                                   const int2 *__restrict__ puv, int64_t nuv,
                                   const int2 *__restrict__ psv, int64_t nsv,
                                   double *__restrict__ Tp, double *__restrict__ Tm) {
+  chain();
   const int64_t total = nuo * nuv + nso * nsv, o2 = o * o, o2v = o2 * v;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -586,6 +598,7 @@ __global__ void ladder_tpm_kernel(int64_t o, int64_t v, const double *__restrict
 // nuo x nuv, Sm nso x nsv, both column-major.
 __global__ void ladder_unpack_kernel(int64_t o, int64_t v, const double *__restrict__ Sp,
                                      const double *__restrict__ Sm, double *__restrict__ R2) {
+  chain();
   const int64_t n = o * o * v * v, nuo = o * (o + 1) / 2, nso = o * (o - 1) / 2;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -603,6 +616,7 @@ __global__ void ladder_unpack_kernel(int64_t o, int64_t v, const double *__restr
 __global__ void denom_kernel(int64_t o, int64_t v, const double *__restrict__ eps,
                              const double *__restrict__ R1, const double *__restrict__ R2,
                              double *__restrict__ t1, double *__restrict__ t2) {
+  chain();
   const int64_t n1 = o * v, n2 = o * o * v * v;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n1 + n2;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -621,6 +635,7 @@ __global__ void denom_kernel(int64_t o, int64_t v, const double *__restrict__ ep
 
 __global__ void plus_transpose_kernel(int64_t o, int64_t v, double alpha,
                                       const double *__restrict__ X, double *__restrict__ out) {
+  chain();
   const int64_t n = o * o * v * v;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -632,6 +647,7 @@ __global__ void plus_transpose_kernel(int64_t o, int64_t v, double alpha,
 
 __global__ void axpby_kernel(int64_t n, double a, const double *__restrict__ x, double b,
                              double *__restrict__ y) {
+  chain();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x)
     y[e] = a * x[e] + (b == 0.0 ? 0.0 : b * y[e]);
@@ -654,6 +670,7 @@ __device__ double block_sum(double v) {
 
 __global__ void dot_partial_kernel(int64_t n, const double *__restrict__ x,
                                    const double *__restrict__ y, double *__restrict__ partials) {
+  chain();
   double s = 0.0;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x)
@@ -665,6 +682,7 @@ __global__ void dot_partial_kernel(int64_t n, const double *__restrict__ x,
 // Dots of nv vectors xs[q] with y, one per blockIdx.y: each is dot_partial_kernel's sum.
 __global__ void dots_partial_kernel(int64_t n, DotVectors xs, const double *__restrict__ y,
                                     double *__restrict__ partials) {
+  chain();
   const double *__restrict__ x = xs.p[blockIdx.y];
   double s = 0.0;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
@@ -676,6 +694,7 @@ __global__ void dots_partial_kernel(int64_t n, DotVectors xs, const double *__re
 
 __global__ void sum_partials_kernel(int np, const double *__restrict__ partials,
                                     double *__restrict__ result) {
+  chain();
   double s = 0.0;
   for (int e = threadIdx.x; e < np; e += blockDim.x) s += partials[(int64_t)blockIdx.x * np + e];
   s = block_sum(s);
@@ -686,6 +705,7 @@ __global__ void tau_energy_partial_kernel(int64_t o, int64_t v, const double *__
                                           const double *__restrict__ t1,
                                           const double *__restrict__ t2,
                                           double *__restrict__ partials) {
+  chain();
   const int64_t n = o * o * v * v;
   double s = 0.0;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
@@ -703,6 +723,7 @@ __global__ void tau_energy_partial_kernel(int64_t o, int64_t v, const double *__
 __global__ void mp2_partial_kernel(int64_t o, int64_t v, const double *__restrict__ g, int64_t si,
                                    int64_t sa, int64_t sj, int64_t sb,
                                    const double *__restrict__ eps, double *__restrict__ partials) {
+  chain();
   const int64_t n = o * v * o * v;
   double s = 0.0;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
@@ -718,6 +739,7 @@ __global__ void mp2_partial_kernel(int64_t o, int64_t v, const double *__restric
 
 // Non-negative doubles order like their bits; a NaN (sign cleared) is above all of them.
 __global__ void pair_asymmetry_kernel(const double *__restrict__ x, Ext4 n, Ext4 st, double *__restrict__ out) {
+  chain();
   const int64_t total = n.e[0] * n.e[1] * n.e[2] * n.e[3];
   unsigned long long d = 0, m = 0;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
@@ -740,6 +762,7 @@ __global__ void pair_asymmetry_kernel(const double *__restrict__ x, Ext4 n, Ext4
 }
 
 __global__ void lincomb_kernel(int64_t n, int nv, LinComb lc, bool first, double *__restrict__ out) {
+  chain();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
     double s = first ? 0.0 : out[e];
@@ -749,6 +772,7 @@ __global__ void lincomb_kernel(int64_t n, int nv, LinComb lc, bool first, double
 }
 
 __global__ void finite_kernel(int64_t n, const double *__restrict__ x, int *flag) {
+  chain();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x)
     if (!isfinite(x[e])) *flag = 1;
@@ -761,67 +785,67 @@ void permute_add(const PermDesc &d, double alpha, const double *X, double beta, 
   int64_t n = 1;
   for (int k = 0; k < d.nd; k++) n *= d.ext[k];
   if (n == 0) return;
-  permute_add_kernel<<<grid_for(n), 256, 0, stream>>>(d, alpha, X, beta, Y, n);
+  launch(permute_add_kernel, grid_for(n), 256, 0, stream, d, alpha, X, beta, Y, n);
   SCESS_CHECK_LAUNCH();
 }
 
 void make_tau(int64_t o, int64_t v, const double *t1, const double *t2, double s, double *tau,
               cudaStream_t stream) {
-  tau_kernel<<<grid_for(o * o * v * v), 256, 0, stream>>>(o, v, t1, t2, s, tau);
+  launch(tau_kernel, grid_for(o * o * v * v), 256, 0, stream, o, v, t1, t2, s, tau);
   SCESS_CHECK_LAUNCH();
 }
 
 void make_tau_delta(int64_t o, int64_t v, const double *t1_0, const double *dt1,
                     const double *dt2, double *dtau, cudaStream_t stream) {
-  tau_delta_kernel<<<grid_for(o * o * v * v), 256, 0, stream>>>(o, v, t1_0, dt1, dt2, dtau);
+  launch(tau_delta_kernel, grid_for(o * o * v * v), 256, 0, stream, o, v, t1_0, dt1, dt2, dtau);
   SCESS_CHECK_LAUNCH();
 }
 
 void ladder_vpm(const double *V, int64_t s0, int64_t s1, int64_t s2, int64_t s3, const int2 *pu,
                 int64_t nu, const int2 *ps, int64_t ns, double *Vp, double *Vm,
                 cudaStream_t stream) {
-  ladder_vpm_kernel<<<grid_for(nu * nu + ns * ns), 256, 0, stream>>>(V, s0, s1, s2, s3, pu, nu, ps,
-                                                                    ns, Vp, Vm);
+  launch(ladder_vpm_kernel, grid_for(nu * nu + ns * ns), 256, 0, stream, V, s0, s1, s2, s3, pu, nu, ps, ns, Vp,
+         Vm);
   SCESS_CHECK_LAUNCH();
 }
 
 void ladder_tpm(int64_t o, int64_t v, const double *tau, const int2 *puo, int64_t nuo,
                 const int2 *pso, int64_t nso, const int2 *puv, int64_t nuv, const int2 *psv,
                 int64_t nsv, double *Tp, double *Tm, cudaStream_t stream) {
-  ladder_tpm_kernel<<<grid_for(nuo * nuv + nso * nsv), 256, 0, stream>>>(
-      o, v, tau, puo, nuo, pso, nso, puv, nuv, psv, nsv, Tp, Tm);
+  launch(ladder_tpm_kernel, grid_for(nuo * nuv + nso * nsv), 256, 0, stream, o, v, tau, puo, nuo, pso, nso,
+         puv, nuv, psv, nsv, Tp, Tm);
   SCESS_CHECK_LAUNCH();
 }
 
 void ladder_unpack(int64_t o, int64_t v, const double *Sp, const double *Sm, double *R2,
                    cudaStream_t stream) {
-  ladder_unpack_kernel<<<grid_for(o * o * v * v), 256, 0, stream>>>(o, v, Sp, Sm, R2);
+  launch(ladder_unpack_kernel, grid_for(o * o * v * v), 256, 0, stream, o, v, Sp, Sm, R2);
   SCESS_CHECK_LAUNCH();
 }
 
 void divide_denominators(int64_t o, int64_t v, const double *eps, const double *R1,
                          const double *R2, double *t1, double *t2, cudaStream_t stream) {
-  denom_kernel<<<grid_for(o * v + o * o * v * v), 256, 0, stream>>>(o, v, eps, R1, R2, t1, t2);
+  launch(denom_kernel, grid_for(o * v + o * o * v * v), 256, 0, stream, o, v, eps, R1, R2, t1, t2);
   SCESS_CHECK_LAUNCH();
 }
 
 void plus_transpose(int64_t o, int64_t v, double alpha, const double *X, double *out,
                     cudaStream_t stream) {
-  plus_transpose_kernel<<<grid_for(o * o * v * v), 256, 0, stream>>>(o, v, alpha, X, out);
+  launch(plus_transpose_kernel, grid_for(o * o * v * v), 256, 0, stream, o, v, alpha, X, out);
   SCESS_CHECK_LAUNCH();
 }
 
 void axpby(int64_t n, double a, const double *x, double b, double *y, cudaStream_t stream) {
   if (n == 0) return;
-  axpby_kernel<<<grid_for(n), 256, 0, stream>>>(n, a, x, b, y);
+  launch(axpby_kernel, grid_for(n), 256, 0, stream, n, a, x, b, y);
   SCESS_CHECK_LAUNCH();
 }
 
 void dot(int64_t n, const double *x, const double *y, double *partials, double *result,
          cudaStream_t stream) {
-  dot_partial_kernel<<<kDotBlocks, 256, 0, stream>>>(n, x, y, partials);
+  launch(dot_partial_kernel, kDotBlocks, 256, 0, stream, n, x, y, partials);
   SCESS_CHECK_LAUNCH();
-  sum_partials_kernel<<<1, 1024, 0, stream>>>(kDotBlocks, partials, result);
+  launch(sum_partials_kernel, 1, 1024, 0, stream, kDotBlocks, partials, result);
   SCESS_CHECK_LAUNCH();
 }
 
@@ -831,9 +855,9 @@ void dots(int64_t n, const double *const *xs, int nv, const double *y, double *p
     DotVectors v{};
     const int m = std::min(kDotVectors, nv - q0);
     for (int q = 0; q < m; q++) v.p[q] = xs[q0 + q];
-    dots_partial_kernel<<<dim3(kDotBlocks, (unsigned)m), 256, 0, stream>>>(n, v, y, partials);
+    launch(dots_partial_kernel, dim3(kDotBlocks, (unsigned)m), 256, 0, stream, n, v, y, partials);
     SCESS_CHECK_LAUNCH();
-    sum_partials_kernel<<<(unsigned)m, 1024, 0, stream>>>(kDotBlocks, partials, result + q0);
+    launch(sum_partials_kernel, (unsigned)m, 1024, 0, stream, kDotBlocks, partials, result + q0);
     SCESS_CHECK_LAUNCH();
   }
 }
@@ -847,38 +871,38 @@ void linear_combination(int64_t n, int nv, const double *const *vecs, const doub
       lc.p[c] = vecs[c0 + c];
       lc.coef[c] = coef[c0 + c];
     }
-    lincomb_kernel<<<grid_for(n), 256, 0, stream>>>(n, m, lc, c0 == 0, out);
+    launch(lincomb_kernel, grid_for(n), 256, 0, stream, n, m, lc, c0 == 0, out);
     SCESS_CHECK_LAUNCH();
   }
 }
 
 void tau_energy(int64_t o, int64_t v, const double *L, const double *t1, const double *t2,
                 double *partials, double *result, cudaStream_t stream) {
-  tau_energy_partial_kernel<<<kDotBlocks, 256, 0, stream>>>(o, v, L, t1, t2, partials);
+  launch(tau_energy_partial_kernel, kDotBlocks, 256, 0, stream, o, v, L, t1, t2, partials);
   SCESS_CHECK_LAUNCH();
-  sum_partials_kernel<<<1, 1024, 0, stream>>>(kDotBlocks, partials, result);
+  launch(sum_partials_kernel, 1, 1024, 0, stream, kDotBlocks, partials, result);
   SCESS_CHECK_LAUNCH();
 }
 
 void mp2_energy(int64_t o, int64_t v, const double *g, int64_t si, int64_t sa, int64_t sj,
                 int64_t sb, const double *eps, double *partials, double *result,
                 cudaStream_t stream) {
-  mp2_partial_kernel<<<kDotBlocks, 256, 0, stream>>>(o, v, g, si, sa, sj, sb, eps, partials);
+  launch(mp2_partial_kernel, kDotBlocks, 256, 0, stream, o, v, g, si, sa, sj, sb, eps, partials);
   SCESS_CHECK_LAUNCH();
-  sum_partials_kernel<<<1, 1024, 0, stream>>>(kDotBlocks, partials, result);
+  launch(sum_partials_kernel, 1, 1024, 0, stream, kDotBlocks, partials, result);
   SCESS_CHECK_LAUNCH();
 }
 
 void pair_asymmetry(const double *x, Ext4 ext, Ext4 str, double *out, cudaStream_t stream) {
   const int64_t n = ext.e[0] * ext.e[1] * ext.e[2] * ext.e[3];
-  pair_asymmetry_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), 8 * kNumSMs)), 256, 0, stream>>>(
-      x, ext, str, out);
+  launch(pair_asymmetry_kernel, (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256),
+         8 * kNumSMs)), 256, 0, stream, x, ext, str, out);
   SCESS_CHECK_LAUNCH();
 }
 
 void check_finite(int64_t n, const double *x, int *flag, cudaStream_t stream) {
   if (n == 0) return;
-  finite_kernel<<<grid_for(n), 256, 0, stream>>>(n, x, flag);
+  launch(finite_kernel, grid_for(n), 256, 0, stream, n, x, flag);
   SCESS_CHECK_LAUNCH();
 }
 
