@@ -18,6 +18,10 @@
 // waits); MMAs issued from uniform registers (see elect_one) 51.6; S_5 between S_2 and
 // S_1, and accumulators released before their arithmetic, 52.3.  Six accumulators of 80
 // columns with a third of the drains: 34 when issue bound it.
+// Joint form (tiles of at most 80 columns): TMEM holds an accumulator for every S_d, in two
+// sets up to 32 columns, and the five are drained together, with one wait and one release a
+// block; three stages where they fit.  313600 x 16 x 140: 315 us -> 144, where the
+// packs' 14 bytes an element read at 4.9 TB/s bound it; 200000 x 16 x 16: 71 -> 43.
 // Every mbarrier wait is bounded (see mbarrier.cuh).
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -38,19 +42,20 @@ namespace scess {
 namespace {
 
 constexpr int BM = 128, BN = 128, BK = kSliceBK;
-constexpr int STAGES = 2;
+constexpr int STAGES = 2, MAX_STAGES = 3;                             // (narrow tiles: three)
 constexpr uint32_t A_SLICE = (uint32_t)BM * BK * 2;                  // one slice of 128 rows
 constexpr uint32_t STAGE_BYTES = kSlices * (BM + BN) * BK * 2;       // 112 KiB
 constexpr int NDIAG = 5;                                             // S_0 .. S_4 are drained
 constexpr int NROT = 3, TAIL = NROT, NACC = NROT + 1;                // accumulators
 constexpr int EPI = 4;                                               // epilogue warpgroups
 constexpr int HC = BN / EPI;                                         // columns of an epilogue thread
+constexpr int BN_JOINT = 80, HC_JOINT = 24;                          // the same of the joint form
 constexpr int THREADS = 128 * (1 + EPI);
 constexpr int kEpiRegs = 104, kCtlRegs = 56, kLaunchRegs = 96;       // 56 + 4 x 104 <= 5 x 96
 static_assert(kSlices == NDIAG + 2, "the tail is S_5 + S_6");
 static_assert(kCtlRegs + EPI * kEpiRegs <= (1 + EPI) * kLaunchRegs, "setmaxnreg draws on the launch's registers");
 struct Ctl {  // behind the stages
-  uint64_t full[STAGES], empty[STAGES], tfull[NACC], tempty[NACC], done;
+  uint64_t full[MAX_STAGES], empty[MAX_STAGES], tfull[NACC], tempty[NACC], done;
   uint32_t tmem;
   alignas(16) int64_t colOff[BN];
   alignas(16) int colE[BN];
@@ -69,7 +74,8 @@ struct SliceMaps {
 };
 struct SliceArgs {
   int M, N, tiles_m, tiles_n;
-  int bn;      // tile width: a multiple of 32, at most 128
+  int bn;      // tile width: a multiple of 32, at most 128, or (joint form) of 16, at most 80
+  int stages;  // joint form
   int fs;      // fraction bits kept of the tail (see slice_value)
   int ny, nz, ng, nseg;
   int kb_total, kb_per_split, splits;
@@ -135,6 +141,7 @@ __device__ __forceinline__ void tmem_wait8(uint32_t *r) {
 }
 
 // What bounds it: long K, the drains (above); short K, the outputs (about 45 instructions each).
+template <bool JOINT>
 __global__ void __launch_bounds__(THREADS, 1)
     slice_gemm_kernel(const __grid_constant__ SliceMaps maps, const __grid_constant__ SliceArgs a) {
   extern __shared__ uint8_t smem_raw[];
@@ -146,9 +153,13 @@ __global__ void __launch_bounds__(THREADS, 1)
   const int units = tiles * nprob * a.splits;
   const int bn = a.bn;
   const uint32_t bslice = (uint32_t)bn * BK * 2;
+  const uint32_t stage_bytes = JOINT ? kSlices * (A_SLICE + bslice) : STAGE_BYTES;
+  const int nst = JOINT ? a.stages : STAGES;
+  const int nset = JOINT && 11 * bn <= 512 ? 2 : 1;                    // sets of S_0 .. S_4
+  const uint32_t tail_col = (uint32_t)((JOINT ? nset * NDIAG : TAIL) * bn);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; s++) {
+    for (int s = 0; s < MAX_STAGES; s++) {
       mbar_init(&ctl.full[s], 1);
       mbar_init(&ctl.empty[s], 1);
     }
@@ -210,25 +221,31 @@ __global__ void __launch_bounds__(THREADS, 1)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kCtlRegs));
   if (warp == 0) {
     if (lane == 0) {
-      int g = 0;
-      int last[STAGES];
-      for (int s = 0; s < STAGES; s++) last[s] = -1;
+      int g = 0, s = 0;
+      uint32_t ph = 0;          // stage and its phase
+      int used = 0;             // stages filled at least once
+      uint32_t lastph = 0;      // phases of their last fills, a bit each
       bool ok = true;
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
         int tm, tn, py, pz, pg, kb0, kb1, sp;
         unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
         for (int kb = kb0; kb < kb1; kb++, g++) {
+          if (s == nst) {
+            s = 0;
+            ph ^= 1u;
+          }
           int sg, lkb;
           seg_at(kb, sg, lkb);
           const SegArgs &S = a.seg[sg];
           const int ya = (int)(S.rowA0[pg] + py * S.rowAy[pg] + pz * S.rowAz[pg]) + tm * BM;
           const int yb = (int)(S.rowB0[pg] + py * S.rowBy[pg] + pz * S.rowBz[pg]) + tn * bn;
-          const int s = g % STAGES;
-          const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
           if (!mbar_wait(&ctl.empty[s], ph ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) { ok = false; break; }
           // diagnostics: the first stage is taken but never filled (see scess_ctx_arm_wait_expiry)
-          if (a.withhold_first && g == 0) continue;
-          uint8_t *st = smem + s * STAGE_BYTES;
+          if (a.withhold_first && g == 0) {
+            s++;
+            continue;
+          }
+          uint8_t *st = smem + s * stage_bytes;
           mbar_expect_tx(&ctl.full[s], kSlices * (A_SLICE + bslice));
 #pragma unroll
           for (int p = kSlices - 1; p >= 0; p--) {
@@ -236,15 +253,18 @@ __global__ void __launch_bounds__(THREADS, 1)
             tma_load_2d(st + kSlices * A_SLICE + p * bslice, &maps.m[S.mapB], p * S.kpad + lkb * BK, yb,
                         &ctl.full[s]);
           }
-          last[s] = g;
+          used |= 1 << s;
+          lastph = (lastph & ~(1u << s)) | (ph << s);
+          s++;
         }
       }
-      for (int s = 0; s < STAGES; s++)
-        if (last[s] >= 0) mbar_drain(&ctl.full[s], (uint32_t)(last[s] / STAGES) & 1u);
+      for (int q = 0; q < nst; q++)
+        if (used >> q & 1) mbar_drain(&ctl.full[q], lastph >> q & 1u);
     }
   } else if (warp == 1) {
     // all lanes, issues by the elected one (see elect_one)
-    int g = 0, c = 0, w = 0;  // stages, rotating fills and units so far
+    int s = 0, c = 0, w = 0;  // stage, rotating fills (joint: K blocks) and units so far
+    uint32_t ph = 0;          // phase of the stage
     const uint64_t desc = sw_desc<64>(smem_u32(smem));
     const uint32_t hi = (uint32_t)(desc >> 32), lo = (uint32_t)desc;
     const uint32_t bq = bslice >> 4;
@@ -257,13 +277,15 @@ __global__ void __launch_bounds__(THREADS, 1)
       int tm, tn, py, pz, pg, kb0, kb1, sp;
       unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
       const uint32_t idesc = idesc_f16kind(BM, min(bn, (a.N - tn * bn + 15) & ~15), 1u);  // BF16
-      for (int kb = kb0; kb < kb1 && ok; kb++, g++) {
-        const int s = g % STAGES;
-        const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
+      for (int kb = kb0; kb < kb1 && ok; kb++, s++) {
+        if (s == nst) {
+          s = 0;
+          ph ^= 1u;
+        }
         if (!wait(&ctl.full[s], ph, ERR_FULL_WAIT)) { ok = false; break; }
         tc_fence_after();
         // slice offsets are added to the stage's descriptors (address field in units of 16 bytes)
-        const uint32_t da = lo + (uint32_t)s * (STAGE_BYTES >> 4), db = da + (kSlices * A_SLICE >> 4);
+        const uint32_t da = lo + (uint32_t)s * (stage_bytes >> 4), db = da + (kSlices * A_SLICE >> 4);
         auto product = [&](uint32_t col, int p, int q, uint32_t acc) {
 #pragma unroll
           for (int k = 0; k < 2; k++)
@@ -272,34 +294,57 @@ __global__ void __launch_bounds__(THREADS, 1)
         auto tail = [&](auto diag, uint32_t acc) {
           constexpr int d = decltype(diag)::value;
 #pragma unroll
-          for (int p = 0; p <= d; p++, acc = 1u) product((uint32_t)(TAIL * bn), p, d - p, acc);
+          for (int p = 0; p <= d; p++, acc = 1u) product(tail_col, p, d - p, acc);
         };
-        // The longest diagonals first and S_5 between S_2 and S_1: a drain is then done
-        // when its accumulator comes round.
-#pragma unroll
-        for (int d = NDIAG - 1; d >= 0; d--) {
-          if (d == 1) {
-            if (kb == kb0) {
-              if (!wait(&ctl.tempty[TAIL], ((uint32_t)w & 1u) ^ 1u, ERR_EMPTY_WAIT)) { ok = false; break; }
-              tc_fence_after();
-            }
-            if (issuer) tail(std::integral_constant<int, NDIAG>{}, kb == kb0 ? 0u : 1u);
-          }
-          const int b = c % NROT;
-          if (ok && !wait(&ctl.tempty[b], (((uint32_t)(c / NROT)) & 1u) ^ 1u, ERR_EMPTY_WAIT)) ok = false;
-          if (!ok) break;
+        auto tail_free = [&]() {
+          if (!wait(&ctl.tempty[TAIL], ((uint32_t)w & 1u) ^ 1u, ERR_EMPTY_WAIT)) return false;
           tc_fence_after();
+          return true;
+        };
+        if constexpr (JOINT) {
+          // S_4 .. S_0 into a set of their own, drained together beside the tail
+          const int set = nset == 2 ? c & 1 : 0;
+          if (!wait(&ctl.tempty[set], (uint32_t)(nset == 2 ? c >> 1 : c) & 1u ^ 1u, ERR_EMPTY_WAIT)) { ok = false; break; }
+          tc_fence_after();
+          c++;
           if (issuer) {
 #pragma unroll
-            for (int p = 0; p <= d; p++) product((uint32_t)(b * bn), p, d - p, p ? 1u : 0u);
-            mma_commit(&ctl.tfull[b]);
+            for (int d = NDIAG - 1; d >= 0; d--)
+#pragma unroll
+              for (int p = 0; p <= d; p++) product((uint32_t)((set * NDIAG + d) * bn), p, d - p, p ? 1u : 0u);
+            mma_commit(&ctl.tfull[set]);
           }
-          c++;
-        }
-        if (!ok) break;
-        if (issuer) {
-          tail(std::integral_constant<int, NDIAG + 1>{}, 1u);
-          mma_commit(&ctl.empty[s]);
+          if (kb == kb0 && !tail_free()) { ok = false; break; }
+          if (issuer) {
+            tail(std::integral_constant<int, NDIAG>{}, kb == kb0 ? 0u : 1u);
+            tail(std::integral_constant<int, NDIAG + 1>{}, 1u);
+            mma_commit(&ctl.empty[s]);
+          }
+        } else {
+          // The longest diagonals first and S_5 between S_2 and S_1: a drain is then done
+          // when its accumulator comes round.
+#pragma unroll
+          for (int d = NDIAG - 1; d >= 0; d--) {
+            if (d == 1) {
+              if (kb == kb0 && !tail_free()) { ok = false; break; }
+              if (issuer) tail(std::integral_constant<int, NDIAG>{}, kb == kb0 ? 0u : 1u);
+            }
+            const int b = c % NROT;
+            if (ok && !wait(&ctl.tempty[b], (((uint32_t)(c / NROT)) & 1u) ^ 1u, ERR_EMPTY_WAIT)) ok = false;
+            if (!ok) break;
+            tc_fence_after();
+            if (issuer) {
+#pragma unroll
+              for (int p = 0; p <= d; p++) product((uint32_t)(b * bn), p, d - p, p ? 1u : 0u);
+              mma_commit(&ctl.tfull[b]);
+            }
+            c++;
+          }
+          if (!ok) break;
+          if (issuer) {
+            tail(std::integral_constant<int, NDIAG + 1>{}, 1u);
+            mma_commit(&ctl.empty[s]);
+          }
         }
       }
       if (ok && issuer) mma_commit(&ctl.tfull[TAIL]);
@@ -312,22 +357,25 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int q = warp & 3;
     const int row = 32 * q + lane;
     const int h = (warp - 4) >> 2;                  // column group
-    const int hc = bn / EPI;                        // its width: 8, 16, 24 or 32
+    // its columns: a quarter of the tile's, or of its groups of eight
+    const int h0 = JOINT ? 8 * ((bn / 8 * h + 3) / 4) : bn / EPI * h;
+    const int hc = (JOINT ? 8 * ((bn / 8 * (h + 1) + 3) / 4) : bn / EPI * (h + 1)) - h0;
+    constexpr int HCT = JOINT ? HC_JOINT : HC;
     const int et = threadIdx.x - 128 - 128 * h;     // 0..127 within the group
     const int bar = 1 + h;
     int c = 0, w = 0;
     bool ok = true;
-    const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(hc * h);
+    const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)h0;
     for (int u = blockIdx.x; u < units && ok; u += gridDim.x, w++) {
       int tm, tn, py, pz, pg, kb0, kb1, sp;
       unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
       const int m = tm * BM + row;
       asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");  // previous unit's column tables read
       if (et < hc) {
-        const int nn = tn * bn + hc * h + et;
+        const int nn = tn * bn + h0 + et;
         const int e = nn < a.N ? a.expB[nn] : kRowNonFinite;
-        ctl.colE[hc * h + et] = e == 0 ? 1023 : e;  // (all zero: any scale)
-        ctl.colOff[hc * h + et] =
+        ctl.colE[h0 + et] = e == 0 ? 1023 : e;  // (all zero: any scale)
+        ctl.colOff[h0 + et] =
             e == kRowNonFinite ? -1
             : a.partial ? (int64_t)sp * a.part_stride + (int64_t)a.M * nn
                         : a.baseC + py * a.cy[pg] + pz * a.cz[pg] + a.cg[pg] + a.colC[pg][nn];
@@ -335,10 +383,10 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int eA = m < a.M ? a.expA[a.expA0[pg] + m] : kRowNonFinite;
       const int64_t rowOff = m < a.M ? (a.partial ? (int64_t)m : a.rowC[pg][m]) : 0;
       const unsigned errv = *(volatile unsigned *)a.err;
-      long long T[HC];
+      long long T[HCT];
       const long long off = magic_sum(kb1 - kb0);
 #pragma unroll
-      for (int j = 0; j < HC; j++) T[j] = -off;
+      for (int j = 0; j < HCT; j++) T[j] = -off;
       auto release = [&](int b) {
         tc_fence_before();
         __syncwarp();
@@ -367,10 +415,38 @@ __global__ void __launch_bounds__(THREADS, 1)
         return true;
       };
       for (int kb = kb0; kb < kb1; kb++) {
-        ok = take(std::integral_constant<int, 4>{}) && take(std::integral_constant<int, 3>{}) &&
-             take(std::integral_constant<int, 2>{}) && take(std::integral_constant<int, 1>{}) &&
-             take(std::integral_constant<int, 0>{});
-        if (!ok) break;
+        if constexpr (JOINT) {
+          const int set = nset == 2 ? c & 1 : 0;
+          ok = mbar_wait(&ctl.tfull[set], (uint32_t)(nset == 2 ? c >> 1 : c) & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles);
+          if (!ok) break;
+          c++;
+          tc_fence_after();
+          const uint32_t t0 = tl + (uint32_t)(set * NDIAG * bn);
+          if (hc == 0) release(set);
+#pragma unroll
+          for (int j = 0; j < HCT; j += 8) {
+            if (j >= hc) continue;
+            uint32_t r[NDIAG][8];
+#pragma unroll
+            for (int d = 0; d < NDIAG; d++) tmem_ld8(t0 + (uint32_t)(d * bn + j), r[d]);
+#pragma unroll
+            for (int d = 0; d < NDIAG; d++) tmem_wait8(r[d]);
+            if (j + 8 >= hc) release(set);  // (all columns are in registers)
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+              add_diag<0>(T[j + i], r[0][i]);
+              add_diag<1>(T[j + i], r[1][i]);
+              add_diag<2>(T[j + i], r[2][i]);
+              add_diag<3>(T[j + i], r[3][i]);
+              add_diag<4>(T[j + i], r[4][i]);
+            }
+          }
+        } else {
+          ok = take(std::integral_constant<int, 4>{}) && take(std::integral_constant<int, 3>{}) &&
+               take(std::integral_constant<int, 2>{}) && take(std::integral_constant<int, 1>{}) &&
+               take(std::integral_constant<int, 0>{});
+          if (!ok) break;
+        }
       }
       if (ok && !mbar_wait(&ctl.tfull[TAIL], (uint32_t)w & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) ok = false;
       asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");  // column tables of this unit written
@@ -388,22 +464,22 @@ __global__ void __launch_bounds__(THREADS, 1)
       // keeps results normal) skip the checks of each output: 42 instructions instead of 90.
       auto fits = [](int e) { return e >= 640 && e <= 1400; };
       const bool rok = fits(eA == 0 ? 1023 : eA) && sc0 >= -1500 && sc0 <= -600;
-      const bool cok = lane >= hc || (ctl.colOff[hc * h + lane] >= 0 && fits(ctl.colE[hc * h + lane]));
+      const bool cok = lane >= hc || (ctl.colOff[h0 + lane] >= 0 && fits(ctl.colE[h0 + lane]));
       const bool plain = __all_sync(0xffffffffu, rok && cok) && !scaled && mode != 2;
       auto finish = [&](auto is_plain) {
         constexpr bool PLAIN = decltype(is_plain)::value;
 #pragma unroll
-        for (int j = 0; j < HC; j += 8) {
+        for (int j = 0; j < HCT; j += 8) {
           if (j >= hc) continue;
           uint32_t r[8];
-          tmem_ld8(tl + (uint32_t)(TAIL * bn + j), r);
+          tmem_ld8(tl + tail_col + (uint32_t)j, r);
           int e[8];
           long long co[8];
-          *reinterpret_cast<int4 *>(e) = *reinterpret_cast<const int4 *>(&ctl.colE[hc * h + j]);
-          *reinterpret_cast<int4 *>(e + 4) = *reinterpret_cast<const int4 *>(&ctl.colE[hc * h + j + 4]);
+          *reinterpret_cast<int4 *>(e) = *reinterpret_cast<const int4 *>(&ctl.colE[h0 + j]);
+          *reinterpret_cast<int4 *>(e + 4) = *reinterpret_cast<const int4 *>(&ctl.colE[h0 + j + 4]);
 #pragma unroll
           for (int i = 0; i < 8; i += 2)
-            *reinterpret_cast<longlong2 *>(co + i) = *reinterpret_cast<const longlong2 *>(&ctl.colOff[hc * h + j + i]);
+            *reinterpret_cast<longlong2 *>(co + i) = *reinterpret_cast<const longlong2 *>(&ctl.colOff[h0 + j + i]);
           tmem_wait8(r);
 #pragma unroll
           for (int i = 0; i < 8; i++) {
@@ -663,10 +739,12 @@ bool kernel_ok() {
   static bool ok = false;
   static std::once_flag once;
   std::call_once(once, [] {
-    cudaFuncAttributes fa;
-    ok = cudaFuncSetAttribute(slice_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)SMEM_BYTES) == cudaSuccess &&
-         cudaFuncGetAttributes(&fa, slice_gemm_kernel) == cudaSuccess && fa.numRegs == kLaunchRegs;
+    auto fits = [](void (*kernel)(SliceMaps, SliceArgs)) {
+      cudaFuncAttributes fa;
+      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES) == cudaSuccess &&
+             cudaFuncGetAttributes(&fa, kernel) == cudaSuccess && fa.numRegs == kLaunchRegs;
+    };
+    ok = fits(slice_gemm_kernel<false>) && fits(slice_gemm_kernel<true>);
     cudaGetLastError();
   });
   return ok;
@@ -685,13 +763,24 @@ SliceEngine::SliceEngine(Ctx &ctx) : ctx_(ctx) {
   SCESS_CUDA(cudaMemsetAsync(err_.as<void>(), 0, sizeof(unsigned) * 4, ctx_.stream));
 }
 
-int SliceEngine::tile_n(int64_t N) { return (int)round_up(ceil_div(N, ceil_div(N, BN)), 8 * EPI); }
+namespace {
+// The joint form's tiles are at most 80 wide.
+bool joint(int bn) { return bn <= BN_JOINT; }
+// Cycles an SM spends on one K block of a unit, measured (152 tiles of 128 rows, K = 1024:
+// widths 16 .. 128): in the rotating form the five drains, one after the other, take as long
+// for 96 columns as for 128.
+double block_cycles(int bn) { return joint(bn) ? 3200.0 + 25.0 * bn : 5750.0; }
+}  // namespace
+
+// The narrow tile where it is cheaper.
+int SliceEngine::tile_n(int64_t N) {
+  auto width = [&](int most, int unit) { return (int)round_up(ceil_div(N, ceil_div(N, most)), unit); };
+  const int wide = width(BN, 8 * EPI), narrow = width(BN_JOINT, 16);
+  const double cw = block_cycles(wide) * (double)ceil_div(N, wide), cn = block_cycles(narrow) * (double)ceil_div(N, narrow);
+  return cn < cw || joint(wide) ? narrow : wide;
+}
 
 namespace {
-// Cycles an SM spends on one K block of a unit, measured: the five drains, one after the
-// other, take as long for few columns as for many.
-double block_cycles(int) { return 5750.0; }
-
 // Split-K of a product and its estimated time in us.  Rounds of units over the SMs times
 // the K blocks of a unit; a unit's epilogue costs about 90 cycles a column, partial sums
 // are written and read again at 5 TB/s, their reduction is one more launch (4 us).
@@ -851,6 +940,7 @@ void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial)
   a.tiles_m = (int)ceil_div(ps.M, BM);
   // column tiles of equal width (the B-side maps have boxes of this many rows)
   a.bn = tile_n(ps.N);
+  a.stages = std::min<int>(MAX_STAGES, (int)(STAGES * STAGE_BYTES / (kSlices * (A_SLICE + (uint32_t)a.bn * BK * 2))));
   a.tiles_n = (int)ceil_div(ps.N, a.bn);
   a.ny = ps.ny;
   a.nz = ps.nz;
@@ -929,7 +1019,7 @@ void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial)
   const int64_t units = (int64_t)a.tiles_m * a.tiles_n * start * a.splits;
   if (units > INT32_MAX) throw Error(SCESS_ERR_INVALID, "slice gemm: too many work units");
   launched_ = true;
-  scess::launch(slice_gemm_kernel, (unsigned)std::min<int64_t>(units, kNumSMs), THREADS, SMEM_BYTES, ctx_.stream, maps, a);
+  scess::launch(joint(a.bn) ? slice_gemm_kernel<true> : slice_gemm_kernel<false>, (unsigned)std::min<int64_t>(units, kNumSMs), THREADS, SMEM_BYTES, ctx_.stream, maps, a);
   SCESS_CHECK_LAUNCH();
   if (a.splits > 1) {
     const bool groups = split_groups(ps.M * ps.N, a.splits);

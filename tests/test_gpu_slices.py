@@ -1,8 +1,8 @@
 """FP64 contractions: on the tensor cores' exact BF16 slices (SliceEngine) and, for
 small products, on the FP64 units; the tuning key f64 selects either for any size.
 
-Sizes sit where the kernels can go wrong: tiles of 128 x 128 and K blocks of 32
-with remainders, one narrow side, K beyond what one unit's integer sum takes
+Sizes sit where the kernels can go wrong: tiles of 128 x 128, of 16 to 80 columns
+(other accumulators) and K blocks of 32 with remainders, one narrow side, K beyond what one unit's integer sum takes
 (16384: split), few tiles (split K) and many.
 
 Tolerance: an output is one rounding of a sum whose operands are cut 60 bits
@@ -24,7 +24,8 @@ def sliced(monkeypatch):
 
 
 SHAPES = [(1, 1, 1), (3, 2, 5), (129, 128, 1217), (128, 127, 1300), (2000, 17, 600), (8, 4001, 700), (1025, 641, 33),
-          (600, 520, 65), (300, 31, 16401), (24, 24, 36000), (2111, 1301, 8)]
+          (600, 520, 65), (300, 31, 16401), (24, 24, 36000), (2111, 1301, 8),
+          (700, 45, 300), (260, 60, 100), (20000, 75, 200), (200, 136, 1000)]
 
 
 def reference(A, B):
