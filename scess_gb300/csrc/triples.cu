@@ -29,6 +29,7 @@
 
 #include "gemm_slice.h"
 #include "gemm_tc.h"
+#include "launch.cuh"
 #include "triples.h"
 
 namespace scess {
@@ -501,7 +502,12 @@ __global__ void __launch_bounds__(256) triples_energy_orbit64_kernel(
   const int n = (int)nb;
   const int al = blockIdx.x / (n * n), bl = (blockIdx.x / n) % n, cl = blockIdx.x % n;
   const int64_t a = A * nb + al, b = Bk * nb + bl, c = C * nb + cl;
-  if (a >= v || b >= v || c >= v || b > a || c > b) return;
+  // the next block triple's GEMM may be placed: it waits for this grid before it writes W
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (a >= v || b >= v || c >= v || b > a || c > b) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
   extern __shared__ __align__(16) unsigned char sm_raw[];
   __shared__ double red[8];
   const int oo = (int)o, o2 = oo * oo, o3 = o2 * oo;
@@ -526,31 +532,39 @@ __global__ void __launch_bounds__(256) triples_energy_orbit64_kernel(
     tc[i] = t1[i + o * c];
     eo[i] = eps[i];
   }
-  // element e of a buffer: u = e % o, column e / o = s + o t; (su, ss, st) are the
-  // strides of u, s, t in Ws.  Eight loads in flight a thread.
-  auto add = [&](const double *Wg, int su, int ss, int st, bool first) {
-    for (int e0 = threadIdx.x; e0 < o3; e0 += 8 * blockDim.x) {
-      double x[8];
+  // S, t1 and eps come from the call's setup, W from the GEMM just before
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // Element e of a buffer: u = e % o, column e / o = s + o t.  W is summed in shared memory,
+  // buffer after buffer; the next chunk's loads (the next buffer's too) go out before a
+  // chunk is added.
+  constexpr int kStage = 5;
+  const int span = kStage * blockDim.x, nch = (o3 + span - 1) / span;
+  double x[kStage], y[kStage];
+  auto load = [&](int step, double *r) {
+    const int g = step / nch;
+    const double *Wg = g == 0 ? W0 : (g == 1 ? W1 : W2);
 #pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const int e = e0 + q * blockDim.x;
-        if (e < o3) x[q] = Wg[e % oo + Mg * (e / oo)];
-      }
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const int e = e0 + q * blockDim.x;
-        if (e < o3) {
-          const int u = e % oo, col = e / oo;
-          double *p = Ws + u * su + (col % oo) * ss + (col / oo) * st;
-          *p = first ? x[q] : *p + x[q];
-        }
-      }
+    for (int q = 0; q < kStage; q++) {
+      const int e = (step - g * nch) * span + (int)threadIdx.x + q * blockDim.x, col = e / oo;
+      if (e < o3) r[q] = Wg[e - col * oo + Mg * col];
     }
-    __syncthreads();
   };
-  add(W0, 1, p1, p2, true);    // (u, s, t) = (i, j, k)
-  add(W1, p1, 1, p2, false);   // (j, i, k)
-  add(W2, p2, 1, p1, false);   // (k, i, j)
+  load(0, x);
+  for (int step = 0; step < 3 * nch; step++) {
+    if (step + 1 < 3 * nch) load(step + 1, y);
+    // (u, s, t) = (i, j, k), (j, i, k), (k, i, j): strides in Ws
+    const int g = step / nch, su = g == 0 ? 1 : (g == 1 ? p1 : p2), ss = g == 0 ? p1 : 1, st = g == 2 ? p1 : p2;
+#pragma unroll
+    for (int q = 0; q < kStage; q++) {
+      const int e = (step - g * nch) * span + (int)threadIdx.x + q * blockDim.x, col = e / oo, t = col / oo;
+      if (e < o3) {
+        double *p = Ws + (e - col * oo) * su + (col - t * oo) * ss + t * st;
+        *p = g == 0 ? x[q] : *p + x[q];
+      }
+      x[q] = y[q];
+    }
+    if (step + 1 == (g + 1) * nch) __syncthreads();
+  }
   const double evirt = eps[o + a] + eps[o + b] + eps[o + c];
   double acc = 0.0;
   for (int q = threadIdx.x; q < norbits; q += blockDim.x) {
@@ -1260,8 +1274,8 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
         }
         se.gemm_grouped(ps, nprob * 2.0 * (double)Mg * Ng * (2.0 * v + 2.0 * o), "slice_gemm[triples]");
         TimedScope ts(ctx.timer, "triples_energy", 0.0, 24.0 * nb * nb * prob, s);
-        triples_energy_orbit64_kernel<<<(unsigned)(nb * nb * nb), threads, smem, s>>>(
-            W.d(), o, v, nb, A, Bk, C, d_eps, d_t1, T.S.p(), orbits.as<uint32_t>(), norbits, energies.p());
+        launch(triples_energy_orbit64_kernel, (unsigned)(nb * nb * nb), threads, smem, s, W.d(), o, v, nb, A, Bk, C,
+               d_eps, d_t1, T.S.p(), orbits.as<uint32_t>(), norbits, energies.p());
         SCESS_CHECK_LAUNCH();
         blocks_done++;
       }
