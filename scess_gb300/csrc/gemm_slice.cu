@@ -74,7 +74,7 @@ struct SliceMaps {
 };
 struct SliceArgs {
   int M, N, tiles_m, tiles_n;
-  int bn;      // tile width: a multiple of 32, at most 128, or (joint form) of 16, at most 80
+  int bn;      // tile width: a multiple of 16, at most 128 (joint form: 80)
   int stages;  // joint form
   int fs;      // fraction bits kept of the tail (see slice_value)
   int ny, nz, ng, nseg;
@@ -357,9 +357,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int q = warp & 3;
     const int row = 32 * q + lane;
     const int h = (warp - 4) >> 2;                  // column group
-    // its columns: a quarter of the tile's, or of its groups of eight
-    const int h0 = JOINT ? 8 * ((bn / 8 * h + 3) / 4) : bn / EPI * h;
-    const int hc = (JOINT ? 8 * ((bn / 8 * (h + 1) + 3) / 4) : bn / EPI * (h + 1)) - h0;
+    // its columns: a quarter of the tile's, in groups of eight
+    const int h0 = 8 * ((bn / 8 * h + 3) / 4), hc = 8 * ((bn / 8 * (h + 1) + 3) / 4) - h0;
     constexpr int HCT = JOINT ? HC_JOINT : HC;
     const int et = threadIdx.x - 128 - 128 * h;     // 0..127 within the group
     const int bar = 1 + h;
@@ -399,16 +398,16 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!mbar_wait(&ctl.tfull[b], (uint32_t)(c / NROT) & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) return false;
         tc_fence_after();
         const uint32_t t0 = tl + (uint32_t)(b * bn);
-        // (16 columns a load: the sums take most of the registers)
+        // (8 columns a load: the sums take most of the registers)
 #pragma unroll
-        for (int j = 0; j < HC; j += 16) {
-          if (j < hc) {  // (columns past hc, within TMEM, are not used)
-            uint32_t r[16];
-            tmem_ld16_async(t0 + (uint32_t)j, r);
-            tmem_wait16(r);
-            if (j + 16 >= hc) release(b);  // (all columns are in registers)
+        for (int j = 0; j < HC; j += 8) {
+          if (j < hc) {
+            uint32_t r[8];
+            tmem_ld8(t0 + (uint32_t)j, r);
+            tmem_wait8(r);
+            if (j + 8 >= hc) release(b);  // (all columns are in registers)
 #pragma unroll
-            for (int i = 0; i < 16; i++) add_diag<D>(T[j + i], r[i]);
+            for (int i = 0; i < 8; i++) add_diag<D>(T[j + i], r[i]);
           }
         }
         c++;
@@ -767,15 +766,14 @@ namespace {
 // The joint form's tiles are at most 80 wide.
 bool joint(int bn) { return bn <= BN_JOINT; }
 // Cycles an SM spends on one K block of a unit, measured (152 tiles of 128 rows, K = 1024:
-// widths 16 .. 128): in the rotating form the five drains, one after the other, take as long
-// for 96 columns as for 128.
-double block_cycles(int bn) { return joint(bn) ? 3200.0 + 25.0 * bn : 5750.0; }
+// widths 16 .. 128; 4096^3 for the scale).
+double block_cycles(int bn) { return joint(bn) ? 2950.0 + 25.0 * bn : 3150.0 + 20.0 * bn; }
 }  // namespace
 
 // The narrow tile where it is cheaper.
 int SliceEngine::tile_n(int64_t N) {
   auto width = [&](int most, int unit) { return (int)round_up(ceil_div(N, ceil_div(N, most)), unit); };
-  const int wide = width(BN, 8 * EPI), narrow = width(BN_JOINT, 16);
+  const int wide = width(BN, 16), narrow = width(BN_JOINT, 16);
   const double cw = block_cycles(wide) * (double)ceil_div(N, wide), cn = block_cycles(narrow) * (double)ceil_div(N, narrow);
   return cn < cw || joint(wide) ? narrow : wide;
 }
