@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(256, 4) triples_energy_orbit_kernel(
 // u the occupied partner of x and (s, t) the other two occupied indices in order;
 // W = (W_0 + W_1) + W_2 is formed in shared memory.  Then as the mixed form: one
 // thread per orbit of (i, j, k), six orderings sharing one denominator.  GB300
-// issues about two FP64 lanes per cycle and SM, so this kernel is FP64-bound: 18 FMAs
+// issues about two FP64 lanes per cycle and SM, so this kernel is FP64-bound (about 70 % at o = 10): 18 FMAs
 // for W + V of an orbit, 18 for r3 and its products, one division, and 12 adds for
 // the sum of the buffers (10 FP64 operations per element; a thread per element with
 // its own denominator took about 30).
@@ -509,7 +509,6 @@ __global__ void __launch_bounds__(256) triples_energy_orbit64_kernel(
     return;
   }
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  __shared__ double red[8];
   const int oo = (int)o, o2 = oo * oo, o3 = o2 * oo;
   // W(i,j,k) at i + p1 j + p2 k and the slices at x + p1 y, p1 and p2 odd: reads along
   // any one index are free of bank conflicts
@@ -592,19 +591,22 @@ __global__ void __launch_bounds__(256) triples_energy_orbit64_kernel(
     num = fma(wo2, fma(3.0, yo2, co), num);
     const double d = ((eo[i] + eo[j]) + eo[k]) - evirt;                             // :155
     // an orbit with two (three) equal indices visits its elements twice (six times)
-    acc += num / (m == 0 ? d : (m == 1 ? d + d : 6.0 * d));                         // :156
+    acc += num * (m == 0 ? 1.0 : (m == 1 ? 0.5 : 1.0 / 6.0)) / d;                   // :156
   }
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) red[w] = acc;
+  // the CTA's sum in one warp: eight warps' shuffles cost more FP64 issue than this
+  __syncthreads();  // (W is read)
+  Ws[threadIdx.x] = acc;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); q++) s += red[q];
-    double deg = 1.0;                                                               // :135-139
-    if (a == c) deg = 6.0;
-    else if (a == b || b == c) deg = 2.0;
-    energies[triple_id(a, b, c)] = s / deg;
+  if (threadIdx.x < 32) {
+    double sum = 0.0;
+    for (int q = threadIdx.x; q < (int)blockDim.x; q += 32) sum += Ws[q];
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
+    if (threadIdx.x == 0) {
+      // degeneracy of the virtual indices                                            :135-139
+      if (a == c) sum /= 6.0;
+      else if (a == b || b == c) sum *= 0.5;
+      energies[triple_id(a, b, c)] = sum;
+    }
   }
 }
 
@@ -1219,9 +1221,9 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
   SCESS_CUDA(cudaMemcpyAsync(orbits.as<void>(), ot.data(), ot.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   ctx.sync();  // (ot is a host vector of this scope)
   const int64_t p1 = o | 1, p2 = (p1 * o) | 1;
-  const size_t smem = (size_t)(p2 * o + 3 * p1 * o + 4 * o) * 8;
-  SCESS_CUDA(cudaFuncSetAttribute(triples_energy_orbit64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const unsigned threads = (unsigned)std::min<int64_t>(256, round_up(norbits, 32));
+  const size_t smem = (size_t)std::max<int64_t>(p2 * o + 3 * p1 * o + 4 * o, threads) * 8;
+  SCESS_CUDA(cudaFuncSetAttribute(triples_energy_orbit64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   SliceProblemSet ps;
   const SlicedPack *packs[6] = {&pP, &pQ, &pQ2, &pR, &pR2, &pTx};
   const int bn = SliceEngine::tile_n(Ng);
