@@ -75,8 +75,7 @@ struct TcArgs {
   const int64_t *rowCg[3], *colCg[3];  // per-group output tables (null: TcOut's)
   int tri[3];                          // group g keeps only the problems with y >= z (ny == nz)
   int gstart[4];                       // first problem index of each group (gstart[ng] = total)
-  int stcol[3];                        // group stores along columns (FP32, beta = 0)
-  int stvec[3];                        // ... in contiguous aligned quads of columns
+  int stvec[3];                        // group stores in contiguous aligned quads of columns
   float *partial;    // split-K partials (nullptr: direct epilogue)
   int64_t part_stride;
   unsigned *err;
@@ -131,7 +130,6 @@ struct TcShape {
   static constexpr int EPI0 = BN == 256 ? 4 : 2;   // first epilogue warp
   static constexpr int NEPI = BN / 32;              // epilogue warps
   static constexpr int THREADS = 32 * (EPI0 + NEPI);
-  static constexpr int CH = BN == 256 ? 16 : 32;    // columns per staged chunk
   static constexpr uint32_t A_BYTES = (uint32_t)TC_BM * BK * 2;
   static constexpr uint32_t B_BYTES = (uint32_t)BNL * BK * 2;
   static constexpr uint32_t STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
@@ -195,9 +193,6 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
   // for the previous store).
   __shared__ int64_t colOff[BN];
   __shared__ int64_t rowOffS[BN / 128][TC_BM];        // row offsets of a column-stored unit
-  // chunk of such a unit; row pitch 129 (CH = 32) or 130 (CH = 16, two rows a
-  // warp step) keeps the column-wise reads free of bank conflicts
-  __shared__ float stage[BN / 128][SH::CH][TC_BM + (SH::CH == 16 ? 2 : 1)];
   // Output scaling, once per CTA: alpha / (sA sB) with power-of-two pack
   // scales sA, sB.  FP32 outputs multiply by it in FP32; FP64 outputs multiply
   // by the user's alpha in FP32 and apply 2^-log2(sA sB) to the exponent field
@@ -628,73 +623,6 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
           }
         }
         __syncwarp();  // rowOffS read before the next unit rewrites it
-        continue;
-      }
-      if (a.stcol[pg] && out.fp32 && (out.beta == 0.0 || accum) && !a.partial) {
-        // Tile staged through shared memory CH columns at a time, then each warp
-        // stores (beta = 1: adds) its 32 rows with the lanes along the columns: for
-        // outputs whose unit-stride index is a column index this writes contiguous runs.
-        // (The (T) launch with o not a multiple of 4: with every lane in a row of its own
-        // the reductions of o = 13, v = 117 took 154 us a launch, now 96.)
-        float *C = (float *)out.C;
-        const float fa = s_falpha;
-        constexpr int CH = SH::CH;
-        rowOffS[h][row] = m < a.M ? rowOff : -1;
-#pragma unroll
-        for (int j0 = 0; j0 < HC; j0 += CH) {
-          // each warp stages and stores only its own 32 rows: warp-level ordering
-          __syncwarp();  // previous chunk read, rowOffS set
-#pragma unroll
-          for (int jj = 0; jj < CH; jj++) stage[h][jj][row] = fa * acc[j0 + jj];
-          __syncwarp();
-          if (BN == 256 && a.stvec[pg] && !accum) {  // (the (T) launch; einsums keep the scalar form)
-            // every aligned quad of columns is a contiguous 16-byte run: lanes
-            // take quad lane % QPR of row rr + lane / QPR (conflict-free reads:
-            // the staging pitch is 2 mod 32 words)
-            constexpr int QPR = CH / 4, RSTEP4 = 32 / QPR;
-            const int cq = lane % QPR, rsub4 = lane / QPR;
-            const int64_t co = colH[j0 + 4 * cq];
-#pragma unroll
-            for (int rr = 0; rr < 32; rr += RSTEP4) {
-              const int r = 32 * q + rr + rsub4;
-              const int64_t ro = rowOffS[h][r];
-              if (ro >= 0 && co >= 0) {
-                const float v0 = stage[h][4 * cq][r], v1 = stage[h][4 * cq + 1][r];
-                const float v2 = stage[h][4 * cq + 2][r], v3 = stage[h][4 * cq + 3][r];
-                float *d = C + ro + co;
-                if (((uintptr_t)d & 15) == 0) {
-                  *reinterpret_cast<float4 *>(d) = make_float4(v0, v1, v2, v3);
-                } else {  // (not expected: the host asks for quads only when aligned)
-                  d[0] = v0;
-                  d[1] = v1;
-                  d[2] = v2;
-                  d[3] = v3;
-                }
-              }
-            }
-          } else {
-            // lanes take column lane % CH of row rr + lane / CH (CH = 16: two rows a step)
-            const int cl = lane % CH;
-            const int rsub = lane / CH;
-            constexpr int RSTEP = 32 / CH;
-            const int64_t co = colH[j0 + cl];
-            if (accum) {
-#pragma unroll 4
-              for (int rr = 0; rr < 32; rr += RSTEP) {
-                const int r = 32 * q + rr + rsub;
-                const int64_t ro = rowOffS[h][r];
-                if (ro >= 0 && co >= 0) atomicAdd(C + ro + co, stage[h][cl][r]);
-              }
-            } else {
-#pragma unroll 4
-              for (int rr = 0; rr < 32; rr += RSTEP) {
-                const int r = 32 * q + rr + rsub;
-                const int64_t ro = rowOffS[h][r];
-                if (ro >= 0 && co >= 0) C[ro + co] = stage[h][cl][r];
-              }
-            }
-          }
-        }
         continue;
       }
       if (m >= a.M) continue;
@@ -1195,8 +1123,7 @@ void tc_gemm_launch_grouped(const TcProblemSet &ps, TcFormat fmt, const TcOut &o
     a.cg[q] = ps.cg[q];
     a.rowCg[q] = ps.rowC[q];
     a.colCg[q] = ps.colC[q];
-    a.stcol[q] = ps.store_by_column[q] ? 1 : 0;
-    a.stvec[q] = ps.store_by_column[q] && ps.store_quads[q] ? 1 : 0;
+    a.stvec[q] = ps.store_quads[q] ? 1 : 0;
   }
   a.partial = splits > 1 ? partial : nullptr;
   a.part_stride = ps.M * ps.N;

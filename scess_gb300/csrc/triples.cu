@@ -149,11 +149,13 @@ __global__ void to_f32_rows_kernel(const double *__restrict__ x, int64_t rows, i
   }
 }
 
-// Layout of the mixed form's W and of the FP32 copy of S its energy kernel
-// reads: rows of o^2 (i, j) pairs are padded to o2p = o^2 rounded up to a
-// multiple of 4 floats, so that every k row and every o^3 block starts on a
-// 16-byte boundary.  W[((a_l nb + b_l) nb + c_l) o3p + i + o j + o2p k] with
-// o3p = o o2p; S as [(a + v b) o2p + i + o j].
+// Layout of the mixed form's W and of the FP32 copy of S its energy kernel reads: runs
+// of o values of i are padded to op = o rounded up to a multiple of 4 floats, so that every
+// quad of i values is aligned: W[((a_l nb + b_l) nb + c_l) o3p + i + op j + o2p k] with
+// o2p = o op, o3p = o o2p; S as [(a + v b) o2p + i + op j].  The grouped GEMM's columns are
+// padded the same way (o op of them), so that its groups add W in 16-byte reductions and
+// the energy kernel reads it in 16-byte loads whatever o.  (With o = 13 unpadded the groups'
+// reductions went through shared memory a float at a time: 97 us a launch at v = 117, 81 this way.)
 __host__ __device__ inline int64_t pad4(int64_t n) { return (n + 3) & ~int64_t(3); }
 
 // FP32 tables of the mixed energy kernel, built once per (T) call: every
@@ -213,13 +215,13 @@ std::vector<uint32_t> orbit_table(int64_t o) {
 // (W_0[b,c][a], W_1[a,c][b], W_2[a,b][c], as laid out by their tables), or
 // NW = 1 buffer the groups reduced into (W[a,b,c]), which this kernel clears
 // after reading so that it starts at zero for the next block triple.  Each
-// block is o^3 floats in (i, j, k) order, i + o j + o2p k.  One CTA per local
+// block is o^3 floats in (i, j, k) order, i + op j + o2p k.  One CTA per local
 // triple (a_l, b_l, c_l).
 //
 // Pass 1: Y = W + V in shared memory, V_ijk = t1_ia (jb|kc) + t1_jb (ia|kc) +
-// t1_kc (ia|jb) (GetV, RCCSD_T.cpp:70-75).  A thread owns a pair (i, j), or four
-// with consecutive i where o is a multiple of four, and some of the k; the loads of
-// several k are issued before any is used, and what was read is cleared at once.
+// t1_kc (ia|jb) (GetV, RCCSD_T.cpp:70-75).  A thread owns four pairs (i, j) with
+// consecutive i and some of the k; the loads of several k are issued before any is
+// used, and what was read is cleared at once.
 // Pass 2 (threads own orbits of (i, j, k)): r3 (:152-154) of an even ordering
 // of the orbit is 3 Y + (S_e - 2 S_o), of an odd one 3 Y + (S_o - 2 S_e)
 // (S_e, S_o: sums of Y over the even / odd orderings), and the denominator
@@ -239,7 +241,7 @@ std::vector<uint32_t> orbit_table(int64_t o) {
 // 45.5 us with V recomputed and the energies added per orbit, 38.3 this way.
 constexpr int kEnergyMaxO = 32;
 template <int NW, bool WS>
-__global__ void __launch_bounds__(256, 4) triples_energy_orbit_kernel(
+__global__ void __launch_bounds__(256, WS ? 4 : 3) triples_energy_orbit_kernel(
     float *__restrict__ W, int64_t o, int64_t v, int64_t nb, int64_t A, int64_t Bk, int64_t C,
     const float2 *__restrict__ ehl, const float *__restrict__ t1f, const float *__restrict__ S,
     const uint4 *__restrict__ orbits, int norbits, double *__restrict__ energies) {
@@ -247,7 +249,7 @@ __global__ void __launch_bounds__(256, 4) triples_energy_orbit_kernel(
             cl = (int)(blockIdx.x % nb);
   const int64_t a = A * nb + al, b = Bk * nb + bl, c = C * nb + cl;
   const int oo = (int)o, o2 = oo * oo;
-  const int o2p = (int)pad4(o2), o3p = oo * o2p;
+  const int op = (int)pad4(oo), o2p = oo * op, o3p = oo * o2p;
   const int64_t nb3o3 = nb * nb * nb * (int64_t)o3p;
   float *W0;
   const float *W1 = nullptr, *W2 = nullptr;
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(256, 4) triples_energy_orbit_kernel(
   // i + p1 j + p2 k.  Odd pitches keep reads along any one index free of bank conflicts
   // (the slices are read that way in pass 2 alone).
   constexpr int EL = WS ? 8 : 4;  // bytes of an element
-  const int p1 = oo | 1, p2 = (p1 * oo) | 1, ps = WS ? oo : p1, slice = WS ? o2p : p1 * oo;
+  const int p1 = oo | 1, p2 = (p1 * oo) | 1, ps = WS ? op : p1, slice = WS ? o2p : p1 * oo;
   float4 *tab = reinterpret_cast<float4 *>(sm_raw);
   float *Sbc = reinterpret_cast<float *>(tab + oo), *Sac = Sbc + slice, *Sab = Sac + slice;
   float *Y = Sab + slice;
@@ -295,9 +297,9 @@ __global__ void __launch_bounds__(256, 4) triples_energy_orbit_kernel(
   } else {
     for (int e = threadIdx.x; e < o2; e += blockDim.x) {
       const int x = e % oo, y = e / oo;
-      Sbc[x + p1 * y] = S_bc[e];
-      Sac[x + p1 * y] = S_ac[e];
-      Sab[x + p1 * y] = S_ab[e];
+      Sbc[x + p1 * y] = S_bc[x + op * y];
+      Sac[x + p1 * y] = S_ac[x + op * y];
+      Sab[x + p1 * y] = S_ab[x + op * y];
     }
   }
   for (int i = threadIdx.x; i < oo; i += blockDim.x)
@@ -316,85 +318,82 @@ __global__ void __launch_bounds__(256, 4) triples_energy_orbit_kernel(
   // before, complete after this wait
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // pass 1; the first loads go out before the barrier that publishes the tables
-  auto pass1 = [&](auto quad) {
-    constexpr int Q = decltype(quad)::value;
-    using Vec = std::conditional_t<Q == 4, float4, float>;
-    constexpr int CH = Q == 4 ? 4 : 8;  // k loads of a thread in flight (more would spill)
-    const int nu = o2 / Q, kgn = max(1, (int)blockDim.x / nu), units = nu * kgn;
-    int t = threadIdx.x, i = 0, j = 0, k0 = 0;
-    Vec r[CH];
-    float *w = W0;
-    auto begin = [&]() {
-      const int kg = t / nu, pr = (t - kg * nu) * Q;
-      j = pr / oo;
-      i = pr - j * oo;
-      k0 = kg;
-      w = W0 + pr;
-    };
-    auto load = [&]() {
+  constexpr int CH = 4;  // k loads of a thread in flight (more would spill)
+  const int nu = o2p / 4, kgn = max(1, (int)blockDim.x / nu), units = nu * kgn;
+  int t = threadIdx.x, i = 0, j = 0, k0 = 0;
+  float4 r[CH];
+  float *w = W0;
+  auto begin = [&]() {
+    k0 = t / nu;
+    const int u = t - k0 * nu;
+    j = u / (op / 4);
+    i = 4 * u - j * op;
+    w = W0 + 4 * u;
+  };
+  auto load = [&]() {
 #pragma unroll
-      for (int n = 0; n < CH; n++) {
-        const int k = k0 + n * kgn;
-        if (k < oo) {
-          r[n] = *reinterpret_cast<const Vec *>(w + k * o2p);
-          if (NW == 3) {
-            const Vec x = *reinterpret_cast<const Vec *>(W1 + (w - W0) + k * o2p),
-                      y = *reinterpret_cast<const Vec *>(W2 + (w - W0) + k * o2p);
-            if constexpr (Q == 4)
-              r[n] = make_float4(r[n].x + (x.x + y.x), r[n].y + (x.y + y.y), r[n].z + (x.z + y.z),
-                                 r[n].w + (x.w + y.w));
-            else
-              r[n] += x + y;
-          }
+    for (int n = 0; n < CH; n++) {
+      const int k = k0 + n * kgn;
+      if (k < oo) {
+        r[n] = *reinterpret_cast<const float4 *>(w + k * o2p);
+        if (NW == 3) {
+          const float4 x = *reinterpret_cast<const float4 *>(W1 + (w - W0) + k * o2p),
+                       y = *reinterpret_cast<const float4 *>(W2 + (w - W0) + k * o2p);
+          r[n] = make_float4(r[n].x + (x.x + y.x), r[n].y + (x.y + y.y), r[n].z + (x.z + y.z), r[n].w + (x.w + y.w));
         }
       }
-    };
-    if (t < units) {
-      begin();
-      load();
     }
-    __syncthreads();
-    while (t < units) {
-      const float tbj = tab[j].y;
-      float tai[Q], sab[Q];
+  };
+  if (t < units) {
+    begin();
+    load();
+  }
+  __syncthreads();
+  while (t < units) {
+    // (values of i from o on are padding: read like the others, not stored)
+    const float tbj = tab[j].y;
+    float tai[4], sab[4];
 #pragma unroll
-      for (int q = 0; q < Q; q++) {
-        tai[q] = tab[i + q].x;
-        sab[q] = Sab[i + q + ps * j];
-      }
-      unsigned char *y0 = yb + EL * (i + p1 * j);
+    for (int q = 0; q < 4; q++) {
+      tai[q] = tab[i + q].x;
+      sab[q] = Sab[i + q + ps * j];
+    }
+    unsigned char *y0 = yb + EL * (i + p1 * j);
 #pragma unroll
-      for (int n = 0; n < CH; n++) {
-        const int k = k0 + n * kgn;
-        if (k < oo) {
-          const float bc = Sbc[j + ps * k], tck = tab[k].z;
-          const Vec sac = *reinterpret_cast<const Vec *>(Sac + i + ps * k);
-          const float *ac = reinterpret_cast<const float *>(&sac), *wr = reinterpret_cast<const float *>(&r[n]);
+    for (int n = 0; n < CH; n++) {
+      const int k = k0 + n * kgn;
+      if (k < oo) {
+        const float bc = Sbc[j + ps * k], tck = tab[k].z;
+        alignas(16) float ac[4];
+        if (WS) {
+          *reinterpret_cast<float4 *>(ac) = *reinterpret_cast<const float4 *>(Sac + i + ps * k);
+        } else {
 #pragma unroll
-          for (int q = 0; q < Q; q++) {
-            const float y = wr[q] + (tai[q] * bc + tbj * ac[q] + tck * sab[q]);
+          for (int q = 0; q < 4; q++) ac[q] = Sac[i + q + ps * k];
+        }
+        const float wr[4] = {r[n].x, r[n].y, r[n].z, r[n].w};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const float y = wr[q] + (tai[q] * bc + tbj * ac[q] + tck * sab[q]);
+          if (i + q < oo) {
             if (WS)
               *reinterpret_cast<float2 *>(y0 + EL * (p2 * k + q)) = make_float2(y, wr[q]);
             else
               *reinterpret_cast<float *>(y0 + EL * (p2 * k + q)) = y;
           }
-          // W is read: cleared for the next block triple's reductions
-          if (NW == 1) *reinterpret_cast<Vec *>(w + k * o2p) = Vec{};
         }
+        // W is read: cleared for the next block triple's reductions
+        if (NW == 1) *reinterpret_cast<float4 *>(w + k * o2p) = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      k0 += CH * kgn;
-      if (k0 >= oo) {
-        t += blockDim.x;
-        if (kgn > 1 || t >= units) break;
-        begin();
-      }
-      load();
     }
-  };
-  if (WS && (oo & 3) == 0)
-    pass1(std::integral_constant<int, 4>{});
-  else
-    pass1(std::integral_constant<int, 1>{});
+    k0 += CH * kgn;
+    if (k0 >= oo) {
+      t += blockDim.x;
+      if (kgn > 1 || t >= units) break;
+      begin();
+    }
+    load();
+  }
   // (shared memory leaves the L1 cache little room: the orbit table comes from L2, an
   // entry ahead of its use)
   int q = threadIdx.x;
@@ -630,6 +629,10 @@ __global__ void sum_energies_kernel(int64_t n, const double *__restrict__ e, dou
 struct TableSpec {
   int nd = 0;
   int64_t ext[6] = {1, 1, 1, 1, 1, 1}, str[6] = {0, 0, 0, 0, 0, 0};
+  // first dimension: entries from `valid` on are padding, and read the last valid index
+  // or (skip) get kNoOffset
+  int64_t valid = INT64_MAX;
+  bool skip = false;
   int64_t size() const {
     int64_t n = 1;
     for (int d = 0; d < nd; d++) n *= ext[d];
@@ -648,6 +651,13 @@ TableSpec table(std::initializer_list<std::pair<int64_t, int64_t>> dims) {
   return t;
 }
 
+TableSpec padded(TableSpec t, int64_t valid, bool skip) {
+  t.valid = valid;
+  t.skip = skip;
+  return t;
+}
+constexpr int64_t kNoOffset = -(int64_t(1) << 60);  // negative with every base added
+
 constexpr int kMaxTables = 24;
 struct TableBatch {
   int nt = 0;
@@ -664,12 +674,18 @@ __global__ void fill_tables_kernel(const __grid_constant__ TableBatch b) {
     while (e >= b.start[t + 1]) t++;
     const TableSpec &sp = b.spec[t];
     int64_t r = e - b.start[t], off = 0;
+    bool none = false;
     for (int d = 0; d < sp.nd; d++) {
       const int64_t q = r / sp.ext[d];
-      off += (r - q * sp.ext[d]) * sp.str[d];
+      int64_t i = r - q * sp.ext[d];
+      if (d == 0 && i >= sp.valid) {
+        none = sp.skip;
+        i = sp.valid - 1;
+      }
+      off += i * sp.str[d];
       r = q;
     }
-    b.out[e] = off;
+    b.out[e] = none ? kNoOffset : off;
   }
 }
 
@@ -1099,7 +1115,7 @@ int choose_nb_grouped(int64_t o, int64_t v) {
   if (forced >= 1) return (int)std::min<int64_t>(forced, v);
   int best = 1;
   double best_score = -1.0;
-  const double o3 = (double)o * o * o, bm = TcEngine::pair_available() ? 256.0 : 128.0;
+  const double o3 = (double)o * o * pad4(o), bm = TcEngine::pair_available() ? 256.0 : 128.0;
   for (int nb = 1; nb <= std::min<int64_t>(v, 64); nb++) {
     if (nb > 1 && (double)nb * nb * nb * o3 * 4.0 > double(64 << 20)) break;
     const double rows = (double)o * nb;
@@ -1329,12 +1345,11 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
   const int64_t ntrip = v * (v + 1) * (v + 2) / 6;
   DTensor energies({std::max<int64_t>(ntrip, 1)});
   SCESS_CUDA(cudaMemsetAsync(energies.p(), 0, energies.size() * sizeof(double), s));
-  // FP64: W in FP64.  MIXED: W in FP32 with rows of (i, j) pairs padded to o2p
-  // floats (see pad4), either three buffers the groups store into (nw = 3) or
+  // FP64: W in FP64.  MIXED: W in FP32 with runs of i padded to op floats (see pad4), either three buffers the groups store into (nw = 3) or
   // one the groups add into with L2 reductions (nw = 1: zeroed here, cleared
   // again by every energy launch after it has read it)
   const int nw = tune_value("t_wbuf", kTriplesWBuffers) == 3 ? 3 : 1;
-  const int64_t o2p = pad4(o2), o3p = o * o2p;
+  const int64_t op = pad4(o), o2p = o * op, o3p = o * o2p;
   const size_t wbytes = (size_t)nb * nb * nb * (mixed ? 4 * nw * o3p : 8 * o3);
   DevMem W(wbytes);
   if (mixed && nw == 1) SCESS_CUDA(cudaMemsetAsync(W.as<void>(), 0, wbytes, s));
@@ -1395,23 +1410,23 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
   uint4 *orb = nullptr;
   float2 *ehl = nullptr;
   float *t1f = nullptr;
-  const int64_t Mg = o * nb, Ng = o2;
+  const int64_t Mg = o * nb, Ng = o2p;  // (columns (s, t), s padded to op)
   if (mixed) {
     TimedScope ts(ctx.timer, "phase:triples_pack", 0.0, 0.0, s);
     TcEngine &tc = ctx.tensor_cores();
     std::vector<TableSpec> pt;
     // P rows r = i + o(x + nb(y + nb(Y + NB X))):  P(i, f, X nb + x, Y nb + y)
     pt.push_back(table({{o, 1}, {nb, o * v}, {nb, o * v * vp}, {NB, o * v * vp * nb}, {NB, o * v * nb}}));
-    // Q rows r = j + o(k + o(z + nb Z)):  Q(f, j, k, Z nb + z)
-    pt.push_back(table({{o, v}, {o, v * o}, {nb, v * o2}, {NB, v * o2 * nb}}));
-    // R rows r = i + o(j + o(x + nb X)):  R(i, j, m, X nb + x)
-    pt.push_back(table({{o, 1}, {o, o}, {nb, o3}, {NB, o3 * nb}}));
+    // Q rows r = j + op(k + o(z + nb Z)):  Q(f, j, k, Z nb + z), padding repeated from j = o - 1
+    pt.push_back(padded(table({{op, v}, {o, v * o}, {nb, v * o2}, {NB, v * o2 * nb}}), o, false));
+    // R rows r = i + op(j + o(x + nb X)):  R(i, j, m, X nb + x)
+    pt.push_back(padded(table({{op, 1}, {o, o}, {nb, o3}, {NB, o3 * nb}}), o, false));
     // t2 rows r = u + o(x + nb(z + nb(X + NB Z))):  t2(m, u, Z nb + z, X nb + x)
     pt.push_back(table({{o, o}, {nb, o2 * vp}, {nb, o2}, {NB, o2 * vp * nb}, {NB, o2 * nb}}));
-    // Q rows in (k, j) order: r = k + o(j + o(z + nb Z))
-    pt.push_back(table({{o, v * o}, {o, v}, {nb, v * o2}, {NB, v * o2 * nb}}));
-    // R rows in (j, i) order: r = j + o(i + o(x + nb X))
-    pt.push_back(table({{o, o}, {o, 1}, {nb, o3}, {NB, o3 * nb}}));
+    // Q rows in (k, j) order: r = k + op(j + o(z + nb Z))
+    pt.push_back(padded(table({{op, v * o}, {o, v}, {nb, v * o2}, {NB, v * o2 * nb}}), o, false));
+    // R rows in (j, i) order: r = j + op(i + o(x + nb X))
+    pt.push_back(padded(table({{op, o}, {o, 1}, {nb, o3}, {NB, o3 * nb}}), o, false));
     DevTables pdt;
     pdt.build(ctx, pt);
     DevMem maxw(2 * sizeof(unsigned));
@@ -1419,14 +1434,14 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
     SCESS_CUDA(cudaMemsetAsync(mx, 0, 2 * sizeof(unsigned), s));
     tc.maxabs_into(P.p(), pdt.ptr[0], o * vp * vp, dt.ptr[kOperand + 1], v, false, mx);
     tc.maxabs_into(T2p.p(), pdt.ptr[3], o * vp * vp, dt.ptr[kOperand + 7], o, true, mx);
-    tc.maxabs_into(Qt.p(), pdt.ptr[1], o2 * vp, dt.ptr[kOperand + 3], v, true, mx + 1);
-    tc.maxabs_into(Rt.p(), pdt.ptr[2], o2 * vp, dt.ptr[kOperand + 5], o, false, mx + 1);
+    tc.maxabs_into(Qt.p(), pdt.ptr[1], o2p * vp, dt.ptr[kOperand + 3], v, true, mx + 1);
+    tc.maxabs_into(Rt.p(), pdt.ptr[2], o2p * vp, dt.ptr[kOperand + 5], o, false, mx + 1);
     tc.pack_with_max(P.p(), pdt.ptr[0], o * vp * vp, dt.ptr[kOperand + 1], v, false, 128, mx, false, pP);
     tc.pack_with_max(T2p.p(), pdt.ptr[3], o * vp * vp, dt.ptr[kOperand + 7], o, true, 128, mx, true, pTx, rbk);
-    tc.pack_with_max(Qt.p(), pdt.ptr[1], o2 * vp, dt.ptr[kOperand + 3], v, true, 128, mx + 1, false, pQ);
-    tc.pack_with_max(Qt.p(), pdt.ptr[4], o2 * vp, dt.ptr[kOperand + 3], v, true, 128, mx + 1, false, pQ2);
-    tc.pack_with_max(Rt.p(), pdt.ptr[2], o2 * vp, dt.ptr[kOperand + 5], o, false, 128, mx + 1, false, pR, rbk);
-    tc.pack_with_max(Rt.p(), pdt.ptr[5], o2 * vp, dt.ptr[kOperand + 5], o, false, 128, mx + 1, false, pR2, rbk);
+    tc.pack_with_max(Qt.p(), pdt.ptr[1], o2p * vp, dt.ptr[kOperand + 3], v, true, 128, mx + 1, false, pQ);
+    tc.pack_with_max(Qt.p(), pdt.ptr[4], o2p * vp, dt.ptr[kOperand + 3], v, true, 128, mx + 1, false, pQ2);
+    tc.pack_with_max(Rt.p(), pdt.ptr[2], o2p * vp, dt.ptr[kOperand + 5], o, false, 128, mx + 1, false, pR, rbk);
+    tc.pack_with_max(Rt.p(), pdt.ptr[5], o2p * vp, dt.ptr[kOperand + 5], o, false, 128, mx + 1, false, pR2, rbk);
     ctx.sync();
     // B side (Q, R rows): tiles of tbn columns; 256 halves the A-operand
     // shared-memory traffic per FLOP (SCESS_T_BN=128 selects the narrow tiles).
@@ -1437,19 +1452,15 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
     mR = TcEngine::map_of(pR, bbox, rbk);
     mR2 = TcEngine::map_of(pR2, bbox, rbk);
     mTx = TcEngine::map_of(pTx, 128, rbk);
-    // Every group writes its (u, s, t) at the triple's (i, j, k), i + o j + o2p k.
-    // Rows (u, x_l), columns (s, t): g = 0 (x = a): (u,s,t) = (i,j,k);
-    // g = 1 (x = b): (j,i,k); g = 2 (x = c): (k,i,j).  nw = 3: buffer g holds
-    // W_g[(y_l nb + z_l) nb + x_l]; nw = 1: W[(a_l nb + b_l) nb + c_l], the
-    // (y_l, z_l) strides being the problem offsets cy, cz.
-    if (nw == 3)
-      gdt.build(ctx, {table({{o, 1}, {nb, o3p}}), table({{o, o}, {o, o2p}}),
-                 table({{o, o}, {nb, o3p}}), table({{o, 1}, {o, o2p}}),
-                 table({{o, o2p}, {nb, o3p}}), table({{o, 1}, {o, o}})});
-    else
-      gdt.build(ctx, {table({{o, 1}, {nb, nb * nb * o3p}}), table({{o, o}, {o, o2p}}),
-                 table({{o, o}, {nb, nb * o3p}}), table({{o, 1}, {o, o2p}}),
-                 table({{o, o2p}, {nb, o3p}}), table({{o, 1}, {o, o}})});
+    // Every group writes its (u, s, t) at the triple's (i, j, k), i + op j + o2p k.
+    // Rows (u, x_l), columns (s, t): g = 0 (x = a): (u,s,t) = (i,j,k), padding skipped;
+    // g = 1 (x = b): (j,i,k); g = 2 (x = c): (k,i,j), both with the padding of i.
+    // nw = 3: buffer g holds W_g[(y_l nb + z_l) nb + x_l]; nw = 1:
+    // W[(a_l nb + b_l) nb + c_l], the (y_l, z_l) strides being the problem offsets cy, cz.
+    const int64_t xa = nw == 3 ? o3p : nb * nb * o3p, xb = nw == 3 ? o3p : nb * o3p;
+    gdt.build(ctx, {table({{o, 1}, {nb, xa}}), padded(table({{op, op}, {o, o2p}}), o, true),
+                    table({{o, op}, {nb, xb}}), table({{op, 1}, {o, o2p}}),
+                    table({{o, o2p}, {nb, o3p}}), table({{op, 1}, {o, op}})});
     Sf.alloc((size_t)o2p * v * v * sizeof(float));
     etab.alloc((size_t)norbits * sizeof(uint4) + (size_t)N * sizeof(float2) + (size_t)o * v * sizeof(float));
     orb = etab.as<uint4>();
@@ -1459,7 +1470,7 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
         d_eps, N, d_t1, o * v, orbits.as<uint32_t>(), norbits, ehl, t1f, orb);
     SCESS_CHECK_LAUNCH();
     to_f32_rows_kernel<<<(unsigned)std::min<int64_t>(ceil_div(o2p * v * v, 256), 16 * kNumSMs), 256, 0, s>>>(
-        T.S.p(), v * v, o2, o2p, Sf.as<float>());
+        T.S.p(), v * v * o, o, op, Sf.as<float>());
     SCESS_CHECK_LAUNCH();
   }
   // (i, j) pairs spread evenly over at most 256 threads
@@ -1511,7 +1522,7 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
             ps.cy[2] = nb * nb * o3p; ps.cz[2] = nb * o3p;
           }
           const int kRoles[3][3] = {{0, 1, 2}, {1, 0, 2}, {2, 0, 1}};  // (x, y, z) of group g
-          const int64_t rp = o * nb * nb, rq = o2 * nb;                 // block strides of the packs
+          const int64_t rp = o * nb * nb, rq = o2p * nb;                // block strides of the packs
           TcSegment &s0 = ps.seg[0], &s1 = ps.seg[1], &s2 = ps.seg[2], &s3 = ps.seg[3];
           s0.mapA = 0; s0.mapB = 1; s0.Kpad = pP.Kpad;   // P(u,f,x,y) Q(f,s,t,z)
           s1.mapA = 0; s1.mapB = 2; s1.Kpad = pP.Kpad;   // P(u,f,x,z) Q(f,t,s,y)
@@ -1522,13 +1533,13 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
             const int64_t X = U[kRoles[g][0]], Yb = U[kRoles[g][1]], Z = U[kRoles[g][2]];
             ps.cg[g] = nw == 3 ? g * nb * nb * nb * o3p : 0;
             s0.rowA0[g] = rp * (Yb + NB * X); s0.rowAy[g] = o * nb;
-            s0.rowB0[g] = rq * Z;             s0.rowBz[g] = o2;
+            s0.rowB0[g] = rq * Z;             s0.rowBz[g] = o2p;
             s1.rowA0[g] = rp * (Z + NB * X);  s1.rowAz[g] = o * nb;
-            s1.rowB0[g] = rq * Yb;            s1.rowBy[g] = o2;
+            s1.rowB0[g] = rq * Yb;            s1.rowBy[g] = o2p;
             s2.rowA0[g] = rp * (X + NB * Z);  s2.rowAz[g] = o * nb;
-            s2.rowB0[g] = rq * Yb;            s2.rowBy[g] = o2;
+            s2.rowB0[g] = rq * Yb;            s2.rowBy[g] = o2p;
             s3.rowA0[g] = rp * (X + NB * Yb); s3.rowAy[g] = o * nb;
-            s3.rowB0[g] = rq * Z;             s3.rowBz[g] = o2;
+            s3.rowB0[g] = rq * Z;             s3.rowBz[g] = o2p;
           }
           TcOut out;
           out.C = W.as<float>();
@@ -1538,10 +1549,8 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
           for (int g = 0; g < 3; g++) {
             ps.rowC[g] = gdt.ptr[2 * g];
             ps.colC[g] = gdt.ptr[2 * g + 1];
-            ps.store_by_column[g] = g > 0;  // i is a column index of groups 1 and 2
-            // columns (i, t) with i fastest: quads of i are contiguous and, with
-            // o % 4 == 0 (o2p, o3p too), 16-byte aligned
-            ps.store_quads[g] = g > 0 && o % 4 == 0;
+            // i is a column index of groups 1 and 2: quads of it, aligned
+            ps.store_quads[g] = g > 0;
           }
           out.alpha = 1.0;
           out.beta = nw == 1 ? 1.0 : 0.0;  // nw = 1: W += each group's product (L2 reductions)
@@ -1554,7 +1563,7 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
           ps.tri[2] = A == Bk;
           double nprob = 0.0;
           for (int g = 0; g < 3; g++) nprob += ps.tri[g] ? nb * (nb + 1) / 2.0 : (double)nb * nb;
-          const double flops = nprob * 2.0 * (double)Mg * Ng * (2.0 * v + 2.0 * o);
+          const double flops = nprob * 2.0 * (double)Mg * o2 * (2.0 * v + 2.0 * o);
           // behind the previous block triple's energy kernel, the launch starts
           // its MMAs while that kernel finishes (W is stored to only after it)
           ps.pdl = pdl && blocks_done > 0;
