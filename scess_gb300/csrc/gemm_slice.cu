@@ -4,23 +4,24 @@
 // bn <= 128:
 //   warp 0     TMA producer: per 32-wide K block one stage with the 7 slices of
 //              128 A rows and bn B rows (64-byte rows, 64B swizzle);
-//   warp 1     owns TMEM (three rotating accumulators of bn columns for S_4 .. S_0,
-//              one for S_5 + S_6) and issues the MMAs (M = 128, N = bn, K = 16);
+//   warp 1     owns TMEM (two rotating accumulators of bn columns for S_4 .. S_0,
+//              one for S_5, one for S_6 + S_7) and issues the MMAs (M = 128, N = bn, K = 16);
 //   warps 4-19 four epilogue warpgroups, bn / 4 columns each: add every drained
 //              S_d, an exact integer, into one 64-bit integer per output, and turn
 //              integer + FP32 tail into FP64 at the end of the unit.
 // The wide tile (an MMA of N = 128 takes 64 cycles, one of N = 80 still 52) leaves TMEM
 // room for four accumulators only, hence the rotation and five drains per K block, which
-// run beside the MMAs.  They bound it: 56 MMAs take 3600 cycles of a K block's 5750, the
-// drains' arithmetic (about four cycles of a scheduler per column, warp and drain) and their waits and
-// releases the rest.  What got it there, TFLOP/s at 4096^3 (68.7 at the tensor pipe's
-// measured rate): two epilogue warps a scheduler 38.8, four 41.8 (they hide each other's
-// waits); MMAs issued from uniform registers (see elect_one) 51.6; S_5 between S_2 and
-// S_1, and accumulators released before their arithmetic, 52.3.  Six accumulators of 80
-// columns with a third of the drains: 34 when issue bound it.
-// Joint form (tiles of at most 80 columns): TMEM holds an accumulator for every S_d, in two
+// run beside the MMAs.  Both bound it: 68 MMAs take 4350 cycles of a K block's 6050, the
+// drains' arithmetic (about four cycles of a scheduler per column, warp and drain) with
+// their waits and releases as long.  What got it there, TFLOP/s at 4096^3: with 28 products
+// and S_5 + S_6 in one accumulator two epilogue warps a scheduler 38.8, four 41.8 (they hide
+// each other's waits); MMAs issued from uniform registers (see elect_one) 51.6; S_5 between
+// S_2 and S_1, and accumulators released before their arithmetic, 52.3.  With 34 products
+// and S_5 apart 45.0 with the tail in two places among the diagonals, 50.1 in three (56.6 at
+// the tensor pipe's measured rate).
+// Joint form (tiles of at most 64 columns): TMEM holds an accumulator for every S_d, in two
 // sets up to 32 columns, and the five are drained together, with one wait and one release a
-// block; three stages where they fit.  313600 x 16 x 140: 315 us -> 144, where the
+// block; three stages where they fit.  313600 x 16 x 140: 315 us -> 150, where the
 // packs' 14 bytes an element read at 4.9 TB/s bound it; 200000 x 16 x 16: 71 -> 43.
 // Every mbarrier wait is bounded (see mbarrier.cuh).
 #include <cuda.h>
@@ -46,13 +47,14 @@ constexpr int STAGES = 2, MAX_STAGES = 3;                             // (narrow
 constexpr uint32_t A_SLICE = (uint32_t)BM * BK * 2;                  // one slice of 128 rows
 constexpr uint32_t STAGE_BYTES = kSlices * (BM + BN) * BK * 2;       // 112 KiB
 constexpr int NDIAG = 5;                                             // S_0 .. S_4 are drained
-constexpr int NROT = 3, TAIL = NROT, NACC = NROT + 1;                // accumulators
+constexpr int NROT = 2, TAIL = NROT, NACC = NROT + 2;                // accumulators: S_5 at TAIL, then S_6 + S_7
+constexpr int kS5Before = 3, kS6Before = 2, kS7Before = 0;           // places in S_4 .. S_0
 constexpr int EPI = 4;                                               // epilogue warpgroups
 constexpr int HC = BN / EPI;                                         // columns of an epilogue thread
-constexpr int BN_JOINT = 80, HC_JOINT = 24;                          // the same of the joint form
+constexpr int BN_JOINT = 64, HC_JOINT = 16;                          // the same of the joint form
 constexpr int THREADS = 128 * (1 + EPI);
 constexpr int kEpiRegs = 104, kCtlRegs = 56, kLaunchRegs = 96;       // 56 + 4 x 104 <= 5 x 96
-static_assert(kSlices == NDIAG + 2, "the tail is S_5 + S_6");
+static_assert(kSlices == NDIAG + 2, "the tail is S_5 .. S_7");
 static_assert(kCtlRegs + EPI * kEpiRegs <= (1 + EPI) * kLaunchRegs, "setmaxnreg draws on the launch's registers");
 struct Ctl {  // behind the stages
   uint64_t full[MAX_STAGES], empty[MAX_STAGES], tfull[NACC], tempty[NACC], done;
@@ -74,7 +76,7 @@ struct SliceMaps {
 };
 struct SliceArgs {
   int M, N, tiles_m, tiles_n;
-  int bn;      // tile width: a multiple of 16, at most 128 (joint form: 80)
+  int bn;      // tile width: a multiple of 16, at most 128 (joint form: 64)
   int stages;  // joint form
   int fs;      // fraction bits kept of the tail (see slice_value)
   int ny, nz, ng, nseg;
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   const uint32_t bslice = (uint32_t)bn * BK * 2;
   const uint32_t stage_bytes = JOINT ? kSlices * (A_SLICE + bslice) : STAGE_BYTES;
   const int nst = JOINT ? a.stages : STAGES;
-  const int nset = JOINT && 11 * bn <= 512 ? 2 : 1;                    // sets of S_0 .. S_4
+  const int nset = JOINT && 12 * bn <= 512 ? 2 : 1;                    // sets of S_0 .. S_4
   const uint32_t tail_col = (uint32_t)((JOINT ? nset * NDIAG : TAIL) * bn);
 
   if (threadIdx.x == 0) {
@@ -291,11 +293,15 @@ __global__ void __launch_bounds__(THREADS, 1)
           for (int k = 0; k < 2; k++)
             mma_f16kind(tmem + col, da + p * (A_SLICE >> 4) + 2 * k, db + q * bq + 2 * k, hi, idesc, k ? 1u : acc);
         };
+        // S_5 into one accumulator, where it stays exact as long as it is below 2^24 of its
+        // units, S_6 and S_7 into another
         auto tail = [&](auto diag, uint32_t acc) {
           constexpr int d = decltype(diag)::value;
 #pragma unroll
-          for (int p = 0; p <= d; p++, acc = 1u) product(tail_col, p, d - p, acc);
+          for (int p = d < kSlices ? 0 : d - kSlices + 1; p <= d && p < kSlices; p++, acc = 1u)
+            product(tail_col + (uint32_t)(d == NDIAG ? 0 : bn), p, d - p, acc);
         };
+        const uint32_t cont = kb == kb0 ? 0u : 1u;
         auto tail_free = [&]() {
           if (!wait(&ctl.tempty[TAIL], ((uint32_t)w & 1u) ^ 1u, ERR_EMPTY_WAIT)) return false;
           tc_fence_after();
@@ -316,19 +322,22 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
           if (kb == kb0 && !tail_free()) { ok = false; break; }
           if (issuer) {
-            tail(std::integral_constant<int, NDIAG>{}, kb == kb0 ? 0u : 1u);
-            tail(std::integral_constant<int, NDIAG + 1>{}, 1u);
+            tail(std::integral_constant<int, NDIAG>{}, cont);
+            tail(std::integral_constant<int, NDIAG + 1>{}, cont);
+            tail(std::integral_constant<int, NDIAG + 2>{}, 1u);
             mma_commit(&ctl.empty[s]);
           }
         } else {
-          // The longest diagonals first and S_5 between S_2 and S_1: a drain is then done
-          // when its accumulator comes round.
+          // The longest diagonals first, S_5 .. S_7 between them: a drain is then done when its
+          // accumulator comes round.
 #pragma unroll
           for (int d = NDIAG - 1; d >= 0; d--) {
-            if (d == 1) {
+            if (d == kS5Before) {
               if (kb == kb0 && !tail_free()) { ok = false; break; }
-              if (issuer) tail(std::integral_constant<int, NDIAG>{}, kb == kb0 ? 0u : 1u);
+              if (issuer) tail(std::integral_constant<int, NDIAG>{}, cont);
             }
+            if (d == kS6Before && issuer) tail(std::integral_constant<int, NDIAG + 1>{}, cont);
+            if (d == kS7Before && issuer) tail(std::integral_constant<int, NDIAG + 2>{}, 1u);
             const int b = c % NROT;
             if (ok && !wait(&ctl.tempty[b], (((uint32_t)(c / NROT)) & 1u) ^ 1u, ERR_EMPTY_WAIT)) ok = false;
             if (!ok) break;
@@ -341,10 +350,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             c++;
           }
           if (!ok) break;
-          if (issuer) {
-            tail(std::integral_constant<int, NDIAG + 1>{}, 1u);
-            mma_commit(&ctl.empty[s]);
-          }
+          if (issuer) mma_commit(&ctl.empty[s]);
         }
       }
       if (ok && issuer) mma_commit(&ctl.tfull[TAIL]);
@@ -470,8 +476,9 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
         for (int j = 0; j < HCT; j += 8) {
           if (j >= hc) continue;
-          uint32_t r[8];
+          uint32_t r[8], r6[8];
           tmem_ld8(tl + tail_col + (uint32_t)j, r);
+          tmem_ld8(tl + tail_col + (uint32_t)(bn + j), r6);
           int e[8];
           long long co[8];
           *reinterpret_cast<int4 *>(e) = *reinterpret_cast<const int4 *>(&ctl.colE[h0 + j]);
@@ -480,9 +487,10 @@ __global__ void __launch_bounds__(THREADS, 1)
           for (int i = 0; i < 8; i += 2)
             *reinterpret_cast<longlong2 *>(co + i) = *reinterpret_cast<const longlong2 *>(&ctl.colOff[h0 + j + i]);
           tmem_wait8(r);
+          tmem_wait8(r6);
 #pragma unroll
           for (int i = 0; i < 8; i++) {
-            const int w = rint_i32(__uint_as_float(r[i]) * ftail);
+            const int w = rint_i32(__uint_as_float(r[i]) * ftail) + rint_i32(__uint_as_float(r6[i]) * ftail);
             double *p = base + co[i];
             if (PLAIN) {
               const double v = slice_value_plain(T[j + i], w, a.fs, sc0 + e[i], flip);
@@ -763,11 +771,11 @@ SliceEngine::SliceEngine(Ctx &ctx) : ctx_(ctx) {
 }
 
 namespace {
-// The joint form's tiles are at most 80 wide.
+// The joint form's tiles are at most 64 wide.
 bool joint(int bn) { return bn <= BN_JOINT; }
 // Cycles an SM spends on one K block of a unit, measured (152 tiles of 128 rows, K = 1024:
 // widths 16 .. 128; 4096^3 for the scale).
-double block_cycles(int bn) { return joint(bn) ? 2950.0 + 25.0 * bn : 3150.0 + 20.0 * bn; }
+double block_cycles(int bn) { return joint(bn) ? 3050.0 + 22.0 * bn : 3450.0 + 20.0 * bn; }
 }  // namespace
 
 // The narrow tile where it is cheaper.
@@ -974,7 +982,7 @@ void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial)
   a.kb_per_split = (int)ceil_div(a.kb_total, splits);
   a.splits = (int)ceil_div(a.kb_total, a.kb_per_split);
   // the 64-bit sum holds 2^12 k 2^36 per output: K <= 2^14 a unit
-  // and the tail, below 2^10 K in units of the integer, in 31 bits
+  // and the tails, together below 2^10 K in units of the integer, in 31 bits
   a.fs = 20;
   for (int64_t k = (int64_t)a.kb_per_split * BK; k > 1; k >>= 1) a.fs--;
   if (a.kb_per_split > 512) throw Error(SCESS_ERR_INVALID, "slice gemm: K of a unit");
