@@ -41,22 +41,34 @@ CurrentCtx::~CurrentCtx() { t_ctx = prev; }
 void *BlockCache::take(size_t bytes) {
   auto it = free_.find(bytes);
   if (it == free_.end()) return nullptr;
-  void *p = it->second;
+  void *p = it->second.p;
+  age_.erase(it->second.stamp);
   free_.erase(it);
   total_ -= bytes;
   return p;
 }
 
-bool BlockCache::give(void *p, size_t bytes) {
-  if (bytes < kMinBytes || total_ + bytes > kMaxCached) return false;
-  free_.emplace(bytes, p);
+bool BlockCache::give(void *p, size_t bytes, size_t &evicted) {
+  evicted = 0;
+  if (bytes < kMinBytes || bytes > kMaxCached) return false;
+  while (total_ + bytes > kMaxCached) {
+    auto old = age_.begin()->second;
+    evicted += old->first;
+    total_ -= old->first;
+    cudaFree(old->second.p);
+    age_.erase(age_.begin());
+    free_.erase(old);
+  }
+  age_[clock_] = free_.emplace(bytes, Block{p, clock_});
+  clock_++;
   total_ += bytes;
   return true;
 }
 
 size_t BlockCache::flush() {
-  for (auto &kv : free_) cudaFree(kv.second);
+  for (auto &kv : free_) cudaFree(kv.second.p);
   free_.clear();
+  age_.clear();
   const size_t t = total_;
   total_ = 0;
   return t;
@@ -125,10 +137,12 @@ void DevMem::release() {
   if (p_) {
     Ctx *c = current_ctx();
     if (c && owner_ == c) {
-      if (!c->blocks.give(p_, bytes_)) {
+      size_t evicted = 0;
+      if (!c->blocks.give(p_, bytes_, evicted)) {
         cudaFree(p_);
-        c->mem_held -= std::min(bytes_, c->mem_held);
+        evicted = bytes_;
       }
+      c->mem_held -= std::min(evicted, c->mem_held);
     } else {
       cudaFree(p_);
     }
