@@ -94,7 +94,6 @@ struct SliceArgs {
   int64_t part_stride;
   unsigned *err;
   long long wait_cycles;
-  int withhold_first;
 };
 
 // T += i 2^(9 (4 - D)) for the drained S_D = i 2^(-9 D) of one K block: |i| is at most
@@ -223,7 +222,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kCtlRegs));
   if (warp == 0) {
     if (lane == 0) {
-      int g = 0, s = 0;
+      int s = 0;
       uint32_t ph = 0;          // stage and its phase
       int used = 0;             // stages filled at least once
       uint32_t lastph = 0;      // phases of their last fills, a bit each
@@ -231,7 +230,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
         int tm, tn, py, pz, pg, kb0, kb1, sp;
         unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
-        for (int kb = kb0; kb < kb1; kb++, g++) {
+        for (int kb = kb0; kb < kb1; kb++) {
           if (s == nst) {
             s = 0;
             ph ^= 1u;
@@ -242,11 +241,6 @@ __global__ void __launch_bounds__(THREADS, 1)
           const int ya = (int)(S.rowA0[pg] + py * S.rowAy[pg] + pz * S.rowAz[pg]) + tm * BM;
           const int yb = (int)(S.rowB0[pg] + py * S.rowBy[pg] + pz * S.rowBz[pg]) + tn * bn;
           if (!mbar_wait(&ctl.empty[s], ph ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) { ok = false; break; }
-          // diagnostics: the first stage is taken but never filled (see scess_ctx_arm_wait_expiry)
-          if (a.withhold_first && g == 0) {
-            s++;
-            continue;
-          }
           uint8_t *st = smem + s * stage_bytes;
           mbar_expect_tx(&ctl.full[s], kSlices * (A_SLICE + bslice));
 #pragma unroll
@@ -1016,10 +1010,7 @@ void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial)
   a.part_stride = ps.M * ps.N;
   if (a.splits > 1 && (!partial || start > 1)) throw Error(SCESS_ERR_INVALID, "slice gemm: split-K");
   a.err = err_.as<unsigned>();
-  a.wait_cycles = wait_cycles_;
-  a.withhold_first = withhold_ ? 1 : 0;
-  wait_cycles_ = 1ll << 32;  // (diagnostics are for one launch)
-  withhold_ = false;
+  a.wait_cycles = 1ll << 32;
   SliceMaps maps;
   for (int i = 0; i < 6; i++) maps.m[i] = ps.maps[std::min(i, ps.nmaps - 1)];
   const int64_t units = (int64_t)a.tiles_m * a.tiles_n * start * a.splits;

@@ -121,10 +121,6 @@ class SliceEngine {
   // Throws SCESS_ERR_CUDA if a bounded wait of a launch since the last check expired.
   void check_error();
   bool launched() const { return launched_; }
-  void arm_wait_expiry(long long wait_cycles) {
-    wait_cycles_ = wait_cycles;
-    withhold_ = true;
-  }
 
  private:
   struct Gather {  // an operand seen through its tables
@@ -161,8 +157,6 @@ class SliceEngine {
   SlicedPack tmpA_, tmpB_;
   DevMem err_, partial_;
   bool launched_ = false, busy_ = false;
-  long long wait_cycles_ = 1ll << 32;
-  bool withhold_ = false;
 };
 
 // Outputs of g whose A row or B column is marked in expA / expB (kRowNonFinite).

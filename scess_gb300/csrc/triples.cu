@@ -12,11 +12,12 @@
 // Y = W + V, r3(Y), the denominators and the degeneracy (:135-157) and writes
 // one partial energy per triple; a fixed-order reduction gives 2 * sum (:167).
 //
-// FP64 form: DFMA GEMMs straight from the padded FP64 repacks, FP64 W and
-// FP64 energy arithmetic.  MIXED form: the same 12 products regroup into three
-// sets of four K segments (one grouped tcgen05 launch per block triple) whose
-// epilogues add them into one FP32 W with L2 reductions, so that W (nb^3 o^3
-// floats, 55 MB at o = 20) stays in L2 between the launch and the energy
+// Both forms regroup the 12 products into three sets of four K segments, one grouped
+// launch per block triple.  FP64 form: the slice GEMM (gemm_slice.h) writes three FP64
+// buffers, kept within L2, that the energy kernel adds (12 DFMA GEMMs into one W where
+// the sliced packs don't fit the device); FP64 energy arithmetic.  MIXED form: the
+// epilogues of the tcgen05 GEMM add the groups into one FP32 W with L2 reductions, so
+// that W (nb^3 o^3 floats, 55 MB at o = 20) stays in L2 between the launch and the energy
 // kernel; the operands are packed once per call into FP16 hi/lo rows grouped
 // by block.  The energy kernel reads W once, clears it for the next block
 // triple and works in FP32 per element with denominators formed from the FP64
