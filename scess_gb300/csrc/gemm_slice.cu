@@ -809,8 +809,8 @@ double plan_us(int64_t M, int64_t N, int64_t Kpad, int64_t &splits) {
 
 double SliceEngine::estimate_us(int64_t M, int64_t N, int64_t K) {
   int64_t z = 1;
-  // packs at 2.5 TB/s, 14 us of launches and latencies
-  return 14.0 + (double)(M + N) * (double)K * 22.0 / 2.5e6 + plan_us(M, N, round_up(std::max<int64_t>(K, 1), BK), z);
+  // packs at 2.9 TB/s, 14 us of launches and latencies
+  return 14.0 + (double)(M + N) * (double)K * 22.0 / 2.9e6 + plan_us(M, N, round_up(std::max<int64_t>(K, 1), BK), z);
 }
 
 bool SliceEngine::usable(int64_t M, int64_t N) {
