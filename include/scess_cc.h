@@ -257,8 +257,7 @@ int scess_rccsd_residual_vjp_df(scess_ctx *ctx, const double *B, int64_t naux, i
  * g_e dE_T/deri (nmo^4, eri layout; nonzero only on the (ov|vv), (oo|vo) and
  * (ov|ov) blocks E_T reads).  e_t (may be NULL) receives E_T.  The forward
  * W is recomputed block by block, so the memory use is that of the FP64 (T).
- * precision: SCESS_PRECISION_FP64 (FP64 accuracy: exact BF16 slices on the
- * tensor cores, small products on the FP64 units), or MIXED (the forward
+ * precision: SCESS_PRECISION_FP64 (see scess_einsum), or MIXED (the forward
  * and transposed GEMMs on the tensor cores: split operands, FP32
  * accumulation; the element-wise gradient of the energy stays FP64). */
 int scess_rccsd_triples_vjp(scess_ctx *ctx, const double *eri, const double *eps, int64_t nmo,
@@ -296,8 +295,13 @@ int scess_rccsd_rdm1(scess_ctx *ctx, const double *eri, const double *eps, int64
  * (src/Tensor/TensorEinsum.h:170-205): spec like "kcld,ilcd->ki", each
  * operand a dense column-major host tensor of rank <= 6 with extents *_ext.
  * Every label of C appears in exactly one of A, B; labels shared by A and B
- * and absent from C are summed.  precision selects the FP64 backend (exact
- * BF16 slices on the tensor cores, small products on the FP64 units) or, for MIXED, the tcgen05 tensor-core backend for any shape. */
+ * and absent from C are summed.  precision selects the FP64 backend or, for
+ * MIXED, the tcgen05 tensor-core backend for any shape.  FP64: small products run on the FP64
+ * units, the others on the tensor cores, operands cut into BF16 slices (60 bits below a
+ * row's largest value) and added exactly; outputs that those bits cannot hold (sum |a b| below
+ * about 2^-7 (row norm^2 + column norm^2)^(1/2) of |row max| |column max|) and those of Inf or NaN
+ * run on the FP64 units.  Either way an output's error is that of FP64 multiply-adds, a few
+ * 2^-53 sum |a b|. */
 int scess_einsum(scess_ctx *ctx, const char *spec, double alpha, const double *A, int32_t a_nd,
                  const int64_t *a_ext, const double *B, int32_t b_nd, const int64_t *b_ext,
                  double beta, double *C, int32_t c_nd, const int64_t *c_ext, int32_t precision);
@@ -310,8 +314,7 @@ int scess_einsum(scess_ctx *ctx, const char *spec, double alpha, const double *A
  * at a time (lam, kap, nu, mu) as the reference does; with chem_to_phys the
  * result is reordered pqrs -> prqs (out is then na x nc x nb x nd), which with
  * A = B = C = D is the physicists' eri of scess_rccsd_solve (RCCSD.cpp:399).
- * precision: FP64 (exact BF16 slices on the tensor cores), or MIXED (tensor cores,
- * split operands). */
+ * precision: FP64 (see scess_einsum), or MIXED (tensor cores, split operands). */
 int scess_transform_tei(scess_ctx *ctx, const double *tei, int64_t nao, const double *A,
                         int64_t na, const double *B, int64_t nb, const double *C, int64_t nc,
                         const double *D, int64_t nd, int32_t chem_to_phys, int32_t precision,

@@ -8,15 +8,20 @@ namespace scess {
 
 constexpr int kDgemmTile = 64, kDgemmBK = 16;
 
+struct DgemmShared {
+  double As[kDgemmBK][kDgemmTile], Bs[kDgemmBK][kDgemmTile];
+  int64_t sRowA[kDgemmTile], sColB[kDgemmTile], sKA[kDgemmBK], sKB[kDgemmBK];
+};
+
 // sum_(kb <= k < ke) A(m, k) B(k, n) of the tile at (m0, n0), each result handed
 // to store(m, n, sum).
 template <class Store>
-__device__ __forceinline__ void dgemm_tile(const TableGemm &g, int64_t m0, int64_t n0, int64_t kb,
+__device__ __forceinline__ void dgemm_tile(DgemmShared &sh, const TableGemm &g, int64_t m0, int64_t n0, int64_t kb,
                                            int64_t ke, Store store) {
   constexpr int BM = kDgemmTile, BN = kDgemmTile, BK = kDgemmBK;
-  __shared__ double As[BK][BM];
-  __shared__ double Bs[BK][BN];
-  __shared__ int64_t sRowA[BM], sColB[BN], sKA[BK], sKB[BK];
+  auto &As = sh.As, &Bs = sh.Bs;
+  auto &sRowA = sh.sRowA, &sColB = sh.sColB;
+  auto &sKA = sh.sKA, &sKB = sh.sKB;
   const int t = threadIdx.x;
   if (t < BM) {
     const int64_t m = m0 + t;

@@ -575,8 +575,8 @@ namespace {
 // tuning key f64: 1 = sliced, 2 = FP64 units).
 bool prefer_slices(const TableGemm &g) {
   const int64_t route = tune_value("f64", 0);
-  if (route == 1) return g.K > 0 && SliceEngine::usable(g.M, g.N);
-  return route != 2 && g.K > 0 && SliceEngine::usable(g.M, g.N) && 
+  if (route == 1) return g.K > 0 && SliceEngine::usable(g.M, g.N, g.K);
+  return route != 2 && g.K > 0 && SliceEngine::usable(g.M, g.N, g.K) &&
          SliceEngine::estimate_us(g.M, g.N, g.K) < std::min(dgemm_small_us(g), skinny64_us(g));
 }
 

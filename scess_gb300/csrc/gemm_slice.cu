@@ -22,11 +22,18 @@
 // Joint form (tiles of at most 64 columns): TMEM holds an accumulator for every S_d, in two
 // sets up to 32 columns, and the five are drained together, with one wait and one release a
 // block; three stages where they fit.  313600 x 16 x 140: 315 us -> 150, where the
-// packs' 14 bytes an element read at 4.9 TB/s bound it; 200000 x 16 x 16: 71 -> 43.
+// packs' 16 bytes an element read at 4.9 TB/s bound it; 200000 x 16 x 16: 71 -> 43.
+// A unit of a product that stands alone begins with the product of the magnitudes: seven K blocks
+// of that plane fill the places of a stage's seven digit slices, and what is added up in the
+// next free accumulator tells which outputs are left to the FP64 units (slice_left).  A warp takes
+// its 32 x 32 outputs at once where their least sum reaches their largest threshold.  Cost, of
+// which a third is the packs': FP64 iterations at o = 10, v = 90 6.9 -> 7.4 ms, at o = 16,
+// v = 140 38.1 -> 40.4, a residual gradient at o = 8, v = 47 5.28 -> 5.54.
 // Every mbarrier wait is bounded (see mbarrier.cuh).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <cmath>
 #include <cstring>
 #include <mutex>
 
@@ -56,6 +63,14 @@ constexpr int THREADS = 128 * (1 + EPI);
 constexpr int kEpiRegs = 104, kCtlRegs = 56, kLaunchRegs = 96;       // 56 + 4 x 104 <= 5 x 96
 static_assert(kSlices == NDIAG + 2, "the tail is S_5 .. S_7");
 static_assert(kCtlRegs + EPI * kEpiRegs <= (1 + EPI) * kLaunchRegs, "setmaxnreg draws on the launch's registers");
+// First column of epilogue group h (0 .. EPI) of a tile of bn columns: a quarter each, in groups of
+// eight; and the group of a column.
+__host__ __device__ constexpr int group_start(int bn, int h) { return 8 * ((bn / 8 * h + 3) / 4); }
+__device__ __forceinline__ int column_group(int bn, int col) {
+  int h = 0;
+  while (h < EPI - 1 && col >= group_start(bn, h + 1)) h++;
+  return h;
+}
 struct Ctl {  // behind the stages
   uint64_t full[MAX_STAGES], empty[MAX_STAGES], tfull[NACC], tempty[NACC], done;
   uint32_t tmem;
@@ -85,6 +100,16 @@ struct SliceArgs {
   int tri[3], gstart[4];
   const int *expA, *expB;
   int64_t expA0[3];
+  // est: sum_k |a_k b_k| first, to find the outputs that are left to the FP64 units (see
+  // slice_left).  Per tile 16 flags (32 rows x a column group each); where one is set, bit
+  // column - group_start of left[tile][column group][row] marks an output.  Split-K: the sums
+  // go to est_partial [split][n][m], and the reduction sets the marks.
+  int est;
+  int rowsA, rowsB;  // of the statistics behind expA, expB (see SlicedPack)
+  float sq_unit;
+  uint32_t *left;
+  uint8_t *flags;
+  float *est_partial;
   double *C;
   int64_t baseC, cy[3], cz[3], cg[3];
   const int64_t *rowC[3], *colC[3];
@@ -139,6 +164,25 @@ __device__ __forceinline__ void tmem_wait8(uint32_t *r) {
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
                :
                : "memory");
+}
+
+// Which outputs the slices cannot hold as well as FP64 multiply-adds would.  A value is rounded at
+// 2^-61 of its row's largest, so that an output's error is, in rms, 2^-61 |row max| |column max|
+// (q / 3)^(1/2) with q = sum (a_k / row max)^2 + (b_k / column max)^2 over the k that both
+// sides have (and 2^-13 each for the digit products that are dropped); a chain of
+// multiply-adds has about 0.4 2^-53 sum_k |a_k b_k|.  So that sum has to reach 1.44 2^-8 q^(1/2)
+// of |row max| |column max|; 2^-7 is asked for.  Exact zeros are exact here too.
+struct RangeRow {
+  float sq, count;  // sum of (value / largest)^2, values that are not zero; negative sq: Inf or NaN
+};
+__device__ __forceinline__ RangeRow range_row(const int *exps, int rows, int64_t r, float sq_unit) {
+  if (r >= rows) return {0.0f, 0.0f};
+  return {exps[r] == kRowNonFinite ? -1.0f : (float)exps[rows + r] * sq_unit, (float)exps[2 * (int64_t)rows + r]};
+}
+__device__ __forceinline__ bool slice_left(float sum, RangeRow a, RangeRow b) {
+  if (a.sq < 0.0f || b.sq < 0.0f) return true;
+  const float q = fminf(a.sq, b.count) + fminf(b.sq, a.count) + 0x1p-13f * fminf(a.count, b.count);
+  return sum != 0.0f && sum * sum < 0x1p-14f * q;
 }
 
 // What bounds it: long K, the drains (above); short K, the outputs (about 45 instructions each).
@@ -230,7 +274,26 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
         int tm, tn, py, pz, pg, kb0, kb1, sp;
         unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
-        for (int kb = kb0; kb < kb1; kb++) {
+        // magnitudes: the places of the digits' seven slices take seven K blocks
+        for (int kb = kb0; a.est && kb < kb1; kb += kSlices) {
+          if (s == nst) {
+            s = 0;
+            ph ^= 1u;
+          }
+          const SegArgs &S = a.seg[0];
+          const int n = min(kSlices, kb1 - kb), x = kSlices * S.kpad + kb * BK;
+          if (!mbar_wait(&ctl.empty[s], ph ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) { ok = false; break; }
+          uint8_t *st = smem + s * stage_bytes;
+          mbar_expect_tx(&ctl.full[s], n * (A_SLICE + bslice));
+          for (int p = 0; p < n; p++) {
+            tma_load_2d(st + p * A_SLICE, &maps.m[S.mapA], x + p * BK, tm * BM, &ctl.full[s]);
+            tma_load_2d(st + kSlices * A_SLICE + p * bslice, &maps.m[S.mapB], x + p * BK, tn * bn, &ctl.full[s]);
+          }
+          used |= 1 << s;
+          lastph = (lastph & ~(1u << s)) | (ph << s);
+          s++;
+        }
+        for (int kb = kb0; kb < kb1 && ok; kb++) {
           if (s == nst) {
             s = 0;
             ph ^= 1u;
@@ -273,6 +336,32 @@ __global__ void __launch_bounds__(THREADS, 1)
       int tm, tn, py, pz, pg, kb0, kb1, sp;
       unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
       const uint32_t idesc = idesc_f16kind(BM, min(bn, (a.N - tn * bn + 15) & ~15), 1u);  // BF16
+      if (a.est) {  // magnitudes into the next accumulator (joint form: the first of a set)
+        const int b = JOINT ? (nset == 2 ? c & 1 : 0) : c % NROT;
+        const int f = JOINT ? (nset == 2 ? c >> 1 : c) : c / NROT;  // fills of it before
+        const uint32_t col = tmem + (uint32_t)(JOINT ? b * NDIAG * bn : b * bn);
+        ok = wait(&ctl.tempty[b], ((uint32_t)f & 1u) ^ 1u, ERR_EMPTY_WAIT);
+        for (int kb = kb0; kb < kb1 && ok; kb += kSlices, s++) {
+          if (s == nst) {
+            s = 0;
+            ph ^= 1u;
+          }
+          if (!wait(&ctl.full[s], ph, ERR_FULL_WAIT)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t da = lo + (uint32_t)s * (stage_bytes >> 4), db = da + (kSlices * A_SLICE >> 4);
+          if (issuer) {
+            const int n = min(kSlices, kb1 - kb);
+            for (int p = 0; p < n; p++)
+#pragma unroll
+              for (int k = 0; k < 2; k++)
+                mma_f16kind(col, da + p * (A_SLICE >> 4) + 2 * k, db + p * bq + 2 * k, hi, idesc, kb > kb0 || p || k ? 1u : 0u);
+            mma_commit(&ctl.empty[s]);
+          }
+        }
+        if (!ok) break;
+        if (issuer) mma_commit(&ctl.tfull[b]);
+        c++;
+      }
       for (int kb = kb0; kb < kb1 && ok; kb++, s++) {
         if (s == nst) {
           s = 0;
@@ -357,8 +446,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int q = warp & 3;
     const int row = 32 * q + lane;
     const int h = (warp - 4) >> 2;                  // column group
-    // its columns: a quarter of the tile's, in groups of eight
-    const int h0 = 8 * ((bn / 8 * h + 3) / 4), hc = 8 * ((bn / 8 * (h + 1) + 3) / 4) - h0;
+    const int h0 = group_start(bn, h), hc = group_start(bn, h + 1) - h0;  // its columns
     constexpr int HCT = JOINT ? HC_JOINT : HC;
     const int et = threadIdx.x - 128 - 128 * h;     // 0..127 within the group
     const int bar = 1 + h;
@@ -382,16 +470,67 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int eA = m < a.M ? a.expA[a.expA0[pg] + m] : kRowNonFinite;
       const int64_t rowOff = m < a.M ? (a.partial ? (int64_t)m : a.rowC[pg][m]) : 0;
       const unsigned errv = *(volatile unsigned *)a.err;
-      long long T[HCT];
-      const long long off = magic_sum(kb1 - kb0);
-#pragma unroll
-      for (int j = 0; j < HCT; j++) T[j] = -off;
       auto release = [&](int b) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0)
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&ctl.tempty[b])) : "memory");
       };
+      uint32_t left = 0;  // columns of this row left to the FP64 units
+      if (a.est) {
+        const int b = JOINT ? (nset == 2 ? c & 1 : 0) : c % NROT;
+        const int f = JOINT ? (nset == 2 ? c >> 1 : c) : c / NROT;
+        const int n0 = tn * bn + h0, nv = min(hc, a.N - n0);  // columns inside the product
+        const RangeRow ra = range_row(a.expA, a.rowsA, m, a.sq_unit);
+        const RangeRow rb = range_row(a.expB, lane < nv ? a.rowsB : 0, n0 + lane, a.sq_unit);  // lane's column
+        ok = mbar_wait(&ctl.tfull[b], (uint32_t)f & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles);
+        if (ok) {
+          c++;
+          tc_fence_after();
+          const uint32_t t0 = tl + (uint32_t)(JOINT ? b * NDIAG * bn : b * bn);
+          // all of a warp's outputs at once, by the largest threshold of theirs; else one by one
+          const RangeRow most = {__int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(fmaxf(rb.sq, 0.0f)))),
+                                 __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(rb.count)))};
+          float least = 3.0e38f;
+          float *p = a.est_partial + (int64_t)sp * a.part_stride + (int64_t)a.M * n0 + m;
+#pragma unroll
+          for (int j = 0; j < HCT; j += 8) {
+            if (j >= hc) continue;
+            uint32_t r[8];
+            tmem_ld8(t0 + (uint32_t)j, r);
+            tmem_wait8(r);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+              if (j + i >= nv) continue;
+              if (!a.partial) least = fminf(least, __uint_as_float(r[i]));
+              else if (m < a.M) p[(int64_t)a.M * (j + i)] = __uint_as_float(r[i]);
+            }
+          }
+          const bool sure = a.partial || m >= a.M || (rb.sq >= 0.0f && least != 0.0f && !slice_left(least, ra, most));
+          if (!__all_sync(0xffffffffu, sure)) {
+#pragma unroll 1
+            for (int j = 0; j < hc; j += 8) {
+              uint32_t r[8];
+              tmem_ld8(t0 + (uint32_t)j, r);
+              tmem_wait8(r);
+#pragma unroll
+              for (int i = 0; i < 8; i++) {
+                const RangeRow x = {__shfl_sync(0xffffffffu, rb.sq, j + i), __shfl_sync(0xffffffffu, rb.count, j + i)};
+                if (j + i < nv && m < a.M && slice_left(__uint_as_float(r[i]), ra, x)) left |= 1u << (j + i);
+              }
+            }
+          }
+          release(b);
+          const bool any = __any_sync(0xffffffffu, left != 0u);
+          // (split-K: cleared here, set by the reduction)
+          if (lane == 0 && sp == 0) a.flags[16 * (u % tiles) + 4 * h + q] = any;
+          if (any || (a.partial && sp == 0)) a.left[(int64_t)(u % tiles * EPI + h) * BM + row] = left;
+        }
+      }
+      long long T[HCT];
+      const long long off = magic_sum(kb1 - kb0);
+#pragma unroll
+      for (int j = 0; j < HCT; j++) T[j] = -off;
       auto take = [&](auto diag) -> bool {
         constexpr int D = decltype(diag)::value;
         const int b = c % NROT;
@@ -413,7 +552,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         c++;
         return true;
       };
-      for (int kb = kb0; kb < kb1; kb++) {
+      for (int kb = kb0; kb < kb1 && ok; kb++) {
         if constexpr (JOINT) {
           const int set = nset == 2 ? c & 1 : 0;
           ok = mbar_wait(&ctl.tfull[set], (uint32_t)(nset == 2 ? c >> 1 : c) & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles);
@@ -464,7 +603,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       auto fits = [](int e) { return e >= 640 && e <= 1400; };
       const bool rok = fits(eA == 0 ? 1023 : eA) && sc0 >= -1500 && sc0 <= -600;
       const bool cok = lane >= hc || (ctl.colOff[h0 + lane] >= 0 && fits(ctl.colE[h0 + lane]));
-      const bool plain = __all_sync(0xffffffffu, rok && cok) && !scaled && mode != 2;
+      const bool plain = __all_sync(0xffffffffu, rok && cok && !left) && !scaled && mode != 2;
       auto finish = [&](auto is_plain) {
         constexpr bool PLAIN = decltype(is_plain)::value;
 #pragma unroll
@@ -490,7 +629,7 @@ __global__ void __launch_bounds__(THREADS, 1)
               const double v = slice_value_plain(T[j + i], w, a.fs, sc0 + e[i], flip);
               if (mode == 0) *p = v;
               else asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
-            } else if (co[i] >= 0 && eA != kRowNonFinite) {
+            } else if (co[i] >= 0 && eA != kRowNonFinite && !(left >> (j + i) & 1u)) {
               double v = slice_value(T[j + i], w, a.fs, sc0 + e[i], flip);
               if (scaled) v *= mul;
               if (mode == 0) *p = v;
@@ -513,12 +652,29 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
 }
 
-// Split-K: C = alpha sum_z partial_z + beta C over unmarked outputs.
+struct PartialSum {
+  double sum = 0.0;
+  float est = 0.0f;
+  __device__ void operator+=(const PartialSum &o) {
+    sum += o.sum;
+    est += o.est;
+  }
+};
+// Split-K: C = alpha sum_z partial_z + beta C over the outputs that are not left.
 template <int ZG>
 __global__ void __launch_bounds__(256) slice_reduce_kernel(const __grid_constant__ SliceArgs a, int splits) {
   chain();
-  split_sum<ZG>(a.partial, a.M, a.N, splits, [&](int64_t m, int64_t n, double s) {
-    if (a.expA[m] == kRowNonFinite || a.expB[n] == kRowNonFinite) return;
+  const int64_t MN = (int64_t)a.M * a.N;
+  auto load = [&](int z, int64_t e) { return PartialSum{a.partial[z * MN + e], a.est_partial[z * MN + e]}; };
+  split_sum<ZG, PartialSum>(a.M, a.N, splits, load, [&](int64_t m, int64_t n, const PartialSum &x) {
+    const double s = x.sum;
+    if (slice_left(x.est, range_row(a.expA, a.rowsA, m, a.sq_unit), range_row(a.expB, a.rowsB, n, a.sq_unit))) {
+      const int tn = (int)n / a.bn, tile = (int)m / BM * a.tiles_n + tn, row = (int)m % BM, col = (int)n - tn * a.bn;
+      const int h = column_group(a.bn, col);
+      a.flags[16 * tile + 4 * h + (row >> 5)] = 1;
+      atomicOr(&a.left[(int64_t)(tile * EPI + h) * BM + row], 1u << (col - group_start(a.bn, h)));
+      return;
+    }
     double *p = a.C + a.baseC + a.rowC[0][m] + a.colC[0][n];
     double val = a.alpha * s;
     if (a.beta != 0.0) val += a.beta * *p;
@@ -535,7 +691,7 @@ __global__ void __launch_bounds__(256) slice_reduce_kernel(const __grid_constant
 // exponents first, the cut in a second launch.  EXPS: exponents only, folded into
 // exps[expIdx[row]] with atomics.  GIVEN: exponents exps[expIdx[row]], K spread over
 // CTAs.
-// HBM-bound with long rows (8 B read and 14 B written per element, 3.2 TB/s at
+// HBM-bound with long rows (8 B read and 16 B written per element, 3.2 TB/s at
 // 4096 x 4096, 2.3 before the loads of the next chunk were in flight while one is cut).
 enum PackMode { PACK_OWN, PACK_PART, PACK_FROM_PART, PACK_EXPS, PACK_GIVEN };
 struct PackOp {
@@ -547,6 +703,8 @@ struct PackOp {
   int mode, unitK, negate, parts;
   uint16_t *dst;
   int *exps, *part;
+  int *stats;     // behind exps: sums of squares, counts (see SlicedPack)
+  float sq_unit;
   const int64_t *expIdx;
   int64_t blocks;  // rt.count times the K ranges
 };
@@ -626,7 +784,10 @@ __global__ void __launch_bounds__(256) slice_pack_kernel(const __grid_constant__
     __syncthreads();
     if (t < ROWS && srow[t] >= 0) {
       if (mode == PACK_EXPS) atomicMax(&op.exps[op.expIdx ? op.expIdx[srow[t]] : srow[t]], se[t]);
-      else if (mode == PACK_PART) op.part[c0 * op.rows + srow[t]] = se[t];
+      else if (mode == PACK_PART) {
+        op.part[c0 * op.rows + srow[t]] = se[t];
+        if (c0 == 0) op.stats[srow[t]] = op.stats[op.rows + srow[t]] = 0;  // (added up by the second launch)
+      }
       else op.exps[srow[t]] = se[t];
     }
     if (mode != PACK_OWN) return;
@@ -639,6 +800,8 @@ __global__ void __launch_bounds__(256) slice_pack_kernel(const __grid_constant__
     load();
   }
   const int rr = t / (KT / 8), ch = t % (KT / 8);
+  int count = 0;
+  float sq = 0.0f;
   for (int64_t c = c0; c < nchunk; c += cs) {
     const bool more = c + cs < nchunk;
     const int64_t nk = (t < KT && more) ? koff((c + cs) * KT + t) : -1;
@@ -654,10 +817,17 @@ __global__ void __launch_bounds__(256) slice_pack_kernel(const __grid_constant__
     const int64_t k0 = c * KT, r = srow[rr];
     if (r < 0 || k0 + ch * 8 >= Kpad) continue;
     const int e = se[rr];
-    uint32_t w[kSlices][4];
+    uint32_t w[kSlices + 1][4];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      int64_t F = e == kRowNonFinite ? 0 : slice_fixed(tile[rr][9 * ch + j], e);
+      const double xv = tile[rr][9 * ch + j];
+      int64_t F = e == kRowNonFinite ? 0 : slice_fixed(xv, e);
+      const float fx = (float)(int)(F >> 32);  // 2^28 x / 2^E
+      sq = fmaf(fx, fx, sq);
+      const uint32_t mag = slice_magnitude(xv, e);
+      count += mag != 0u;
+      if (j & 1) w[kSlices][j >> 1] |= mag << 16;
+      else w[kSlices][j >> 1] = mag;
       if (op.negate) F = -F;
       const int64_t G = F + kDigitBias;
 #pragma unroll
@@ -674,10 +844,27 @@ __global__ void __launch_bounds__(256) slice_pack_kernel(const __grid_constant__
         else w[p][j >> 1] = b;
       }
     }
-    uint16_t *d = op.dst + r * kSlices * Kpad + k0 + ch * 8;
+    uint16_t *d = op.dst + r * kPlanes * Kpad + k0 + ch * 8;
 #pragma unroll
-    for (int p = 0; p < kSlices; p++)
+    for (int p = 0; p < kPlanes; p++)
       *reinterpret_cast<uint4 *>(d + p * Kpad) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+  }
+  if (!op.stats) return;
+#pragma unroll
+  for (int off = KT / 16; off > 0; off >>= 1) {
+    count += __shfl_xor_sync(0xffffffffu, count, off);
+    sq += __shfl_xor_sync(0xffffffffu, sq, off);
+  }
+  if (ch == 0 && srow[rr] >= 0) {
+    int *u = op.stats + srow[rr], *n = u + op.rows;
+    const int squares = (int)ceilf(sq * 0x1p-56f / op.sq_unit);
+    if (cs == 1) {
+      *u = squares;
+      *n = count;
+    } else {
+      atomicAdd(u, squares);
+      atomicAdd(n, count);
+    }
   }
 }
 
@@ -697,25 +884,115 @@ void launch_packs(const PackOp *op, int n, cudaStream_t stream) {  // (the opera
   SCESS_CHECK_LAUNCH();
 }
 
-__global__ void __launch_bounds__(256) dgemm_masked_kernel(TableGemm g, const int *__restrict__ expA,
-                                                           const int *__restrict__ expB) {
+// The outputs that the slice GEMM has left (see SliceArgs::est), on the FP64 units: a thread looks
+// at a GEMM tile's 16 flags, and the CTA walks the 64 x 64 pieces of those that have any.  Items
+// are dealt out one by one; ks CTAs share a tile's K where there are few tiles, the last one
+// adds their ranges in order.  Returns at once where nothing was left.
+struct LeftArgs {
+  const uint32_t *left;
+  const uint8_t *flags;
+  int bn, tiles_m, tiles_n, ks;
+  int64_t kper;
+  double *partial;  // ks > 1: [tile][ks][4][64 x 64]
+  int *counters;    // of a tile; zero between launches
+};
+__global__ void __launch_bounds__(256) slice_left_kernel(TableGemm g, LeftArgs a) {
   chain();
-  const int64_t tm = (g.M + kDgemmTile - 1) / kDgemmTile, tn = (g.N + kDgemmTile - 1) / kDgemmTile;
-  const int t = threadIdx.x;
-  for (int64_t tile = blockIdx.x; tile < tm * tn; tile += gridDim.x) {
-    const int64_t m0 = (tile % tm) * kDgemmTile, n0 = (tile / tm) * kDgemmTile;
-    bool bad = false;
-    if (t < kDgemmTile) bad = m0 + t < g.M && expA[m0 + t] == kRowNonFinite;
-    else if (t < 2 * kDgemmTile) bad = n0 + t - kDgemmTile < g.N && expB[n0 + t - kDgemmTile] == kRowNonFinite;
-    if (!__syncthreads_or(bad)) continue;
-    dgemm_tile(g, m0, n0, 0, g.K, [&](int64_t m, int64_t n, double acc) {
-      if (expA[m] != kRowNonFinite && expB[n] != kRowNonFinite) return;
-      const int64_t off = g.baseC + g.rowC[m] + g.colC[n];
-      double val = g.alpha * acc;
-      if (g.beta != 0.0) val += g.beta * g.C[off];
-      g.C[off] = val;
-    });
+  constexpr int T = kDgemmTile;
+  __shared__ DgemmShared sh;
+  constexpr int FEW = 128;  // outputs of a piece that are computed one by one, a warp each
+  __shared__ int todo[256], ntodo, few[FEW], nfew, last;
+  const int64_t items = (int64_t)a.tiles_m * a.tiles_n * a.ks;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+  for (int64_t i0 = 0; i0 * gridDim.x + blockIdx.x < items; i0 += 256) {
+    if (t == 0) ntodo = 0;
     __syncthreads();
+    const int64_t mine = (i0 + t) * gridDim.x + blockIdx.x;
+    if (mine < items) {
+      const uint4 f = *reinterpret_cast<const uint4 *>(a.flags + 16 * (mine / a.ks));
+      if (f.x | f.y | f.z | f.w) todo[atomicAdd(&ntodo, 1)] = t;
+    }
+    __syncthreads();
+    for (int q = 0; q < ntodo; q++) {
+      const int64_t item = (i0 + todo[q]) * gridDim.x + blockIdx.x;
+      const int tile = (int)(item / a.ks), z = (int)(item % a.ks);
+      const int64_t M0 = (int64_t)(tile / a.tiles_n) * BM, N0 = (int64_t)(tile % a.tiles_n) * a.bn;
+      const uint8_t *flags = a.flags + 16 * tile;
+      // outputs (m0 + tx + 16 i, n0 + ty + 16 j) of a piece at bit 4 i + j
+      auto marks = [&](int64_t m0, int64_t n0) {
+        uint32_t b = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const int64_t m = m0 + tx + 16 * i, n = n0 + ty + 16 * j;
+            if (m >= g.M || n >= g.N || n >= N0 + a.bn) continue;
+            const int h = column_group(a.bn, (int)(n - N0)), row = (int)(m - M0);
+            if (flags[4 * h + (row >> 5)] &&
+                (a.left[(int64_t)(tile * EPI + h) * BM + row] >> ((int)(n - N0) - group_start(a.bn, h)) & 1u))
+              b |= 1u << (4 * i + j);
+          }
+        return b;
+      };
+      auto finish = [&](int64_t m, int64_t n, double acc) {
+        const int64_t off = g.baseC + g.rowC[m] + g.colC[n];
+        double val = g.alpha * acc;
+        if (g.beta != 0.0) val += g.beta * g.C[off];
+        g.C[off] = val;
+      };
+      double *p = a.partial + (int64_t)tile * a.ks * 4 * T * T;
+      const int64_t kb = z * a.kper, ke = min(g.K, kb + a.kper);
+      for (int piece = 0; piece < 4; piece++) {
+        const int64_t m0 = M0 + (piece & 1) * T, n0 = N0 + (piece >> 1) * T;
+        const uint32_t b = marks(m0, n0);
+        if (t == 0) nfew = 0;
+        if (!__syncthreads_or(b)) continue;
+        auto store = [&](int x, int y, double acc) {
+          if (a.ks == 1) finish(m0 + x, n0 + y, acc);
+          else p[(z * 4 + piece) * (T * T) + x + T * y] = acc;
+        };
+        for (uint32_t r = b; r; r &= r - 1) {
+          const int bit = __ffs((int)r) - 1, at = atomicAdd(&nfew, 1);
+          if (at < FEW) few[at] = tx + 16 * (bit >> 2) + T * (ty + 16 * (bit & 3));
+        }
+        __syncthreads();
+        if (nfew <= FEW) {
+          for (int f = t >> 5; f < nfew; f += 8) {
+            const int x = few[f] % T, y = few[f] / T;
+            const double *A = g.A + g.baseA + g.rowA[m0 + x], *B = g.B + g.baseB + g.colB[n0 + y];
+            double acc = 0.0;
+#pragma unroll 4
+            for (int64_t k = kb + (t & 31); k < ke; k += 32) acc = fma(A[g.kA[k]], B[g.kB[k]], acc);
+            for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+            if ((t & 31) == 0) store(x, y, acc);
+          }
+        } else {
+          dgemm_tile(sh, g, m0, n0, kb, ke, [&](int64_t m, int64_t n, double acc) {
+            const int x = (int)(m - m0), y = (int)(n - n0);
+            if (b >> (4 * (x >> 4) + (y >> 4)) & 1u) store(x, y, acc);
+          });
+        }
+        __syncthreads();
+      }
+      if (a.ks == 1) continue;
+      __threadfence();
+      __syncthreads();
+      if (t == 0) last = atomicAdd(&a.counters[tile], 1) == a.ks - 1;
+      __syncthreads();
+      if (!last) continue;
+      __threadfence();
+      if (t == 0) a.counters[tile] = 0;
+      for (int piece = 0; piece < 4; piece++) {
+        const int64_t m0 = M0 + (piece & 1) * T, n0 = N0 + (piece >> 1) * T;
+        for (uint32_t b = marks(m0, n0); b; b &= b - 1) {
+          const int bit = __ffs((int)b) - 1, x = tx + 16 * (bit >> 2), y = ty + 16 * (bit & 3);
+          double s = 0.0;
+          for (int r = 0; r < a.ks; r++) s += __ldcg(p + (r * 4 + piece) * (T * T) + x + T * y);
+          finish(m0 + x, n0 + y, s);
+        }
+      }
+    }
+    __syncthreads();  // (the list is used up)
   }
 }
 
@@ -753,18 +1030,18 @@ bool kernel_ok() {
 
 }  // namespace
 
-void dgemm_masked(const TableGemm &g, const int *expA, const int *expB, cudaStream_t stream) {
-  const int64_t tiles = ceil_div(g.M, kDgemmTile) * ceil_div(g.N, kDgemmTile);
-  launch(dgemm_masked_kernel, (unsigned)std::min<int64_t>(tiles, 4 * kNumSMs), 256, 0, stream, g, expA, expB);
-  SCESS_CHECK_LAUNCH();
-}
-
 SliceEngine::SliceEngine(Ctx &ctx) : ctx_(ctx) {
   err_.alloc(sizeof(unsigned) * 4);
   SCESS_CUDA(cudaMemsetAsync(err_.as<void>(), 0, sizeof(unsigned) * 4, ctx_.stream));
 }
 
 namespace {
+// Unit of the rows' sums of squares: as fine as 31 bits allow (a CTA's part is rounded up).
+float square_unit(int64_t K) {
+  int e = -12;
+  while (std::ldexp(1.0, 30 + e) < (double)K) e++;
+  return std::ldexp(1.0f, e);
+}
 // The joint form's tiles are at most 64 wide.
 bool joint(int bn) { return bn <= BN_JOINT; }
 // Cycles an SM spends on one K block of a unit, measured (152 tiles of 128 rows, K = 1024:
@@ -813,15 +1090,15 @@ double SliceEngine::estimate_us(int64_t M, int64_t N, int64_t K) {
   return 14.0 + (double)(M + N) * (double)K * 22.0 / 2.9e6 + plan_us(M, N, round_up(std::max<int64_t>(K, 1), BK), z);
 }
 
-bool SliceEngine::usable(int64_t M, int64_t N) {
-  return kernel_ok() && M <= INT32_MAX / 2 && N <= INT32_MAX / 2;
+bool SliceEngine::usable(int64_t M, int64_t N, int64_t K) {
+  return kernel_ok() && M <= INT32_MAX / 2 && N <= INT32_MAX / 2 && K < (int64_t(1) << 26);
 }
 
 CUtensorMap SliceEngine::map_of(const SlicedPack &p, int box_rows) {
   CUtensorMap m;
   std::memset(&m, 0, sizeof(m));
-  cuuint64_t dims[2] = {(cuuint64_t)(kSlices * p.Kpad), (cuuint64_t)p.rows};
-  cuuint64_t strides[1] = {(cuuint64_t)(kSlices * p.Kpad * 2)};
+  cuuint64_t dims[2] = {(cuuint64_t)(kPlanes * p.Kpad), (cuuint64_t)p.rows};
+  cuuint64_t strides[1] = {(cuuint64_t)(kPlanes * p.Kpad * 2)};
   cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.mem.as<void>(), dims, strides, box, estr,
@@ -834,7 +1111,7 @@ CUtensorMap SliceEngine::map_of(const SlicedPack &p, int box_rows) {
 
 void SliceEngine::alloc(SlicedPack &out, int64_t rows, int64_t K) {
   const int64_t Kpad = round_up(std::max<int64_t>(K, 1), BK);
-  const size_t bytes = (size_t)rows * kSlices * Kpad * sizeof(uint16_t), eb = (size_t)rows * sizeof(int);
+  const size_t bytes = (size_t)rows * kPlanes * Kpad * sizeof(uint16_t), eb = (size_t)rows * 3 * sizeof(int);
   if (out.mem.bytes() < bytes) out.mem.alloc(bytes);
   if (out.exps.bytes() < eb) out.exps.alloc(round_up((int64_t)eb, 4096));
   out.rows = rows;
@@ -863,7 +1140,7 @@ void SliceEngine::pack_with_exps(const double *src, const int64_t *rowOff, int64
                                  int64_t K, bool unitK, const int *exps, const int64_t *expIdx, bool negate,
                                  SlicedPack &out) {
   alloc(out, rows, K);
-  TimedScope ts(ctx_.timer, "slice_pack", 0.0, (double)rows * K * 8 + (double)rows * out.Kpad * 14, ctx_.stream);
+  TimedScope ts(ctx_.timer, "slice_pack", 0.0, (double)rows * K * 8 + (double)rows * out.Kpad * 16, ctx_.stream);
   PackOp op = {};
   op.src = src;
   op.row = rowOff;
@@ -904,7 +1181,9 @@ void SliceEngine::pack(const Gather *g, SlicedPack *const *out, int n) {
     op.unitK = g[i].unitK ? 1 : 0;
     op.dst = o.mem.as<uint16_t>();
     op.exps = o.exps.as<int>();
-    bytes += (double)g[i].rows * g[i].K * 8 + (double)g[i].rows * o.Kpad * 14;
+    op.stats = op.exps + g[i].rows;
+    op.sq_unit = square_unit(g[i].K);
+    bytes += (double)g[i].rows * g[i].K * 8 + (double)g[i].rows * o.Kpad * 16;
     const int64_t chunks = ceil_div(o.Kpad, 64);
     // one walk per CTA over its rows' whole K while that fills the device or K is
     // short; else the exponents first, then the cut, each spread over K too
@@ -948,7 +1227,7 @@ void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial)
   a.nseg = ps.nseg;
   for (int s = 0; s < ps.nseg; s++) {
     const SliceSegment &g = ps.seg[s];
-    if (g.Kpad % BK != 0 || g.Kpad <= 0 || kSlices * g.Kpad > INT32_MAX)
+    if (g.Kpad % BK != 0 || g.Kpad <= 0 || kPlanes * g.Kpad > INT32_MAX)
       throw Error(SCESS_ERR_INVALID, "slice gemm: segment K");
     for (int q = 0; q < ps.ng; q++) {
       const int64_t maxA = g.rowA0[q] + (int64_t)(ps.ny - 1) * g.rowAy[q] + (int64_t)(ps.nz - 1) * g.rowAz[q] + a.tiles_m * BM;
@@ -997,6 +1276,12 @@ void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial)
   a.gstart[ps.ng] = (int)start;
   a.expA = ps.expA;
   a.expB = ps.expB;
+  a.est = ps.est;
+  a.sq_unit = ps.sq_unit;
+  a.rowsA = (int)ps.M;
+  a.rowsB = (int)ps.N;
+  a.left = ps.left;
+  a.flags = ps.flags;
   a.C = ps.C;
   a.baseC = ps.baseC;
   a.alpha = ps.alpha;
@@ -1008,7 +1293,9 @@ void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial)
   a.alpha_neg = f < 0;
   a.partial = a.splits > 1 ? partial : nullptr;
   a.part_stride = ps.M * ps.N;
-  if (a.splits > 1 && (!partial || start > 1)) throw Error(SCESS_ERR_INVALID, "slice gemm: split-K");
+  a.est_partial = reinterpret_cast<float *>(partial + a.splits * a.part_stride);
+  if (a.est && (start > 1 || ps.nseg > 1)) throw Error(SCESS_ERR_INVALID, "slice gemm: estimates of one problem");
+  if (a.splits > 1 && (!partial || !a.est || start > 1)) throw Error(SCESS_ERR_INVALID, "slice gemm: split-K");
   a.err = err_.as<unsigned>();
   a.wait_cycles = 1ll << 32;
   SliceMaps maps;
@@ -1031,32 +1318,55 @@ void SliceEngine::gemm_grouped(const SliceProblemSet &ps, double flops, const ch
   launch(ps, 1, nullptr);
 }
 
-void SliceEngine::gemm(const SlicedPack &A, const SlicedPack &B, double alpha, double beta, double *C,
-                       const int64_t *rowC, const int64_t *colC, const char *name) {
+void SliceEngine::product(const TableGemm &g, const SlicedPack &A, const SlicedPack &B, const char *name) {
   SliceProblemSet ps;
-  ps.M = A.rows;
-  ps.N = B.rows;
+  ps.M = g.M;
+  ps.N = g.N;
   int64_t splits = 1;
   plan_us(ps.M, ps.N, A.Kpad, splits);
-  double *partial = nullptr;
-  if (splits > 1) {
-    const size_t need = (size_t)splits * ps.M * ps.N * sizeof(double);
-    if (partial_.bytes() < need) partial_.alloc(need);
-    partial = partial_.d();
-  }
-  TimedScope ts(ctx_.timer, name, 2.0 * ps.M * ps.N * A.K, 0.0, ctx_.stream);
+  LeftArgs la = {};
+  la.bn = tile_n(g.N);
+  la.tiles_m = (int)ceil_div(g.M, BM);
+  la.tiles_n = (int)ceil_div(g.N, la.bn);
+  la.counters = ctx_.counters.as<int>();
+  const int64_t tiles = (int64_t)la.tiles_m * la.tiles_n;
+  static_assert(kNumSMs <= kSmallCounters, "a counter a tile");
+  // few tiles: their K over several CTAs (one takes 4 ms per thousand k)
+  const int64_t ks = tiles >= kNumSMs ? 1 : std::min(4 * kNumSMs / tiles, ceil_div(g.K, 64));
+  la.kper = ks == 1 ? g.K : round_up(ceil_div(g.K, ks), 16);
+  la.ks = (int)ceil_div(g.K, la.kper);
+  // (everything is allocated before anything is launched: the caller falls back to the FP64
+  // units when it does not fit)
+  auto room = [](DevMem &m, size_t bytes) {
+    if (m.bytes() < bytes) m.alloc(bytes);
+  };
+  const size_t mn = (size_t)g.M * g.N, words = (size_t)tiles * EPI * BM;
+  room(left_, words * sizeof(uint32_t) + 16 * tiles);
+  room(partial_, std::max(splits > 1 ? splits * mn * (sizeof(double) + sizeof(float)) : 0,
+                          la.ks > 1 ? (size_t)tiles * la.ks * 4 * kDgemmTile * kDgemmTile * sizeof(double) : 0));
+  ps.est = 1;
+  ps.sq_unit = square_unit(g.K);
+  ps.left = left_.as<uint32_t>();
+  ps.flags = reinterpret_cast<uint8_t *>(ps.left + words);
+  la.left = ps.left;
+  la.flags = ps.flags;
+  la.partial = partial_.d();
+  TimedScope ts(ctx_.timer, name, 2.0 * g.M * g.N * g.K, 0.0, ctx_.stream);
   ps.maps[0] = map_of(A, BM);
   ps.maps[1] = map_of(B, tile_n(ps.N));
   ps.nmaps = 2;
   ps.seg[0].Kpad = A.Kpad;
   ps.expA = A.e();
   ps.expB = B.e();
-  ps.C = C;
-  ps.rowC[0] = rowC;
-  ps.colC[0] = colC;
-  ps.alpha = alpha;
-  ps.beta = beta;
-  launch(ps, (int)splits, partial);
+  ps.C = g.C;
+  ps.baseC = g.baseC;
+  ps.rowC[0] = g.rowC;
+  ps.colC[0] = g.colC;
+  ps.alpha = g.alpha;
+  ps.beta = g.beta;
+  launch(ps, (int)splits, partial_.d());
+  scess::launch(slice_left_kernel, (unsigned)std::min<int64_t>(tiles * la.ks, 4 * kNumSMs), 256, 0, ctx_.stream, g, la);
+  SCESS_CHECK_LAUNCH();
 }
 
 void SliceEngine::reclaim() {
@@ -1064,6 +1374,7 @@ void SliceEngine::reclaim() {
   tmpA_ = SlicedPack();
   tmpB_ = SlicedPack();
   partial_.release();
+  left_.release();
   spare_.clear();
   cache_.clear();
 }
@@ -1074,6 +1385,25 @@ struct Busy {
   explicit Busy(bool &x) : b(x) { b = true; }
   ~Busy() { b = false; }
 };
+// The same product with its sides exchanged: C^T = B^T A^T.
+TableGemm exchanged(const TableGemm &g) {
+  TableGemm h = g;
+  h.A = g.B;
+  h.B = g.A;
+  h.rowA = g.colB;
+  h.kA = g.kB;
+  h.colB = g.rowA;
+  h.kB = g.kA;
+  h.rowC = g.colC;
+  h.colC = g.rowC;
+  h.baseA = g.baseB;
+  h.baseB = g.baseA;
+  h.M = g.N;
+  h.N = g.M;
+  h.aUnitM = g.bUnitN;
+  h.bUnitN = g.aUnitM;
+  return h;
+}
 }  // namespace
 
 bool SliceEngine::table_gemm(const TableGemm &g, const char *name) {
@@ -1083,13 +1413,12 @@ bool SliceEngine::table_gemm(const TableGemm &g, const char *name) {
                           {g.B + g.baseB, g.colB, g.N, g.kB, g.K, !g.bUnitN}};
     SlicedPack *const out[2] = {&tmpA_, &tmpB_};
     pack(ga, out, 2);
-    if (g.M <= 64 && g.M < g.N) gemm(tmpB_, tmpA_, g.alpha, g.beta, g.C + g.baseC, g.colC, g.rowC, name);
-    else gemm(tmpA_, tmpB_, g.alpha, g.beta, g.C + g.baseC, g.rowC, g.colC, name);
+    if (g.M <= 64 && g.M < g.N) product(exchanged(g), tmpB_, tmpA_, name);
+    else product(g, tmpA_, tmpB_, name);
   } catch (const Error &e) {
     if (e.code != SCESS_ERR_OOM) throw;
     return false;
   }
-  dgemm_masked(g, tmpA_.e(), tmpB_.e(), ctx_.stream);
   return true;
 }
 
@@ -1157,22 +1486,6 @@ bool SliceEngine::contract(const EinsumPlan &pl, double alpha, const double *A, 
     out[n++] = p;
     return p;
   };
-  const std::string tname = "slice_gemm[" + pl.spec + "]";
-  const SlicedPack *pa = nullptr, *pb = nullptr;
-  try {
-    pa = get(gA, true, constA, tmpA_);
-    pb = get(gB, false, constB, tmpB_);
-    if (n) pack(todo, out, n);
-    if (swap) gemm(*pb, *pa, alpha, beta, C, pl.d_colC, pl.d_rowC, tname.c_str());
-    else gemm(*pa, *pb, alpha, beta, C, pl.d_rowC, pl.d_colC, tname.c_str());
-  } catch (const Error &e) {
-    // packs listed above may not have been made
-    reuse_.clear();
-    spare_.clear();
-    cache_.clear();
-    if (e.code != SCESS_ERR_OOM) throw;
-    return false;  // no room for the packs: the DFMA kernel needs none
-  }
   TableGemm g;
   g.A = A;
   g.B = B;
@@ -1190,7 +1503,20 @@ bool SliceEngine::contract(const EinsumPlan &pl, double alpha, const double *A, 
   g.beta = beta;
   g.aUnitM = pl.aUnitM;
   g.bUnitN = pl.bUnitN;
-  dgemm_masked(g, pa->e(), pb->e(), ctx_.stream);
+  const std::string tname = "slice_gemm[" + pl.spec + "]";
+  try {
+    const SlicedPack *pa = get(gA, true, constA, tmpA_), *pb = get(gB, false, constB, tmpB_);
+    if (n) pack(todo, out, n);
+    if (swap) product(exchanged(g), *pb, *pa, tname.c_str());
+    else product(g, *pa, *pb, tname.c_str());
+  } catch (const Error &e) {
+    // packs listed above may not have been made
+    reuse_.clear();
+    spare_.clear();
+    cache_.clear();
+    if (e.code != SCESS_ERR_OOM) throw;
+    return false;  // no room for the packs: the DFMA kernel needs none
+  }
   return true;
 }
 

@@ -23,11 +23,14 @@
 // products (kc|ld) t2 of the iterations o5 v19 .1e-16, 1.5e-16; o8 v47 .9e-16, 1.6e-16;
 // o10 v90 .7e-16, 4.5e-16; o16 v140 .8e-16, 12e-16.  (With S_5 + S_6 in one accumulator and
 // S_7 dropped, 28 products: 1.4, 2.6, 4.8 and 9.6e-16.)  Values far below their row's
-// largest are held to that row's 60 bits, not to 53 of their own.
-//
-// Rows holding Inf or NaN are marked by the pack kernel; their outputs are left to
-// the DFMA kernel (dgemm_masked), which is launched behind every GEMM and returns
-// at once where nothing is marked.
+// largest are held to that row's 60 bits, not to 53 of their own: where they decide an
+// output, sum_k |a_k b_k| is small beside |row max| |column max|.  An eighth plane of the packs
+// holds the values' magnitudes, whose product tells that sum for every output (two MMAs for
+// the digits' 68).  Outputs that are short of the rule at slice_left, and those of rows and
+// columns with Inf or NaN, are left to the FP64 units (slice_left_kernel, behind every GEMM; it
+// returns at once where nothing is left).  So an output's error is of the size of a chain of
+// FP64 multiply-adds', relative to sum_k |a_k b_k|, whatever the values.  The grouped launches of
+// (T) do without (see triples_fp64_sliced).
 #pragma once
 #include <cuda.h>
 
@@ -42,12 +45,14 @@
 
 namespace scess {
 
-constexpr int kSlices = 7;
+constexpr int kSlices = 7, kPlanes = kSlices + 1;  // digits, magnitudes
 constexpr int kSliceBK = 32;        // K block of the kernel: 32 x 16 bit = 64 B rows, SWIZZLE_64B
 constexpr int kRowNonFinite = 2047;  // row exponent of a row that holds Inf or NaN
 
-// rows x [kSlices][Kpad] BF16 digits, Kpad a multiple of 32, and one biased FP64
-// exponent per row (0: all values zero; kRowNonFinite: Inf or NaN).
+// rows x [kPlanes][Kpad] BF16 values, Kpad a multiple of 32, and per row one biased FP64
+// exponent (0: all values zero; kRowNonFinite: Inf or NaN); behind the exponents, for products
+// that stand alone, the rows' sums of squares relative to their largest value (in units of
+// square_unit), and then their numbers of values that are not zero.
 struct SlicedPack {
   DevMem mem, exps;
   DevMem part;  // partial row exponents of long rows
@@ -72,6 +77,11 @@ struct SliceProblemSet {
   // exponents of output row m / column n of group g: expA[expA0[g] + m], expB[n]
   const int *expA = nullptr, *expB = nullptr;
   int64_t expA0[3] = {0, 0, 0};
+  // outputs left to the FP64 units (see SliceArgs)
+  int est = 0;
+  float sq_unit = 0.0f;
+  uint32_t *left = nullptr;
+  uint8_t *flags = nullptr;
   // output element (m, n) of problem (y, z, g): C[baseC + y cy + z cz + cg + rowC[m] + colC[n]]
   double *C = nullptr;
   int64_t baseC = 0, cy[3] = {0, 0, 0}, cz[3] = {0, 0, 0}, cg[3] = {0, 0, 0};
@@ -83,7 +93,7 @@ class SliceEngine {
  public:
   explicit SliceEngine(Ctx &ctx);
   // The device runs the kernel and the sizes are within its coordinates.
-  static bool usable(int64_t M, int64_t N);
+  static bool usable(int64_t M, int64_t N, int64_t K);
   // Estimated time of a product with its packs, in us.
   static double estimate_us(int64_t M, int64_t N, int64_t K);
   // C = alpha A.B + beta C through the tables of g (the FP64 engine's GEMM).
@@ -135,8 +145,8 @@ class SliceEngine {
   // Packs of up to two operands in one launch (two where K is long).
   void pack(const Gather *g, SlicedPack *const *out, int n);
   void alloc(SlicedPack &out, int64_t rows, int64_t K);
-  void gemm(const SlicedPack &A, const SlicedPack &B, double alpha, double beta, double *C,
-            const int64_t *rowC, const int64_t *colC, const char *name);
+  // The product of g's operands, packed as A and B.
+  void product(const TableGemm &g, const SlicedPack &A, const SlicedPack &B, const char *name);
   void launch(const SliceProblemSet &ps, int splits, double *partial);
 
   Ctx &ctx_;
@@ -155,11 +165,8 @@ class SliceEngine {
   std::set<const double *> stable_;
   const void *owner_ = nullptr;
   SlicedPack tmpA_, tmpB_;
-  DevMem err_, partial_;
+  DevMem err_, partial_, left_;
   bool launched_ = false, busy_ = false;
 };
-
-// Outputs of g whose A row or B column is marked in expA / expB (kRowNonFinite).
-void dgemm_masked(const TableGemm &g, const int *expA, const int *expB, cudaStream_t stream);
 
 }  // namespace scess

@@ -754,7 +754,9 @@ __global__ void __launch_bounds__(256) tc_reduce_kernel(TcOut out, int64_t M, in
   }
   __syncthreads();
   const double alpha = s_alpha;
-  split_sum<ZG>(partial, M, N, splits, [&](int64_t m, int64_t n, double s) {
+  const int64_t MN = M * N;
+  auto load = [&](int z, int64_t e) { return (double)partial[z * MN + e]; };
+  split_sum<ZG, double>(M, N, splits, load, [&](int64_t m, int64_t n, double s) {
     const int64_t off = out.baseC + out.rowC[m] + out.colC[n];
     double val = alpha * s;
     if (out.fp32) {

@@ -19,8 +19,9 @@ constexpr int BM = kDgemmTile, BN = kDgemmTile, BK = kDgemmBK;
 __global__ void __launch_bounds__(256) dgemm_table_kernel(TableGemm g, int64_t kChunk,
                                                           double *partial) {
   chain();
+  __shared__ DgemmShared sh;
   const int64_t kb = (int64_t)blockIdx.z * kChunk;
-  dgemm_tile(g, (int64_t)blockIdx.x * BM, (int64_t)blockIdx.y * BN, kb, min(g.K, kb + kChunk),
+  dgemm_tile(sh, g, (int64_t)blockIdx.x * BM, (int64_t)blockIdx.y * BN, kb, min(g.K, kb + kChunk),
              [&](int64_t m, int64_t n, double acc) {
                if (partial) {
                  partial[(int64_t)blockIdx.z * g.M * g.N + m + g.M * n] = acc;

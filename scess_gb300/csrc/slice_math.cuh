@@ -72,6 +72,15 @@ SCESS_HD int64_t slice_fixed(double x, int emax) {
   return (b >> 63) ? -F : F;
 }
 
+// |x| relative to its row's largest exponent as BF16 bits, rounded down: |x| 2^(1022 - emax), at least
+// 2^-60 unless x is zero.
+SCESS_HD uint32_t slice_magnitude(double x, int emax) {
+  const uint64_t b = bits_of(x) & 0x7fffffffffffffffull;
+  const int be = (int)(b >> 52), gap = emax - be;
+  if (b == 0) return 0u;
+  return be == 0 || gap > 58 ? (127 - 60) << 7 : (uint32_t)(126 - gap) << 7 | ((uint32_t)(b >> 45) & 0x7fu);
+}
+
 // F + kDigitBias has digit p (p = 1 .. 6) in bits [9 (6 - p), 9 (6 - p) + 9)
 // offset by 256, and digit 0 above bit 54.
 constexpr int64_t kDigitBias = 256ll * (1ll + (1ll << 9) + (1ll << 18) + (1ll << 27) + (1ll << 36) +

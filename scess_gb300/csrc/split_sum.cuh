@@ -1,5 +1,5 @@
 // Sums over the K ranges of a split product, shared by the reductions of both
-// tensor-core engines: partial[z][e], z in a fixed order, added in FP64.
+// tensor-core engines: load(z, e), z in a fixed order, added as V.
 #pragma once
 #include <cstdint>
 
@@ -15,10 +15,9 @@ inline unsigned split_blocks(int64_t MN, bool groups) {
   return (unsigned)(groups || n < 2048 ? n : 2048);
 }
 
-// finish(m, n, sum) for every output m + M n.
-template <int ZG, typename T, typename F>
-__device__ __forceinline__ void split_sum(const T *__restrict__ partial, int64_t M, int64_t N, int splits,
-                                          const F &finish) {
+// finish(m, n, sum) for every output e = m + M n.
+template <int ZG, typename V, typename L, typename F>
+__device__ __forceinline__ void split_sum(int64_t M, int64_t N, int splits, const L &load, const F &finish) {
   const int64_t MN = M * N;
   auto indices = [&](int64_t e, int64_t &m, int64_t &n) {
     if (MN <= UINT32_MAX) {
@@ -32,21 +31,22 @@ __device__ __forceinline__ void split_sum(const T *__restrict__ partial, int64_t
   };
   if constexpr (ZG == 1) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < MN; e += (int64_t)gridDim.x * blockDim.x) {
-      double s = 0.0;
+      V s{};
 #pragma unroll 4
-      for (int z = 0; z < splits; z++) s += (double)partial[(int64_t)z * MN + e];
+      for (int z = 0; z < splits; z++) s += load(z, e);
       int64_t m, n;
       indices(e, m, n);
       finish(m, n, s);
     }
   } else {
-    __shared__ double red[ZG][32];
+    __shared__ __align__(16) unsigned char raw[ZG * 32 * sizeof(V)];
+    V(*red)[32] = reinterpret_cast<V(*)[32]>(raw);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t e = blockIdx.x * (int64_t)32 + lane;
-    double s = 0.0;
+    V s{};
     if (e < MN) {
 #pragma unroll 4
-      for (int z = w; z < splits; z += ZG) s += (double)partial[(int64_t)z * MN + e];
+      for (int z = w; z < splits; z += ZG) s += load(z, e);
     }
     red[w][lane] = s;
     __syncthreads();
