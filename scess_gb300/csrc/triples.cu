@@ -22,6 +22,7 @@
 // by block.  The energy kernel reads W once, clears it for the next block
 // triple and works in FP32 per element with denominators formed from the FP64
 // orbital energies in double-float, compensated sums and FP64 per triple.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -1158,7 +1159,8 @@ int choose_nb_sliced(int64_t o, int64_t v) {
 // tensor cores' exact slices (gemm_slice.h), in the three groups of four K segments
 // described in rccsd_triples.  All segments of a group add up in one sum per output,
 // so P and t2 rows share the exponent of their (u, x) and Q and R rows that of their
-// (s, t).  False (nothing computed) when the packs do not fit into device memory.
+// (s, t).  False (nothing computed) when the packs do not fit into device memory or the
+// operands hold Inf or NaN.
 bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, const double *d_eps,
                          const double *d_t1, const double *d_t2, const Control &ctl, TriplesStats *stats,
                          const double *d_B, int64_t naux, double &e_t) {
@@ -1236,7 +1238,11 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
   }
   SCESS_CUDA(cudaMemsetAsync(energies.p(), 0, energies.size() * sizeof(double), s));
   SCESS_CUDA(cudaMemcpyAsync(orbits.as<void>(), ot.data(), ot.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-  ctx.sync();  // (ot is a host vector of this scope)
+  std::vector<int> he(o * vp + o2);
+  SCESS_CUDA(cudaMemcpyAsync(he.data(), exps.as<void>(), he.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+  ctx.sync();  // (ot and he are host vectors of this scope)
+  // Inf or NaN among the operands: the digits hold neither
+  if (std::find(he.begin(), he.end(), kRowNonFinite) != he.end()) return false;
   const int64_t p1 = o | 1, p2 = (p1 * o) | 1;
   const unsigned threads = (unsigned)std::min<int64_t>(256, round_up(norbits, 32));
   const size_t smem = (size_t)std::max<int64_t>(p2 * o + 3 * p1 * o + 4 * o, threads) * 8;
