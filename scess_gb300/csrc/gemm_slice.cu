@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(256) slice_pack_kernel(const __grid_constant__
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       const double xv = tile[rr][9 * ch + j];
-      int64_t F = e == kRowNonFinite ? 0 : slice_fixed(xv, e);
+      int64_t F = e == kRowNonFinite ? 0 : slice_fixed(xv, e);  // (GIVEN: the caller rejects such rows)
       const float fx = (float)(int)(F >> 32);  // 2^28 x / 2^E
       sq = fmaf(fx, fx, sq);
       const uint32_t mag = slice_magnitude(xv, e);

@@ -30,7 +30,7 @@
 // columns with Inf or NaN, are left to the FP64 units (slice_left_kernel, behind every GEMM; it
 // returns at once where nothing is left).  So an output's error is of the size of a chain of
 // FP64 multiply-adds', relative to sum_k |a_k b_k|, whatever the values.  The grouped launches of
-// (T) do without (see triples_fp64_sliced).
+// (T) do without (see triples_slices_hold).
 #pragma once
 #include <cuda.h>
 

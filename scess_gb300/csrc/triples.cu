@@ -32,6 +32,7 @@
 #include "gemm_slice.h"
 #include "gemm_tc.h"
 #include "launch.cuh"
+#include "slice_math.cuh"
 #include "triples.h"
 
 namespace scess {
@@ -1155,12 +1156,119 @@ int choose_nb_sliced(int64_t o, int64_t v) {
   return best;
 }
 
+// Exponents of the sliced FP64 form.  All four segments of a group add up in one sum per
+// output, so P and t2 rows of a (u, x) share an exponent, and Q (t2 too) and R rows of an (s, t);
+// t2 2^s meets R 2^-s there, with one shift s for the call that brings amplitudes and
+// integrals to one size on either side (unshifted, amplitudes of 2^-30 had 33 bits of their 53).
+// raw: P, t2 ([nA] each), Q, R ([nB] each), 0 for all zeros; out: the exponents to cut P, t2, Q and
+// R with, kRowNonFinite kept; mx: the four tensors' largest.
+__global__ void __launch_bounds__(1024) triples_exps_kernel(const int *__restrict__ raw, int64_t nA, int64_t nB,
+                                                            int *__restrict__ out, int *__restrict__ mx) {
+  chain();
+  __shared__ int m[4];
+  if (threadIdx.x < 4) m[threadIdx.x] = 0;
+  __syncthreads();
+  const int64_t n[4] = {nA, nA, nB, nB}, at[4] = {0, nA, 2 * nA, 2 * nA + nB};
+  for (int q = 0; q < 4; q++) {
+    int e = 0;
+    for (int64_t i = threadIdx.x; i < n[q]; i += blockDim.x) e = max(e, raw[at[q] + i]);
+    atomicMax(&m[q], e);
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) mx[threadIdx.x] = m[threadIdx.x];
+  const int s = (m[0] && m[1] && m[2] && m[3]) ? ((m[0] - m[1]) + (m[3] - m[2])) / 2 : 0;
+  for (int side = 0; side < 2; side++) {
+    const int sh = side ? -s : s;  // of the second tensor of the side
+    const int *x = raw + at[2 * side], *y = x + n[2 * side];
+    int *ox = out + at[2 * side], *oy = ox + n[2 * side];
+    for (int64_t i = threadIdx.x; i < n[2 * side]; i += blockDim.x) {
+      const bool bad = x[i] == kRowNonFinite || y[i] == kRowNonFinite;
+      const int e = x[i] || y[i] ? max(1, max(x[i] ? x[i] : 1, y[i] ? y[i] + sh : 1)) : 0;
+      ox[i] = bad ? kRowNonFinite : e;
+      oy[i] = bad ? kRowNonFinite : (e ? e - sh : 0);
+    }
+  }
+}
+
+// Sums of squares of P and Q for every f, t2 and R for every m, relative to the tensor's largest
+// exponent: out[column][part], columns P (v), Q (v), t2 (o), R (o).
+constexpr int kSquareParts = 8;
+struct SquareOps {
+  const double *src[4];
+  const int64_t *row[4], *k[4];
+  int64_t rows[4];
+  int v, o;
+};
+__global__ void __launch_bounds__(256) triples_squares_kernel(SquareOps ops, const int *__restrict__ mx,
+                                                              float *__restrict__ out) {
+  chain();
+  __shared__ float red[8];
+  int c = blockIdx.x / kSquareParts;
+  const int part = blockIdx.x % kSquareParts;
+  const int q = c < ops.v ? 0 : c < 2 * ops.v ? 1 : c < 2 * ops.v + ops.o ? 2 : 3;
+  c -= q < 2 ? q * ops.v : 2 * ops.v + (q - 2) * ops.o;
+  const int e = mx[q == 0 ? 0 : q == 1 ? 2 : q == 2 ? 1 : 3];  // (mx in the order P, t2, Q, R)
+  const double *src = ops.src[q] + ops.k[q][c];
+  float s = 0.0f;
+  for (int64_t r = part * 256 + threadIdx.x; r < ops.rows[q]; r += 256 * kSquareParts) {
+    const float x = __uint_as_float(slice_magnitude(src[ops.row[q][r]], e) << 16);
+    s = fmaf(x, x, s);
+  }
+  for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) s += red[w];
+    out[blockIdx.x] = s;
+  }
+}
+
+// Whether the sliced form is as accurate as FP64 multiply-adds for the energy, a sum over all W of
+// a block: the squared errors of all outputs (see slice_left, gemm_slice.cu) are compared,
+//   2^-122 / 3 sum [(column max)^2 a_k^2 + (row max)^2 b_k^2]  <=  0.16 2^-106 sum (a_k b_k)^2
+// with a factor of 2 to spare; dense tensors pass by a factor of 50 and more.  False also
+// where an exponent leaves the range of FP64's.
+bool triples_slices_hold(const std::vector<int> &exps, const int mx[4], const std::vector<float> &squares, int64_t o,
+                         int64_t v, int64_t nA, int64_t nB) {
+  for (int e : exps)
+    if (e >= kRowNonFinite) return false;
+  auto col = [&](int64_t c) {
+    double s = 0.0;
+    for (int p = 0; p < kSquareParts; p++) s += squares[c * kSquareParts + p];
+    return s;
+  };
+  const int *eA = exps.data(), *eB = eA + 2 * nA;
+  int a = 1, b = 1;  // largest exponents of the two sides
+  for (int64_t i = 0; i < nA; i++) a = std::max(a, eA[i]);
+  for (int64_t i = 0; i < nB; i++) b = std::max(b, eB[i]);
+  double ra = 0.0, rb = 0.0;  // sums of (row max)^2, (column max)^2 over (u, x), (s, t)
+  for (int64_t i = 0; i < nA; i++)
+    if (eA[i]) ra += std::exp2(2.0 * (eA[i] - a));
+  for (int64_t i = 0; i < nB; i++)
+    if (eB[i]) rb += std::exp2(2.0 * (eB[i] - b));
+  // the tensors' largest relative to their side's: t2 and R carry the shift
+  int64_t shift = 0;
+  for (int64_t i = 0; i < nA; i++)
+    if (eA[i]) shift = eA[i] - eA[nA + i];
+  const double scale[4] = {2.0 * (mx[0] - a), 2.0 * (mx[2] - b), 2.0 * (mx[1] + shift - a), 2.0 * (mx[3] - shift - b)};
+  double norms[2] = {0.0, 0.0}, products = 0.0;
+  for (int pair = 0; pair < 2; pair++) {
+    const int64_t n = pair ? o : v, c0 = pair ? 2 * v : 0;
+    const double fa = std::exp2(scale[2 * pair]), fb = std::exp2(scale[2 * pair + 1]);
+    for (int64_t f = 0; f < n; f++) {
+      const double x = col(c0 + f) * fa, y = col(c0 + n + f) * fb;
+      norms[0] += x;
+      norms[1] += y;
+      products += x * y;
+    }
+  }
+  return (double)v * (rb * norms[0] + ra * norms[1]) <= 16384.0 * products;
+}
+
 // FP64 (T) with the 12 products of a block triple as one grouped launch on the
 // tensor cores' exact slices (gemm_slice.h), in the three groups of four K segments
-// described in rccsd_triples.  All segments of a group add up in one sum per output,
-// so P and t2 rows share the exponent of their (u, x) and Q and R rows that of their
-// (s, t).  False (nothing computed) when the packs do not fit into device memory or the
-// operands hold Inf or NaN.
+// described in rccsd_triples.  False (nothing computed) when the packs do not fit into device
+// memory or the slices do not hold the operands.
 bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, const double *d_eps,
                          const double *d_t1, const double *d_t2, const Control &ctl, TriplesStats *stats,
                          const double *d_B, int64_t naux, double &e_t) {
@@ -1181,8 +1289,10 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
   SliceEngine &se = ctx.slice_engine();
   SlicedPack pP, pQ, pQ2, pR, pR2, pTx;
   DevTables pdt, gdt;
-  DevMem exps, W, orbits;
+  DevMem exps, squares, W, orbits;
   DTensor energies;
+  const int64_t nA = o * vp, nexp = 2 * nA + 2 * o2;
+  std::vector<float> hsq;
   std::vector<uint32_t> ot = orbit_table(o);
   const int norbits = (int)ot.size();
   try {
@@ -1203,9 +1313,10 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
                     table({{o, 1}, {nb, o}, {nb, 0}, {NB, 0}, {NB, o * nb}}),
                     table({{o, 1}, {nb, o}, {nb, 0}, {NB, o * nb}, {NB, 0}}),
                     table({{o, 1}, {o, o}, {nb, 0}, {NB, 0}})});
-    exps.alloc((size_t)(o * vp + o2) * sizeof(int));
-    int *eA = exps.as<int>(), *eB = eA + o * vp;
-    SCESS_CUDA(cudaMemsetAsync(eA, 0, (size_t)(o * vp + o2) * sizeof(int), s));
+    // P, t2 (o vp each), Q, R (o^2 each): exponents as found, then as used; then the largest
+    exps.alloc((size_t)(2 * nexp + 4) * sizeof(int));
+    int *raw = exps.as<int>(), *use = raw + nexp;
+    SCESS_CUDA(cudaMemsetAsync(raw, 0, (size_t)nexp * sizeof(int), s));
     const int64_t *kP = T.dt.ptr[T.kOperand + 1], *kT = T.dt.ptr[T.kOperand + 7], *kQ = T.dt.ptr[T.kOperand + 3],
                   *kR = T.dt.ptr[T.kOperand + 5];
     const int64_t rP = o * vp * vp, rQ = o2 * vp;
@@ -1216,18 +1327,35 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
       const int64_t *k;
       int64_t K;
       bool unitK;
-      int *e;
+      int64_t e;  // of its exponents
       int idx;
       bool neg;
       SlicedPack &out;
     };
-    const Op ops[6] = {{T.P, 0, rP, kP, v, false, eA, 6, false, pP},  {T.T2p, 3, rP, kT, o, true, eA, 7, true, pTx},
-                       {T.Qt, 1, rQ, kQ, v, true, eB, 8, false, pQ},  {T.Qt, 4, rQ, kQ, v, true, eB, 8, false, pQ2},
-                       {T.Rt, 2, rQ, kR, o, false, eB, 8, false, pR}, {T.Rt, 5, rQ, kR, o, false, eB, 8, false, pR2}};
+    const int64_t oT = nA, oQ = 2 * nA, oR = 2 * nA + o2;
+    const Op ops[6] = {{T.P, 0, rP, kP, v, false, 0, 6, false, pP},   {T.T2p, 3, rP, kT, o, true, oT, 7, true, pTx},
+                       {T.Qt, 1, rQ, kQ, v, true, oQ, 8, false, pQ},  {T.Qt, 4, rQ, kQ, v, true, oQ, 8, false, pQ2},
+                       {T.Rt, 2, rQ, kR, o, false, oR, 8, false, pR}, {T.Rt, 5, rQ, kR, o, false, oR, 8, false, pR2}};
     for (const Op &q : ops)
-      se.row_exps(q.t.p(), pdt.ptr[q.row], q.rows, q.k, q.K, q.unitK, q.e, pdt.ptr[q.idx]);
+      se.row_exps(q.t.p(), pdt.ptr[q.row], q.rows, q.k, q.K, q.unitK, raw + q.e, pdt.ptr[q.idx]);
+    launch(triples_exps_kernel, 1, 1024, 0, s, (const int *)raw, nA, o2, use, use + nexp);
+    SCESS_CHECK_LAUNCH();
+    SquareOps sq = {};
+    sq.v = (int)v;
+    sq.o = (int)o;
+    for (int q = 0; q < 4; q++) {
+      const Op &x = ops[q == 0 ? 0 : q == 1 ? 2 : q == 2 ? 1 : 4];
+      sq.src[q] = x.t.p();
+      sq.row[q] = pdt.ptr[x.row];
+      sq.k[q] = x.k;
+      sq.rows[q] = x.rows;
+    }
+    hsq.resize((size_t)(2 * v + 2 * o) * kSquareParts);
+    squares.alloc(hsq.size() * sizeof(float));
+    launch(triples_squares_kernel, (unsigned)hsq.size(), 256, 0, s, sq, (const int *)(use + nexp), squares.as<float>());
+    SCESS_CHECK_LAUNCH();
     for (const Op &q : ops)
-      se.pack_with_exps(q.t.p(), pdt.ptr[q.row], q.rows, q.k, q.K, q.unitK, q.e, pdt.ptr[q.idx], q.neg, q.out);
+      se.pack_with_exps(q.t.p(), pdt.ptr[q.row], q.rows, q.k, q.K, q.unitK, use + q.e, pdt.ptr[q.idx], q.neg, q.out);
     gdt.build(ctx, {table({{Mg, 1}}), table({{Ng, Mg}})});
     W.alloc((size_t)(3 * nb * nb * prob) * sizeof(double));
     energies = DTensor({std::max<int64_t>(ntrip, 1)});
@@ -1238,11 +1366,15 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
   }
   SCESS_CUDA(cudaMemsetAsync(energies.p(), 0, energies.size() * sizeof(double), s));
   SCESS_CUDA(cudaMemcpyAsync(orbits.as<void>(), ot.data(), ot.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-  std::vector<int> he(o * vp + o2);
-  SCESS_CUDA(cudaMemcpyAsync(he.data(), exps.as<void>(), he.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
-  ctx.sync();  // (ot and he are host vectors of this scope)
-  // Inf or NaN among the operands: the digits hold neither
-  if (std::find(he.begin(), he.end(), kRowNonFinite) != he.end()) return false;
+  std::vector<int> he(nexp + 4);
+  const int *use = exps.as<int>() + nexp;
+  SCESS_CUDA(cudaMemcpyAsync(he.data(), use, he.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+  SCESS_CUDA(cudaMemcpyAsync(hsq.data(), squares.as<void>(), hsq.size() * sizeof(float), cudaMemcpyDeviceToHost, s));
+  ctx.sync();  // (ot, he and hsq are host vectors of this scope)
+  int mx[4];
+  std::copy(he.end() - 4, he.end(), mx);
+  he.resize(nexp);
+  if (!triples_slices_hold(he, mx, hsq, o, v, nA, o2)) return false;
   const int64_t p1 = o | 1, p2 = (p1 * o) | 1;
   const unsigned threads = (unsigned)std::min<int64_t>(256, round_up(norbits, 32));
   const size_t smem = (size_t)std::max<int64_t>(p2 * o + 3 * p1 * o + 4 * o, threads) * 8;
@@ -1263,8 +1395,8 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
     ps.seg[q].mapB = mB[q];
     ps.seg[q].Kpad = q < 2 ? pP.Kpad : pTx.Kpad;
   }
-  ps.expA = exps.as<int>();
-  ps.expB = ps.expA + o * vp;
+  ps.expA = use;
+  ps.expB = use + 2 * nA;
   ps.C = W.d();
   for (int g = 0; g < 3; g++) {
     ps.cy[g] = prob;
