@@ -647,18 +647,26 @@ bool RccsdState::inputs_symmetric() {
   const int64_t o = B_.o, v = B_.v;
   cudaStream_t s = ctx_.stream;
   double *d = ctx_.dscalars;
-  SCESS_CUDA(cudaMemsetAsync(d, 0, 6 * sizeof(double), s));
-  pair_asymmetry(amp_.p() + n1_, {{o, o, v, v}}, {{1, o, o * o, o * o * v}}, d, s);
-  if (drv_.p()) pair_asymmetry(drv_.p(), {{o, o, v, v}}, {{1, o, o * o, o * o * v}}, d + 2, s);
-  if (eri_.p()) {  // (a DF state's <ab|cd> is symmetric as it is formed)
-    const int64_t *st = B_.vvvv.str;
-    pair_asymmetry(B_.vvvv.p, {{v, v, v, v}}, {{st[0], st[1], st[2], st[3]}}, d + 4, s);
+  // t2 and what enters it outside the symmetrised terms (the driver, <ij|ab>, Woooo from <kl|ij>
+  // and <kl|cd>: else t2 loses the symmetry in the first iteration), and <ab|cd>
+  int n = 0;
+  auto check = [&](const double *p, int64_t a, int64_t b, const int64_t *st) {
+    pair_asymmetry(p, {{a, a, b, b}}, {{st[0], st[1], st[2], st[3]}}, d + 2 * n++, s);
+  };
+  SCESS_CUDA(cudaMemsetAsync(d, 0, 10 * sizeof(double), s));
+  const int64_t st2[4] = {1, o, o * o, o * o * v};
+  check(amp_.p() + n1_, o, v, st2);
+  if (drv_.p()) check(drv_.p(), o, v, st2);
+  if (eri_.p()) {  // (a DF state's integrals are symmetric as they are formed)
+    check(B_.vvvv.p, v, v, B_.vvvv.str);
+    check(B_.oovv_phys.p, o, v, B_.oovv_phys.str);
+    check(B_.oooo.p, o, o, B_.oooo.str);
   }
-  SCESS_CUDA(cudaMemcpyAsync(ctx_.hscalars, d, 6 * sizeof(double), cudaMemcpyDeviceToHost, s));
+  SCESS_CUDA(cudaMemcpyAsync(ctx_.hscalars, d, 2 * n * sizeof(double), cudaMemcpyDeviceToHost, s));
   ctx_.sync();
   const double *h = ctx_.hscalars;
   // rounding of a solver's own amplitudes, no more
-  for (int q = 0; q < 3; q++)
+  for (int q = 0; q < n; q++)
     if (!(h[2 * q] <= 16.0 * DBL_EPSILON * h[2 * q + 1])) return false;
   return true;
 }
@@ -687,7 +695,8 @@ bool RccsdState::iterate(int max_steps, const Control &ctl) {
       rccsd_residual(ctx_, B_, amp_.p(), drv_.p(), Backend::MIXED, w_, R_.p());       // :350
     } else if (ph == Phase::FP64) {
       // the reassociated list has a quarter of the ladder's FLOPs and forms no v^4
-      // intermediate, but takes t2(ijab) = t2(jiba) and <ab|cd> = <ba|dc> for granted
+      // intermediate, but takes t2(ijab) = t2(jiba) and <ab|cd> = <ba|dc> for granted in every
+      // iteration
       if (symmetric_ < 0) symmetric_ = inputs_symmetric() ? 1 : 0;
       if (!symmetric_ && !w_.Wvvvv.p()) w_.Wvvvv = DTensor({v, v, v, v});
       rccsd_residual(ctx_, B_, amp_.p(), drv_.p(), Backend::FP64, w_, R_.p(),

@@ -123,7 +123,8 @@ class RccsdState {
   int64_t nmo() const { return B_.N; }
 
  private:
-  bool inputs_symmetric();  // t2 and the driver under (ia <-> jb), <ab|cd> under (ac <-> bd)
+  // t2 stays symmetric under (ia <-> jb): amplitudes, driver, <ij|ab>, <kl|ij>; and <ab|cd>
+  bool inputs_symmetric();
   void reset_history();
   void init(const SolveInput &in, const scess_rccsd_options &opts);
   Ctx &ctx_;
