@@ -134,7 +134,7 @@ int64_t scess_ctx_memory_held(const scess_ctx *ctx);
 
 /* Diagnostics of the tensor-core kernels' failure path (no counterpart in the
  * reference).  Every pipeline wait inside those kernels is bounded; this arms
- * the NEXT tensor-core launch of the context with a bound of `wait_cycles` GPU
+ * the NEXT tensor-core launch of the context (mixed or FP64 form) with a bound of `wait_cycles` GPU
  * clock cycles (2^16 .. 2^40; production launches use ~2^32) and makes its
  * copy thread leave the first operand stage unfilled, so that the MMA
  * thread's wait on it runs out.  The kernel then records the expiry, lets the

@@ -251,7 +251,7 @@ int64_t scess_ctx_memory_held(const scess_ctx *ctx) {
 
 int scess_ctx_arm_wait_expiry(scess_ctx *ctx, int64_t wait_cycles) {
   if (wait_cycles < (int64_t(1) << 16) || wait_cycles > (int64_t(1) << 40)) return SCESS_ERR_INVALID;
-  return guard(ctx, [&](scess::Ctx &c) { c.tensor_cores().arm_wait_expiry(wait_cycles); });
+  return guard(ctx, [&](scess::Ctx &c) { c.wait_diag = {wait_cycles, true}; });
 }
 
 int scess_ctx_set_callbacks(scess_ctx *ctx, scess_cancel_fn cancel, scess_log_fn log, void *user) {

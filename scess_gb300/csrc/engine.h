@@ -223,6 +223,14 @@ struct TimedScope {
   }
 };
 
+// Bounds of the tensor-core kernels' pipeline waits.  The defaults are the production
+// ones; the diagnostics entry point arms a short bound and a withheld first
+// stage for one launch, to exercise the expiry path.
+struct WaitDiag {
+  long long wait_cycles = 1ll << 32;
+  bool withhold_first = false;
+};
+
 struct Ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -256,6 +264,12 @@ struct Ctx {
   void logf(int level, const char *fmt, ...) const;
   TcEngine &tensor_cores();
   SliceEngine &slice_engine();
+  WaitDiag wait_diag;  // of the next tensor-core launch (either engine's)
+  WaitDiag take_wait_diag() {
+    const WaitDiag d = wait_diag;
+    wait_diag = WaitDiag();
+    return d;
+  }
 };
 
 // C = alpha A.B + beta C in FP64 through the tables of g: small products on the

@@ -119,6 +119,7 @@ struct SliceArgs {
   int64_t part_stride;
   unsigned *err;
   long long wait_cycles;
+  int withhold_first;
 };
 
 // T += i 2^(9 (4 - D)) for the drained S_D = i 2^(-9 D) of one K block: |i| is at most
@@ -183,6 +184,20 @@ __device__ __forceinline__ bool slice_left(float sum, RangeRow a, RangeRow b) {
   if (a.sq < 0.0f || b.sq < 0.0f) return true;
   const float q = fminf(a.sq, b.count) + fminf(b.sq, a.count) + 0x1p-13f * fminf(a.count, b.count);
   return sum != 0.0f && sum * sum < 0x1p-14f * q;
+}
+
+// Whether any of the barrier's 128 threads says so (all of them wait for one another).
+__device__ __forceinline__ bool group_any(int bar, bool x) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.or.pred q, %2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"((uint32_t)x), "r"(bar)
+      : "memory");
+  return r != 0;
 }
 
 // What bounds it: long K, the drains (above); short K, the outputs (about 45 instructions each).
@@ -270,6 +285,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       uint32_t ph = 0;          // stage and its phase
       int used = 0;             // stages filled at least once
       uint32_t lastph = 0;      // phases of their last fills, a bit each
+      bool withhold = a.withhold_first;  // diagnostics: the first stage is taken but never filled
       bool ok = true;
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
         int tm, tn, py, pz, pg, kb0, kb1, sp;
@@ -283,6 +299,11 @@ __global__ void __launch_bounds__(THREADS, 1)
           const SegArgs &S = a.seg[0];
           const int n = min(kSlices, kb1 - kb), x = kSlices * S.kpad + kb * BK;
           if (!mbar_wait(&ctl.empty[s], ph ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) { ok = false; break; }
+          if (withhold) {
+            withhold = false;
+            s++;
+            continue;
+          }
           uint8_t *st = smem + s * stage_bytes;
           mbar_expect_tx(&ctl.full[s], n * (A_SLICE + bslice));
           for (int p = 0; p < n; p++) {
@@ -304,6 +325,11 @@ __global__ void __launch_bounds__(THREADS, 1)
           const int ya = (int)(S.rowA0[pg] + py * S.rowAy[pg] + pz * S.rowAz[pg]) + tm * BM;
           const int yb = (int)(S.rowB0[pg] + py * S.rowBy[pg] + pz * S.rowBz[pg]) + tn * bn;
           if (!mbar_wait(&ctl.empty[s], ph ^ 1u, a.err, ERR_EMPTY_WAIT, a.wait_cycles)) { ok = false; break; }
+          if (withhold) {
+            withhold = false;
+            s++;
+            continue;
+          }
           uint8_t *st = smem + s * stage_bytes;
           mbar_expect_tx(&ctl.full[s], kSlices * (A_SLICE + bslice));
 #pragma unroll
@@ -453,6 +479,10 @@ __global__ void __launch_bounds__(THREADS, 1)
     int c = 0, w = 0;
     bool ok = true;
     const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)h0;
+    // (one answer for a warp: what follows a wait is done by all its lanes or by none)
+    auto wait = [&](uint64_t *barrier, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait(barrier, parity, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) != 0;
+    };
     for (int u = blockIdx.x; u < units && ok; u += gridDim.x, w++) {
       int tm, tn, py, pz, pg, kb0, kb1, sp;
       unit_coords(u, tm, tn, py, pz, pg, kb0, kb1, sp);
@@ -483,7 +513,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         const int n0 = tn * bn + h0, nv = min(hc, a.N - n0);  // columns inside the product
         const RangeRow ra = range_row(a.expA, a.rowsA, m, a.sq_unit);
         const RangeRow rb = range_row(a.expB, lane < nv ? a.rowsB : 0, n0 + lane, a.sq_unit);  // lane's column
-        ok = mbar_wait(&ctl.tfull[b], (uint32_t)f & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles);
+        ok = wait(&ctl.tfull[b], (uint32_t)f & 1u);
         if (ok) {
           c++;
           tc_fence_after();
@@ -534,7 +564,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       auto take = [&](auto diag) -> bool {
         constexpr int D = decltype(diag)::value;
         const int b = c % NROT;
-        if (!mbar_wait(&ctl.tfull[b], (uint32_t)(c / NROT) & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) return false;
+        if (!wait(&ctl.tfull[b], (uint32_t)(c / NROT) & 1u)) return false;
         tc_fence_after();
         const uint32_t t0 = tl + (uint32_t)(b * bn);
         // (8 columns a load: the sums take most of the registers)
@@ -555,7 +585,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int kb = kb0; kb < kb1 && ok; kb++) {
         if constexpr (JOINT) {
           const int set = nset == 2 ? c & 1 : 0;
-          ok = mbar_wait(&ctl.tfull[set], (uint32_t)(nset == 2 ? c >> 1 : c) & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles);
+          ok = wait(&ctl.tfull[set], (uint32_t)(nset == 2 ? c >> 1 : c) & 1u);
           if (!ok) break;
           c++;
           tc_fence_after();
@@ -586,9 +616,10 @@ __global__ void __launch_bounds__(THREADS, 1)
           if (!ok) break;
         }
       }
-      if (ok && !mbar_wait(&ctl.tfull[TAIL], (uint32_t)w & 1u, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) ok = false;
-      asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");  // column tables of this unit written
-      if (!ok || errv) break;
+      if (ok && !wait(&ctl.tfull[TAIL], (uint32_t)w & 1u)) ok = false;
+      // Column tables of this unit written.  The group's four warps leave together or not at all:
+      // one that left alone would be missed at the next unit's barrier, which has no bound.
+      if (group_any(bar, !ok || errv)) break;
       tc_fence_after();
       const double mul = a.alpha;
       const bool scaled = !a.partial && !a.alpha_pow2;
@@ -1297,7 +1328,9 @@ void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial)
   if (a.est && (start > 1 || ps.nseg > 1)) throw Error(SCESS_ERR_INVALID, "slice gemm: estimates of one problem");
   if (a.splits > 1 && (!partial || !a.est || start > 1)) throw Error(SCESS_ERR_INVALID, "slice gemm: split-K");
   a.err = err_.as<unsigned>();
-  a.wait_cycles = 1ll << 32;
+  const WaitDiag diag = ctx_.take_wait_diag();
+  a.wait_cycles = diag.wait_cycles;
+  a.withhold_first = diag.withhold_first ? 1 : 0;
   SliceMaps maps;
   for (int i = 0; i < 6; i++) maps.m[i] = ps.maps[std::min(i, ps.nmaps - 1)];
   const int64_t units = (int64_t)a.tiles_m * a.tiles_n * start * a.splits;

@@ -1045,7 +1045,7 @@ bool TcEngine::pair_available() { return kernel_setup().pair_ok; }
 
 void tc_gemm_launch_grouped(const TcProblemSet &ps, TcFormat fmt, const TcOut &out, int nseg,
                             int splits, float *partial, unsigned *err, cudaStream_t stream,
-                            const TcWaitDiag &diag) {
+                            const WaitDiag &diag) {
   const KernelSetup &ks = kernel_setup();
   const bool wide_ok = ks.wide_ok, pair_ok = ks.pair_ok;
   const int pair_clusters = ks.pair_clusters;
@@ -1186,7 +1186,7 @@ void tc_gemm_launch_grouped(const TcProblemSet &ps, TcFormat fmt, const TcOut &o
 void tc_gemm_launch_maps(const CUtensorMap &ma, const CUtensorMap &mb, int64_t Kpad, int64_t rowA0,
                          int64_t M, int64_t rowB0, int64_t N, int bn, TcFormat fmt,
                          const TcOut &out, int nseg, int splits, float *partial, unsigned *err,
-                         cudaStream_t stream, const TcWaitDiag &diag) {
+                         cudaStream_t stream, const WaitDiag &diag) {
   (void)bn;
   TcProblemSet ps;
   ps.maps[0] = ma;
@@ -1208,13 +1208,7 @@ void TcEngine::gemm_maps(const CUtensorMap &ma, const CUtensorMap &mb, int64_t K
                          int nseg, cudaStream_t stream) {
   TimedScope ts(ctx_.timer, "tc_gemm", 2.0 * M * N * Kreal, 0.0, stream ? stream : ctx_.stream);
   tc_gemm_launch_maps(ma, mb, Kpad, rowA0, M, rowB0, N, tile_n(N), fmt_, out, nseg, 1, nullptr,
-                      err_.as<unsigned>(), stream ? stream : ctx_.stream, take_diag());
-}
-
-TcWaitDiag TcEngine::take_diag() {
-  TcWaitDiag d = diag_;
-  diag_ = TcWaitDiag();  // one launch only
-  return d;
+                      err_.as<unsigned>(), stream ? stream : ctx_.stream, ctx_.take_wait_diag());
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1232,7 +1226,7 @@ void TcEngine::gemm_grouped(const TcProblemSet &ps, const TcOut &out, double flo
                             const char *name, cudaStream_t stream) {
   TimedScope ts(ctx_.timer, name, flops, 0.0, stream ? stream : ctx_.stream);
   tc_gemm_launch_grouped(ps, fmt_, out, 3, 1, nullptr, err_.as<unsigned>(),
-                         stream ? stream : ctx_.stream, take_diag());
+                         stream ? stream : ctx_.stream, ctx_.take_wait_diag());
 }
 
 // GB300's FP64 units run the table GEMM at ~1 TFLOP/s for large tiles and at a
@@ -1432,7 +1426,7 @@ void TcEngine::gemm(const Packed &A, int64_t rowA0, int64_t M, const Packed &B, 
   const int bn = tile_n(N);
   const CUtensorMap ma = map_of(A, TC_BM), mb = map_of(B, bn);
   tc_gemm_launch_maps(ma, mb, A.Kpad, rowA0, M, rowB0, N, bn, fmt_, o, nseg, splits, partial,
-                      err_.as<unsigned>(), ctx_.stream, take_diag());
+                      err_.as<unsigned>(), ctx_.stream, ctx_.take_wait_diag());
 }
 
 std::unique_ptr<Packed> TcEngine::take_spare(size_t bytes) {

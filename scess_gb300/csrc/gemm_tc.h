@@ -103,14 +103,6 @@ struct TcProblemSet {
   bool pdl = false;
 };
 
-// Bounds of the kernels' pipeline waits.  The defaults are the production
-// ones; the diagnostics entry point arms a short bound and a withheld first
-// stage for one launch, to exercise the expiry path.
-struct TcWaitDiag {
-  long long wait_cycles = 1ll << 32;
-  bool withhold_first = false;
-};
-
 class TcEngine {
  public:
   explicit TcEngine(Ctx &ctx);
@@ -175,12 +167,6 @@ class TcEngine {
                  int nseg = 3, cudaStream_t stream = nullptr);
   // Device error word set by bounded waits inside the kernels (0 = fine).
   void check_error();
-  // The next launch bounds its waits by wait_cycles and withholds its first
-  // operand stage (its MMA thread's wait then runs out).
-  void arm_wait_expiry(long long wait_cycles) {
-    diag_.wait_cycles = wait_cycles;
-    diag_.withhold_first = true;
-  }
   // Cached packings of constant operands are keyed by device pointer and
   // tagged with the owner that keeps those pointers alive: a resident
   // RccsdState (its address) or 0 for a single C-ABI call.  clear_cache(owner)
@@ -223,17 +209,15 @@ class TcEngine {
   DevMem hint_words_;  // one max word per hint slot
   DevMem partial_;
   DevMem err_;
-  TcWaitDiag diag_;
-  TcWaitDiag take_diag();
 };
 
 // Raw launchers.
 void tc_gemm_launch_grouped(const TcProblemSet &ps, TcFormat fmt, const TcOut &out, int nseg,
                             int splits, float *partial, unsigned *err, cudaStream_t stream,
-                            const TcWaitDiag &diag = TcWaitDiag());
+                            const WaitDiag &diag = WaitDiag());
 void tc_gemm_launch_maps(const CUtensorMap &ma, const CUtensorMap &mb, int64_t Kpad, int64_t rowA0,
                          int64_t M, int64_t rowB0, int64_t N, int bn, TcFormat fmt,
                          const TcOut &out, int nseg, int splits, float *partial, unsigned *err,
-                         cudaStream_t stream, const TcWaitDiag &diag = TcWaitDiag());
+                         cudaStream_t stream, const WaitDiag &diag = WaitDiag());
 
 }  // namespace scess
