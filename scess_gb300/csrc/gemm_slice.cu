@@ -186,20 +186,6 @@ __device__ __forceinline__ bool slice_left(float sum, RangeRow a, RangeRow b) {
   return sum != 0.0f && sum * sum < 0x1p-14f * q;
 }
 
-// Whether any of the barrier's 128 threads says so (all of them wait for one another).
-__device__ __forceinline__ bool group_any(int bar, bool x) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.or.pred q, %2, 128, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}\n"
-      : "=r"(r)
-      : "r"((uint32_t)x), "r"(bar)
-      : "memory");
-  return r != 0;
-}
-
 // What bounds it: long K, the drains (above); short K, the outputs (about 45 instructions each).
 template <bool JOINT>
 __global__ void __launch_bounds__(THREADS, 1)

@@ -461,6 +461,10 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
     const int et = threadIdx.x - 32 * SH::EPI0 - 128 * h;  // 0..127 within the half
     const int bar = 1 + h;                                // named barrier of the half
     int64_t *colH = colOff + HC * h;
+    // (one answer for a warp: what follows a wait is done by all its lanes or by none)
+    auto wait = [&](uint64_t *barrier, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait(barrier, parity, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) != 0;
+    };
     int c = 0;
     bool ok = true;
     for (int it = 0; it * nwork < units && ok; it++) {
@@ -508,7 +512,7 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
         for (int kb = kb0; kb < kb1; kb += a.kbd, c++) {
           const int b = c % NBUF;
           const uint32_t bph = (uint32_t)(c / NBUF) & 1u;
-          if (!mbar_wait(&tfull[b], bph, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) { ok = false; break; }
+          if (!wait(&tfull[b], bph)) { ok = false; break; }
           tc_fence_after();
           const uint32_t t0 = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(b * BN + HC * h);
           // acc[64 L + 4 j + e]: lane 32 q + 16 L + 8 (e / 2) + lane / 4,
@@ -534,7 +538,7 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
         for (int kb = kb0; kb < kb1; kb += a.kbd, c++) {
           const int b = c % NBUF;
           const uint32_t bph = (uint32_t)(c / NBUF) & 1u;
-          if (!mbar_wait(&tfull[b], bph, a.err, ERR_ACCUM_WAIT, a.wait_cycles)) { ok = false; break; }
+          if (!wait(&tfull[b], bph)) { ok = false; break; }
           tc_fence_after();
           const uint32_t t0 = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(b * BN + HC * h);
 #pragma unroll
@@ -556,8 +560,9 @@ __global__ void __launch_bounds__(TcShape<BN, BK, PAIR>::THREADS, 1)
           }
         }
       }
-      asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");  // colOff of this unit written
-      if (!ok || errv) break;
+      // colOff of this unit written; the half's four warps leave together or not at all (one that
+      // left alone would be missed at the next unit's barrier, which has no bound)
+      if (group_any(bar, !ok || errv)) break;
       if (pc) {
         float *C = (float *)out.C;
         const float fa = s_falpha;

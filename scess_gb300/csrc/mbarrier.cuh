@@ -62,4 +62,18 @@ __device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity) {
     if (clock64() - t0 > (1ll << 32)) return;
 }
 
+// Whether any of the barrier's 128 threads says so (all of them wait for one another).
+__device__ __forceinline__ bool group_any(int bar, bool x) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.or.pred q, %2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"((uint32_t)x), "r"(bar)
+      : "memory");
+  return r != 0;
+}
+
 }  // namespace scess
