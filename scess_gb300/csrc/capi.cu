@@ -495,9 +495,9 @@ int scess_rccsd_state_iterate(scess_rccsd_state *state, int32_t n_iterations,
     ctl.time_limit_s = state->impl->options().time_limit_s;
     struct Reset {
       scess::Ctx &c;
-      ~Reset() {
-        c.tensor_cores().set_cache_owner(nullptr);
-        c.slice_engine().set_cache_owner(nullptr);
+      ~Reset() {  // (an engine whose construction has failed is not there)
+        if (c.tc) c.tc->set_cache_owner(nullptr);
+        if (c.slices) c.slices->set_cache_owner(nullptr);
       }
     } reset{c};
     c.tensor_cores().set_cache_owner(state->impl);
