@@ -501,7 +501,7 @@ int scess_rccsd_state_iterate(scess_rccsd_state *state, int32_t n_iterations,
       }
     } reset{c};
     c.tensor_cores().set_cache_owner(state->impl);
-    c.slice_engine().set_cache_owner(state->impl);
+    if (scess::SliceEngine *e = c.slice_engine()) e->set_cache_owner(state->impl);
     state->impl->iterate(n_iterations, ctl);
     if (result) *result = state->impl->result();
     if (device_ms) *device_ms = state->impl->last_device_ms();

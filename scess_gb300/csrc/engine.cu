@@ -240,9 +240,15 @@ TcEngine &Ctx::tensor_cores() {
   return *tc;
 }
 
-SliceEngine &Ctx::slice_engine() {
-  if (!slices) slices = std::make_unique<SliceEngine>(*this);
-  return *slices;
+SliceEngine *Ctx::slice_engine() {
+  if (!slices) {
+    try {
+      slices = std::make_unique<SliceEngine>(*this);
+    } catch (const Error &e) {
+      if (e.code != SCESS_ERR_OOM) throw;
+    }
+  }
+  return slices.get();
 }
 
 void HostPages::start(double *p, int64_t n) {
@@ -571,13 +577,15 @@ const EinsumPlan &plan_einsum(Ctx &ctx, const char *spec, const TV &A, const TV 
 }
 
 namespace {
-// Whether the sliced form is usable and faster than the FP64 units (estimates of both;
-// tuning key f64: 1 = sliced, 2 = FP64 units).
-bool prefer_slices(const TableGemm &g) {
+// The slice engine where it is usable and faster than the FP64 units (estimates of both;
+// tuning key f64: 1 = sliced, 2 = FP64 units), else null.
+SliceEngine *slices_for(Ctx &ctx, const TableGemm &g) {
   const int64_t route = tune_value("f64", 0);
-  if (route == 1) return g.K > 0 && SliceEngine::usable(g.M, g.N, g.K);
-  return route != 2 && g.K > 0 && SliceEngine::usable(g.M, g.N, g.K) &&
-         SliceEngine::estimate_us(g.M, g.N, g.K) < std::min(dgemm_small_us(g), skinny64_us(g));
+  if (g.K <= 0 || route == 2) return nullptr;
+  if (route != 1 && SliceEngine::estimate_us(g.M, g.N, g.K) >= std::min(dgemm_small_us(g), skinny64_us(g)))
+    return nullptr;
+  SliceEngine *e = ctx.slice_engine();
+  return e && e->usable(g.M, g.N, g.K) ? e : nullptr;
 }
 
 // C = alpha A.B + beta C on the FP64 units: short K against a long side, or cut finely
@@ -679,15 +687,14 @@ void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, 
     dgemv_table(h, ctx.stream);
     return;
   }
-  if (prefer_slices(g) &&
-      ctx.slice_engine().contract(pl, alpha, A.p, B.p, beta, C.p, constA, constB))
-    return;
+  if (SliceEngine *e = slices_for(ctx, g))
+    if (e->contract(pl, alpha, A.p, B.p, beta, C.p, constA, constB)) return;
   dfma_gemm(ctx, g, pl.cUnitM, pl.cUnitN);
 }
 
 void fp64_table_gemm(Ctx &ctx, const TableGemm &g, const char *name) {
-  if (prefer_slices(g) && ctx.slice_engine().table_gemm(g, name))
-    return;
+  if (SliceEngine *e = slices_for(ctx, g))
+    if (e->table_gemm(g, name)) return;
   dfma_gemm(ctx, g, false, false);
 }
 

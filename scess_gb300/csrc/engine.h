@@ -263,7 +263,7 @@ struct Ctx {
   double *ensure_workspace(int64_t doubles);
   void logf(int level, const char *fmt, ...) const;
   TcEngine &tensor_cores();
-  SliceEngine &slice_engine();
+  SliceEngine *slice_engine();  // null: no room for it
   WaitDiag wait_diag;  // of the next tensor-core launch (either engine's)
   WaitDiag take_wait_diag() {
     const WaitDiag d = wait_diag;

@@ -1028,26 +1028,18 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// The kernel's setmaxnreg split assumes it is launched with exactly kLaunchRegs
-// registers a thread.
-bool kernel_ok() {
-  static bool ok = false;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    auto fits = [](void (*kernel)(SliceMaps, SliceArgs)) {
-      cudaFuncAttributes fa;
-      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES) == cudaSuccess &&
-             cudaFuncGetAttributes(&fa, kernel) == cudaSuccess && fa.numRegs == kLaunchRegs;
-    };
-    ok = fits(slice_gemm_kernel<false>) && fits(slice_gemm_kernel<true>);
-    cudaGetLastError();
-  });
-  return ok;
-}
-
 }  // namespace
 
+// The kernel's setmaxnreg split assumes it is launched with exactly kLaunchRegs registers a
+// thread; its shared memory is an attribute of each device's copy of it.
 SliceEngine::SliceEngine(Ctx &ctx) : ctx_(ctx) {
+  auto fits = [](void (*kernel)(SliceMaps, SliceArgs)) {
+    cudaFuncAttributes fa;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES) == cudaSuccess &&
+           cudaFuncGetAttributes(&fa, kernel) == cudaSuccess && fa.numRegs == kLaunchRegs;
+  };
+  kernel_ok_ = fits(slice_gemm_kernel<false>) && fits(slice_gemm_kernel<true>);
+  cudaGetLastError();
   err_.alloc(sizeof(unsigned) * 4);
   SCESS_CUDA(cudaMemsetAsync(err_.as<void>(), 0, sizeof(unsigned) * 4, ctx_.stream));
 }
@@ -1107,8 +1099,8 @@ double SliceEngine::estimate_us(int64_t M, int64_t N, int64_t K) {
   return 14.0 + (double)(M + N) * (double)K * 22.0 / 2.9e6 + plan_us(M, N, round_up(std::max<int64_t>(K, 1), BK), z);
 }
 
-bool SliceEngine::usable(int64_t M, int64_t N, int64_t K) {
-  return kernel_ok() && M <= INT32_MAX / 2 && N <= INT32_MAX / 2 && K < (int64_t(1) << 26);
+bool SliceEngine::usable(int64_t M, int64_t N, int64_t K) const {
+  return kernel_ok_ && M <= INT32_MAX / 2 && N <= INT32_MAX / 2 && K < (int64_t(1) << 26);
 }
 
 CUtensorMap SliceEngine::map_of(const SlicedPack &p, int box_rows) {
@@ -1226,7 +1218,7 @@ void SliceEngine::pack(const Gather *g, SlicedPack *const *out, int n) {
 }
 
 void SliceEngine::launch(const SliceProblemSet &ps, int splits, double *partial) {
-  if (!kernel_ok()) throw Error(SCESS_ERR_UNSUPPORTED, "slice gemm: kernel unavailable");
+  if (!kernel_ok_) throw Error(SCESS_ERR_UNSUPPORTED, "slice gemm: kernel unavailable");
   if (ps.M <= 0 || ps.N <= 0 || ps.ny <= 0 || ps.nz <= 0 || ps.ng <= 0) return;
   if (ps.ng > 3 || ps.nseg < 1 || ps.nseg > 4) throw Error(SCESS_ERR_INVALID, "slice gemm: groups or segments");
   SliceArgs a;

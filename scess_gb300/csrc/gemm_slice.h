@@ -93,7 +93,7 @@ class SliceEngine {
  public:
   explicit SliceEngine(Ctx &ctx);
   // The device runs the kernel and the sizes are within its coordinates.
-  static bool usable(int64_t M, int64_t N, int64_t K);
+  bool usable(int64_t M, int64_t N, int64_t K) const;
   // Estimated time of a product with its packs, in us.
   static double estimate_us(int64_t M, int64_t N, int64_t K);
   // C = alpha A.B + beta C through the tables of g (the FP64 engine's GEMM).
@@ -166,7 +166,7 @@ class SliceEngine {
   const void *owner_ = nullptr;
   SlicedPack tmpA_, tmpB_;
   DevMem err_, partial_, left_;
-  bool launched_ = false, busy_ = false;
+  bool launched_ = false, busy_ = false, kernel_ok_ = false;
 };
 
 }  // namespace scess

@@ -218,15 +218,15 @@ struct MaxHints {
   SliceEngine *slices = nullptr;  // FP64: packs of the tensors shared between einsums
   MaxHints(Ctx &ctx, Backend be) {
     if (be != Backend::FP64) tc = &ctx.tensor_cores();
-    else slices = &ctx.slice_engine();
+    else slices = ctx.slice_engine();
   }
   void add(const double *p, int64_t n) {
     if (tc) tc->add_max_hint(p, n);
-    else slices->add_stable(p);
+    else if (slices) slices->add_stable(p);
   }
   ~MaxHints() {
     if (tc) tc->clear_max_hints();
-    else slices->clear_stable();
+    else if (slices) slices->clear_stable();
   }
   MaxHints(const MaxHints &) = delete;
   MaxHints &operator=(const MaxHints &) = delete;

@@ -1277,7 +1277,7 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
   const int nb = choose_nb_sliced(o, v);
   const int64_t NB = ceil_div(v, nb), vp = NB * nb;
   const int64_t Mg = o * nb, Ng = o2, prob = Mg * Ng;
-  if (!SliceEngine::usable(o * vp * vp, o2 * vp, v)) return false;
+  if (!ctx.slice_engine() || !ctx.slice_engine()->usable(o * vp * vp, o2 * vp, v)) return false;
   const int64_t ntrip = v * (v + 1) * (v + 2) / 6;
   TriplesSetup T;
   T.o = o;
@@ -1286,7 +1286,7 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
   T.nb = nb;
   T.NB = NB;
   T.vp = vp;
-  SliceEngine &se = ctx.slice_engine();
+  SliceEngine &se = *ctx.slice_engine();
   SlicedPack pP, pQ, pQ2, pR, pR2, pTx;
   DevTables pdt, gdt;
   DevMem exps, squares, W, orbits;
