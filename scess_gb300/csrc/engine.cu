@@ -578,11 +578,12 @@ const EinsumPlan &plan_einsum(Ctx &ctx, const char *spec, const TV &A, const TV 
 
 namespace {
 // The slice engine where it is usable and faster than the FP64 units (estimates of both;
-// tuning key f64: 1 = sliced, 2 = FP64 units), else null.
-SliceEngine *slices_for(Ctx &ctx, const TableGemm &g) {
+// tuning key f64: 1 = sliced, 2 = FP64 units), else null.  cUnitM, cUnitN: C's unit stride, if known.
+SliceEngine *slices_for(Ctx &ctx, const TableGemm &g, bool cUnitM, bool cUnitN) {
   const int64_t route = tune_value("f64", 0);
   if (g.K <= 0 || route == 2) return nullptr;
-  if (route != 1 && SliceEngine::estimate_us(g.M, g.N, g.K) >= std::min(dgemm_small_us(g), skinny64_us(g)))
+  if (route != 1 && SliceEngine::estimate_us(g.M, g.N, g.K, cUnitM, cUnitN) >=
+                        std::min(dgemm_small_us(g), skinny64_us(g)))
     return nullptr;
   SliceEngine *e = ctx.slice_engine();
   return e && e->usable(g.M, g.N, g.K) ? e : nullptr;
@@ -687,13 +688,13 @@ void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, 
     dgemv_table(h, ctx.stream);
     return;
   }
-  if (SliceEngine *e = slices_for(ctx, g))
+  if (SliceEngine *e = slices_for(ctx, g, pl.cUnitM, pl.cUnitN))
     if (e->contract(pl, alpha, A.p, B.p, beta, C.p, constA, constB)) return;
   dfma_gemm(ctx, g, pl.cUnitM, pl.cUnitN);
 }
 
 void fp64_table_gemm(Ctx &ctx, const TableGemm &g, const char *name) {
-  if (SliceEngine *e = slices_for(ctx, g))
+  if (SliceEngine *e = slices_for(ctx, g, false, false))
     if (e->table_gemm(g, name)) return;
   dfma_gemm(ctx, g, false, false);
 }

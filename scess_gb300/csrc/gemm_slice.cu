@@ -1093,10 +1093,12 @@ double plan_us(int64_t M, int64_t N, int64_t Kpad, int64_t &splits) {
 }
 }  // namespace
 
-double SliceEngine::estimate_us(int64_t M, int64_t N, int64_t K) {
+double SliceEngine::estimate_us(int64_t M, int64_t N, int64_t K, bool cUnitM, bool cUnitN) {
   int64_t z = 1;
-  // packs at 2.9 TB/s, 14 us of launches and latencies
-  return 14.0 + (double)(M + N) * (double)K * 22.0 / 2.9e6 + plan_us(M, N, round_up(std::max<int64_t>(K, 1), BK), z);
+  if (exchanges(M, N, cUnitM, cUnitN)) std::swap(M, N);
+  // packs at 2.9 TB/s, 14 us of launches and latencies (6 x 5766 x 1116, either way round: 105
+  // us measured, 94 by this; on the FP64 units 94 and 95)
+  return 14.0 + (double)(M + N) * (double)K * 24.0 / 2.9e6 + plan_us(M, N, round_up(std::max<int64_t>(K, 1), BK), z);
 }
 
 bool SliceEngine::usable(int64_t M, int64_t N, int64_t K) const {
@@ -1424,7 +1426,7 @@ bool SliceEngine::table_gemm(const TableGemm &g, const char *name) {
                           {g.B + g.baseB, g.colB, g.N, g.kB, g.K, !g.bUnitN}};
     SlicedPack *const out[2] = {&tmpA_, &tmpB_};
     pack(ga, out, 2);
-    if (g.M <= 64 && g.M < g.N) product(exchanged(g), tmpB_, tmpA_, name);
+    if (exchanges(g.M, g.N, false, false)) product(exchanged(g), tmpB_, tmpA_, name);
     else product(g, tmpA_, tmpB_, name);
   } catch (const Error &e) {
     if (e.code != SCESS_ERR_OOM) throw;
@@ -1464,9 +1466,7 @@ void SliceEngine::check_error() {
 bool SliceEngine::contract(const EinsumPlan &pl, double alpha, const double *A, const double *B, double beta,
                            double *C, bool constA, bool constB) {
   Busy busy(busy_);
-  // Epilogue lanes walk the GEMM rows: put C's unit-stride index there, unless
-  // that side is short: rows come in tiles of 128, columns in steps of 16.
-  const bool swap = std::min(pl.M, pl.N) <= 64 ? pl.M < pl.N : (!pl.cUnitM && pl.cUnitN);
+  const bool swap = exchanges(pl.M, pl.N, pl.cUnitM, pl.cUnitN);
   const Gather gA{A, pl.d_rowA, pl.M, pl.d_kA, pl.K, pl.aUnitK, pl.aRowStride, pl.aKStride, pl.aRowP, pl.aRowE};
   const Gather gB{B, pl.d_colB, pl.N, pl.d_kB, pl.K, pl.bUnitK, pl.bColStride, pl.bKStride, pl.bColP, pl.bColE};
   Gather todo[2];

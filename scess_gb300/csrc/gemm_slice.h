@@ -34,6 +34,7 @@
 #pragma once
 #include <cuda.h>
 
+#include <algorithm>
 #include <map>
 #include <memory>
 #include <set>
@@ -94,8 +95,14 @@ class SliceEngine {
   explicit SliceEngine(Ctx &ctx);
   // The device runs the kernel and the sizes are within its coordinates.
   bool usable(int64_t M, int64_t N, int64_t K) const;
-  // Estimated time of a product with its packs, in us.
-  static double estimate_us(int64_t M, int64_t N, int64_t K);
+  // Whether an M x N product is launched with its sides exchanged (as N x M): lanes of the
+  // epilogue walk the GEMM rows, so C's unit-stride index (cUnitM, cUnitN, if known) is put there,
+  // unless a side is short: rows come in tiles of 128, columns in steps of 16.
+  static bool exchanges(int64_t M, int64_t N, bool cUnitM, bool cUnitN) {
+    return std::min(M, N) <= 64 ? M < N : (!cUnitM && cUnitN);
+  }
+  // Estimated time of a product with its packs, in us, in the orientation it is launched in.
+  static double estimate_us(int64_t M, int64_t N, int64_t K, bool cUnitM, bool cUnitN);
   // C = alpha A.B + beta C through the tables of g (the FP64 engine's GEMM).
   // False when the packs do not fit into device memory: nothing was launched
   // and the caller uses the DFMA kernel.
