@@ -3,10 +3,6 @@
 #include <cstdarg>
 #include <cstdlib>
 #include <cstring>
-#include <system_error>
-
-#include <sys/mman.h>
-#include <unistd.h>
 
 #include "engine.h"
 #include "gemm_slice.h"
@@ -249,37 +245,6 @@ SliceEngine *Ctx::slice_engine() {
     }
   }
   return slices.get();
-}
-
-void HostPages::start(double *p, int64_t n) {
-#ifdef __linux__
-#ifndef MADV_POPULATE_WRITE
-#define MADV_POPULATE_WRITE 23
-#endif
-  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-  const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + page - 1) / page * page;
-  const uintptr_t e = (reinterpret_cast<uintptr_t>(p) + (size_t)std::max<int64_t>(n, 0) * sizeof(double)) / page * page;
-  if (!p || e <= a || e - a < (size_t(8) << 20)) return;
-  constexpr int kThreads = 4;  // (more contend for the address space's lock)
-  const size_t part = ((e - a) / kThreads + page - 1) / page * page;
-  try {
-    for (int i = 0; i < kThreads; i++) {
-      const uintptr_t b = a + (size_t)i * part;
-      if (b >= e) break;
-      const size_t len = std::min<size_t>(part, e - b);
-      threads_.emplace_back([b, len] { (void)madvise(reinterpret_cast<void *>(b), len, MADV_POPULATE_WRITE); });
-    }
-  } catch (const std::system_error &) {  // no more threads: the copy faults the rest in
-  }
-#else
-  (void)p;
-  (void)n;
-#endif
-}
-
-void HostPages::wait() {
-  for (auto &t : threads_) t.join();
-  threads_.clear();
 }
 
 void upload(Ctx &ctx, double *dst, const double *src, int64_t n) {

@@ -4,10 +4,10 @@
 #include <map>
 #include <memory>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "common.cuh"
+#include "host_pages.h"
 #include "kernels.h"
 
 namespace scess {
@@ -290,26 +290,6 @@ void einsum(Ctx &ctx, const char *spec, double alpha, const TV &A, const TV &B, 
 void permute(Ctx &ctx, const char *spec, double alpha, const TV &X, double beta, const TV &Y);
 
 const EinsumPlan &plan_einsum(Ctx &ctx, const char *spec, const TV &A, const TV &B, const TV &C);
-
-// Page-faults a host output buffer in while the GPU works: a copy into pages that
-// the caller has never touched (a fresh allocation) runs at the speed of the faults,
-// 230 MB in 8.5 ms where the copy alone takes 1.3 (GB300 with Grace, 64 KiB pages);
-// four threads fault the same range in in 2.8 ms.  The contents are not touched
-// (MADV_POPULATE_WRITE); ranges below 8 MiB and systems without it are left alone.
-// The destructor waits for the threads.
-class HostPages {
- public:
-  HostPages() = default;
-  HostPages(double *p, int64_t n) { start(p, n); }
-  ~HostPages() { wait(); }
-  HostPages(const HostPages &) = delete;
-  HostPages &operator=(const HostPages &) = delete;
-  void start(double *p, int64_t n);  // n doubles at p (null: nothing)
-  void wait();
-
- private:
-  std::vector<std::thread> threads_;
-};
 
 // Upload helpers (synchronous w.r.t. the host buffer).
 void upload(Ctx &ctx, double *dst, const double *src, int64_t n);
