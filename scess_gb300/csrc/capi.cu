@@ -53,7 +53,12 @@ int guard(scess_ctx *ctx, F &&f) {
   cudaStreamSynchronize(ctx->impl->stream);
   if (ctx->impl->tc) ctx->impl->tc->clear_cache(nullptr);
   if (ctx->impl->slices) ctx->impl->slices->clear_cache(nullptr);
-  if (code != SCESS_OK) cudaGetLastError();
+  if (code != SCESS_OK) {
+    // a call that failed otherwise may have left the mark of an expired wait behind
+    if (ctx->impl->tc) ctx->impl->tc->clear_error();
+    if (ctx->impl->slices) ctx->impl->slices->clear_error();
+    cudaGetLastError();
+  }
   return code;
 }
 

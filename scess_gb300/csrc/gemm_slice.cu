@@ -1451,6 +1451,11 @@ void SliceEngine::clear_stable() {
   stable_.clear();
 }
 
+void SliceEngine::clear_error() {
+  launched_ = false;
+  cudaMemsetAsync(err_.as<void>(), 0, sizeof(unsigned), ctx_.stream);
+}
+
 void SliceEngine::check_error() {
   if (!launched_) return;
   launched_ = false;
@@ -1520,12 +1525,13 @@ bool SliceEngine::contract(const EinsumPlan &pl, double alpha, const double *A, 
     if (n) pack(todo, out, n);
     if (swap) product(exchanged(g), *pb, *pa, tname.c_str());
     else product(g, *pa, *pb, tname.c_str());
-  } catch (const Error &e) {
+  } catch (const std::exception &x) {
     // packs listed above may not have been made
     reuse_.clear();
     spare_.clear();
     cache_.clear();
-    if (e.code != SCESS_ERR_OOM) throw;
+    const Error *e = dynamic_cast<const Error *>(&x);
+    if (!e || e->code != SCESS_ERR_OOM) throw;
     return false;  // no room for the packs: the DFMA kernel needs none
   }
   return true;

@@ -137,6 +137,7 @@ class SliceEngine {
   void clear_stable();
   // Throws SCESS_ERR_CUDA if a bounded wait of a launch since the last check expired.
   void check_error();
+  void clear_error();
   bool launched() const { return launched_; }
 
  private:

@@ -1470,6 +1470,8 @@ void TcEngine::check_error() {
   }
 }
 
+void TcEngine::clear_error() { cudaMemsetAsync(err_.as<void>(), 0, sizeof(unsigned), ctx_.stream); }
+
 void TcEngine::table_gemm(const TableGemm &g, const char *name) {
   const std::string tname = std::string("tc_gemm[") + name + "]";
   timer_name_ = tname.c_str();

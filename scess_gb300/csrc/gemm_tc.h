@@ -167,6 +167,7 @@ class TcEngine {
                  int nseg = 3, cudaStream_t stream = nullptr);
   // Device error word set by bounded waits inside the kernels (0 = fine).
   void check_error();
+  void clear_error();
   // Cached packings of constant operands are keyed by device pointer and
   // tagged with the owner that keeps those pointers alive: a resident
   // RccsdState (its address) or 0 for a single C-ABI call.  clear_cache(owner)
