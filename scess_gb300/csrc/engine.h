@@ -51,7 +51,8 @@ class BlockCache {
 // every call.  Keys: t_nb (virtual block size of (T), both forms; default: the
 // size chosen from o and v), t_kbd (K blocks of 64 per TMEM drain in the
 // mixed (T) launch: 1, 2 or 4), t_wbuf (W buffers of the mixed (T): 1 or 3) and f64
-// (FP64 products: 1 on the tensor cores' slices, 2 on the FP64 units).
+// (FP64 products: 1 on the tensor cores' slices, 2 on the FP64 units, there with the 12
+// products a block triple of (T)).
 // Returns `def` for an unset key.
 int64_t tune_value(const char *key, int64_t def);
 // TMEM drain cadence of the mixed (T) launch (K blocks of 64 per drain).

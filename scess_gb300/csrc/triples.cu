@@ -1457,7 +1457,7 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
   cudaStream_t s = ctx.stream;
   {
     const int64_t q1 = o | 1, q2 = (q1 * o) | 1;
-    if (!mixed && (q2 * o + 3 * o * o + 4 * o) * 8 <= 200 * 1024 && o <= 255) {  // (else refused below)
+    if (!mixed && tune_value("f64", 0) != 2 && (q2 * o + 3 * o * o + 4 * o) * 8 <= 200 * 1024 && o <= 255) {  // (else refused below)
       double e_t = 0.0;
       if (triples_fp64_sliced(ctx, d_eri, nmo, o, d_eps, d_t1, d_t2, ctl, stats, d_B, naux, e_t)) return e_t;
     }
