@@ -129,6 +129,12 @@ const TV &RccsdBlocks::l_ovoo(Ctx &ctx) const {
   return L_ovoo.v;
 }
 
+void RccsdBlocks::release_reassociated() {
+  ladder.reset();
+  L_ovvv = DTensor();
+  L_ovoo = DTensor();
+}
+
 void RccsdBlocks::build_l(Ctx &ctx) {
   // L_oovv = 2 <ij|ab> - <ij|ba>                                                   :68-69
   L_oovv = DTensor({o, o, v, v});
@@ -698,9 +704,22 @@ bool RccsdState::iterate(int max_steps, const Control &ctl) {
       // intermediate, but takes t2(ijab) = t2(jiba) and <ab|cd> = <ba|dc> for granted in every
       // iteration
       if (symmetric_ < 0) symmetric_ = inputs_symmetric() ? 1 : 0;
-      if (!symmetric_ && !w_.Wvvvv.p()) w_.Wvvvv = DTensor({v, v, v, v});
-      rccsd_residual(ctx_, B_, amp_.p(), drv_.p(), Backend::FP64, w_, R_.p(),
-                     symmetric_ ? ResidualList::REASSOCIATED : ResidualList::LITERAL);
+      bool done = false;
+      if (symmetric_) {
+        try {
+          rccsd_residual(ctx_, B_, amp_.p(), drv_.p(), Backend::FP64, w_, R_.p(), ResidualList::REASSOCIATED);
+          done = true;
+        } catch (const Error &e) {  // its combined integrals don't fit: with few virtuals the literal list may
+          if (e.code != SCESS_ERR_OOM) throw;
+          symmetric_ = 0;
+          if (ctx_.slices) ctx_.slices->reclaim();  // (their packs)
+          B_.release_reassociated();
+        }
+      }
+      if (!done) {
+        if (!w_.Wvvvv.p()) w_.Wvvvv = DTensor({v, v, v, v});
+        rccsd_residual(ctx_, B_, amp_.p(), drv_.p(), Backend::FP64, w_, R_.p(), ResidualList::LITERAL);
+      }
     } else if (ph == Phase::REFINED) {
       // R = R0 + dR(T0, T - T0)
       SCESS_CUDA(cudaMemcpyAsync(damp_.p(), amp_.p(), n_ * sizeof(double), cudaMemcpyDeviceToDevice, s));

@@ -35,6 +35,7 @@ struct RccsdBlocks {
   mutable DTensor L_ovvv, L_ovoo;
   const TV &l_ovvv(Ctx &ctx) const;
   const TV &l_ovoo(Ctx &ctx) const;
+  void release_reassociated();  // the three above, when memory is short
   // views into the device eri (nmo^4)
   void build(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t nocc);
   // from DF factors B (naux x nmo x nmo): only the seven regions of <pq|rs> the
