@@ -1448,21 +1448,12 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
   return true;
 }
 
-}  // namespace
-
-double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, const double *d_eps,
-                     const double *d_t1, const double *d_t2, bool mixed, const Control &ctl,
-                     TriplesStats *stats, const double *d_B, int64_t naux) {
+// (T) with blocks of nb virtuals: the mixed form, or FP64 with 12 products a block triple.
+double triples_blocked(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, const double *d_eps, const double *d_t1,
+                       const double *d_t2, bool mixed, const Control &ctl, TriplesStats *stats, const double *d_B,
+                       int64_t naux, int nb) {
   const int64_t v = nmo - o, N = nmo;
   cudaStream_t s = ctx.stream;
-  {
-    const int64_t q1 = o | 1, q2 = (q1 * o) | 1;
-    if (!mixed && tune_value("f64", 0) != 2 && (q2 * o + 3 * o * o + 4 * o) * 8 <= 200 * 1024 && o <= 255) {  // (else refused below)
-      double e_t = 0.0;
-      if (triples_fp64_sliced(ctx, d_eri, nmo, o, d_eps, d_t1, d_t2, ctl, stats, d_B, naux, e_t)) return e_t;
-    }
-  }
-  const int nb = mixed ? choose_nb_grouped(o, v) : choose_nb(o, v, 8, size_t(128) << 20);
   const int64_t NB = ceil_div(v, nb), vp = NB * nb;
   const int64_t o2 = o * o, o3 = o2 * o;
 
@@ -1747,6 +1738,31 @@ double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, cons
     stats->block_triples = blocks_done;
   }
   return ctx.hscalars[0];
+}
+
+}  // namespace
+
+double rccsd_triples(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, const double *d_eps,
+                     const double *d_t1, const double *d_t2, bool mixed, const Control &ctl,
+                     TriplesStats *stats, const double *d_B, int64_t naux) {
+  const int64_t v = nmo - o;
+  {
+    const int64_t q1 = o | 1, q2 = (q1 * o) | 1;
+    if (!mixed && tune_value("f64", 0) != 2 && (q2 * o + 3 * o * o + 4 * o) * 8 <= 200 * 1024 &&
+        o <= 255) {  // (else refused below)
+      double e_t = 0.0;
+      if (triples_fp64_sliced(ctx, d_eri, nmo, o, d_eps, d_t1, d_t2, ctl, stats, d_B, naux, e_t)) return e_t;
+    }
+  }
+  int nb = mixed ? choose_nb_grouped(o, v) : choose_nb(o, v, 8, size_t(128) << 20);
+  for (;;) {
+    try {
+      return triples_blocked(ctx, d_eri, nmo, o, d_eps, d_t1, d_t2, mixed, ctl, stats, d_B, naux, nb);
+    } catch (const Error &e) {  // W doesn't fit: smaller blocks (unless a size was asked for)
+      if (e.code != SCESS_ERR_OOM || nb == 1 || tune_value("t_nb", 0) >= 1) throw;
+      nb = (nb + 1) / 2;
+    }
+  }
 }
 
 double rccsd_triples_vjp(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o,

@@ -47,3 +47,25 @@ def test_iterations_with_few_virtuals_under_a_cap():
         t1, t2 = oracle.update_amplitudes(ints, eia, eijab, None, t1, t2)
     assert rel_err(got[0], t1) < 1e-12 and rel_err(got[1], t2) < 1e-12
     assert np.all(np.isfinite(got[1]))
+
+
+@pytest.mark.parametrize('precision,tol', [('mixed', 1e-5), ('fp64', 1e-12)])
+def test_triples_under_a_cap_take_smaller_blocks(monkeypatch, precision, tol):
+    o, v = 13, 40
+    w = make_workload(o, v, seed=7, with_amplitudes=True)
+
+    def energy(cap, tune):
+        monkeypatch.setenv('SCESS_TUNE', tune)
+        with s.Context(0) as ctx:
+            ctx.set_memory_limit(cap)
+            try:
+                return ctx.triples(None, w.eps, o, w.t1, w.t2, B=w.B, precision=precision)
+            except cc.ScessError as e:
+                assert e.status == cc.SCESS_ERR_OOM
+                return None
+
+    ample = energy(0, '')
+    small = 'f64=2,t_nb=2'  # (blocks of two virtuals; FP64: the form without packs)
+    cap = next(c for c in range(8 << 20, 1 << 30, 2 << 20) if energy(c, small) is not None)
+    got = energy(cap + (2 << 20), '')
+    assert got is not None and abs(got - ample) <= tol * abs(ample)
