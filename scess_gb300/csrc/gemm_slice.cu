@@ -1382,12 +1382,16 @@ void SliceEngine::product(const TableGemm &g, const SlicedPack &A, const SlicedP
   SCESS_CHECK_LAUNCH();
 }
 
-void SliceEngine::reclaim() {
-  if (busy_) return;
+void SliceEngine::release_workspaces() {
   tmpA_ = SlicedPack();
   tmpB_ = SlicedPack();
   partial_.release();
   left_.release();
+}
+
+void SliceEngine::reclaim() {
+  if (busy_) return;
+  release_workspaces();
   spare_.clear();
   cache_.clear();
 }
@@ -1440,7 +1444,10 @@ void SliceEngine::clear_cache(const void *owner) {
     if (it->first.owner == owner) it = cache_.erase(it);
     else ++it;
   }
-  if (!owner) spare_.clear();  // (the end of an API call)
+  if (owner) return;
+  // the end of an API call: what is kept beyond it is bounded here, the rest by the block cache
+  spare_.clear();
+  if (workspace_bytes() > kKeptBytes) release_workspaces();
 }
 
 void SliceEngine::clear_stable() {

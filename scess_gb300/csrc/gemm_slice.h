@@ -135,10 +135,10 @@ class SliceEngine {
   // through equal tables share one pack.
   void add_stable(const double *p) { stable_.insert(p); }
   void clear_stable();
+  int64_t workspace_bytes() const { return (int64_t)(tmpA_.mem.bytes() + tmpB_.mem.bytes() + partial_.bytes() + left_.bytes()); }
   // Throws SCESS_ERR_CUDA if a bounded wait of a launch since the last check expired.
   void check_error();
   void clear_error();
-  bool launched() const { return launched_; }
 
  private:
   struct Gather {  // an operand seen through its tables
@@ -172,6 +172,9 @@ class SliceEngine {
   std::vector<std::unique_ptr<SlicedPack>> spare_;  // packs of stable tensors, done with
   std::set<const double *> stable_;
   const void *owner_ = nullptr;
+  // Workspaces of products: kept between calls up to this size.
+  static constexpr int64_t kKeptBytes = int64_t(256) << 20;
+  void release_workspaces();
   SlicedPack tmpA_, tmpB_;
   DevMem err_, partial_, left_;
   bool launched_ = false, busy_ = false, kernel_ok_ = false;
