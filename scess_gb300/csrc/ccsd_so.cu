@@ -273,14 +273,12 @@ SoResult so_ccsd(Ctx &ctx, const double *d_g, const double *d_eps, int64_t nmo, 
 
   // DIIS subspace (CCSD-DIIS.cpp:73-80): amplitudes and errors, oldest first
   const int slots = kMaxDiis + 1;
-  DevMem vamp, verr, vptr, vcoef;
+  DevMem vamp, verr;
   std::deque<int> order;
   std::vector<std::vector<double>> gram;
   if (diis) {
     vamp.alloc((size_t)slots * n * sizeof(double));
     verr.alloc((size_t)slots * n * sizeof(double));
-    vptr.alloc(slots * sizeof(double *));
-    vcoef.alloc(slots * sizeof(double));
   }
 
   SoResult res;
