@@ -78,7 +78,7 @@ SCESS_HD uint32_t slice_magnitude(double x, int emax) {
   const uint64_t b = bits_of(x) & 0x7fffffffffffffffull;
   const int be = (int)(b >> 52), gap = emax - be;
   if (b == 0) return 0u;
-  return be == 0 || gap > 58 ? (127 - 60) << 7 : (uint32_t)(126 - gap) << 7 | ((uint32_t)(b >> 45) & 0x7fu);
+  return be == 0 || gap > 59 ? (127 - 60) << 7 : (uint32_t)(126 - gap) << 7 | ((uint32_t)(b >> 45) & 0x7fu);
 }
 
 // F + kDigitBias has digit p (p = 1 .. 6) in bits [9 (6 - p), 9 (6 - p) + 9)
@@ -96,16 +96,17 @@ SCESS_HD double power_of_two(int n) {
 }
 
 // (T + w 2^-fs) 2^sc rounded to FP64 (|T| < 2^62, 1 <= fs <= 31, -900 <= sc <= 800),
-// its sign bit xor-ed by flip unless it is zero.  A negative sum is complemented
-// rather than negated: one part in 2^32 of T's last place.
+// its sign bit xor-ed by flip unless it is zero.
 SCESS_HD double slice_value_plain(int64_t T, int w, int fs, int sc, uint32_t flip) {
   const uint64_t H = (uint64_t)(T + (int64_t)(w >> fs));
   const uint32_t f = (uint32_t)w << (32 - fs);
   const uint32_t sgn = (uint32_t)((int64_t)H >> 63);
   const uint32_t h1 = (uint32_t)(H >> 32) ^ sgn, h0 = (uint32_t)H ^ sgn, l = f ^ sgn;
-  // the leading nonzero word first: (a, b, c) of (h1, h0, l)
+  // The leading nonzero word first: (a, b, c) of (h1, h0, l).  The magnitude of a negative sum is
+  // its complement and one more in the last place, which is the complement with ones without end:
+  // they follow l, and the rounding carries them up.
   const bool m1 = h1 == 0u, m2 = m1 && h0 == 0u;
-  const uint32_t a = m2 ? l : (m1 ? h0 : h1), b = m2 ? 0u : (m1 ? l : h0), c = m1 ? 0u : l;
+  const uint32_t a = m2 ? l : (m1 ? h0 : h1), b = m2 ? sgn : (m1 ? l : h0), c = m1 ? sgn : l;
   const int lz = clz32(a);
   const uint32_t x1 = funnel_l(a, b, lz & 31), x0 = funnel_l(b, c, lz & 31);
   const int be = sc + 1023 + 63 - lz - (m1 ? 32 : 0) - (m2 ? 32 : 0);
