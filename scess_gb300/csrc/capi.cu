@@ -54,6 +54,7 @@ int guard(scess_ctx *ctx, F &&f) {
   if (ctx->impl->tc) ctx->impl->tc->clear_cache(nullptr);
   if (ctx->impl->slices) ctx->impl->slices->clear_cache(nullptr);
   if (code != SCESS_OK) {
+    ctx->impl->tape = nullptr;  // (a recording that was cut short: its tape is gone)
     // a call that failed otherwise may have left the mark of an expired wait behind
     if (ctx->impl->tc) ctx->impl->tc->clear_error();
     if (ctx->impl->slices) ctx->impl->slices->clear_error();
