@@ -1228,16 +1228,20 @@ __global__ void __launch_bounds__(256) triples_squares_kernel(SquareOps ops, con
 //   2^-122 / 3 sum [(column max)^2 a_k^2 + (row max)^2 b_k^2]  <=  0.16 2^-106 sum (a_k b_k)^2
 // with a factor of 2 to spare; dense tensors pass by a factor of 50 and more.  False also
 // where an exponent leaves the range of FP64's.
-bool triples_slices_hold(const std::vector<int> &exps, const int mx[4], const std::vector<float> &squares, int64_t o,
-                         int64_t v, int64_t nA, int64_t nB) {
-  for (int e : exps)
-    if (e >= kRowNonFinite) return false;
+// eA: exponents as used, the tensors' largest, the sums of squares.
+bool triples_slices_hold(const int *eA, int64_t o, int64_t v, int64_t nA, int64_t nB) {
+  const int *eB = eA + 2 * nA, *mx = eB + 2 * nB, *squares = mx + 4;
+  for (const int *e = eA; e < mx; e++)
+    if (*e >= kRowNonFinite) return false;
   auto col = [&](int64_t c) {
     double s = 0.0;
-    for (int p = 0; p < kSquareParts; p++) s += squares[c * kSquareParts + p];
+    for (int p = 0; p < kSquareParts; p++) {
+      float x;
+      std::memcpy(&x, squares + c * kSquareParts + p, sizeof(x));
+      s += x;
+    }
     return s;
   };
-  const int *eA = exps.data(), *eB = eA + 2 * nA;
   int a = 1, b = 1;  // largest exponents of the two sides
   for (int64_t i = 0; i < nA; i++) a = std::max(a, eA[i]);
   for (int64_t i = 0; i < nB; i++) b = std::max(b, eB[i]);
@@ -1289,10 +1293,9 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
   SliceEngine &se = *ctx.slice_engine();
   SlicedPack pP, pQ, pQ2, pR, pR2, pTx;
   DevTables pdt, gdt;
-  DevMem exps, squares, W, orbits;
+  DevMem exps, W, orbits;
   DTensor energies;
-  const int64_t nA = o * vp, nexp = 2 * nA + 2 * o2;
-  std::vector<float> hsq;
+  const int64_t nA = o * vp, nexp = 2 * nA + 2 * o2, nsq = (2 * v + 2 * o) * kSquareParts;
   std::vector<uint32_t> ot = orbit_table(o);
   const int norbits = (int)ot.size();
   try {
@@ -1313,8 +1316,9 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
                     table({{o, 1}, {nb, o}, {nb, 0}, {NB, 0}, {NB, o * nb}}),
                     table({{o, 1}, {nb, o}, {nb, 0}, {NB, o * nb}, {NB, 0}}),
                     table({{o, 1}, {o, o}, {nb, 0}, {NB, 0}})});
-    // P, t2 (o vp each), Q, R (o^2 each): exponents as found, then as used; then the largest
-    exps.alloc((size_t)(2 * nexp + 4) * sizeof(int));
+    // P, t2 (o vp each), Q, R (o^2 each): exponents as found, then as used; the largest; the
+    // sums of squares
+    exps.alloc((size_t)(2 * nexp + 4 + nsq) * sizeof(int));
     int *raw = exps.as<int>(), *use = raw + nexp;
     SCESS_CUDA(cudaMemsetAsync(raw, 0, (size_t)nexp * sizeof(int), s));
     const int64_t *kP = T.dt.ptr[T.kOperand + 1], *kT = T.dt.ptr[T.kOperand + 7], *kQ = T.dt.ptr[T.kOperand + 3],
@@ -1350,9 +1354,8 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
       sq.k[q] = x.k;
       sq.rows[q] = x.rows;
     }
-    hsq.resize((size_t)(2 * v + 2 * o) * kSquareParts);
-    squares.alloc(hsq.size() * sizeof(float));
-    launch(triples_squares_kernel, (unsigned)hsq.size(), 256, 0, s, sq, (const int *)(use + nexp), squares.as<float>());
+    launch(triples_squares_kernel, (unsigned)nsq, 256, 0, s, sq, (const int *)(use + nexp),
+           reinterpret_cast<float *>(use + nexp + 4));
     SCESS_CHECK_LAUNCH();
     for (const Op &q : ops)
       se.pack_with_exps(q.t.p(), pdt.ptr[q.row], q.rows, q.k, q.K, q.unitK, use + q.e, pdt.ptr[q.idx], q.neg, q.out);
@@ -1366,15 +1369,11 @@ bool triples_fp64_sliced(Ctx &ctx, const double *d_eri, int64_t nmo, int64_t o, 
   }
   SCESS_CUDA(cudaMemsetAsync(energies.p(), 0, energies.size() * sizeof(double), s));
   SCESS_CUDA(cudaMemcpyAsync(orbits.as<void>(), ot.data(), ot.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-  std::vector<int> he(nexp + 4);
+  std::vector<int> he(nexp + 4 + nsq);
   const int *use = exps.as<int>() + nexp;
   SCESS_CUDA(cudaMemcpyAsync(he.data(), use, he.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
-  SCESS_CUDA(cudaMemcpyAsync(hsq.data(), squares.as<void>(), hsq.size() * sizeof(float), cudaMemcpyDeviceToHost, s));
-  ctx.sync();  // (ot, he and hsq are host vectors of this scope)
-  int mx[4];
-  std::copy(he.end() - 4, he.end(), mx);
-  he.resize(nexp);
-  if (!triples_slices_hold(he, mx, hsq, o, v, nA, o2)) return false;
+  ctx.sync();  // (ot and he are host vectors of this scope)
+  if (!triples_slices_hold(he.data(), o, v, nA, o2)) return false;
   const int64_t p1 = o | 1, p2 = (p1 * o) | 1;
   const unsigned threads = (unsigned)std::min<int64_t>(256, round_up(norbits, 32));
   const size_t smem = (size_t)std::max<int64_t>(p2 * o + 3 * p1 * o + 4 * o, threads) * 8;
