@@ -901,112 +901,101 @@ void launch_packs(const PackOp *op, int n, cudaStream_t stream) {  // (the opera
   SCESS_CHECK_LAUNCH();
 }
 
-// The outputs that the slice GEMM has left (see SliceArgs::est), on the FP64 units: a thread looks
-// at a GEMM tile's 16 flags, and the CTA walks the 64 x 64 pieces of those that have any.  Items
-// are dealt out one by one; ks CTAs share a tile's K where there are few tiles, the last one
-// adds their ranges in order.  Returns at once where nothing was left.
+// The outputs that the slice GEMM has left (see SliceArgs::est), on the FP64 units.  Items are the
+// 64 x 64 pieces of the GEMM's tiles, dealt out one by one; a thread looks at an item's tile, of
+// 16 flags, and the CTA walks those that have any.  ks CTAs share an item's K where there are few,
+// and the last one adds their ranges in order.  Returns at once where nothing was left (3 us).
 struct LeftArgs {
   const uint32_t *left;
   const uint8_t *flags;
-  int bn, tiles_m, tiles_n, ks;
-  int64_t kper;
-  double *partial;  // ks > 1: [tile][ks][4][64 x 64]
-  int *counters;    // of a tile; zero between launches
+  int bn, pieces, tiles_n, ks;  // pieces of a tile: two by one or two
+  int64_t items, kper;          // items: tiles, pieces, ks
+  double *partial;              // ks > 1: [tile, piece][ks][64 x 64]
+  int *counters;                // of a tile and piece; zero between launches
 };
 __global__ void __launch_bounds__(256) slice_left_kernel(TableGemm g, LeftArgs a) {
   chain();
   constexpr int T = kDgemmTile;
-  __shared__ DgemmShared sh;
   constexpr int FEW = 128;  // outputs of a piece that are computed one by one, a warp each
+  __shared__ DgemmShared sh;
   __shared__ int todo[256], ntodo, few[FEW], nfew, last;
-  const int64_t items = (int64_t)a.tiles_m * a.tiles_n * a.ks;
   const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  for (int64_t i0 = 0; i0 * gridDim.x + blockIdx.x < items; i0 += 256) {
+  for (int64_t i0 = 0; i0 * gridDim.x + blockIdx.x < a.items; i0 += 256) {
     if (t == 0) ntodo = 0;
     __syncthreads();
     const int64_t mine = (i0 + t) * gridDim.x + blockIdx.x;
-    if (mine < items) {
-      const uint4 f = *reinterpret_cast<const uint4 *>(a.flags + 16 * (mine / a.ks));
+    if (mine < a.items) {
+      const uint4 f = *reinterpret_cast<const uint4 *>(a.flags + 16 * (mine / a.ks / a.pieces));
       if (f.x | f.y | f.z | f.w) todo[atomicAdd(&ntodo, 1)] = t;
     }
     __syncthreads();
     for (int q = 0; q < ntodo; q++) {
-      const int64_t item = (i0 + todo[q]) * gridDim.x + blockIdx.x;
-      const int tile = (int)(item / a.ks), z = (int)(item % a.ks);
+      const int64_t item = (i0 + todo[q]) * gridDim.x + blockIdx.x, piece = item / a.ks;
+      const int z = (int)(item % a.ks), tile = (int)(piece / a.pieces), sub = (int)(piece % a.pieces);
       const int64_t M0 = (int64_t)(tile / a.tiles_n) * BM, N0 = (int64_t)(tile % a.tiles_n) * a.bn;
-      const uint8_t *flags = a.flags + 16 * tile;
-      // outputs (m0 + tx + 16 i, n0 + ty + 16 j) of a piece at bit 4 i + j
-      auto marks = [&](int64_t m0, int64_t n0) {
-        uint32_t b = 0;
+      const int64_t m0 = M0 + (sub & 1) * T, n0 = N0 + (sub >> 1) * T;
+      // outputs (m0 + tx + 16 i, n0 + ty + 16 j) at bit 4 i + j
+      uint32_t b = 0;
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+      for (int i = 0; i < 4; i++)
 #pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const int64_t m = m0 + tx + 16 * i, n = n0 + ty + 16 * j;
-            if (m >= g.M || n >= g.N || n >= N0 + a.bn) continue;
-            const int h = column_group(a.bn, (int)(n - N0)), row = (int)(m - M0);
-            if (flags[4 * h + (row >> 5)] &&
-                (a.left[(int64_t)(tile * EPI + h) * BM + row] >> ((int)(n - N0) - group_start(a.bn, h)) & 1u))
-              b |= 1u << (4 * i + j);
-          }
-        return b;
-      };
-      auto finish = [&](int64_t m, int64_t n, double acc) {
-        const int64_t off = g.baseC + g.rowC[m] + g.colC[n];
+        for (int j = 0; j < 4; j++) {
+          const int row = (int)(m0 - M0) + tx + 16 * i, col = (int)(n0 - N0) + ty + 16 * j;
+          if (M0 + row >= g.M || N0 + col >= g.N || col >= a.bn) continue;
+          const int h = column_group(a.bn, col);
+          if (a.flags[16 * tile + 4 * h + (row >> 5)] &&
+              (a.left[(int64_t)(tile * EPI + h) * BM + row] >> (col - group_start(a.bn, h)) & 1u))
+            b |= 1u << (4 * i + j);
+        }
+      if (t == 0) nfew = 0;
+      if (!__syncthreads_or(b)) continue;
+      auto finish = [&](int x, int y, double acc) {
+        const int64_t off = g.baseC + g.rowC[m0 + x] + g.colC[n0 + y];
         double val = g.alpha * acc;
         if (g.beta != 0.0) val += g.beta * g.C[off];
         g.C[off] = val;
       };
-      double *p = a.partial + (int64_t)tile * a.ks * 4 * T * T;
-      const int64_t kb = z * a.kper, ke = min(g.K, kb + a.kper);
-      for (int piece = 0; piece < 4; piece++) {
-        const int64_t m0 = M0 + (piece & 1) * T, n0 = N0 + (piece >> 1) * T;
-        const uint32_t b = marks(m0, n0);
-        if (t == 0) nfew = 0;
-        if (!__syncthreads_or(b)) continue;
-        auto store = [&](int x, int y, double acc) {
-          if (a.ks == 1) finish(m0 + x, n0 + y, acc);
-          else p[(z * 4 + piece) * (T * T) + x + T * y] = acc;
-        };
-        for (uint32_t r = b; r; r &= r - 1) {
-          const int bit = __ffs((int)r) - 1, at = atomicAdd(&nfew, 1);
-          if (at < FEW) few[at] = tx + 16 * (bit >> 2) + T * (ty + 16 * (bit & 3));
-        }
-        __syncthreads();
-        if (nfew <= FEW) {
-          for (int f = t >> 5; f < nfew; f += 8) {
-            const int x = few[f] % T, y = few[f] / T;
-            const double *A = g.A + g.baseA + g.rowA[m0 + x], *B = g.B + g.baseB + g.colB[n0 + y];
-            double acc = 0.0;
-#pragma unroll 4
-            for (int64_t k = kb + (t & 31); k < ke; k += 32) acc = fma(A[g.kA[k]], B[g.kB[k]], acc);
-            for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
-            if ((t & 31) == 0) store(x, y, acc);
-          }
-        } else {
-          dgemm_tile(sh, g, m0, n0, kb, ke, [&](int64_t m, int64_t n, double acc) {
-            const int x = (int)(m - m0), y = (int)(n - n0);
-            if (b >> (4 * (x >> 4) + (y >> 4)) & 1u) store(x, y, acc);
-          });
-        }
-        __syncthreads();
+      double *p = a.partial + piece * a.ks * (T * T);
+      auto store = [&](int x, int y, double acc) {
+        if (a.ks == 1) finish(x, y, acc);
+        else p[z * (T * T) + x + T * y] = acc;
+      };
+      for (uint32_t r = b; r; r &= r - 1) {
+        const int bit = __ffs((int)r) - 1, at = atomicAdd(&nfew, 1);
+        if (at < FEW) few[at] = tx + 16 * (bit >> 2) + T * (ty + 16 * (bit & 3));
       }
+      __syncthreads();
+      const int64_t kb = z * a.kper, ke = min(g.K, kb + a.kper);
+      if (nfew <= FEW) {
+        for (int f = t >> 5; f < nfew; f += 8) {
+          const int x = few[f] % T, y = few[f] / T;
+          const double *A = g.A + g.baseA + g.rowA[m0 + x], *B = g.B + g.baseB + g.colB[n0 + y];
+          double acc = 0.0;
+#pragma unroll 4
+          for (int64_t k = kb + (t & 31); k < ke; k += 32) acc = fma(A[g.kA[k]], B[g.kB[k]], acc);
+          for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+          if ((t & 31) == 0) store(x, y, acc);
+        }
+      } else {
+        dgemm_tile(sh, g, m0, n0, kb, ke, [&](int64_t m, int64_t n, double acc) {
+          const int x = (int)(m - m0), y = (int)(n - n0);
+          if (b >> (4 * (x >> 4) + (y >> 4)) & 1u) store(x, y, acc);
+        });
+      }
+      __syncthreads();
       if (a.ks == 1) continue;
       __threadfence();
       __syncthreads();
-      if (t == 0) last = atomicAdd(&a.counters[tile], 1) == a.ks - 1;
+      if (t == 0) last = atomicAdd(&a.counters[piece], 1) == a.ks - 1;
       __syncthreads();
       if (!last) continue;
       __threadfence();
-      if (t == 0) a.counters[tile] = 0;
-      for (int piece = 0; piece < 4; piece++) {
-        const int64_t m0 = M0 + (piece & 1) * T, n0 = N0 + (piece >> 1) * T;
-        for (uint32_t b = marks(m0, n0); b; b &= b - 1) {
-          const int bit = __ffs((int)b) - 1, x = tx + 16 * (bit >> 2), y = ty + 16 * (bit & 3);
-          double s = 0.0;
-          for (int r = 0; r < a.ks; r++) s += __ldcg(p + (r * 4 + piece) * (T * T) + x + T * y);
-          finish(m0 + x, n0 + y, s);
-        }
+      if (t == 0) a.counters[piece] = 0;
+      for (uint32_t r = b; r; r &= r - 1) {
+        const int bit = __ffs((int)r) - 1, x = tx + 16 * (bit >> 2), y = ty + 16 * (bit & 3);
+        double s = 0.0;
+        for (int w = 0; w < a.ks; w++) s += __ldcg(p + w * (T * T) + x + T * y);
+        finish(x, y, s);
       }
     }
     __syncthreads();  // (the list is used up)
@@ -1339,15 +1328,16 @@ void SliceEngine::product(const TableGemm &g, const SlicedPack &A, const SlicedP
   plan_us(ps.M, ps.N, A.Kpad, splits);
   LeftArgs la = {};
   la.bn = tile_n(g.N);
-  la.tiles_m = (int)ceil_div(g.M, BM);
+  la.pieces = la.bn > kDgemmTile ? 4 : 2;
   la.tiles_n = (int)ceil_div(g.N, la.bn);
   la.counters = ctx_.counters.as<int>();
-  const int64_t tiles = (int64_t)la.tiles_m * la.tiles_n;
-  static_assert(kNumSMs <= kSmallCounters, "a counter a tile");
-  // few tiles: their K over several CTAs (one takes 4 ms per thousand k)
-  const int64_t ks = tiles >= kNumSMs ? 1 : std::min(4 * kNumSMs / tiles, ceil_div(g.K, 64));
+  const int64_t tiles = ceil_div(g.M, BM) * la.tiles_n, pieces = tiles * la.pieces;
+  static_assert(2 * kNumSMs <= kSmallCounters, "a counter a piece");
+  // few pieces: their K over several CTAs (one takes a millisecond per thousand k)
+  const int64_t ks = pieces >= 2 * kNumSMs ? 1 : std::min(4 * kNumSMs / pieces, ceil_div(g.K, 64));
   la.kper = ks == 1 ? g.K : round_up(ceil_div(g.K, ks), 16);
   la.ks = (int)ceil_div(g.K, la.kper);
+  la.items = pieces * la.ks;
   // (everything is allocated before anything is launched: the caller falls back to the FP64
   // units when it does not fit)
   auto room = [](DevMem &m, size_t bytes) {
@@ -1356,7 +1346,7 @@ void SliceEngine::product(const TableGemm &g, const SlicedPack &A, const SlicedP
   const size_t mn = (size_t)g.M * g.N, words = (size_t)tiles * EPI * BM;
   room(left_, words * sizeof(uint32_t) + 16 * tiles);
   room(partial_, std::max(splits > 1 ? splits * mn * (sizeof(double) + sizeof(float)) : 0,
-                          la.ks > 1 ? (size_t)tiles * la.ks * 4 * kDgemmTile * kDgemmTile * sizeof(double) : 0));
+                          la.ks > 1 ? (size_t)la.items * kDgemmTile * kDgemmTile * sizeof(double) : 0));
   ps.est = 1;
   ps.sq_unit = square_unit(g.K);
   ps.left = left_.as<uint32_t>();
@@ -1378,7 +1368,7 @@ void SliceEngine::product(const TableGemm &g, const SlicedPack &A, const SlicedP
   ps.alpha = g.alpha;
   ps.beta = g.beta;
   launch(ps, (int)splits, partial_.d());
-  scess::launch(slice_left_kernel, (unsigned)std::min<int64_t>(tiles * la.ks, 4 * kNumSMs), 256, 0, ctx_.stream, g, la);
+  scess::launch(slice_left_kernel, (unsigned)std::min<int64_t>(la.items, 4 * kNumSMs), 256, 0, ctx_.stream, g, la);
   SCESS_CHECK_LAUNCH();
 }
 
