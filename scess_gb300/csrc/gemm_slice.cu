@@ -22,13 +22,15 @@
 // Joint form (tiles of at most 64 columns): TMEM holds an accumulator for every S_d, in two
 // sets up to 32 columns, and the five are drained together, with one wait and one release a
 // block; three stages where they fit.  313600 x 16 x 140: 315 us -> 150, where the
-// packs' 16 bytes an element read at 4.9 TB/s bound it; 200000 x 16 x 16: 71 -> 43.
+// packs' bytes read at 4.9 TB/s bound it; 200000 x 16 x 16: 71 -> 43 (both before the
+// magnitudes, below).
 // A unit of a product that stands alone begins with the product of the magnitudes: seven K blocks
 // of that plane fill the places of a stage's seven digit slices, and what is added up in the
 // next free accumulator tells which outputs are left to the FP64 units (slice_left).  A warp takes
-// its 32 x 32 outputs at once where their least sum reaches their largest threshold.  Cost, of
-// which a third is the packs': FP64 iterations at o = 10, v = 90 6.9 -> 7.4 ms, at o = 16,
-// v = 140 38.1 -> 40.4, a residual gradient at o = 8, v = 47 5.28 -> 5.54.
+// its 32 x 32 outputs at once where their least sum reaches their largest threshold.  Cost, with
+// the packs' eighth plane: 4096^3 49.9 -> 47.3 TFLOP/s, 8192 x 8192 x 32 293 -> 344 us,
+// 313600 x 16 x 140 161 -> 207; FP64 iterations at o = 10, v = 90 6.9 -> 7.4 ms, at o = 16,
+// v = 140 38.1 -> 41.1, a residual gradient at o = 8, v = 47 5.28 -> 5.46.
 // Every mbarrier wait is bounded (see mbarrier.cuh).
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -708,7 +710,7 @@ __global__ void __launch_bounds__(256) slice_reduce_kernel(const __grid_constant
 // exponents first, the cut in a second launch.  EXPS: exponents only, folded into
 // exps[expIdx[row]] with atomics.  GIVEN: exponents exps[expIdx[row]], K spread over
 // CTAs.
-// HBM-bound with long rows (8 B read and 16 B written per element, 3.2 TB/s at
+// HBM-bound with long rows (8 B read and 16 B written per element, 3.4 TB/s at
 // 4096 x 4096, 2.3 before the loads of the next chunk were in flight while one is cut).
 enum PackMode { PACK_OWN, PACK_PART, PACK_FROM_PART, PACK_EXPS, PACK_GIVEN };
 struct PackOp {
