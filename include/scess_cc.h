@@ -296,12 +296,12 @@ int scess_rccsd_rdm1(scess_ctx *ctx, const double *eri, const double *eps, int64
  * operand a dense column-major host tensor of rank <= 6 with extents *_ext.
  * Every label of C appears in exactly one of A, B; labels shared by A and B
  * and absent from C are summed.  precision selects the FP64 backend or, for
- * MIXED, the tcgen05 tensor-core backend for any shape.  FP64: small products run on the FP64
- * units, the others on the tensor cores, operands cut into BF16 slices (60 bits below a
- * row's largest value) and added exactly; outputs that those bits cannot hold (sum |a b| below
- * about 2^-7 (row norm^2 + column norm^2)^(1/2) of |row max| |column max|) and those of Inf or NaN
- * run on the FP64 units.  Either way an output's error is that of FP64 multiply-adds, a few
- * 2^-53 sum |a b|. */
+ * MIXED, the tcgen05 tensor-core backend for any shape.  FP64: small products
+ * run on the FP64 units, the others on the tensor cores, operands cut into
+ * BF16 slices that hold 60 bits below a row's largest value; outputs that
+ * those bits cannot hold (sum |a b| small beside |row max| |column max|) and
+ * those of Inf or NaN run on the FP64 units.  Either way an output's error is
+ * that of FP64 multiply-adds, a few 2^-53 sum |a b|. */
 int scess_einsum(scess_ctx *ctx, const char *spec, double alpha, const double *A, int32_t a_nd,
                  const int64_t *a_ext, const double *B, int32_t b_nd, const int64_t *b_ext,
                  double beta, double *C, int32_t c_nd, const int64_t *c_ext, int32_t precision);

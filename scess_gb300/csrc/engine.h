@@ -274,10 +274,10 @@ struct Ctx {
 };
 
 // C = alpha A.B + beta C in FP64 through the tables of g: small products on the
-// FP64 units, the others on the tensor cores' exact slices.
+// FP64 units, the others on the tensor cores' slices (gemm_slice.h).
 void fp64_table_gemm(Ctx &ctx, const TableGemm &g, const char *name);
 
-// FP64: DFMA engine.  MIXED: tensor cores for contractions large enough to pay
+// FP64: FP64 units and slices.  MIXED: tensor cores for contractions large enough to pay
 // for packing, FP64 for the rest.  TENSOR: tensor cores for every contraction.
 enum class Backend { FP64 = 0, MIXED = 1, TENSOR = 2 };
 

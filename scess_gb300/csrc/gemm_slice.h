@@ -1,4 +1,4 @@
-// FP64 contractions on the tensor cores: operands cut into exact BF16 slices.
+// FP64 contractions on the tensor cores: operands cut into BF16 slices.
 //
 // GB300's FP64 units run at about 1 TFLOP/s, 1/1900 of its BF16 tensor rate.  An
 // FP64 value is therefore cut into kSlices = 7 signed base-512 digits of a fixed

@@ -60,10 +60,10 @@ struct RccsdWork {
 // reference's contraction list literally; Backend::MIXED evaluates the large
 // contractions on tensor cores and folds the T1 dressing of Wvvvv into the
 // ladder (vvvv tau plus two o^3v^3 contractions), so no v^4 tensor is formed.
-// list: the reference's literal contraction list (AUTO for the FP64 backend:
-// the drop-in path) or the reassociated one (AUTO for the tensor cores; also
-// the FP64 base evaluations of the refined mixed solve, which then write no
-// v^4 tensor).  Both compute the same function.
+// list: the reference's literal contraction list (AUTO for the FP64 backend)
+// or the reassociated one (AUTO for the tensor cores; also the FP64 iterations
+// of symmetric inputs and the FP64 base evaluations of the refined mixed solve,
+// which then write no v^4 tensor).  Both compute the same function.
 enum class ResidualList { AUTO = 0, LITERAL = 1, REASSOCIATED = 2 };
 void rccsd_residual(Ctx &ctx, const RccsdBlocks &B, const double *amp, const double *t2driver,
                     Backend be, RccsdWork &w, double *R, ResidualList list = ResidualList::AUTO);
