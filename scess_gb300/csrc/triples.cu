@@ -1233,6 +1233,7 @@ bool triples_slices_hold(const int *eA, int64_t o, int64_t v, int64_t nA, int64_
   const int *eB = eA + 2 * nA, *mx = eB + 2 * nB, *squares = mx + 4;
   for (const int *e = eA; e < mx; e++)
     if (*e >= kRowNonFinite) return false;
+  if (mx[1] == 0) return true;  // no t2: every W is exactly zero
   auto col = [&](int64_t c) {
     double s = 0.0;
     for (int p = 0; p < kSquareParts; p++) {
