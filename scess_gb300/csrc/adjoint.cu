@@ -381,12 +381,10 @@ LambdaResult rccsd_lambda(Ctx &ctx, const double *d_eri, const double *eps_host,
     const int nv = (int)order.size();
     std::vector<const double *> hp(nv);
     for (int q = 0; q < nv; q++) hp[q] = de.d() + (size_t)order[q] * n;
-    dots(n, hp.data(), nv, ve, ctx.partials, ctx.dscalars, s);
-    SCESS_CUDA(cudaMemcpyAsync(ctx.hscalars, ctx.dscalars, nv * sizeof(double), cudaMemcpyDeviceToHost, s));
-    ctx.sync();
-    for (int q = 0; q < nv - 1; q++) gram[q].push_back(ctx.hscalars[q]);
-    gram.emplace_back(ctx.hscalars, ctx.hscalars + nv);
-    const double rms = std::sqrt(ctx.hscalars[nv - 1] / (double)n);
+    const std::vector<double> row = dots_on_host(ctx, n, hp.data(), nv, ve);
+    for (int q = 0; q < nv - 1; q++) gram[q].push_back(row[q]);
+    gram.push_back(row);
+    const double rms = std::sqrt(row[nv - 1] / (double)n);
     if (it >= opts.diis_start) {
       std::vector<double> c = diis_coefficients(gram);
       for (int q = 0; q < nv; q++) hp[q] = dv.d() + (size_t)order[q] * n;

@@ -302,12 +302,9 @@ SoResult so_ccsd(Ctx &ctx, const double *d_g, const double *d_eps, int64_t nmo, 
       const int m = (int)order.size();
       std::vector<const double *> hp(m);
       for (int q = 0; q < m; q++) hp[q] = verr.d() + (size_t)order[q] * n;
-      dots(n, hp.data(), m, ve, ctx.partials, ctx.dscalars, s);
-      SCESS_CUDA(cudaMemcpyAsync(ctx.hscalars, ctx.dscalars, m * sizeof(double),
-                                 cudaMemcpyDeviceToHost, s));
-      ctx.sync();
-      for (int q = 0; q < m - 1; q++) gram[q].push_back(ctx.hscalars[q]);
-      gram.emplace_back(ctx.hscalars, ctx.hscalars + m);
+      const std::vector<double> row = dots_on_host(ctx, n, hp.data(), m, ve);
+      for (int q = 0; q < m - 1; q++) gram[q].push_back(row[q]);
+      gram.push_back(row);
       if (it >= kDiisStart) {                                                      // :119-166
         if ((int)order.size() > kMaxDiis) {
           order.pop_front();

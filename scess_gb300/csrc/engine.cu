@@ -247,6 +247,20 @@ SliceEngine *Ctx::slice_engine() {
   return slices.get();
 }
 
+std::vector<double> dots_on_host(Ctx &ctx, int64_t n, const double *const *xs, int nv, const double *y) {
+  constexpr int kAtOnce = 3 * kDotVectors;
+  std::vector<double> r;
+  r.reserve(nv);
+  for (int q = 0; q < nv; q += kAtOnce) {
+    const int m = std::min(kAtOnce, nv - q);
+    dots(n, xs + q, m, y, ctx.partials, ctx.dscalars, ctx.stream);
+    SCESS_CUDA(cudaMemcpyAsync(ctx.hscalars, ctx.dscalars, m * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
+    ctx.sync();
+    r.insert(r.end(), ctx.hscalars, ctx.hscalars + m);
+  }
+  return r;
+}
+
 void upload(Ctx &ctx, double *dst, const double *src, int64_t n) {
   if (n <= 0) return;
   SCESS_CUDA(cudaMemcpyAsync(dst, src, (size_t)n * sizeof(double), cudaMemcpyHostToDevice,

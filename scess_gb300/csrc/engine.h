@@ -292,6 +292,10 @@ void permute(Ctx &ctx, const char *spec, double alpha, const TV &X, double beta,
 
 const EinsumPlan &plan_einsum(Ctx &ctx, const char *spec, const TV &A, const TV &B, const TV &C);
 
+// xs[q] . y for nv vectors (host array of device pointers), on the host.  Any nv: the context's
+// device and pinned scalars hold 64 at a time.
+std::vector<double> dots_on_host(Ctx &ctx, int64_t n, const double *const *xs, int nv, const double *y);
+
 // Upload helpers (synchronous w.r.t. the host buffer).
 void upload(Ctx &ctx, double *dst, const double *src, int64_t n);
 void download(Ctx &ctx, double *dst, const double *src, int64_t n);

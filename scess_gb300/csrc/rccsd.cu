@@ -761,13 +761,10 @@ bool RccsdState::iterate(int max_steps, const Control &ctl) {
     const int nv = (int)order_.size();
     std::vector<const double *> vecs(nv);
     for (int q = 0; q < nv; q++) vecs[q] = diis_err_.d() + (size_t)order_[q] * n_;
-    dots(n_, vecs.data(), nv, ve, ctx_.partials, ctx_.dscalars, s);
-    SCESS_CUDA(cudaMemcpyAsync(ctx_.hscalars, ctx_.dscalars, nv * sizeof(double),
-                               cudaMemcpyDeviceToHost, s));
-    ctx_.sync();
-    for (int q = 0; q < nv - 1; q++) gram_[q].push_back(ctx_.hscalars[q]);
-    gram_.emplace_back(ctx_.hscalars, ctx_.hscalars + nv);
-    const double errdot = ctx_.hscalars[nv - 1];
+    const std::vector<double> row = dots_on_host(ctx_, n_, vecs.data(), nv, ve);
+    for (int q = 0; q < nv - 1; q++) gram_[q].push_back(row[q]);
+    gram_.push_back(row);
+    const double errdot = row[nv - 1];
     if (it_ - phase_start_ >= opts_.diis_start) {                                    // :354-357
       if (it_ - phase_start_ == opts_.diis_start) ctx_.logf(1, "Turning on DIIS");
       std::vector<double> c = diis_coefficients(gram_);
